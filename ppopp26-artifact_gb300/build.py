@@ -29,7 +29,7 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 # Montgomery multiply formulation (csrc/fr.cuh), the transform's twiddle
 # multiply (PP_NTT_MUL) and the pass kernels' blocks per SM (PP_NTT_MINB);
 # overridable for experiments
-MUL_VARIANT = os.environ.get("PP_MUL_VARIANT", "9")
+MUL_VARIANT = os.environ.get("PP_MUL_VARIANT", "14")
 NTT_MUL = os.environ.get("PP_NTT_MUL", "")
 NTT_MINB = os.environ.get("PP_NTT_MINB", "")
 NVCC_FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "-DPP_MUL_VARIANT=" + MUL_VARIANT,

@@ -14,8 +14,9 @@
 // comparing Montgomery multiplication algorithms", IEEE Micro 1996) on 32-bit
 // words.  r = 1 (mod 2^32) gives -r^-1 = 0xffffffff, so each row's m is a
 // negation, and the two lowest words of r (1 and 0xffffffff) make m*r[0] and
-// m*r[1] multiply-free: each row costs 16 + 12 integer multiplies instead of
-// 16 + 16.
+// m*r[1] multiply-free: each row costs 8 + 6 wide products instead of 8 + 8.
+// The form the kernels run is fr_mul_cells (below); the others are earlier
+// formulations kept as its cross-checks on the host.
 #pragma once
 #include <stdint.h>
 
@@ -534,7 +535,7 @@ PP_HD fr fr_mul_kara(const fr &a, const fr &b) {
 }
 
 #ifndef PP_MUL_VARIANT
-#define PP_MUL_VARIANT 0
+#define PP_MUL_VARIANT 14  // fr_mul_cells
 #endif
 
 // ---------------------------------------------------------------------------
@@ -884,6 +885,186 @@ PP_HD fr fr_mul_sos(const fr &a, const fr &b) {
   return mont_redc16(t);
 }
 
+// ---------------------------------------------------------------------------
+// Variant 14 (the kernels' form): carry-chained cells.
+//
+// A mad.lo.cc / madc.hi.cc pair on one product is a single wide multiply-add
+// that takes the carry in and leaves the carry out.  Products that sit two
+// words apart therefore chain without any separate addition: the running sum
+// is held as two arrays of 64-bit cells, X at even word positions and Y at
+// odd ones, and a row a_i * b is two chains (b's even words into X, its odd
+// words into Y) with one add for the carry out of each.  The row forms above
+// spend 9 to 18 ALU additions per row, and a register move per product to
+// zero-extend its 32-bit addend, where this one spends 2.
+//
+// The reduction subtracts: r = 1 (mod 2^32), so with L the lowest word
+// t - L r is divisible by 2^32 and
+//   -L r = -L + L 2^32 + L N 2^64 - L 2^256,  N = 2^192 - (r >> 64) - 1,
+// i.e. the lowest word vanishes without a carry, L is added one word up, six
+// products L * N[j] follow, and the L at word 8 is collected (M below) and
+// subtracted once at the end.  112 wide products in all, as the row forms.
+//
+// Measured on GB300 (two chains per thread, 256-thread blocks): 78.4 G
+// multiplies/s (lazy) and 77.5 G/s (canonical) against 55.7 and 53.4 G/s for
+// variant 9: 4.6 cycles per wide product and sub-partition, against 6.5.
+// ---------------------------------------------------------------------------
+#define PP_N0 0x0001a401u
+#define PP_N1 0xac425bfdu
+#define PP_N2 0xf65e27fau
+#define PP_N3 0xccc627f7u
+#define PP_N4 0xd66282b7u
+#define PP_N5 0x8c1258acu
+
+// acc[0 .. 2N) += a * (b[0], b[2], .. b[2N-2]), product k at words 2k and
+// 2k+1, with the carry flag added in when CIN; the carry out goes to acc[2N]
+template <int N, bool CIN = false>
+PP_HD void mad_cells(uint32_t *acc, uint32_t a, const uint32_t *b) {
+  acc[0] = CIN ? madloc_cc(a, b[0], acc[0]) : madlo_cc(a, b[0], acc[0]);
+  acc[1] = madhic_cc(a, b[0], acc[1]);
+#pragma unroll
+  for (int k = 1; k < N; ++k) {
+    acc[2 * k] = madloc_cc(a, b[2 * k], acc[2 * k]);
+    acc[2 * k + 1] = madhic_cc(a, b[2 * k], acc[2 * k + 1]);
+  }
+  acc[2 * N] = addc(acc[2 * N], 0);
+}
+// the same products into fresh words acc[0 .. 2N)
+template <int N>
+PP_HD void mul_cells(uint32_t *acc, uint32_t a, const uint32_t *b) {
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    const uint64_t p = (uint64_t)a * b[2 * k];
+    acc[2 * k] = (uint32_t)p;
+    acc[2 * k + 1] = (uint32_t)(p >> 32);
+  }
+}
+
+// One reduction step: x holds cells at positions 0, 2, 4, 6 (x[8]: position
+// 8), y at 1, 3, 5, 7 (y[8]: position 9); L = x[0] is the whole word at
+// position 0.  Returns the whole word at position 1; afterwards y's cells are
+// at even and x + 2's at odd positions of the value shifted down one word.
+PP_HD uint32_t fr_red_cells(uint32_t *x, uint32_t *y, uint32_t L) {
+  const uint32_t nr[6] = {PP_N0, PP_N1, PP_N2, PP_N3, PP_N4, PP_N5};
+  y[0] = add_cc(y[0], L);
+  y[1] = addc_cc(y[1], 0);
+  mad_cells<3, true>(y + 2, L, nr + 1);
+  const uint32_t next = add_cc(y[0], x[1]);
+  mad_cells<3, true>(x + 2, L, nr);
+  return next;
+}
+
+// after a reduction step: shift the cells down one word (renaming only)
+PP_HD void fr_shift_cells(uint32_t x[9], uint32_t y[9]) {
+  uint32_t t[9];
+#pragma unroll
+  for (int k = 0; k < 9; ++k) t[k] = x[k];
+#pragma unroll
+  for (int k = 0; k < 9; ++k) x[k] = y[k];
+#pragma unroll
+  for (int k = 0; k < 7; ++k) y[k] = t[k + 2];
+  y[7] = 0;
+  y[8] = 0;
+}
+
+// o + r where mask is all ones (o where it is 0), modulo 2^256
+PP_HD void fr_add_r_masked(uint32_t o[8], uint32_t mask) {
+  o[0] = add_cc(o[0], PP_R0 & mask);
+  o[1] = addc_cc(o[1], PP_R1 & mask);
+  o[2] = addc_cc(o[2], PP_R2 & mask);
+  o[3] = addc_cc(o[3], PP_R3 & mask);
+  o[4] = addc_cc(o[4], PP_R4 & mask);
+  o[5] = addc_cc(o[5], PP_R5 & mask);
+  o[6] = addc_cc(o[6], PP_R6 & mask);
+  o[7] = addc(o[7], PP_R7 & mask);
+}
+
+// a b 2^-256 mod r.  The value before the last step is (a b - M r) / 2^256
+// with 0 <= M < 2^256: above -r, and below r when a b < r 2^256 (b < r and
+// any 256-bit a).  Canonical form adds r to a negative value; LAZY always
+// adds it, leaving 0 < result < 2r.
+template <bool LAZY = false>
+PP_HD fr fr_mul_cells(const fr &a, const fr &b) {
+  uint32_t X[9], Y[9], M[8];
+  mul_cells<4>(X, a.v[0], b.v);
+  mul_cells<4>(Y, a.v[0], b.v + 1);
+  X[8] = Y[8] = 0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    if (i) {
+      mad_cells<4>(X, a.v[i], b.v);
+      mad_cells<4>(Y, a.v[i], b.v + 1);
+    }
+    M[i] = X[0];
+    Y[0] = fr_red_cells(X, Y, X[0]);
+    fr_shift_cells(X, Y);
+  }
+  fr o;
+  o.v[0] = X[0];
+  o.v[1] = add_cc(X[1], Y[0]);
+#pragma unroll
+  for (int k = 2; k < 8; ++k) o.v[k] = addc_cc(X[k], Y[k - 1]);
+  const uint32_t top = addc(X[8], 0);
+  o.v[0] = sub_cc(o.v[0], M[0]);
+#pragma unroll
+  for (int k = 1; k < 8; ++k) o.v[k] = subc_cc(o.v[k], M[k]);
+  const uint32_t neg = subc(top, 0);  // top - borrow: all ones when negative, else 0
+  if (LAZY) fr_add_r_masked(o.v, 0xffffffffu);
+  else fr_add_r_masked(o.v, neg);
+  return o;
+}
+
+// r[0..16) = a * b with carry-chained cells
+PP_HD void mul8_cells(uint32_t r[16], const uint32_t a[8], const uint32_t b[8]) {
+  uint32_t E[18], O[18];  // words 0 .. and 1 ..
+  mul_cells<4>(E, a[0], b);
+  mul_cells<4>(O, a[0], b + 1);
+#pragma unroll
+  for (int k = 8; k < 18; ++k) E[k] = O[k] = 0;
+#pragma unroll
+  for (int i = 1; i < 8; ++i) {
+    // a_i b_j at word i + j: even words into E, odd words into O
+    if (i & 1) {
+      mad_cells<4>(O + i - 1, a[i], b);
+      mad_cells<4>(E + i + 1, a[i], b + 1);
+    } else {
+      mad_cells<4>(E + i, a[i], b);
+      mad_cells<4>(O + i, a[i], b + 1);
+    }
+  }
+  r[0] = E[0];
+  r[1] = add_cc(E[1], O[0]);
+#pragma unroll
+  for (int k = 2; k < 15; ++k) r[k] = addc_cc(E[k], O[k - 1]);
+  r[15] = addc(E[15], O[14]);
+}
+
+// (t[0..8) - M r) / 2^256 for the M that makes it whole, in 8 words and a top
+// word (all ones when negative): the value is in (-r, 1)
+PP_HD uint32_t fr_redc8_cells(uint32_t o[8], const uint32_t *t) {
+  uint32_t X[9], Y[9], M[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    X[k] = t[k];
+    Y[k] = 0;
+  }
+  X[8] = Y[8] = 0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    M[i] = X[0];
+    Y[0] = fr_red_cells(X, Y, X[0]);
+    fr_shift_cells(X, Y);
+  }
+  o[0] = X[0];
+  o[1] = add_cc(X[1], Y[0]);
+#pragma unroll
+  for (int k = 2; k < 8; ++k) o[k] = addc_cc(X[k], Y[k - 1]);
+  const uint32_t top = addc(X[8], 0);
+  o[0] = sub_cc(o[0], M[0]);
+#pragma unroll
+  for (int k = 1; k < 8; ++k) o[k] = subc_cc(o[k], M[k]);
+  return subc(top, 0);
+}
+
 PP_HD fr fr_mul(const fr &a, const fr &b) {
 #if PP_MUL_VARIANT == 2
   return fr_mul_w(a, b);
@@ -909,66 +1090,67 @@ PP_HD fr fr_mul(const fr &a, const fr &b) {
   return fr_mul_mix<1, 0>(a, b);
 #elif PP_MUL_VARIANT == 13
   return fr_mul_mix<0, 2>(a, b);
+#elif PP_MUL_VARIANT == 14
+  return fr_mul_cells(a, b);
 #else
   return fr_mul_v<PP_MUL_VARIANT>(a, b);
 #endif
 }
 
-// r[0..16) = a^2 for a < 2^255: the 28 cross products a_i a_j (i < j) in rows
-// of independent products (row i: a_i times a_(i+1..7), each row's top word
-// new), doubled, plus the 8 squares a_i^2 in one add-with-carry chain: 36 wide
-// products where a general product needs 64.
-PP_HD void sqr8_rows(uint32_t r[16], const uint32_t a[8]) {
-#pragma unroll
-  for (int k = 0; k < 16; ++k) r[k] = 0;
-#pragma unroll
-  for (int i = 0; i < 7; ++i) {
-    const int n = 7 - i;  // partners a[i + 1 .. 7] at words 2i + 1 .. i + 7
-    uint32_t lo[7], hi[7];
-#pragma unroll
-    for (int j = 0; j < n; ++j) {
-      const uint64_t s = (uint64_t)a[i] * a[i + 1 + j] + r[2 * i + 1 + j];
-      lo[j] = (uint32_t)s;
-      hi[j] = (uint32_t)(s >> 32);
-    }
-    r[2 * i + 1] = lo[0];
-    if (n == 1) {
-      r[2 * i + 2] = hi[0];
-    } else {
-      r[2 * i + 2] = add_cc(lo[1], hi[0]);
-#pragma unroll
-      for (int j = 2; j < n; ++j) r[2 * i + 1 + j] = addc_cc(lo[j], hi[j - 1]);
-      r[i + 8] = addc(hi[n - 1], 0);
-    }
+// rows I .. 6 of the cross products a_I a_j (j > I) of a square: words I + j,
+// even ones in E, odd ones in O (word k at O[k - 1])
+template <int I>
+PP_HD void sqr8_cross(uint32_t *E, uint32_t *O, const uint32_t a[8]) {
+  constexpr int N1 = (8 - I) / 2, N2 = (7 - I) / 2;  // j = I + 1, I + 3 ..; j = I + 2, ..
+  if constexpr (I == 0) {
+    mul_cells<N1>(O, a[0], a + 1);
+    mul_cells<N2>(E + 2, a[0], a + 2);
+  } else {
+    mad_cells<N1>(O + 2 * I, a[I], a + I + 1);
+    if constexpr (N2 > 0) mad_cells<N2>(E + 2 * I + 2, a[I], a + I + 2);
   }
+  if constexpr (I < 6) sqr8_cross<I + 1>(E, O, a);
+}
+
+// r[0..16) = a^2 for a < 2^255: the 28 cross products, doubled, plus the 8
+// squares a_i^2 in one carry chain: 36 wide products where a general product
+// needs 64.
+PP_HD void sqr8_cells(uint32_t r[16], const uint32_t a[8]) {
+  uint32_t E[18], O[18];
+#pragma unroll
+  for (int k = 0; k < 18; ++k) E[k] = O[k] = 0;
+  sqr8_cross<0>(E, O, a);
+  r[0] = 0;
+  r[1] = O[0];
+  r[2] = add_cc(E[2], O[1]);
+#pragma unroll
+  for (int k = 3; k < 15; ++k) r[k] = addc_cc(E[k], O[k - 1]);
+  r[15] = addc(E[15], O[14]);
   // 2 x (the cross products) < a^2 < 2^510: the shift loses no bit
 #pragma unroll
   for (int k = 15; k > 0; --k) r[k] = (r[k] << 1) | (r[k - 1] >> 31);
-  r[0] <<= 1;
-  uint32_t sl[8], sh[8];
+  r[0] = madlo_cc(a[0], a[0], r[0]);
+  r[1] = madhic_cc(a[0], a[0], r[1]);
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const uint64_t s = (uint64_t)a[i] * a[i];
-    sl[i] = (uint32_t)s;
-    sh[i] = (uint32_t)(s >> 32);
+  for (int i = 1; i < 8; ++i) {
+    r[2 * i] = madloc_cc(a[i], a[i], r[2 * i]);
+    r[2 * i + 1] = madhic_cc(a[i], a[i], r[2 * i + 1]);
   }
-  r[0] = add_cc(r[0], sl[0]);
-  r[1] = addc_cc(r[1], sh[0]);
-#pragma unroll
-  for (int i = 1; i < 7; ++i) {
-    r[2 * i] = addc_cc(r[2 * i], sl[i]);
-    r[2 * i + 1] = addc_cc(r[2 * i + 1], sh[i]);
-  }
-  r[14] = addc_cc(r[14], sl[7]);
-  r[15] = addc(r[15], sh[7]);
 }
 
-// a^2 for canonical a (a^2 < r 2^256, as the reduction needs): the square's
-// 36 wide products, then the row-form Montgomery reduction (48)
+// a^2 2^-256 mod r for canonical a (a^2 < r 2^256): the square's 36 wide
+// products, then the reduction's 48
 PP_HD fr fr_sqr(const fr &a) {
   uint32_t t[16];
-  sqr8_rows(t, a.v);
-  return mont_redc16_rows(t);
+  sqr8_cells(t, a.v);
+  fr o;
+  // (-r, 1) + the upper half (below r): above -r and below r
+  const uint32_t top = fr_redc8_cells(o.v, t);
+  o.v[0] = add_cc(o.v[0], t[8]);
+#pragma unroll
+  for (int k = 1; k < 8; ++k) o.v[k] = addc_cc(o.v[k], t[8 + k]);
+  fr_add_r_masked(o.v, addc(top, 0));
+  return o;
 }
 
 // ---- lazy arithmetic on [0, 2r) for the NTT's inner rounds: values stay
@@ -976,7 +1158,9 @@ PP_HD fr fr_sqr(const fr &a) {
 // result.  fr_mul_lazy takes a < 2r and b < r (the twiddle) and returns a
 // value < 2r.
 PP_HD fr fr_mul_lazy(const fr &a, const fr &b) {
-#if PP_MUL_VARIANT == 9
+#if PP_MUL_VARIANT == 14
+  return fr_mul_cells<true>(a, b);
+#elif PP_MUL_VARIANT == 9
   return fr_mul_row9<true>(a, b);
 #else
   fr c = a;
@@ -1069,31 +1253,10 @@ PP_HD fr fr_canon(const fr &a) {
 // subtractions gives the canonical result: 64 wide products per term and one
 // reduction per group, where a multiply per term costs 112.
 // ---------------------------------------------------------------------------
-// r[0..16) = a * b, rows of independent products + one add chain per row
-PP_HD void mul8_rows(uint32_t r[16], const uint32_t a[8], const uint32_t b[8]) {
-#pragma unroll
-  for (int k = 0; k < 16; ++k) r[k] = 0;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    uint32_t lo[8], hi[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const uint64_t s = (uint64_t)a[i] * b[j] + r[i + j];
-      lo[j] = (uint32_t)s;
-      hi[j] = (uint32_t)(s >> 32);
-    }
-    r[i] = lo[0];
-    r[i + 1] = add_cc(lo[1], hi[0]);
-#pragma unroll
-    for (int j = 2; j < 8; ++j) r[i + j] = addc_cc(lo[j], hi[j - 1]);
-    r[i + 8] = addc(hi[7], 0);
-  }
-}
-
 // acc[0..17) += a * b
 PP_HD void fr_mac17(uint32_t acc[17], const fr &a, const fr &b) {
   uint32_t p[16];
-  mul8_rows(p, a.v, b.v);
+  mul8_cells(p, a.v, b.v);
   acc[0] = add_cc(acc[0], p[0]);
 #pragma unroll
   for (int k = 1; k < 16; ++k) acc[k] = addc_cc(acc[k], p[k]);
@@ -1112,40 +1275,21 @@ PP_HD void sub_if_ge9(uint32_t x[9], const uint32_t kr[9]) {
 }
 
 // acc * 2^-256 mod r, canonical, for acc < 2^543 whose reduction is below
-// 16 r (a sum of at most 16 products of canonical values: acc < 16 r^2, so
+// 15 r (a sum of at most 16 products of canonical values: acc < 16 r^2, so
 // the reduced value is below 16 r^2 / 2^256 + r < 8.3 r)
 PP_HD fr fr_redc17(uint32_t t[17]) {
   const uint32_t r[8] = {PP_R0, PP_R1, PP_R2, PP_R3, PP_R4, PP_R5, PP_R6, PP_R7};
-  uint32_t hc = 0;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    // round i: t += m r 2^(32 i) with m = -t[i] (r = 1 mod 2^32), as
-    // mont_redc16_rows; the carry out of word i + 8 rides into round i + 1
-    const uint32_t t0 = t[i];
-    const uint32_t m = 0u - t0;
-    uint32_t lo[8], hi[8];
-#pragma unroll
-    for (int j = 2; j < 8; ++j) {
-      const uint64_t s = (uint64_t)m * r[j] + t[i + j];
-      lo[j] = (uint32_t)s;
-      hi[j] = (uint32_t)(s >> 32);
-    }
-    (void)sub_cc(0, m);
-    const uint32_t h1 = subc(m, 0);
-    (void)add_cc(t0, 0xffffffffu);
-    t[i + 1] = addc_cc(t[i + 1], t0);
-    t[i + 2] = addc_cc(lo[2], h1);
-#pragma unroll
-    for (int j = 3; j < 8; ++j) t[i + j] = addc_cc(lo[j], hi[j - 1]);
-    t[i + 8] = addc_cc(t[i + 8], hi[7]);
-    const uint32_t c1 = addc(0, 0);
-    t[i + 8] = add_cc(t[i + 8], hc);
-    hc = addc(c1, 0);
-  }
-  t[16] += hc;  // the value t[8..17) is below 2^260: no carry leaves word 16
+  // (-r, 1) + the upper nine words + r: above 0 and below 9.3 r
   uint32_t x[9];
+  x[8] = fr_redc8_cells(x, t);
+  x[0] = add_cc(x[0], t[8]);
 #pragma unroll
-  for (int i = 0; i < 9; ++i) x[i] = t[8 + i];
+  for (int i = 1; i < 8; ++i) x[i] = addc_cc(x[i], t[8 + i]);
+  x[8] = addc(x[8], t[16]);
+  x[0] = add_cc(x[0], r[0]);
+#pragma unroll
+  for (int i = 1; i < 8; ++i) x[i] = addc_cc(x[i], r[i]);
+  x[8] = addc(x[8], 0);
   // k r for k = 8, 4, 2, 1
   uint32_t kr[9];
 #pragma unroll

@@ -27,22 +27,41 @@ namespace pp {
 
 // Blocks per SM each operator's geometry aims for (scan_geom): longer chunks
 // cut the summaries to scan, more blocks hide more latency.  Swept over 1, 2,
-// 4, 8 and 16 on GB300 at 2^20 / 2^22 elements: grand product 2 (80.0 us
-// against 86.5 for 4; 4 is 3 % faster at 2^22), division 2 (94.5 / 222
-// against 128 / 252), permutation product 8 (574 / 2125 against 592 / 2180;
-// its local pass runs 2 blocks per SM, so it needs more of them to hide
-// latency).  Evaluation has its own geometry (k_eval_tree).
+// 3 and 4 on GB300 (us at 2^20 / 2^22 / 2^24): division 2 (77 / 170 / 529;
+// 1: 72 / 171 / 559, 4: 115 / 207 / 546); permutation product 8 at 2^20 / 2^22
+// (424 / 1702; 4: 425 / 1632, 6: 451 / 1721; its local pass runs 2 blocks per
+// SM, so it needs more of them to hide latency).  Evaluation has its own
+// geometry (k_eval_tree).
 constexpr uint32_t kGpBlocksPerSm = 2, kDivBlocksPerSm = 2,
                    kPermBlocksPerSm = 8;
-// The grand product's chains grow with n while its block trees do not: at
-// 2^22 3 blocks per SM beat 2 (0.210 against 0.220 ms), at 2^24 4 beat 2 and 3
-// (0.712 against 0.764 / 0.730 ms); at 2^20 2 stays best (4: 0.081 against
-// 0.075 ms).  The division's replay was best at 2 for all three sizes.
+// The grand product's chains grow with n while its block trees do not: us with
+// 2 / 3 / 4 blocks per SM at 2^20 57.4 / 57.4 / 65.6, at 2^22 159.5 / 156.1 /
+// 162.0, at 2^24 563 / 547 / 545.
 inline uint32_t gp_blocks_per_sm(uint64_t n) {
   return n <= (1ull << 21) ? kGpBlocksPerSm : n <= (1ull << 23) ? 3 : 4;
 }
 
 // ---------------------------------------------------------------- helpers
+// A field element in shared memory as two 16-byte accesses (p 16-byte
+// aligned).  Read through a plain fr lvalue the compiler issues eight 4-byte
+// loads, and where the address is the same for the whole warp it keeps the
+// words in uniform registers, from which a wide multiply-add runs slower: the
+// dot products' 64-product term took 471 cycles per warp that way, 318 so.
+__device__ __forceinline__ fr lds_fr(const fr *p) {
+  const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+  fr r;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3])
+               : "r"(a)
+               : "memory");
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r.v[4]), "=r"(r.v[5]), "=r"(r.v[6]), "=r"(r.v[7])
+               : "r"(a + 16)
+               : "memory");
+  return r;
+}
+__device__ __forceinline__ void sts_fr(fr *p, const fr &v) { st_fr(p, v); }
+
 // Block scans are work-efficient (Blelloch, "Prefix sums and their
 // applications", 1990): an up-sweep and a down-sweep over a balanced tree,
 // 2(n-1) combines for n = blockDim.x (a power of two) instead of the n log n
@@ -52,37 +71,141 @@ inline uint32_t gp_blocks_per_sm(uint64_t n) {
 // scans (9 dependent steps instead of 16) made the 2^20 grand product,
 // evaluation and division 13-36 % slower on GB300.
 
-// prod p[i], lo <= i < hi (hi > lo), in ascending order
-__device__ __forceinline__ fr chunk_product(const fr *p, uint64_t lo, uint64_t hi) {
-  fr acc = ld_fr(p + lo);
-  for (uint64_t i = lo + 1; i < hi; ++i) acc = fr_mul(acc, ld_fr(p + i));
-  return acc;
+// A warp's view of its 32 chunks (lane l owns the K contiguous elements from
+// (gt0 + l) K): tiles of kTileElems elements per lane go through shared memory,
+// so global accesses are whole 64-byte segments (a lane reading its own chunk
+// touches 32 lines per instruction), and the next tile's cp.async copies run
+// while this one is multiplied.  In-place kernels write their results into the
+// tile and store it the same way: with plain accesses each load hits the line
+// the previous iteration's store went to, and the replay loops ran 2 to 9x
+// slower depending on how the compiler placed the two (carry-chained multiply,
+// 2^20 / 2^24: grand product 189 / 2885 us with plain accesses, 57 / 547 us
+// through the tiles; division 221 / 5686 us, 77 / 529 us).
+constexpr uint32_t kTileElems = 2, kTileUnits = 32 * 2 * kTileElems;  // 16-byte units per tile
+
+// 16 bytes, or 16 zero bytes when !valid (src is not read then)
+__device__ __forceinline__ void cp_async16(uint4 *dst, const uint4 *src, bool valid) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(valid ? 16 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() {
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// sum_{lo <= i < hi} p[i] x^(i - lo) (hi > lo) from pw[k] = x^k, k <= 16, in
-// shared memory: groups of 16 coefficients are dot products with one
-// reduction each (fr_mac17 / fr_redc17), joined by Horner steps with x^16
-__device__ __forceinline__ fr chunk_dot(const fr *p, uint64_t lo, uint64_t hi, const fr *pw) {
-  const uint64_t ng = (hi - lo + 15) >> 4;
-  fr L = fr_zero();
-#pragma unroll 1
-  for (uint64_t g = ng; g-- > 0;) {
-    const uint64_t b = lo + (g << 4);
-    const uint32_t cnt = (uint32_t)(hi - b < 16 ? hi - b : 16);
-    uint32_t acc[17];
-#pragma unroll
-    for (int k = 0; k < 17; ++k) acc[k] = 0;
-    // each coefficient is loaded one term ahead of its multiply
-    fr cur = ld_fr(p + b);
-#pragma unroll 1
-    for (uint32_t i = 0; i < cnt; ++i) {
-      const fr nxt = i + 1 < cnt ? ld_fr(p + b + i + 1) : cur;
-      fr_mac17(acc, cur, pw[i]);
-      cur = nxt;
-    }
-    const fr S = fr_redc17(acc);
-    L = g + 1 == ng ? S : fr_add(fr_mul(L, pw[16]), S);
+struct ChunkTiles {
+  uint4 *buf;     // 2 tiles of this warp
+  uint64_t base;  // first element of lane 0's chunk
+  uint64_t n, k;
+  uint32_t tiles;  // tiles per chunk
+
+  __device__ __forceinline__ ChunkTiles(uint4 *sm, uint32_t warp, uint64_t gt0, uint64_t n_, uint64_t k_)
+      : buf(sm + warp * 2 * kTileUnits), base(gt0 * k_), n(n_), k(k_),
+        tiles((uint32_t)((k_ + kTileElems - 1) / kTileElems)) {}
+
+  // unit p of row r: conflict-free for a lane's own row and for whole segments
+  static __device__ __forceinline__ uint32_t at(uint32_t r, uint32_t p) {
+    return r * 4 + (p ^ ((r >> 1) & 3));
   }
+  // element of unit u of tile t; n when it lies past the chunk or the vector
+  // (its tile slot reads as zero and is not stored)
+  __device__ __forceinline__ uint64_t elem(uint32_t u, uint32_t t) const {
+    const uint64_t off = (uint64_t)t * kTileElems + ((u & 3) >> 1);
+    const uint64_t i = base + (u >> 2) * k + off;
+    return off < k && i < n ? i : n;
+  }
+  __device__ __forceinline__ void load(const fr *p, uint32_t t, uint32_t slot) const {
+    const uint32_t lane = threadIdx.x & 31;
+    uint4 *s = buf + slot * kTileUnits;
+#pragma unroll
+    for (uint32_t q = 0; q < kTileUnits / 32; ++q) {
+      const uint32_t u = q * 32 + lane;
+      const uint64_t i = elem(u, t);
+      const bool valid = i < n;
+      cp_async16(s + at(u >> 2, u & 3), reinterpret_cast<const uint4 *>(p + (valid ? i : 0)) + (u & 1), valid);
+    }
+  }
+  __device__ __forceinline__ void store(fr *p, uint32_t t, uint32_t slot) const {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint4 *s = buf + slot * kTileUnits;
+#pragma unroll
+    for (uint32_t q = 0; q < kTileUnits / 32; ++q) {
+      const uint32_t u = q * 32 + lane;
+      const uint64_t i = elem(u, t);
+      if (i < n) reinterpret_cast<uint4 *>(p + i)[u & 1] = s[at(u >> 2, u & 3)];
+    }
+  }
+  // element e of this lane's row of the tile in `slot`
+  __device__ __forceinline__ fr get(uint32_t slot, uint32_t e) const {
+    const uint4 *s = buf + slot * kTileUnits;
+    const uint32_t lane = threadIdx.x & 31;
+    const uint4 a = s[at(lane, 2 * e)], b = s[at(lane, 2 * e + 1)];
+    return fr{{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}};
+  }
+  __device__ __forceinline__ void put(uint32_t slot, uint32_t e, const fr &v) const {
+    uint4 *s = buf + slot * kTileUnits;
+    const uint32_t lane = threadIdx.x & 31;
+    s[at(lane, 2 * e)] = make_uint4(v.v[0], v.v[1], v.v[2], v.v[3]);
+    s[at(lane, 2 * e + 1)] = make_uint4(v.v[4], v.v[5], v.v[6], v.v[7]);
+  }
+
+  // body(step, tile, slot) for steps 0 .. tiles-1 in the order tile_of(step);
+  // with out, the tile is stored there after its body
+  template <typename Order, typename Body>
+  __device__ __forceinline__ void run(const fr *in, fr *out, Order tile_of, Body body) const {
+    load(in, tile_of(0u), 0);
+    cp_async_commit();
+#pragma unroll 1
+    for (uint32_t s = 0; s < tiles; ++s) {
+      if (s + 1 < tiles) load(in, tile_of(s + 1), (s + 1) & 1);
+      cp_async_commit();
+      cp_async_wait<1>();  // this step's tile has landed
+      __syncwarp();
+      const uint32_t t = tile_of(s);
+      body(s, t, s & 1);
+      __syncwarp();
+      if (out) {
+        store(out, t, s & 1);
+        __syncwarp();
+      }
+    }
+  }
+};
+constexpr uint32_t kTileSmemUnits = (kScanThreads / 32) * 2 * kTileUnits;  // 32 KiB
+static_assert(kTileSmemUnits * sizeof(uint4) >= 2 * kScanThreads * sizeof(fr),
+              "the block scans reuse the tiles' shared memory");
+
+// sum p[lo + i] x^i over this lane's chunk (lo = its first element; elements
+// past the vector read as zero) from pw[k] = x^k, k <= 16, in shared memory: groups of
+// 16 coefficients are dot products with one reduction each (fr_mac17 /
+// fr_redc17), joined by Horner steps with x^16.  Whole warps only.
+__device__ __forceinline__ fr chunk_dot(const ChunkTiles &ct, const fr *p, const fr *pw) {
+  constexpr uint32_t TG = 16 / kTileElems;  // tiles per group
+  const uint32_t ng = (ct.tiles + TG - 1) / TG, top = ct.tiles - (ng - 1) * TG;
+  fr L = fr_zero();
+  uint32_t acc[17];
+#pragma unroll
+  for (int k = 0; k < 17; ++k) acc[k] = 0;
+  // groups from the top down, the tiles of a group upwards
+  const auto order = [&](uint32_t s) {
+    return s < top ? (ng - 1) * TG + s : (ng - 2 - (s - top) / TG) * TG + (s - top) % TG;
+  };
+  ct.run(p, nullptr, order, [&](uint32_t, uint32_t t, uint32_t slot) {
+    const uint32_t e0 = (t % TG) * kTileElems;
+#pragma unroll
+    for (uint32_t e = 0; e < kTileElems; ++e)
+      fr_mac17(acc, ct.get(slot, e), lds_fr(pw + e0 + e));
+    if (t % TG == TG - 1 || t == ct.tiles - 1) {  // the group's last tile
+      const fr S = fr_redc17(acc);
+      L = t / TG == ng - 1 ? S : fr_add(fr_mul(L, lds_fr(pw + 16)), S);
+#pragma unroll
+      for (int k = 0; k < 17; ++k) acc[k] = 0;
+    }
+  });
   return L;
 }
 
@@ -101,7 +224,7 @@ __device__ __forceinline__ void warp_power_table17(const fr &x, fr *pw) {
     }
     if (lane > h && lane <= 2 * h) v = fr_mul(lowv, hv);
   }
-  if (lane <= 16) pw[lane] = v;
+  if (lane <= 16) sts_fr(pw + lane, v);
 }
 
 // inclusive prefix product over a block of 256 threads (commutative);
@@ -117,35 +240,35 @@ __device__ fr block_prefix_product(fr v, fr *s) {
   const int t = threadIdx.x;
   constexpr int n = kScanThreads;
   static_assert(kScanThreads == 256, "32 runs of 8");
-  s[t] = v;
+  sts_fr(s + t, v);
   __syncthreads();
   for (int d = 1; d < 8; d <<= 1) {
     const int idx = (t + 1) * 2 * d - 1;
-    if (idx < n) s[idx] = fr_mul(s[idx - d], s[idx]);
+    if (idx < n) sts_fr(s + idx, fr_mul(lds_fr(s + idx - d), lds_fr(s + idx)));
     __syncthreads();
   }
   if (t < 32) {
-    fr inc = s[8 * t + 7];
+    fr inc = lds_fr(s + 8 * t + 7);
     for (int o = 1; o < 32; o <<= 1) {
       const fr u = shfl_up_fr(inc, o);
       if (t >= o) inc = fr_mul(u, inc);
     }
     const fr ex = shfl_up_fr(inc, 1);
-    s[8 * t + 7] = t ? ex : fr_one();
+    sts_fr(s + 8 * t + 7, t ? ex : fr_one());
   }
   __syncthreads();
   for (int d = 4; d >= 1; d >>= 1) {
     const int idx = (t + 1) * 2 * d - 1;
     if (idx < n) {
-      const fr left = s[idx - d];
-      s[idx - d] = s[idx];
-      s[idx] = fr_mul(s[idx], left);
+      const fr left = lds_fr(s + idx - d);
+      sts_fr(s + idx - d, lds_fr(s + idx));
+      sts_fr(s + idx, fr_mul(lds_fr(s + idx), left));
     }
     __syncthreads();
   }
-  const fr incl = fr_mul(s[t], v);
+  const fr incl = fr_mul(lds_fr(s + t), v);
   __syncthreads();
-  s[t] = incl;
+  sts_fr(s + t, incl);
   __syncthreads();
   return incl;
 }
@@ -176,20 +299,20 @@ __device__ fr warp_block_prefix_product(fr v, fr *s) {
     const fr u = shfl_up_fr(v, o);
     if (lane >= o) v = fr_mul(u, v);
   }
-  if (lane == 31) s[w] = v;  // warp totals
+  if (lane == 31) sts_fr(s + w, v);  // warp totals
   __syncthreads();
   if (w == 0) {
-    fr x = lane < nw ? s[lane] : fr_one();
+    fr x = lane < nw ? lds_fr(s + lane) : fr_one();
     for (int o = 1; o < nw; o <<= 1) {
       const fr u = shfl_up_fr(x, o);
       if (lane >= o) x = fr_mul(u, x);
     }
-    if (lane < nw) s[lane] = x;  // warps 0 .. lane
+    if (lane < nw) sts_fr(s + lane, x);  // warps 0 .. lane
   }
   __syncthreads();
-  if (w > 0) v = fr_mul(s[w - 1], v);
+  if (w > 0) v = fr_mul(lds_fr(s + w - 1), v);
   __syncthreads();
-  s[t] = v;
+  sts_fr(s + t, v);
   __syncthreads();
   return v;
 }
@@ -200,20 +323,20 @@ __device__ fr warp_block_suffix_product(fr v, fr *s) {
     const fr u = shfl_down_fr(v, o);
     if (lane + o < 32) v = fr_mul(v, u);
   }
-  if (lane == 0) s[w] = v;  // warp totals
+  if (lane == 0) sts_fr(s + w, v);  // warp totals
   __syncthreads();
   if (w == 0) {
-    fr x = lane < nw ? s[lane] : fr_one();
+    fr x = lane < nw ? lds_fr(s + lane) : fr_one();
     for (int o = 1; o < nw; o <<= 1) {
       const fr u = shfl_down_fr(x, o);
       if (lane + o < nw) x = fr_mul(x, u);
     }
-    if (lane < nw) s[lane] = x;  // warps lane .. nw-1
+    if (lane < nw) sts_fr(s + lane, x);  // warps lane .. nw-1
   }
   __syncthreads();
-  if (w + 1 < nw) v = fr_mul(v, s[w + 1]);
+  if (w + 1 < nw) v = fr_mul(v, lds_fr(s + w + 1));
   __syncthreads();
-  s[t] = v;
+  sts_fr(s + t, v);
   __syncthreads();
   return v;
 }
@@ -236,8 +359,8 @@ template <bool NAMED = false>
 __device__ void block_affine_suffix(fr &a, fr &b, fr *sa, fr *sb, bool all = true) {
   const int t = threadIdx.x, n = NAMED ? kScanThreads : blockDim.x;
   const int u = n - 1 - t;
-  sa[u] = a;
-  sb[u] = b;
+  sts_fr(sa + u, a);
+  sts_fr(sb + u, b);
   scan_sync<NAMED>();
   // The full scan of 256 maps takes the hybrid form of block_prefix_product:
   // three up-sweep levels, one warp scanning the 32 run maps, three
@@ -247,19 +370,19 @@ __device__ void block_affine_suffix(fr &a, fr &b, fr *sa, fr *sb, bool all = tru
   for (int d = 1; d < (hybrid ? 8 : n); d <<= 1) {
     const int idx = (t + 1) * 2 * d - 1;
     if (idx < n) {
-      const fr la = sa[idx - d], lb = sb[idx - d], ra = sa[idx], rb = sb[idx];
-      sa[idx] = fr_add(ra, fr_mul(rb, la));
-      sb[idx] = fr_mul(rb, lb);
+      const fr la = lds_fr(sa + idx - d), lb = lds_fr(sb + idx - d), ra = lds_fr(sa + idx), rb = lds_fr(sb + idx);
+      sts_fr(sa + idx, fr_add(ra, fr_mul(rb, la)));
+      sts_fr(sb + idx, fr_mul(rb, lb));
     }
     scan_sync<NAMED>();
   }
   if (!all) {
     // sa[n-1], sb[n-1] = G_{n-1} = F_0
     if (t == 0) {
-      a = sa[n - 1];
-      b = sb[n - 1];
-      sa[0] = a;
-      sb[0] = b;
+      a = lds_fr(sa + n - 1);
+      b = lds_fr(sb + n - 1);
+      sts_fr(sa, a);
+      sts_fr(sb, b);
     }
     scan_sync<NAMED>();
     return;
@@ -267,7 +390,7 @@ __device__ void block_affine_suffix(fr &a, fr &b, fr *sa, fr *sb, bool all = tru
   if (hybrid) {
     if (t < 32) {
       // exclusive scan of the run maps at u = 8k + 7, in u order
-      fr xa = sa[8 * t + 7], xb = sb[8 * t + 7];
+      fr xa = lds_fr(sa + 8 * t + 7), xb = lds_fr(sb + 8 * t + 7);
       for (int o = 1; o < 32; o <<= 1) {
         const fr ua = shfl_up_fr(xa, o), ub = shfl_up_fr(xb, o);
         if (t >= o) {
@@ -276,31 +399,31 @@ __device__ void block_affine_suffix(fr &a, fr &b, fr *sa, fr *sb, bool all = tru
         }
       }
       const fr ea = shfl_up_fr(xa, 1), eb = shfl_up_fr(xb, 1);
-      sa[8 * t + 7] = t ? ea : fr_zero();
-      sb[8 * t + 7] = t ? eb : fr_one();
+      sts_fr(sa + 8 * t + 7, t ? ea : fr_zero());
+      sts_fr(sb + 8 * t + 7, t ? eb : fr_one());
     }
   } else if (t == 0) {
-    sa[n - 1] = fr_zero();
-    sb[n - 1] = fr_one();
+    sts_fr(sa + n - 1, fr_zero());
+    sts_fr(sb + n - 1, fr_one());
   }
   scan_sync<NAMED>();
   for (int d = hybrid ? 4 : n >> 1; d >= 1; d >>= 1) {
     const int idx = (t + 1) * 2 * d - 1;
     if (idx < n) {
-      const fr la = sa[idx - d], lb = sb[idx - d], pa = sa[idx], pb = sb[idx];
-      sa[idx - d] = pa;
-      sb[idx - d] = pb;
-      sa[idx] = fr_add(la, fr_mul(lb, pa));  // left o P
-      sb[idx] = fr_mul(lb, pb);
+      const fr la = lds_fr(sa + idx - d), lb = lds_fr(sb + idx - d), pa = lds_fr(sa + idx), pb = lds_fr(sb + idx);
+      sts_fr(sa + idx - d, pa);
+      sts_fr(sb + idx - d, pb);
+      sts_fr(sa + idx, fr_add(la, fr_mul(lb, pa)));  // left o P
+      sts_fr(sb + idx, fr_mul(lb, pb));
     }
     scan_sync<NAMED>();
   }
   // exclusive E_u in (sa[u], sb[u]); inclusive G_u = g_u o E_u = F_t
-  const fr ea = sa[u], eb = sb[u];
+  const fr ea = lds_fr(sa + u), eb = lds_fr(sb + u);
   const fr ia = fr_add(a, fr_mul(b, ea)), ib = fr_mul(b, eb);
   scan_sync<NAMED>();
-  sa[t] = ia;
-  sb[t] = ib;
+  sts_fr(sa + t, ia);
+  sts_fr(sb + t, ib);
   a = ia;
   b = ib;
   scan_sync<NAMED>();
@@ -309,13 +432,22 @@ __device__ void block_affine_suffix(fr &a, fr &b, fr *sa, fr *sb, bool all = tru
 // ------------------------------------------------------------ grand product
 __device__ __forceinline__ void gp_local_body(const fr *__restrict__ in, const ScanGeom &g,
                                               fr *__restrict__ thread_excl,
-                                              fr *__restrict__ block_total, uint32_t blk, fr *s) {
+                                              fr *__restrict__ block_total, uint32_t blk, uint4 *sm) {
+  fr *s = reinterpret_cast<fr *>(sm);
   const uint64_t gt = blk * (uint64_t)kScanThreads + threadIdx.x;
-  const uint64_t lo = gt * g.k, hi = lo + g.k < g.n ? lo + g.k : g.n;
-  const fr p = lo < hi ? chunk_product(in, lo, hi) : fr_one();
+  const ChunkTiles ct(sm, threadIdx.x >> 5, gt - (threadIdx.x & 31), g.n, g.k);
+  // elements past the vector read as zero: only lanes after the last element
+  // see those products, and nothing reads theirs
+  fr p = fr_one();
+  ct.run(in, nullptr, [](uint32_t st) { return st; }, [&](uint32_t, uint32_t t, uint32_t slot) {
+#pragma unroll
+    for (uint32_t e = 0; e < kTileElems; ++e)
+      if (e == 0 || t * kTileElems + e < g.k) p = t + e ? fr_mul(p, ct.get(slot, e)) : ct.get(slot, e);
+  });
+  __syncthreads();
   const fr incl = block_prefix_product(p, s);
   // exclusive = inclusive of the previous thread
-  const fr excl = threadIdx.x ? s[threadIdx.x - 1] : fr_one();
+  const fr excl = threadIdx.x ? lds_fr(s + threadIdx.x - 1) : fr_one();
   if (gt < g.threads) st_fr(thread_excl + gt, excl);
   if (threadIdx.x == blockDim.x - 1) st_fr(block_total + blk, incl);
 }
@@ -323,8 +455,8 @@ __device__ __forceinline__ void gp_local_body(const fr *__restrict__ in, const S
 __global__ void __launch_bounds__(kScanThreads) k_gp_local(const fr *__restrict__ in, ScanGeom g,
                                                             fr *__restrict__ thread_excl,
                                                             fr *__restrict__ block_total) {
-  __shared__ fr s[kScanThreads];
-  gp_local_body(in, g, thread_excl, block_total, blockIdx.x, s);
+  __shared__ uint4 sm[kTileSmemUnits];
+  gp_local_body(in, g, thread_excl, block_total, blockIdx.x, sm);
 }
 
 // out_excl[i] = prod_{j<i} in[j] and/or out_incl[i] = prod_{j<=i} in[j]; either
@@ -332,35 +464,47 @@ __global__ void __launch_bounds__(kScanThreads) k_gp_local(const fr *__restrict_
 __device__ __forceinline__ void gp_apply_body(const fr *in, fr *out_excl, fr *out_incl,
                                               const ScanGeom &g, const fr *__restrict__ thread_excl,
                                               const fr *__restrict__ block_total, uint32_t blk,
-                                              fr *s) {
+                                              uint4 *sm) {
   // product of the totals of all earlier blocks
+  fr *s = reinterpret_cast<fr *>(sm);
   fr p = fr_one();
   for (uint32_t b = threadIdx.x; b < blk; b += blockDim.x) p = fr_mul(p, ld_fr(block_total + b));
-  s[threadIdx.x] = p;
+  sts_fr(s + threadIdx.x, p);
   __syncthreads();
   for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) s[threadIdx.x] = fr_mul(s[threadIdx.x], s[threadIdx.x + o]);
+    if ((int)threadIdx.x < o) sts_fr(s + threadIdx.x, fr_mul(lds_fr(s + threadIdx.x), lds_fr(s + threadIdx.x + o)));
     __syncthreads();
   }
-  const fr block_prefix = s[0];
+  const fr block_prefix = lds_fr(s);
+  __syncthreads();  // the tiles reuse s
   const uint64_t gt = blk * (uint64_t)kScanThreads + threadIdx.x;
-  if (gt >= g.threads) return;
-  fr run = fr_mul(block_prefix, ld_fr(thread_excl + gt));
-  const uint64_t lo = gt * g.k, hi = lo + g.k < g.n ? lo + g.k : g.n;
-  for (uint64_t i = lo; i < hi; ++i) {
-    const fr v = ld_fr(in + i);
-    if (out_excl) st_fr(out_excl + i, run);
-    run = fr_mul(run, v);
-    if (out_incl) st_fr(out_incl + i, run);
-  }
+  const uint64_t lo = gt * g.k;
+  fr run = gt < g.threads ? fr_mul(block_prefix, ld_fr(thread_excl + gt)) : fr_one();
+  const ChunkTiles ct(sm, threadIdx.x >> 5, gt - (threadIdx.x & 31), g.n, g.k);
+  // the tile leaves with the exclusive products (or, without out_excl, the
+  // inclusive ones); when both are wanted the lanes store the inclusive ones
+  ct.run(in, out_excl ? out_excl : out_incl, [](uint32_t st) { return st; },
+         [&](uint32_t, uint32_t t, uint32_t slot) {
+#pragma unroll
+           for (uint32_t e = 0; e < kTileElems; ++e) {
+             const uint64_t i = (uint64_t)t * kTileElems + e;
+             if (e == 0 || i < g.k) {
+               const fr v = ct.get(slot, e);
+               if (out_excl) ct.put(slot, e, run);
+               run = fr_mul(run, v);
+               if (!out_excl) ct.put(slot, e, run);
+               else if (out_incl && lo + i < g.n) st_fr(out_incl + lo + i, run);
+             }
+           }
+         });
 }
 
 __global__ void __launch_bounds__(kScanThreads) k_gp_apply(const fr *in, fr *out_excl, fr *out_incl,
                                                             ScanGeom g,
                                                             const fr *__restrict__ thread_excl,
                                                             const fr *__restrict__ block_total) {
-  __shared__ fr s[kScanThreads];
-  gp_apply_body(in, out_excl, out_incl, g, thread_excl, block_total, blockIdx.x, s);
+  __shared__ uint4 sm[kTileSmemUnits];
+  gp_apply_body(in, out_excl, out_incl, g, thread_excl, block_total, blockIdx.x, sm);
 }
 
 // Batched grand products: the blocks of all jobs are numbered consecutively
@@ -379,20 +523,20 @@ __device__ __forceinline__ uint32_t find_job(const uint32_t *__restrict__ start,
 __global__ void __launch_bounds__(kScanThreads) k_gp_local_batch(const GpBatchJob *__restrict__ jobs,
                                                                   const uint32_t *__restrict__ start,
                                                                   uint32_t count) {
-  __shared__ fr s[kScanThreads];
+  __shared__ uint4 sm[kTileSmemUnits];
   const uint32_t j = find_job(start, count, blockIdx.x);
   const GpBatchJob jb = jobs[j];
-  gp_local_body(jb.in, jb.g, jb.thread_excl, jb.block_total, blockIdx.x - start[j], s);
+  gp_local_body(jb.in, jb.g, jb.thread_excl, jb.block_total, blockIdx.x - start[j], sm);
 }
 
 __global__ void __launch_bounds__(kScanThreads) k_gp_apply_batch(const GpBatchJob *__restrict__ jobs,
                                                                   const uint32_t *__restrict__ start,
                                                                   uint32_t count) {
-  __shared__ fr s[kScanThreads];
+  __shared__ uint4 sm[kTileSmemUnits];
   const uint32_t j = find_job(start, count, blockIdx.x);
   const GpBatchJob jb = jobs[j];
   gp_apply_body(jb.in, jb.out, nullptr, jb.g, jb.thread_excl, jb.block_total, blockIdx.x - start[j],
-                s);
+                sm);
 }
 
 int gp_batch_launch(const GpBatchJob *d_jobs, const uint32_t *d_block_start, uint32_t count,
@@ -430,7 +574,7 @@ __global__ void __launch_bounds__(kScanThreads, 2)
     k_perm_local(const PermArgs a, ScanGeom g, fr *__restrict__ thread_num,
                  fr *__restrict__ thread_den, fr *__restrict__ block_num,
                  fr *__restrict__ block_den) {
-  __shared__ fr s1[kScanThreads], s2[kScanThreads];
+  __shared__ __align__(16) fr s1[kScanThreads], s2[kScanThreads];
   const fr beta = ld_fr(a.params), gamma = ld_fr(a.params + 1);
   const fr bk0 = fr_mul(beta, ld_fr(a.params + 2));
   const fr bk1 = fr_mul(beta, ld_fr(a.params + 3));
@@ -460,8 +604,8 @@ __global__ void __launch_bounds__(kScanThreads, 2)
   const fr incl_n = warp_block_prefix_product(N, s1);  // s1[t] = N_0 .. N_t
   const fr incl_d = warp_block_suffix_product(D, s2);  // s2[t] = D_t .. D_last
   if (gt < g.threads) {
-    st_fr(thread_num + gt, threadIdx.x ? s1[threadIdx.x - 1] : fr_one());
-    st_fr(thread_den + gt, threadIdx.x + 1 < blockDim.x ? s2[threadIdx.x + 1] : fr_one());
+    st_fr(thread_num + gt, threadIdx.x ? lds_fr(s1 + threadIdx.x - 1) : fr_one());
+    st_fr(thread_den + gt, threadIdx.x + 1 < blockDim.x ? lds_fr(s2 + threadIdx.x + 1) : fr_one());
   }
   if (threadIdx.x == blockDim.x - 1) st_fr(block_num + blockIdx.x, incl_n);
   if (threadIdx.x == 0) st_fr(block_den + blockIdx.x, incl_d);
@@ -472,7 +616,7 @@ __global__ void __launch_bounds__(kScanThreads, 2)
 // denominator totals of the blocks after b, divided by all denominators.
 __global__ void __launch_bounds__(kScanThreads) k_perm_carry(fr *block_num, fr *block_den,
                                                               uint32_t nb) {
-  __shared__ fr s1[kScanThreads], s2[kScanThreads];
+  __shared__ __align__(16) fr s1[kScanThreads], s2[kScanThreads];
   __shared__ fr s_inv;
   const uint32_t per = (nb + blockDim.x - 1) / blockDim.x;
   const uint32_t lo = threadIdx.x * per < nb ? threadIdx.x * per : nb;
@@ -484,10 +628,10 @@ __global__ void __launch_bounds__(kScanThreads) k_perm_carry(fr *block_num, fr *
   }
   warp_block_prefix_product(N, s1);
   warp_block_suffix_product(D, s2);  // s2[0]: every denominator (none is zero)
-  if (threadIdx.x == 0) s_inv = fr_inv_fast(s2[0]);
+  if (threadIdx.x == 0) s_inv = fr_inv_fast(lds_fr(s2));
   __syncthreads();
-  fr run_n = threadIdx.x ? s1[threadIdx.x - 1] : fr_one();
-  fr run_d = fr_mul(s_inv, threadIdx.x + 1 < blockDim.x ? s2[threadIdx.x + 1] : fr_one());
+  fr run_n = threadIdx.x ? lds_fr(s1 + threadIdx.x - 1) : fr_one();
+  fr run_d = fr_mul(s_inv, threadIdx.x + 1 < blockDim.x ? lds_fr(s2 + threadIdx.x + 1) : fr_one());
   for (uint32_t b = lo; b < hi; ++b) {
     const fr v = ld_fr(block_num + b);
     st_fr(block_num + b, run_n);
@@ -533,14 +677,15 @@ __global__ void __launch_bounds__(kScanThreads)
 // with kScanThreads + 32 threads: the extra warp computes m^K while the
 // others evaluate their chunks (chunk_dot, after the first warp's table of
 // m^0 .. m^16), which do not need it.
-__global__ void __launch_bounds__(kScanThreads + 32) k_affine_local(const fr *__restrict__ p, ScanGeom g,
+__global__ void __launch_bounds__(kScanThreads + 32, 2) k_affine_local(const fr *__restrict__ p, ScanGeom g,
                                                                      const fr *__restrict__ m_ptr,
                                                                      int negate_m, fr *thread_a,
                                                                      fr *thread_b, fr *block_a,
                                                                      fr *block_b) {
-  __shared__ fr sa[kScanThreads], sb[kScanThreads];
+  __shared__ uint4 sm[kTileSmemUnits];  // the chunks' tiles, then the scan
+  fr *sa = reinterpret_cast<fr *>(sm), *sb = sa + kScanThreads;
   __shared__ fr s_mk;
-  __shared__ fr s_pw[17];  // m^k, k <= 16, for the chunks' dot products
+  __shared__ __align__(16) fr s_pw[17];  // m^k, k <= 16, for the chunks' dot products
   fr m = ld_fr(m_ptr);
   if (negate_m) m = fr_neg(m);
   if (threadIdx.x >= kScanThreads) {
@@ -553,14 +698,15 @@ __global__ void __launch_bounds__(kScanThreads + 32) k_affine_local(const fr *__
   const uint64_t gt = blockIdx.x * (uint64_t)kScanThreads + threadIdx.x;
   const uint64_t lo = gt * g.k < g.n ? gt * g.k : g.n;
   const uint64_t hi = lo + g.k < g.n ? lo + g.k : g.n;
-  const fr L = hi > lo ? chunk_dot(p, lo, hi, s_pw) : fr_zero();
-  __syncthreads();  // m^K ready
+  const ChunkTiles ct(sm, threadIdx.x >> 5, gt - (threadIdx.x & 31), g.n, g.k);
+  const fr L = chunk_dot(ct, p, s_pw);
+  __syncthreads();  // m^K ready, tiles free
   fr a = L, b = hi - lo == g.k ? s_mk : hi > lo ? fr_pow_u64(m, hi - lo) : fr_one();
   block_affine_suffix<true>(a, b, sa, sb, thread_a != nullptr);
   if (thread_a && gt < g.threads) {
     const bool last = threadIdx.x == kScanThreads - 1;
-    st_fr(thread_a + gt, last ? fr_zero() : sa[threadIdx.x + 1]);
-    st_fr(thread_b + gt, last ? fr_one() : sb[threadIdx.x + 1]);
+    st_fr(thread_a + gt, last ? fr_zero() : lds_fr(sa + threadIdx.x + 1));
+    st_fr(thread_b + gt, last ? fr_one() : lds_fr(sb + threadIdx.x + 1));
   }
   if (threadIdx.x == 0) {
     st_fr(block_a + blockIdx.x, a);
@@ -584,8 +730,8 @@ __device__ void compose_blocks(const fr *block_a, const fr *block_b, uint32_t fi
     b = fr_mul(bi, b);
   }
   block_affine_suffix(a, b, sa, sb, false);
-  A = sa[0];
-  B = sb[0];
+  A = lds_fr(sa);
+  B = lds_fr(sb);
 }
 
 __global__ void __launch_bounds__(kScanThreads) k_div_apply(fr *inout, ScanGeom g,
@@ -594,26 +740,34 @@ __global__ void __launch_bounds__(kScanThreads) k_div_apply(fr *inout, ScanGeom 
                                                              const fr *__restrict__ thread_b,
                                                              const fr *__restrict__ block_a,
                                                              const fr *__restrict__ block_b) {
-  __shared__ fr sa[kScanThreads], sb[kScanThreads];
+  __shared__ uint4 sm[kTileSmemUnits];  // the composition's scan, then the tiles
+  fr *sa = reinterpret_cast<fr *>(sm), *sb = sa + kScanThreads;
   const fr m = fr_neg(ld_fr(m_ptr));
   fr A, B;
   compose_blocks(block_a, block_b, blockIdx.x + 1, g.blocks, A, B, sa, sb);
+  __syncthreads();
   const fr s_end_block = A;  // S at the end of this block (S_n = 0)
   const uint64_t gt = blockIdx.x * (uint64_t)kScanThreads + threadIdx.x;
-  if (gt >= g.threads) return;
-  fr s = fr_add(ld_fr(thread_a + gt), fr_mul(ld_fr(thread_b + gt), s_end_block));
-  const uint64_t lo = gt * g.k, hi = lo + g.k < g.n ? lo + g.k : g.n;
-  for (uint64_t i = hi; i > lo; --i) {
-    const fr pi = ld_fr(inout + i - 1);
-    st_fr(inout + i - 1, s);  // q_{i-1} = S_i
-    s = fr_add(pi, fr_mul(m, s));
-  }
+  // past the vector S = 0 and elements read as zero, so s stays 0 there
+  fr s = gt < g.threads ? fr_add(ld_fr(thread_a + gt), fr_mul(ld_fr(thread_b + gt), s_end_block))
+                        : fr_zero();
+  const ChunkTiles ct(sm, threadIdx.x >> 5, gt - (threadIdx.x & 31), g.n, g.k);
+  const uint32_t last = ct.tiles - 1;
+  ct.run(inout, inout, [&](uint32_t st) { return last - st; }, [&](uint32_t, uint32_t t, uint32_t slot) {
+#pragma unroll
+    for (int e = (int)kTileElems - 1; e >= 0; --e)
+      if (e == 0 || t * kTileElems + e < g.k) {
+        const fr pi = ct.get(slot, e);
+        ct.put(slot, e, s);  // q_i = S_(i+1)
+        s = fr_add(pi, fr_mul(m, s));
+      }
+  });
 }
 
 __global__ void __launch_bounds__(kScanThreads) k_eval_final(const fr *__restrict__ block_a,
                                                               const fr *__restrict__ block_b,
                                                               uint32_t count, fr *y) {
-  __shared__ fr sa[kScanThreads], sb[kScanThreads];
+  __shared__ __align__(16) fr sa[kScanThreads], sb[kScanThreads];
   fr A, B;
   compose_blocks(block_a, block_b, 0, count, A, B, sa, sb);
   if (threadIdx.x == 0) st_fr(y, A);
@@ -642,8 +796,9 @@ __global__ void __launch_bounds__(kScanThreads) k_eval_final(const fr *__restric
 // Blocks per SM: 1 up to 2^21 coefficients, 2 above.  At 2^20 the helpers'
 // powers (a chain of about 25 dependent multiplies, slowed by the Horner warps
 // that share their SM) end after the chains, so fewer Horner warps per SM
-// finish the block sooner (41.8 against 46.1 us); at 2^22 the chains are the
-// longer part and two blocks per SM are as fast (106 against 108 us).
+// finish the block sooner (30.8 against 32.9 us); at 2^22 and 2^24 the chains
+// are the longer part and two blocks per SM are faster (70.3 against 73.9 us,
+// 223 against 246 us).
 constexpr uint32_t kEvalBlocksPerSmSmall = 1, kEvalBlocksPerSm = 2;
 constexpr uint64_t kEvalSmallMax = 1ull << 21;
 constexpr uint32_t kEvalHelperWarps = 2;
@@ -678,10 +833,11 @@ __global__ void __launch_bounds__(HT + 32 * kEvalHelperWarps)
                 fr *__restrict__ block_val, uint32_t *__restrict__ ticket, fr *__restrict__ y) {
   static_assert(HT % 32 == 0 && HT <= 256, "Horner threads: whole warps, at most 256");
   constexpr uint32_t kHelpers = 32 * kEvalHelperWarps, kWarps = HT / 32;
-  __shared__ fr tab[32];  // tab[a] = x^(K a), tab[16 + a] = x^(16 K a), a < 16
+  __shared__ uint4 sm[kWarps * 2 * kTileUnits];
+  __shared__ __align__(16) fr tab[32];  // tab[a] = x^(K a), tab[16 + a] = x^(16 K a), a < 16
   __shared__ fr s_wb;     // x^(HT K b)
-  __shared__ fr s_pw[17]; // x^k, k <= 16, for the Horner threads' dot products
-  __shared__ fr s_warp[kWarps];
+  __shared__ __align__(16) fr s_pw[17]; // x^k, k <= 16, for the Horner threads' dot products
+  __shared__ __align__(16) fr s_warp[kWarps];
   __shared__ uint32_t s_last;
   // warps 0 and 1 are the helpers
   const uint32_t lane = threadIdx.x & 31;
@@ -694,7 +850,7 @@ __global__ void __launch_bounds__(HT + 32 * kEvalHelperWarps)
     fr u = v;
 #pragma unroll 1
     for (int i = 0; i < 4; ++i) u = fr_sqr(u);
-    tab[lane] = fr_pow_u64(lane < 16 ? v : u, lane & 15);
+    sts_fr(tab + lane, fr_pow_u64(lane < 16 ? v : u, lane & 15));
   } else if (threadIdx.x < kHelpers) {
     // the block's weight: (x^(HT K))^b
     fr v = fr_pow_u64(x, g.k);
@@ -707,18 +863,18 @@ __global__ void __launch_bounds__(HT + 32 * kEvalHelperWarps)
     // it on a named barrier (the helper warps do not)
     if (warp == 0) warp_power_table17(x, s_pw);
     asm volatile("bar.sync 1, %0;" ::"n"(HT) : "memory");
-    const uint64_t lo = ((uint64_t)blockIdx.x * HT + t) * g.k;
-    if (lo < g.n) L = chunk_dot(p, lo, lo + g.k < g.n ? lo + g.k : g.n, s_pw);
+    const ChunkTiles ct(sm, warp, (uint64_t)blockIdx.x * HT + t - lane, g.n, g.k);
+    L = chunk_dot(ct, p, s_pw);
   }
   __syncthreads();  // the tables, the block weight and the chunk values are ready
   if (threadIdx.x >= kHelpers) {
-    const fr w = fr_mul(tab[t & 15], tab[16 + (t >> 4)]);  // x^(K t)
+    const fr w = fr_mul(lds_fr(tab + (t & 15)), lds_fr(tab + 16 + (t >> 4)));  // x^(K t)
     const fr sum = warp_sum_fr(fr_mul(L, w));
-    if (lane == 0) s_warp[warp] = sum;
+    if (lane == 0) sts_fr(s_warp + warp, sum);
   }
   __syncthreads();
   if (threadIdx.x < 32) {
-    fr v = warp_sum_fr(lane < kWarps ? s_warp[lane] : fr_zero());
+    fr v = warp_sum_fr(lane < kWarps ? lds_fr(s_warp + lane) : fr_zero());
     if (lane == 0) {
       st_fr(block_val + blockIdx.x, fr_mul(v, s_wb));
       __threadfence();
@@ -733,11 +889,11 @@ __global__ void __launch_bounds__(HT + 32 * kEvalHelperWarps)
     fr acc = fr_zero();
     for (uint32_t b = t; b < gridDim.x; b += HT) acc = fr_add(acc, ldcg_fr(block_val + b));
     acc = warp_sum_fr(acc);
-    if (lane == 0) s_warp[warp] = acc;
+    if (lane == 0) sts_fr(s_warp + warp, acc);
   }
   __syncthreads();
   if (threadIdx.x < 32) {
-    const fr v = warp_sum_fr(lane < kWarps ? s_warp[lane] : fr_zero());
+    const fr v = warp_sum_fr(lane < kWarps ? lds_fr(s_warp + lane) : fr_zero());
     if (lane == 0) {
       st_fr(y, v);
       *ticket = 0;
