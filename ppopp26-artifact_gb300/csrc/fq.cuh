@@ -96,8 +96,10 @@ PP_HD fq fq_dbl(const fq &a) { return fq_add(a, a); }
 
 PP_HD fq fq_neg(const fq &a) { return fq_sub(fq_zero(), a); }
 
-// Montgomery product a b R^-1 mod q: CIOS with the rows of Fr's variant 9
-// (independent wide products per row, one add chain), m_i = t_0 * q' per row.
+// ---- row forms of the Montgomery product a b R^-1 mod q, CIOS with
+// m_i = t_0 * q' per row: the host tests hold them against fq_mul's
+// carry-chained cells (below), which replaced them in the kernels.
+// Row 0: independent wide products per row, one add chain.
 PP_HD void fq_row_ab(uint32_t t[14], uint32_t ai, const uint32_t b[12]) {
   uint32_t lo[12], hi[12];
 #pragma unroll
@@ -138,9 +140,7 @@ PP_HD void fq_row_red(uint32_t t[14]) {
 }
 
 // The same rows with bare wide products and two add chains (low words, then
-// high words).  A wide multiply with a 64-bit addend holds the integer-
-// multiply pipe about 1.4 times as long as a bare one; the second add chain
-// runs on the ALU pipe instead.
+// high words).
 PP_HD void fq_row_ab_wide(uint32_t t[14], uint32_t ai, const uint32_t b[12]) {
   uint32_t lo[12], hi[12];
 #pragma unroll
@@ -185,24 +185,7 @@ PP_HD void fq_row_red_wide(uint32_t t[14]) {
   t[13] = 0;
 }
 
-// Row forms: AB / RED = 0 for the single-chain rows above, 1 for bare wide
-// products.  Every form leaves the same 14-word window after each row.  The
-// MSM's bucket sums keep the integer-multiply pipe ~84 % busy and the ALU
-// pipe ~32 %, so moving the product rows' additions to the ALU pays there:
-// the 2^20 MSM took 15.21 ms with (0, 0), 14.02 with (1, 0), 14.73 with
-// (0, 1) and 14.84 with (1, 1) on GB300.
-#ifndef PP_FQ_AB
-#define PP_FQ_AB 1
-#endif
-#ifndef PP_FQ_RED
-#define PP_FQ_RED 0
-#endif
-// the squaring's product rows: 0 single chain, 1 bare wide products (the
-// same 2^20 MSM time, 14.13 against 14.12 ms)
-#ifndef PP_FQ_SQ_WIDE
-#define PP_FQ_SQ_WIDE 0
-#endif
-
+// AB / RED = 0 for the single-chain rows, 1 for bare wide products
 template <int AB, int RED>
 PP_HD fq fq_mul_rows(const fq &a, const fq &b) {
   uint32_t t[14];
@@ -223,6 +206,89 @@ PP_HD fq fq_mul_rows(const fq &a, const fq &b) {
   return r;
 }
 
+// ---- the kernels' multiply: carry-chained cells (mad_cells, fr.cuh).  The
+// running sum is two arrays of 64-bit cells, X at even and Y at odd word
+// positions; a row a_i b is two chains of six wide multiply-adds that pass the
+// carry along, and so is the reduction row m q.  After a reduction row the
+// lowest word is zero; the arrays shift one word by renaming, and the odd word
+// left over (H) joins the next row's lowest cell.  288 wide products, as the
+// row forms, but about 75 additions where those take 400 and more.
+// GB300, two chains per thread: 26.8 against 22.3 G multiplies/s (bare product
+// rows); squaring 36.9 against 26.0 G/s.
+PP_HD void fq_shift_cells(uint32_t x[13], uint32_t y[13]) {
+  uint32_t t[13];
+#pragma unroll
+  for (int k = 0; k < 13; ++k) t[k] = x[k];
+#pragma unroll
+  for (int k = 0; k < 13; ++k) x[k] = y[k];
+#pragma unroll
+  for (int k = 0; k < 11; ++k) y[k] = t[k + 2];
+  y[11] = 0;
+  y[12] = 0;
+}
+
+PP_HD fq fq_mul_cells(const fq &a, const fq &b) {
+  const uint32_t q[12] = {PP_Q0, PP_Q1, PP_Q2, PP_Q3, PP_Q4, PP_Q5,
+                          PP_Q6, PP_Q7, PP_Q8, PP_Q9, PP_Q10, PP_Q11};
+  uint32_t X[13], Y[13], H = 0;
+  mul_cells<6>(X, a.v[0], b.v);
+  mul_cells<6>(Y, a.v[0], b.v + 1);
+  X[12] = Y[12] = 0;
+#pragma unroll
+  for (int i = 0; i < 12; ++i) {
+    if (i) {
+      X[0] = add_cc(X[0], H);  // its carry enters Y, one word up
+      mad_cells<6, true>(Y, a.v[i], b.v + 1);
+      mad_cells<6>(X, a.v[i], b.v);
+    }
+    const uint32_t m = X[0] * PP_QP;
+    mad_cells<6>(X, m, q);
+    mad_cells<6>(Y, m, q + 1);
+    H = X[1];
+    fq_shift_cells(X, Y);
+  }
+  fq r;
+  r.v[0] = add_cc(X[0], H);
+#pragma unroll
+  for (int k = 1; k < 12; ++k) r.v[k] = addc_cc(X[k], Y[k - 1]);
+  fq_reduce_once(r.v);  // below 2q < 2^383
+  return r;
+}
+
+// T (24 words, below q 2^384) -> T 2^-384 mod q: the reduction rows of the
+// lower half, then the upper half added
+PP_HD fq fq_redc24_cells(const uint32_t T[24]) {
+  const uint32_t q[12] = {PP_Q0, PP_Q1, PP_Q2, PP_Q3, PP_Q4, PP_Q5,
+                          PP_Q6, PP_Q7, PP_Q8, PP_Q9, PP_Q10, PP_Q11};
+  uint32_t X[13], Y[13], H = 0;
+#pragma unroll
+  for (int k = 0; k < 12; ++k) X[k] = T[k];
+  X[12] = 0;
+#pragma unroll
+  for (int i = 0; i < 12; ++i) {
+    const uint32_t l = X[0] + H, m = l * PP_QP;
+    if (i) {
+      X[0] = add_cc(X[0], H);
+      mad_cells<6, true>(Y, m, q + 1);
+    } else {
+      mul_cells<6>(Y, m, q + 1);
+      Y[12] = 0;
+    }
+    mad_cells<6>(X, m, q);
+    H = X[1];
+    fq_shift_cells(X, Y);
+  }
+  fq r;
+  r.v[0] = add_cc(X[0], H);
+#pragma unroll
+  for (int k = 1; k < 12; ++k) r.v[k] = addc_cc(X[k], Y[k - 1]);
+  r.v[0] = add_cc(r.v[0], T[12]);
+#pragma unroll
+  for (int k = 1; k < 12; ++k) r.v[k] = addc_cc(r.v[k], T[12 + k]);
+  fq_reduce_once(r.v);  // below q + q
+  return r;
+}
+
 // One out-of-line copy per translation unit: the point formulas call it
 // ~10-14 times per addition, and with every call inlined the bucket-sum
 // kernels outgrew the instruction cache (instruction-fetch stalls led; the
@@ -232,103 +298,47 @@ PP_HD fq fq_mul_rows(const fq &a, const fq &b) {
 #else
 #define PP_FQ_MUL static inline
 #endif
-PP_FQ_MUL fq fq_mul(const fq &a, const fq &b) { return fq_mul_rows<PP_FQ_AB, PP_FQ_RED>(a, b); }
+PP_FQ_MUL fq fq_mul(const fq &a, const fq &b) { return fq_mul_cells(a, b); }
 
-// ---- squaring: a^2 = sum_i a_i C_i 2^(64 i) with C_i = a_i + 2^32 D_i and
-// D_i = 2 floor(a / 2^(32 (i + 1))), so row i multiplies a_i by the 13 - i
-// words of C_i instead of all 12 words of a: 78 wide products instead of 144
-// before the (unchanged) reduction rows.  After i reduction rows the CIOS
-// window has moved i words, so row i's term starts at window word i.
-// A2 = 2a in 13 words; D_i's words are A2[i + 1 ..] with the bit that a_i
-// shifted in cleared.
-// the same row with bare wide products and two add chains
+// rows I .. 10 of the cross products a_I a_j (j > I): word I + j, even ones in
+// E, odd ones in O (word k at O[k - 1])
 template <int I>
-PP_HD void fq_row_sq_wide(uint32_t t[14], uint32_t ai, const uint32_t A2[13]) {
-  constexpr int L = I < 11 ? 13 - I : 1;  // words I .. 12 (I = 11: word 11 only)
-  uint32_t lo[13], hi[13];
-  uint64_t p = (uint64_t)ai * ai;
-  lo[0] = (uint32_t)p;
-  hi[0] = (uint32_t)(p >> 32);
-#pragma unroll
-  for (int k = 1; k + 1 < L; ++k) {
-    const uint32_t dk = k == 1 ? (A2[I + 1] & ~1u) : A2[I + k];
-    p = (uint64_t)ai * dk;
-    lo[k] = (uint32_t)p;
-    hi[k] = (uint32_t)(p >> 32);
-  }
-  if constexpr (L > 1) {  // word 12: a_i times the top bit of 2a, no high word
-    lo[L - 1] = A2[12] ? ai : 0u;
-    hi[L - 1] = 0;
-  }
-  t[I] = add_cc(t[I], lo[0]);
-#pragma unroll
-  for (int k = 1; k < L; ++k) t[I + k] = addc_cc(t[I + k], lo[k]);
-#pragma unroll
-  for (int k = I + L; k < 13; ++k) t[k] = addc_cc(t[k], 0);
-  t[13] = addc(t[13], 0);
-  // high words land on I + 1 .. 12 for every row (the select's is 0)
-  t[I + 1] = add_cc(t[I + 1], hi[0]);
-#pragma unroll
-  for (int k = 1; k + 1 < L; ++k) t[I + 1 + k] = addc_cc(t[I + 1 + k], hi[k]);
-  t[13] = addc(t[13], 0);
-}
-
-template <int I>
-PP_HD void fq_row_sq(uint32_t t[14], uint32_t ai, const uint32_t A2[13]) {
-  uint32_t lo[13], hi[13];
-  uint64_t s = (uint64_t)ai * ai + t[I];
-  lo[0] = (uint32_t)s;
-  hi[0] = (uint32_t)(s >> 32);
-  if constexpr (I == 11) {  // C_11 = a_11
-    t[11] = lo[0];
-    t[12] = add_cc(t[12], hi[0]);
-    t[13] = addc(t[13], 0);
+PP_HD void fq_sqr_cross(uint32_t *E, uint32_t *O, const uint32_t a[12]) {
+  constexpr int N1 = (12 - I) / 2, N2 = (11 - I) / 2;  // j = I + 1, I + 3 ..; j = I + 2, ..
+  if constexpr (I == 0) {
+    mul_cells<N1>(O, a[0], a + 1);
+    mul_cells<N2>(E + 2, a[0], a + 2);
   } else {
-    constexpr int L = 13 - I;  // words I .. 12
-#pragma unroll
-    for (int k = 1; k + 1 < L; ++k) {  // a_i D_i[k - 1] at word I + k
-      const uint32_t dk = k == 1 ? (A2[I + 1] & ~1u) : A2[I + k];
-      s = (uint64_t)ai * dk + t[I + k];
-      lo[k] = (uint32_t)s;
-      hi[k] = (uint32_t)(s >> 32);
-    }
-    s = (uint64_t)(A2[12] ? ai : 0u) + t[12];  // a_i times the top bit of 2a
-    lo[L - 1] = (uint32_t)s;
-    hi[L - 1] = (uint32_t)(s >> 32);
-    t[I] = lo[0];
-    t[I + 1] = add_cc(lo[1], hi[0]);
-#pragma unroll
-    for (int k = 2; k < L; ++k) t[I + k] = addc_cc(lo[k], hi[k - 1]);
-    t[13] = addc(t[13], hi[L - 1]);
+    mad_cells<N1>(O + 2 * I, a[I], a + I + 1);
+    if constexpr (N2 > 0) mad_cells<N2>(E + 2 * I + 2, a[I], a + I + 2);
   }
+  if constexpr (I < 10) fq_sqr_cross<I + 1>(E, O, a);
 }
 
-template <int I>
-PP_HD void fq_sq_rows(uint32_t t[14], const fq &a, const uint32_t A2[13]) {
-  if (PP_FQ_SQ_WIDE) fq_row_sq_wide<I>(t, a.v[I], A2);
-  else fq_row_sq<I>(t, a.v[I], A2);
-  if (PP_FQ_RED) fq_row_red_wide(t);
-  else fq_row_red(t);
-  if constexpr (I < 11) fq_sq_rows<I + 1>(t, a, A2);
-}
-
-// a^2 R^-1 mod q for a < q (same result as fq_mul(a, a)); the window stays
-// below 2^448 (row 0 adds up to 2^417) and ends below 2q
+// a^2 R^-1 mod q for a < q (same result as fq_mul(a, a)): 66 cross products,
+// doubled, and 12 squares instead of 144 products, then the same reduction
 PP_FQ_MUL fq fq_sqr(const fq &a) {
-  uint32_t A2[13];
-  A2[0] = a.v[0] << 1;
+  uint32_t E[26], O[26], T[24];
 #pragma unroll
-  for (int k = 1; k < 12; ++k) A2[k] = (a.v[k] << 1) | (a.v[k - 1] >> 31);
-  A2[12] = a.v[11] >> 31;
-  uint32_t t[14];
+  for (int k = 0; k < 26; ++k) E[k] = O[k] = 0;
+  fq_sqr_cross<0>(E, O, a.v);
+  T[0] = 0;
+  T[1] = O[0];
+  T[2] = add_cc(E[2], O[1]);
 #pragma unroll
-  for (int j = 0; j < 14; ++j) t[j] = 0;
-  fq_sq_rows<0>(t, a, A2);
-  fq_reduce_once(t);
-  fq r;
+  for (int k = 3; k < 23; ++k) T[k] = addc_cc(E[k], O[k - 1]);
+  T[23] = addc(E[23], O[22]);
+  // twice the cross products < a^2 < 2^762: the shift loses no bit
 #pragma unroll
-  for (int i = 0; i < 12; ++i) r.v[i] = t[i];
-  return r;
+  for (int k = 23; k > 0; --k) T[k] = (T[k] << 1) | (T[k - 1] >> 31);
+  T[0] = madlo_cc(a.v[0], a.v[0], T[0]);
+  T[1] = madhic_cc(a.v[0], a.v[0], T[1]);
+#pragma unroll
+  for (int k = 1; k < 12; ++k) {
+    T[2 * k] = madloc_cc(a.v[k], a.v[k], T[2 * k]);
+    T[2 * k + 1] = madhic_cc(a.v[k], a.v[k], T[2 * k + 1]);
+  }
+  return fq_redc24_cells(T);
 }
 
 // ---- binary extended-GCD inverse: shifts and subtractions instead of the
