@@ -12,12 +12,17 @@
 //  * A thread block owns a tile of R_p x T_p elements (R_p * T_p <= 2048,
 //    64 KiB of shared memory, XOR-swizzled 16-byte units); T_p adjacent
 //    columns give >= 128-byte contiguous row segments for coalesced HBM
-//    access.  Inside the tile each column's DFT runs as radix-8 rounds held in
-//    registers (8 elements per thread), with a final radix-4/2 round.
-//  * Every Montgomery multiply is on the integer pipe; the transform is
-//    compute-bound (~11 multiplies per element at 2^24 against 3 HBM passes),
-//    so the inter-pass twiddles are read from HBM tables (one load instead of
-//    a multiply), and inverse transforms fold 2^-L into the first layer table.
+//    access.  Each column's DFT runs as radix-8 rounds held in registers (8
+//    elements per thread), with a final radix-4/2 round; the first round reads
+//    its elements straight from global memory and the last one writes them
+//    there, so shared memory only carries the exchanges in between.
+//  * Every multiply is on the integer pipe; the transform is compute-bound
+//    (~11 multiplies per element at 2^24 against 3 HBM passes), so the
+//    inter-pass twiddles are read from HBM tables (one load instead of a
+//    multiply), and inverse transforms fold 2^-L into the first layer table.
+//    The twiddles inside a pass are few, so they are kept in the four-part
+//    form of fr_mul_const4 (82 wide products instead of 112): per-round tables
+//    read through L1, and the 8-point DFT's three roots in constant memory.
 //
 // Reference behaviour restated: natural order in and out, w_N =
 // forward_roots_of_unity[lg N] = 7^((r-1)/N) (PLONK/utils/zkp/cuda/
@@ -89,6 +94,17 @@ struct SmemTile {
     s[swz(u)] = make_uint4(v.v[0], v.v[1], v.v[2], v.v[3]);
     s[swz(u + 1)] = make_uint4(v.v[4], v.v[5], v.v[6], v.v[7]);
   }
+  // asynchronous copy of *p into the slot (cp.async, 16 bytes each)
+  __device__ __forceinline__ void fetch(uint32_t row, uint32_t col, const fr *p) const {
+    const uint32_t u = ((row << lgT) + col) << 1;
+#pragma unroll
+    for (uint32_t h = 0; h < 2; ++h) {
+      const uint32_t d = (uint32_t)__cvta_generic_to_shared(s + swz(u + h));
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d),
+                   "l"(reinterpret_cast<const uint4 *>(p) + h)
+                   : "memory");
+    }
+  }
 };
 
 // Inside a transform values are kept below 2r (fr_*_lazy); the last round of
@@ -99,25 +115,90 @@ __device__ __forceinline__ void bfly(fr &a, fr &b) {
   b = fr_sub_lazy(t, b);
 }
 
-// 8-point DFT, decimation in frequency; afterwards x[i] = X[bitrev3(i)]
-__device__ __forceinline__ void dft8(fr x[8], const fr &w1, const fr &w2, const fr &w3) {
+// g, g^2, g^3 for g = 7^((r - 1) / 8), the forward 8-point DFT's root, each as
+// the four products of fr_mul_const4
+__constant__ fr c_root8[3][4] = {
+    {
+        {{0xcef49ea0u, 0xdcd5caa8u, 0xbd6d1816u, 0x69201e87u,
+          0xcf28faf2u, 0x783ec6b6u, 0x87a05b34u, 0x1e0586d8u}},
+        {{0xde0a24a3u, 0xdfaa358fu, 0x8f1ab3c9u, 0x3a13d616u,
+          0x407da03fu, 0xd862d68du, 0x17ac7fefu, 0x0b97f08eu}},
+        {{0x9b12398eu, 0x4b53ca4eu, 0x7624ef38u, 0xa0d9e7f3u,
+          0x9524919bu, 0x47e4ef53u, 0xe24cf722u, 0x5fe27ea0u}},
+        {{0x44eb37e9u, 0xe757b80eu, 0x4229cdacu, 0x9df71901u,
+          0x5bdd56fdu, 0xcbb407acu, 0xf1dfe463u, 0x3ba5b74du}},
+    },
+    {
+        {{0xc7edfb36u, 0x381204c8u, 0xc7ed6ccbu, 0xc59889a0u,
+          0x307d7343u, 0x26b07cdau, 0xd246eae2u, 0x274ed2c8u}},
+        {{0xcc3033f3u, 0xdd027557u, 0x3d5071f7u, 0xda5fec58u,
+          0x53ff4e10u, 0xd6b1d7c9u, 0x8bee15e0u, 0x1c496903u}},
+        {{0x9e3a2626u, 0x234eedafu, 0x05d6a1f7u, 0xce1bb45du,
+          0xb4dc675bu, 0x44ba87bbu, 0x600997adu, 0x26b36dfau}},
+        {{0x5593a1d4u, 0x54f62ddcu, 0x689ce4a1u, 0x29f28715u,
+          0x4630a8abu, 0xa058db80u, 0x070dfcaau, 0x2c58143fu}},
+    },
+    {
+        {{0x2fb113e9u, 0x11d87474u, 0xdfb3fc26u, 0x319788e0u,
+          0x92036cf2u, 0xf41937d2u, 0x80f69024u, 0x4d0272cbu}},
+        {{0xfa7a5327u, 0x5b7707ecu, 0x2ed969adu, 0x17f947e5u,
+          0xfceb0de1u, 0x9a8fc772u, 0x8d46ac2cu, 0x67ccda1au}},
+        {{0x4fd24120u, 0xcaf5f51cu, 0x9d075bc9u, 0xdd83221cu,
+          0x6588868cu, 0x410bf77cu, 0xfd335d4du, 0x57893116u}},
+        {{0x3a74abb7u, 0x043dfd25u, 0x6cf2b08cu, 0xf7b43b7eu,
+          0xe1196756u, 0x7c149dabu, 0x91e39a97u, 0x0ac07ea6u}},
+    },
+};
+
+// 8-point forward DFT, natural order in and out (decimation in frequency; the
+// output permutation is a renaming).  The inverse DFT is the same values with
+// output k at (8 - k) mod 8, so one set of roots serves both directions.
+// inputs_used() is called once every input has been read.
+template <typename F>
+__device__ __forceinline__ void dft8(fr x[8], F inputs_used) {
   bfly(x[0], x[4]);
   bfly(x[1], x[5]);
   bfly(x[2], x[6]);
   bfly(x[3], x[7]);
-  x[5] = fr_mul_twiddle(x[5], w1);
-  x[6] = fr_mul_twiddle(x[6], w2);
-  x[7] = fr_mul_twiddle(x[7], w3);
+  inputs_used();
+  x[5] = fr_mul_const4(x[5], c_root8[0]);
+  x[6] = fr_mul_const4(x[6], c_root8[1]);
+  x[7] = fr_mul_const4(x[7], c_root8[2]);
   bfly(x[0], x[2]);
   bfly(x[1], x[3]);
   bfly(x[4], x[6]);
   bfly(x[5], x[7]);
-  x[3] = fr_mul_twiddle(x[3], w2);
-  x[7] = fr_mul_twiddle(x[7], w2);
+  x[3] = fr_mul_const4(x[3], c_root8[1]);
+  x[7] = fr_mul_const4(x[7], c_root8[1]);
   bfly(x[0], x[1]);
   bfly(x[2], x[3]);
   bfly(x[4], x[5]);
   bfly(x[6], x[7]);
+  fr t = x[1];
+  x[1] = x[4];
+  x[4] = t;
+  t = x[3];
+  x[3] = x[6];
+  x[6] = t;
+}
+
+// Round twiddles.  A round of 8-point DFTs with 2^lgSj columns (lgSj = 1 .. 8)
+// multiplies output k of column c by w_R^(c k), R = 2^(lgSj + 3).  The tables
+// of all lgSj follow one another; each is laid out [k - 1][plane][c] in
+// 16-byte planes (two per part of fr_mul_const4's four), so the lanes of a
+// warp, on neighbouring columns, read contiguous bytes.
+constexpr uint32_t kRoundUnits = 56 * (512 - 2);  // 16-byte units, lgSj = 1 .. 8
+__host__ __device__ __forceinline__ uint32_t round_offset(uint32_t lgSj) {
+  return 56 * ((1u << lgSj) - 2);
+}
+__device__ __forceinline__ fr mul_round_twiddle(const fr &x, const uint4 *t, uint32_t lgSj) {
+  fr w[4];
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    const uint4 a = __ldg(t + ((2 * p) << lgSj)), b = __ldg(t + ((2 * p + 1) << lgSj));
+    w[p] = fr{{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}};
+  }
+  return fr_mul_const4(x, w);
 }
 
 __device__ __forceinline__ uint32_t digit_reverse(uint32_t o, uint32_t lgR) {
@@ -132,13 +213,78 @@ __device__ __forceinline__ uint32_t digit_reverse(uint32_t o, uint32_t lgR) {
   return p;
 }
 
+// the output index held at position p of a finished column (the inverse of
+// digit_reverse; additive over disjoint bits of p)
+__device__ __forceinline__ uint32_t digit_index(uint32_t p, uint32_t lgR) {
+  uint32_t rem = lgR, o = 0, sh = 0;
+  while (rem > 0) {
+    const uint32_t lgr = rem >= 3 ? 3 : rem;
+    rem -= lgr;
+    o += ((p >> rem) & ((1u << lgr) - 1)) << sh;
+    sh += lgr;
+  }
+  return o;
+}
+
 // w_{R S}^(o c) from the split tables (both canonical, so the product is)
 __device__ __forceinline__ fr split_layer_twiddle(const PassArgs &a, uint32_t o, uint64_t c) {
   const uint64_t e = (uint64_t)o * c;
   return fr_mul(ldg_fr(a.tw_hi + (e >> a.tw_lgh)), ldg_fr(a.tw_lo + (e & ((1ull << a.tw_lgh) - 1))));
 }
 
-// One tile of one pass.  The block may be wider than the tile needs (batched
+// The layer multiply as a call: inlined eight times per thread it is 24 KB of
+// code that every tile walks through (2^22: 714 us inlined, 702 called; 2^24:
+// 2760 and 2738).  The round twiddles, in the loop, are faster inlined.
+__device__ __noinline__ fr mul_layer(fr a, fr b) { return fr_mul_lazy(a, b); }
+
+// where a tile's elements lie
+struct TileGeom {
+  uint64_t base = 0, col0 = 0;         // intermediate pass: first element, first column
+  uint64_t in_base = 0, out_base = 0;  // last pass: first input and output element
+  uint32_t lgS1 = 0;
+  __device__ __forceinline__ uint64_t src(const PassArgs &a, uint32_t n, uint32_t col) const {
+    if (!a.last) return base + ((uint64_t)n << a.lgS) + col;
+    return in_base + ((uint64_t)col << lgS1) + n;  // one pass: in_base = col = 0
+  }
+};
+
+__device__ __forceinline__ TileGeom tile_geom(const PassArgs &a, const uint64_t tileid) {
+  TileGeom t;
+  if (!a.last) {
+    const uint32_t lgtpq = a.lgS - a.lgT;
+    const uint64_t q = tileid >> lgtpq, ct = tileid & ((1ull << lgtpq) - 1);
+    t.col0 = ct << a.lgT;
+    t.base = (q << (a.lgR + a.lgS)) + t.col0;
+  } else if (a.P > 1) {
+    const uint32_t lgR1 = a.lgRp[0];
+    t.lgS1 = a.lgN - lgR1;
+    const uint32_t lgkb = lgR1 - a.lgT;
+    const uint64_t kb = tileid & ((1ull << lgkb) - 1), rest = tileid >> lgkb;
+    uint64_t rin = 0, r = rest;
+    uint32_t acc = lgR1;
+    for (uint32_t j = 1; j + 1 < a.P; ++j) {
+      const uint32_t bits = a.lgRp[j];
+      acc += bits;
+      rin += (r & ((1ull << bits) - 1)) << (a.lgN - acc);
+      r >>= bits;
+    }
+    t.in_base = ((kb << a.lgT) << t.lgS1) + rin;
+    t.out_base = (kb << a.lgT) + (rest << lgR1);
+  }
+  return t;
+}
+
+// One tile of one pass: load (+ input multiply), column DFTs, layer twiddle or
+// scale, store.  Bound by the integer-multiply pipe (68 % busy: 16 warps per SM
+// at 128 registers) and by the loads' latency around it.  GB300, 2^24 points:
+// 3.32 ms with general multiplies and every round through shared memory, 2.87
+// with the four-part twiddles and the first and last round on global memory,
+// 2.74 with the layer twiddles fetched during the last round and multiplied by
+// a called function (pieces left out, for scale: layer multiplies 370 us, their
+// loads 220 before the asynchronous fetch, input loads 250, round-twiddle loads
+// 224).  Asking L2 for the next wave's tiles made it 1.4 % slower, 1024-element
+// tiles with four blocks per SM 7 %.
+// The block may be wider than the tile needs (batched
 // launches use 256 threads for every job); surplus threads only join the
 // barriers.
 template <bool HOSTIO>
@@ -152,51 +298,19 @@ __device__ __forceinline__ void ntt_tile(const PassArgs &a, const uint64_t tilei
   const uint32_t tid = threadIdx.x;
   const bool active = tid < nthr;
 
-  uint64_t base = 0, col0 = 0, in_base = 0, out_base = 0;
-  uint32_t lgS1 = 0;
-  if (!a.last) {
-    const uint32_t lgtpq = a.lgS - a.lgT;
-    const uint64_t q = tileid >> lgtpq, ct = tileid & ((1ull << lgtpq) - 1);
-    col0 = ct << a.lgT;
-    base = (q << (a.lgR + a.lgS)) + col0;
-  } else if (a.P > 1) {
-    const uint32_t lgR1 = a.lgRp[0];
-    lgS1 = a.lgN - lgR1;
-    const uint32_t lgkb = lgR1 - a.lgT;
-    const uint64_t kb = tileid & ((1ull << lgkb) - 1), rest = tileid >> lgkb;
-    uint64_t rin = 0, r = rest;
-    uint32_t acc = lgR1;
-    for (uint32_t j = 1; j + 1 < a.P; ++j) {
-      const uint32_t bits = a.lgRp[j];
-      acc += bits;
-      rin += (r & ((1ull << bits) - 1)) << (a.lgN - acc);
-      r >>= bits;
-    }
-    in_base = ((kb << a.lgT) << lgS1) + rin;
-    out_base = (kb << a.lgT) + (rest << lgR1);
-  }
+  const TileGeom geo = tile_geom(a, tileid);
+  const uint64_t base = geo.base, col0 = geo.col0, out_base = geo.out_base;
 
-  // ---- load the tile (coalesced) into shared memory.  A host-memory input
-  // without a multiply on the way in moves 16-byte halves, so one warp
-  // instruction reads whole 128-byte lines; a thread's 16 loads issue in two
-  // groups of eight before their shared-memory stores, so it waits on host
-  // memory twice per tile instead of sixteen times.
-  auto tile_src = [&](uint32_t e, uint32_t &n, uint32_t &col) -> uint64_t {
-    if (!a.last) {
-      n = e >> a.lgT;
-      col = e & (T - 1);
-      return base + ((uint64_t)n << a.lgS) + col;
-    }
-    if (a.P == 1) {
-      n = e;
-      col = 0;
-      return n;
-    }
-    n = e & (R - 1);
-    col = e >> a.lgR;
-    return in_base + ((uint64_t)col << lgS1) + n;
-  };
-  if (unit_in && !(a.first && a.in_kind == NTT_IN_DIAG)) {
+  // ---- a host-memory input without a multiply on the way in goes through
+  // shared memory in 16-byte halves, so one warp instruction reads whole
+  // 128-byte lines; a thread's 16 loads issue in two groups of eight before
+  // their shared-memory stores, so it waits on host memory twice per tile
+  // instead of sixteen times.
+  const bool stage_in = unit_in && !(a.first && a.in_kind == NTT_IN_DIAG);
+  // a host-memory output without a scale leaves the tile the same way
+  const bool stage_out = unit_out && !(a.last && a.has_post_scale);
+  auto tile_src = [&](uint32_t n, uint32_t col) -> uint64_t { return geo.src(a, n, col); };
+  if (stage_in) {
     const uint4 zero4 = make_uint4(0, 0, 0, 0);
     if (active) {
 #pragma unroll
@@ -207,8 +321,8 @@ __device__ __forceinline__ void ntt_tile(const PassArgs &a, const uint64_t tilei
         for (uint32_t i = 0; i < 8; ++i) {
           const uint32_t u = tid + (k0 + i) * nthr;
           const uint32_t e = u >> 1, h = u & 1;
-          uint32_t n, col;
-          const uint64_t g = tile_src(e, n, col);
+          const uint32_t n = a.last ? e & (R - 1) : e >> a.lgT, col = a.last ? e >> a.lgR : e & (T - 1);
+          const uint64_t g = tile_src(n, col);
           dst[i] = swz((((n << a.lgT) + col) << 1) + h);
           v[i] = zero4;
           if (!a.first) {
@@ -224,116 +338,110 @@ __device__ __forceinline__ void ntt_tile(const PassArgs &a, const uint64_t tilei
         for (uint32_t i = 0; i < 8; ++i) tile.s[dst[i]] = v[i];
       }
     }
-  } else {
-    for (uint32_t e = tid; active && e < E; e += nthr) {
-      uint32_t n, col;
-      uint64_t g;
-      if (!a.last) {
-        n = e >> a.lgT;
-        col = e & (T - 1);
-        g = base + ((uint64_t)n << a.lgS) + col;
-      } else if (a.P == 1) {
-        n = e;
-        col = 0;
-        g = n;
-      } else {
-        n = e & (R - 1);
-        col = e >> a.lgR;
-        g = in_base + ((uint64_t)col << lgS1) + n;
-      }
-      fr v;
-      if (a.first) {
-        if (a.in_kind == NTT_IN_SPREAD) {
-          v = (g & ((1ull << a.spread) - 1)) == 0 ? ldcs_fr(a.in + (g >> a.spread)) : fr_zero();
-        } else if (g < a.n_valid) {
-          v = ldcs_fr(a.in + g);
-          if (a.in_kind == NTT_IN_DIAG) {
-            const fr d = a.diag_hi ? fr_mul(ldg_fr(a.diag + (g & ((1ull << a.diag_lgh) - 1))),
-                                            ldg_fr(a.diag_hi + (g >> a.diag_lgh)))
-                                   : ldcs_fr(a.diag + g);
-            v = fr_mul_twiddle(v, d);
-          }
-        } else {
-          v = fr_zero();
-        }
-      } else {
-        v = ldcs_fr(a.in + g);
-      }
-      tile.put(n, col, v);
-    }
+    __syncthreads();
   }
-  __syncthreads();
+  auto load = [&](uint32_t n, uint32_t col) -> fr {
+    const uint64_t g = tile_src(n, col);
+    if (!a.first) return ldcs_fr(a.in + g);
+    if (a.in_kind == NTT_IN_SPREAD)
+      return (g & ((1ull << a.spread) - 1)) == 0 ? ldcs_fr(a.in + (g >> a.spread)) : fr_zero();
+    if (g >= a.n_valid) return fr_zero();
+    const fr v = ldcs_fr(a.in + g);
+    if (a.in_kind != NTT_IN_DIAG) return v;
+    const fr d = a.diag_hi ? fr_mul(ldg_fr(a.diag + (g & ((1ull << a.diag_lgh) - 1))),
+                                    ldg_fr(a.diag_hi + (g >> a.diag_lgh)))
+                           : ldcs_fr(a.diag + g);
+    return fr_mul_lazy(v, d);
+  };
 
-  // ---- column DFTs: radix-8 rounds, final radix-4/2 round
+  // ---- column DFTs: radix-8 rounds, final radix-4/2 round.  A thread holds
+  // the 8 positions pb + (j << lgs) of one column.  Neighbouring lanes take
+  // neighbouring columns (contiguous in global memory, and few distinct
+  // twiddles per warp), except where the last pass reads: there a column is
+  // contiguous.
   {
     const uint32_t lgcpt = a.lgR - 3;
-    const uint32_t col = tid >> lgcpt, d = tid & ((1u << lgcpt) - 1);
     uint32_t lgP = 0, rem = a.lgR;
-    while (rem > 0) {
+#pragma unroll 1
+    for (;;) {
       const uint32_t lgr = rem >= 3 ? 3 : rem;
       const uint32_t lgSj = rem - lgr;
-      if (!active) {
-        // surplus thread of a wider block: barriers only
-      } else if (lgr == 3) {
-        const uint32_t c = d & ((1u << lgSj) - 1), prefix = d >> lgSj;
-        const uint32_t pb = (prefix << (lgSj + 3)) + c;
+      if (active) {  // surplus threads of a wider block: barriers only
+        const bool by_row = a.last && lgP == 0;
+        const uint32_t col = by_row ? tid >> lgcpt : tid & (T - 1);
+        const uint32_t d = by_row ? tid & ((1u << lgcpt) - 1) : tid >> a.lgT;
+        const uint32_t lgs = lgr == 3 ? lgSj : 0;
+        const uint32_t c = d & ((1u << lgs) - 1);
+        const uint32_t pb = ((d >> lgs) << (lgs + 3)) + c;
+        // over zero padding only the first 8 >> zero_lg inputs can be non-zero
+        const uint32_t zlg = lgP == 0 ? a.zero_lg : 0;
         fr x[8];
-        const fr w1 = ldg_fr(a.tw_inner + (R >> 3));
-        const fr w2 = ldg_fr(a.tw_inner + (R >> 2));
-        const fr w3 = ldg_fr(a.tw_inner + 3 * (R >> 3));
-        if (lgP == 0 && a.zero_lg >= 3) {
-          // first round over zero padding: only x[0] can be non-zero, and the
-          // 8-point DFT of (x0, 0, ..., 0) is x0 in every output
-          x[0] = tile.get(pb, col);
-#pragma unroll
-          for (int i = 1; i < 8; ++i) x[i] = x[0];
-        } else if (lgP == 0 && a.zero_lg == 2) {
-          // only x[0], x[1] can be non-zero: X[k] = x0 + x1 w^k, w^4 = -1,
-          // stored bit-reversed like dft8 (x[i] = X[bitrev3(i)])
-          const fr x0 = tile.get(pb, col), x1 = tile.get(pb + (1u << lgSj), col);
-          const fr t1 = fr_mul_twiddle(x1, w1), t2 = fr_mul_twiddle(x1, w2), t3 = fr_mul_twiddle(x1, w3);
-          x[0] = fr_add_lazy(x0, x1);
-          x[1] = fr_sub_lazy(x0, x1);
-          x[2] = fr_add_lazy(x0, t2);
-          x[3] = fr_sub_lazy(x0, t2);
-          x[4] = fr_add_lazy(x0, t1);
-          x[5] = fr_sub_lazy(x0, t1);
-          x[6] = fr_add_lazy(x0, t3);
-          x[7] = fr_sub_lazy(x0, t3);
-        } else {
-#pragma unroll
-          for (int i = 0; i < 8; ++i) x[i] = tile.get(pb + ((uint32_t)i << lgSj), col);
-          dft8(x, w1, w2, w3);
-        }
-        // x[i] holds output k = bitrev3(i)
-        if (lgSj > 0) {
-#pragma unroll
-          for (int i = 1; i < 8; ++i) {
-            const uint32_t k = ((i & 1) << 2) | (i & 2) | ((i >> 2) & 1);
-            x[i] = fr_mul_twiddle(x[i], ldg_fr(a.tw_inner + ((c * k) << lgP)));
-          }
-        } else if (a.last && unit_out) {
-          // the 16-byte store path copies tile words: canonical here
-#pragma unroll
-          for (int i = 0; i < 8; ++i) x[i] = fr_canon(x[i]);
-        }
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          const uint32_t k = ((i & 1) << 2) | (i & 2) | ((i >> 2) & 1);
-          tile.put(pb + (k << lgSj), col, x[i]);
+          if (i > 0 && zlg >= 3) break;
+          if (i > 1 && zlg == 2) break;
+          const uint32_t n = pb + ((uint32_t)i << lgs);
+          x[i] = lgP == 0 && !stage_in ? load(n, col) : tile.get(n, col);
         }
-      } else {
-        // last round (S = 1): this thread owns positions 8d .. 8d+7
-        fr x[8];
+        // output j of the round goes to position pb + (at(j) << lgs): the
+        // inverse transform takes the forward DFT's outputs in reverse
+        const auto at = [&](uint32_t j) -> uint32_t {
+          if (!a.inverse || lgr == 1) return j;
+          return lgr == 3 ? (8 - j) & 7 : (j & 4) | ((4 - (j & 3)) & 3);
+        };
+        // the last round of an intermediate pass fetches its layer twiddles
+        // into the tile slots it has just read (nobody else uses them), so
+        // they arrive while the round computes
+        const bool fetch = lgSj == 0 && !stage_out && a.tw_layer;
+        const uint32_t o0 = digit_index(pb, a.lgR);
+        const auto fetch_layer = [&] {
+          if (!fetch) return;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) x[i] = tile.get((d << 3) + i, col);
-        if (lgr == 2) {
-          const fr w4 = ldg_fr(a.tw_inner + (R >> 2));
+          for (uint32_t j = 0; j < 8; ++j) {
+            const uint64_t o = o0 + digit_index(j << lgs, a.lgR);
+            tile.fetch(pb + (j << lgs), col, a.tw_layer + (o << a.lgS) + col0 + col);
+          }
+          asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        if (lgr == 3) {
+          if (zlg >= 3) {
+            fetch_layer();
+            // the 8-point DFT of (x0, 0, ..., 0) is x0 in every output
+#pragma unroll
+            for (int i = 1; i < 8; ++i) x[i] = x[0];
+          } else if (zlg == 2) {
+            // X[k] = x0 + x1 g^k, g^4 = -1
+            const fr x0 = x[0], x1 = x[1];
+            fetch_layer();
+            const fr t1 = fr_mul_const4(x1, c_root8[0]), t2 = fr_mul_const4(x1, c_root8[1]);
+            const fr t3 = fr_mul_const4(x1, c_root8[2]);
+            x[0] = fr_add_lazy(x0, x1);
+            x[4] = fr_sub_lazy(x0, x1);
+            x[1] = fr_add_lazy(x0, t1);
+            x[5] = fr_sub_lazy(x0, t1);
+            x[2] = fr_add_lazy(x0, t2);
+            x[6] = fr_sub_lazy(x0, t2);
+            x[3] = fr_add_lazy(x0, t3);
+            x[7] = fr_sub_lazy(x0, t3);
+          } else {
+            dft8(x, fetch_layer);
+          }
+          if (lgSj > 0) {
+            const uint4 *tw = a.tw_round + round_offset(lgSj) + c;
+#pragma unroll
+            for (uint32_t j = 1; j < 8; ++j)
+              x[j] = mul_round_twiddle(x[j], tw + (((at(j) - 1) * 8) << lgSj), lgSj);
+          }
+        } else if (lgr == 2) {
 #pragma unroll
           for (int h = 0; h < 8; h += 4) {
             bfly(x[h + 0], x[h + 2]);
             bfly(x[h + 1], x[h + 3]);
-            x[h + 3] = fr_mul_twiddle(x[h + 3], w4);
+          }
+          fetch_layer();
+#pragma unroll
+          for (int h = 0; h < 8; h += 4) {
+            x[h + 3] = fr_mul_const4(x[h + 3], c_root8[1]);
             bfly(x[h + 0], x[h + 1]);
             bfly(x[h + 2], x[h + 3]);
             const fr t = x[h + 1];  // bit-reversed -> natural
@@ -343,82 +451,68 @@ __device__ __forceinline__ void ntt_tile(const PassArgs &a, const uint64_t tilei
         } else {
 #pragma unroll
           for (int h = 0; h < 8; h += 2) bfly(x[h], x[h + 1]);
+          fetch_layer();
         }
-        if (a.last && unit_out) {
+        if (lgSj > 0 || stage_out) {
+          // the 16-byte output path copies tile words: canonical here
+          if (lgSj == 0 && a.last) {
 #pragma unroll
-          for (int i = 0; i < 8; ++i) x[i] = fr_canon(x[i]);
+            for (int i = 0; i < 8; ++i) x[i] = fr_canon(x[i]);
+          }
+#pragma unroll
+          for (uint32_t j = 0; j < 8; ++j) tile.put(pb + (at(j) << lgs), col, x[j]);
+        } else {
+          // ---- the last round stores (coalesced), with the layer twiddle or
+          // the final scale
+          if (fetch) asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+          for (uint32_t j = 0; j < 8; ++j) {
+            const uint32_t pos = at(j) << lgs;
+            const uint64_t o = o0 + digit_index(pos, a.lgR);
+            if (!a.last) {
+              fr v = x[j];
+              if (fetch) v = mul_layer(v, tile.get(pb + pos, col));
+              st_fr(a.out + base + (o << a.lgS) + col, v);
+            } else {
+              fr v = fr_canon(x[j]);
+              if (a.has_post_scale) v = fr_mul(v, a.post_scale);
+              st_fr(a.out + out_base + col + (o << (a.lgN - a.lgR)), v);
+            }
+          }
         }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) tile.put((d << 3) + i, col, x[i]);
       }
-      __syncthreads();
+      if (lgSj == 0) break;
+      // the next round exchanges among 2^lgSj threads of a column, and with
+      // neighbouring lanes on neighbouring columns those T 2^lgSj threads are
+      // one warp in the later rounds
+      if ((T << lgSj) <= 32 && !(a.last && lgP == 0)) __syncwarp();
+      else __syncthreads();
       lgP += lgr;
       rem -= lgr;
     }
   }
+  if (!stage_out) return;
+  __syncthreads();
 
-  // ---- store (coalesced), with the layer twiddle or the final scale.  A
-  // host-memory output without a scale moves 16-byte halves, so one warp
-  // instruction writes whole 128-byte lines (partial lines cost C2C bandwidth).
-  if (a.last && unit_out && !a.has_post_scale) {
-    for (uint32_t u = tid; active && u < 2 * E; u += nthr) {
-      const uint32_t e = u >> 1, h = u & 1;
-      uint32_t o, col;
-      if (a.P == 1) {
-        o = e;
-        col = 0;
-      } else {
-        o = e >> a.lgT;
-        col = e & (T - 1);
-      }
-      const uint4 v = tile.s[swz((((digit_reverse(o, a.lgR) << a.lgT) + col) << 1) + h)];
-      const uint64_t g =
-          a.P == 1 ? (uint64_t)o : out_base + col + ((uint64_t)o << (a.lgN - a.lgR));
-      reinterpret_cast<uint4 *>(a.out + g)[h] = v;
+  // ---- host output through the tile: whole 128-byte lines leave it (partial
+  // lines cost C2C bandwidth)
+  if (!a.last && (a.tw_layer || a.tw_lo)) {
+    // an intermediate pass: the layer twiddles go into the tile first
+    for (uint32_t e = tid; active && e < E; e += nthr) {
+      const uint32_t o = e >> a.lgT, col = e & (T - 1), r = digit_reverse(o, a.lgR);
+      const fr w = a.tw_layer ? ldcs_fr(a.tw_layer + ((uint64_t)o << a.lgS) + col0 + col)
+                              : split_layer_twiddle(a, o, col0 + col);
+      tile.put(r, col, fr_mul_lazy(tile.get(r, col), w));
     }
-    return;
+    __syncthreads();
   }
-  if (!a.last && unit_out) {
-    // host output of an intermediate pass: the layer twiddles go into the
-    // tile first, then whole 128-byte lines leave it
-    if (a.tw_layer || a.tw_lo) {
-      for (uint32_t e = tid; active && e < E; e += nthr) {
-        const uint32_t o = e >> a.lgT, col = e & (T - 1), r = digit_reverse(o, a.lgR);
-        const fr w = a.tw_layer ? ldcs_fr(a.tw_layer + ((uint64_t)o << a.lgS) + col0 + col)
-                                : split_layer_twiddle(a, o, col0 + col);
-        tile.put(r, col, fr_mul_twiddle(tile.get(r, col), w));
-      }
-      __syncthreads();
-    }
-    for (uint32_t u = tid; active && u < 2 * E; u += nthr) {
-      const uint32_t e = u >> 1, h = u & 1;
-      const uint32_t o = e >> a.lgT, col = e & (T - 1);
-      const uint4 v = tile.s[swz((((digit_reverse(o, a.lgR) << a.lgT) + col) << 1) + h)];
-      reinterpret_cast<uint4 *>(a.out + base + ((uint64_t)o << a.lgS) + col)[h] = v;
-    }
-    return;
-  }
-  for (uint32_t e = tid; active && e < E; e += nthr) {
-    uint32_t o, col;
-    if (a.P == 1) {
-      o = e;
-      col = 0;
-    } else {
-      o = e >> a.lgT;
-      col = e & (T - 1);
-    }
-    fr v = tile.get(digit_reverse(o, a.lgR), col);
-    if (!a.last) {
-      if (a.tw_layer) v = fr_mul_twiddle(v, ldcs_fr(a.tw_layer + ((uint64_t)o << a.lgS) + col0 + col));
-      else if (a.tw_lo) v = fr_mul_twiddle(v, split_layer_twiddle(a, o, col0 + col));
-      st_fr(a.out + base + ((uint64_t)o << a.lgS) + col, v);
-    } else {
-      v = fr_canon(v);  // one element at a time here, not 8 live in the last round
-      if (a.has_post_scale) v = fr_mul(v, a.post_scale);
-      const uint64_t g =
-          a.P == 1 ? (uint64_t)o : out_base + col + ((uint64_t)o << (a.lgN - a.lgR));
-      st_fr(a.out + g, v);
-    }
+  for (uint32_t u = tid; active && u < 2 * E; u += nthr) {
+    const uint32_t e = u >> 1, h = u & 1;
+    const uint32_t o = e >> a.lgT, col = e & (T - 1);
+    const uint4 v = tile.s[swz((((digit_reverse(o, a.lgR) << a.lgT) + col) << 1) + h)];
+    const uint64_t g = a.last ? out_base + col + ((uint64_t)o << (a.lgN - a.lgR))
+                              : base + ((uint64_t)o << a.lgS) + col;
+    reinterpret_cast<uint4 *>(a.out + g)[h] = v;
   }
 }
 
@@ -446,138 +540,122 @@ __global__ void __launch_bounds__(256, PP_NTT_MINB) k_ntt_batch_level(const __gr
   ntt_tile<false>(p.args[lo], t - p.tile_start[lo], sm);  // device endpoints
 }
 
-// Transforms of 2^3 .. 2^11 points (single-pass plans) in one block: the
-// input goes to shared memory in bit-reversed order, then radix-2
-// decimation-in-time layers with w_N^(j N / 2m) from the plan's inner table
-// leave the natural-order result.  Transforms this small are bound by
-// latency, not by the multiply pipe.  The tiled pass kernel runs its unrolled
-// radix-8 rounds once over a large code body and waits on instruction fetch
-// (ncu at 2^11: no_instruction stalls 4.3 warps per issue; 46 us per call);
-// this kernel's rolled loops keep its code small.  The input is read in full
-// before anything is written, so in == out is allowed.
-__global__ void __launch_bounds__(512) k_ntt_small(const PassArgs a) {
-  extern __shared__ uint4 sm[];
-  fr *x = reinterpret_cast<fr *>(sm);
-  const uint32_t lg = a.lgN, N = 1u << lg, half = N >> 1;
-#pragma unroll 1
-  for (uint32_t i = threadIdx.x; i < N; i += blockDim.x) {
-    fr v;
-    if (a.in_kind == NTT_IN_SPREAD) {
-      v = (i & ((1u << a.spread) - 1)) == 0 ? ldcs_fr(a.in + (i >> a.spread)) : fr_zero();
-    } else if (i < a.n_valid) {
-      v = ldcs_fr(a.in + i);
-      if (a.in_kind == NTT_IN_DIAG) v = fr_mul(v, ldcs_fr(a.diag + i));
-    } else {
-      v = fr_zero();
-    }
-    st_fr(x + (__brev(i) >> (32 - lg)), v);
-  }
-  __syncthreads();
-#pragma unroll 1
-  for (uint32_t s = 0; s < lg; ++s) {
-#pragma unroll 1
-    for (uint32_t b = threadIdx.x; b < half; b += blockDim.x) {
-      const uint32_t j = b & ((1u << s) - 1);
-      const uint32_t p = ((b >> s) << (s + 1)) + j, q = p + (1u << s);
-      const fr t = fr_mul(ld_fr(x + q), ldg_fr(a.tw_inner + (j << (lg - 1 - s))));
-      const fr u = ld_fr(x + p);
-      st_fr(x + p, fr_add(u, t));
-      st_fr(x + q, fr_sub(u, t));
-    }
-    __syncthreads();
-  }
-#pragma unroll 1
-  for (uint32_t i = threadIdx.x; i < N; i += blockDim.x) {
-    fr v = ld_fr(x + i);
-    if (a.has_post_scale) v = fr_mul(v, a.post_scale);
-    st_fr(a.out + i, v);
-  }
+// Latency form (single calls of 2^3 .. 2^17 points): one column of R points per
+// block, R / 2 threads (at least a warp), one pass up to 2^8 points and two
+// above.  Transforms this small are bound by the length of the dependent chain,
+// not by the multiply pipe, and the tile kernel's unrolled rounds (60 KB of
+// code) by instruction fetch.  So each thread holds one butterfly of a radix-2
+// decimation-in-time layer:
+//  * the first layer reads its two rows straight from global memory (bit
+//    reversal is the address) and has no multiply; the last one stores its two
+//    outputs, in natural order, from registers;
+//  * a layer's twiddle, in the four-part form (557 cycles a multiply for a lone
+//    warp, the general one takes 765), is loaded before the barrier that the
+//    layer waits on;
+//  * the first six layers' exchanges stay inside a warp (__syncwarp);
+//  * the second pass's blocks are placed while the first pass drains.
+// GB300, us per call, against the form before it (general multiply, canonical
+// additions, a barrier and a dependent twiddle load per layer): 2^9 11.0 (14.4),
+// 2^12 12.3 (18.4), 2^14 14.3 (20.5), 2^16 18.5 (30.7), 2^17 34.8 (49.0); up to
+// 2^8 the host's call takes longer than the kernel.  2^18: 54.9 here, 55.3 with
+// the tile kernel; 2^19: 109 and 94.
+// Values are lazy (below 2r) until the last pass stores them.  Every input of
+// the block is read before the first barrier, so one pass may run in place
+// (with one warp: before the first __syncwarp).
+__device__ __forceinline__ uint32_t small_swz(uint32_t i) {
+  return i ^ (((i >> 3) ^ (i >> 6) ^ (i >> 9)) & 7u);
 }
+// twiddles of layer s >= 1 (w_{2^(s+1)}^j, j < 2^s), planes as mul_round_twiddle
+__host__ __device__ __forceinline__ uint32_t layer_offset(uint32_t s) { return 8 * ((1u << s) - 1); }
+constexpr uint32_t kLayerUnits = 8 * 1023;  // layers 0 .. 9
 
-// One tile of a latency-form pass (2^9 .. 2^17 points, one column per tile):
-// the tile geometry, inputs and outputs of ntt_tile, with each column's DFT
-// as rolled radix-2 decimation-in-time layers over its bit-reversed copy in
-// shared memory (so the result is in natural order), canonical throughout.
-__global__ void __launch_bounds__(256) k_ntt_small_pass(const PassArgs a) {
+__global__ void __launch_bounds__(512) k_ntt_small_pass(const PassArgs a) {
   extern __shared__ uint4 sm[];
-  fr *x = reinterpret_cast<fr *>(sm);  // column col at x[col R ..]
-  const uint32_t lgR = a.lgR, R = 1u << lgR, T = 1u << a.lgT, E = R << a.lgT;
-  const uint64_t tileid = blockIdx.x;
-  uint64_t base = 0, col0 = 0, in_base = 0, out_base = 0;
-  uint32_t lgS1 = 0;
-  if (!a.last) {
-    const uint32_t lgtpq = a.lgS - a.lgT;
-    const uint64_t q = tileid >> lgtpq, ct = tileid & ((1ull << lgtpq) - 1);
-    col0 = ct << a.lgT;
-    base = (q << (a.lgR + a.lgS)) + col0;
-  } else {
-    const uint32_t lgR1 = a.lgRp[0];
-    lgS1 = a.lgN - lgR1;
-    const uint32_t lgkb = lgR1 - a.lgT;
-    const uint64_t kb = tileid & ((1ull << lgkb) - 1), rest = tileid >> lgkb;
-    uint64_t rin = 0, r = rest;
-    uint32_t acc = lgR1;
-    for (uint32_t j = 1; j + 1 < a.P; ++j) {
-      const uint32_t bits = a.lgRp[j];
-      acc += bits;
-      rin += (r & ((1ull << bits) - 1)) << (a.lgN - acc);
-      r >>= bits;
+  const uint32_t lgR = a.lgR, R = 1u << lgR, half = R >> 1, b = threadIdx.x;
+  uint4 *lo = sm, *hi = sm + R;  // element i: words 0..3 at lo[swz(i)], 4..7 at hi
+  const auto put = [&](uint32_t i, const fr &v) {
+    lo[small_swz(i)] = make_uint4(v.v[0], v.v[1], v.v[2], v.v[3]);
+    hi[small_swz(i)] = make_uint4(v.v[4], v.v[5], v.v[6], v.v[7]);
+  };
+  const auto get = [&](uint32_t i) {
+    const uint4 u = lo[small_swz(i)], v = hi[small_swz(i)];
+    return fr{{u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w}};
+  };
+  const TileGeom geo = tile_geom(a, blockIdx.x);
+  const bool active = b < half;
+  const uint32_t bn = __brev(b) >> (33 - lgR);  // row of the thread's first input
+  // a dependent pass may start while the one before it drains
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  fr x[2];
+  if (active) {
+#pragma unroll
+    for (uint32_t i = 0; i < 2; ++i) {
+      const uint64_t g = geo.src(a, bn + i * half, 0);
+      if (!a.first) {
+        x[i] = ldcs_fr(a.in + g);
+      } else if (a.in_kind == NTT_IN_SPREAD) {
+        x[i] = (g & ((1ull << a.spread) - 1)) == 0 ? ldcs_fr(a.in + (g >> a.spread)) : fr_zero();
+      } else {
+        x[i] = g < a.n_valid ? ldcs_fr(a.in + g) : fr_zero();
+      }
     }
-    in_base = ((kb << a.lgT) << lgS1) + rin;
-    out_base = (kb << a.lgT) + (rest << lgR1);
-  }
+    if (a.first && a.in_kind == NTT_IN_DIAG) {
 #pragma unroll 1
-  for (uint32_t e = threadIdx.x; e < E; e += blockDim.x) {
-    uint32_t n, col;
-    uint64_t g;
+      for (uint32_t i = 0; i < 2; ++i) {
+        const uint64_t g = geo.src(a, bn + i * half, 0);
+        const fr d = g < a.n_valid ? ldcs_fr(a.diag + g) : fr_zero();
+        const fr v = fr_mul_lazy(i ? x[1] : x[0], d);
+        if (i) x[1] = v;
+        else x[0] = v;
+      }
+    }
+    bfly(x[0], x[1]);
+    put(2 * b, x[0]);
+    put(2 * b + 1, x[1]);
+  }
+  uint32_t p = 2 * b, q = 2 * b + 1;
+#pragma unroll 1
+  for (uint32_t s = 1; s < lgR; ++s) {
+    const uint32_t j = b & ((1u << s) - 1);
+    uint4 w[8];
+    if (active) {
+      const uint4 *t = a.tw_dit + layer_offset(s) + j;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) w[k] = __ldg(t + (k << s));
+    }
+    // layers 0 .. 5 stay within the 64 elements of a warp
+    if (s <= 5) __syncwarp();
+    else __syncthreads();
+    p = ((b >> s) << (s + 1)) + j;
+    q = p + (1u << s);
+    if (active) {
+      fr wp[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        wp[k] = fr{{w[2 * k].x, w[2 * k].y, w[2 * k].z, w[2 * k].w, w[2 * k + 1].x, w[2 * k + 1].y,
+                    w[2 * k + 1].z, w[2 * k + 1].w}};
+      x[0] = get(p);
+      x[1] = fr_mul_const4(get(q), wp);
+      bfly(x[0], x[1]);
+      if (s + 1 < lgR) {
+        put(p, x[0]);
+        put(q, x[1]);
+      }
+    }
+  }
+  if (!active) return;
+#pragma unroll 1
+  for (uint32_t i = 0; i < 2; ++i) {
+    const uint64_t o = i ? q : p;
+    fr v = i ? x[1] : x[0];
     if (!a.last) {
-      n = e >> a.lgT;
-      col = e & (T - 1);
-      g = base + ((uint64_t)n << a.lgS) + col;
+      v = fr_mul_lazy(v, ldcs_fr(a.tw_layer + (o << a.lgS) + geo.col0));
+      st_fr(a.out + geo.base + (o << a.lgS), v);
     } else {
-      n = e & (R - 1);
-      col = e >> a.lgR;
-      g = in_base + ((uint64_t)col << lgS1) + n;
-    }
-    fr v;
-    if (!a.first) {
-      v = ldcs_fr(a.in + g);
-    } else if (a.in_kind == NTT_IN_SPREAD) {
-      v = (g & ((1ull << a.spread) - 1)) == 0 ? ldcs_fr(a.in + (g >> a.spread)) : fr_zero();
-    } else if (g < a.n_valid) {
-      v = ldcs_fr(a.in + g);
-      if (a.in_kind == NTT_IN_DIAG) v = fr_mul(v, ldcs_fr(a.diag + g));
-    } else {
-      v = fr_zero();
-    }
-    st_fr(x + (col << lgR) + (__brev(n) >> (32 - lgR)), v);
-  }
-  __syncthreads();
-  const uint32_t half = E >> 1, hmask = (R >> 1) - 1;
-#pragma unroll 1
-  for (uint32_t s = 0; s < lgR; ++s) {
-#pragma unroll 1
-    for (uint32_t b = threadIdx.x; b < half; b += blockDim.x) {
-      fr *xc = x + ((b >> (lgR - 1)) << lgR);
-      const uint32_t bb = b & hmask, j = bb & ((1u << s) - 1);
-      const uint32_t p = ((bb >> s) << (s + 1)) + j, q = p + (1u << s);
-      const fr t = fr_mul(ld_fr(xc + q), ldg_fr(a.tw_inner + (j << (lgR - 1 - s))));
-      const fr u = ld_fr(xc + p);
-      st_fr(xc + p, fr_add(u, t));
-      st_fr(xc + q, fr_sub(u, t));
-    }
-    __syncthreads();
-  }
-#pragma unroll 1
-  for (uint32_t e = threadIdx.x; e < E; e += blockDim.x) {
-    const uint32_t o = e >> a.lgT, col = e & (T - 1);
-    fr v = ld_fr(x + (col << lgR) + o);
-    if (!a.last) {
-      if (a.tw_layer) v = fr_mul(v, ldcs_fr(a.tw_layer + ((uint64_t)o << a.lgS) + col0 + col));
-      st_fr(a.out + base + ((uint64_t)o << a.lgS) + col, v);
-    } else {
+      v = fr_canon(v);
       if (a.has_post_scale) v = fr_mul(v, a.post_scale);
-      st_fr(a.out + out_base + col + ((uint64_t)o << (a.lgN - a.lgR)), v);
+      st_fr(a.out + geo.out_base + (o << (a.lgN - a.lgR)), v);
     }
   }
 }
@@ -622,18 +700,48 @@ __global__ void k_pow_table(fr *out, uint64_t count, const fr *__restrict__ win,
   }
 }
 
+// the round tables (round_offset, mul_round_twiddle) from inner[e] = w_2048^e:
+// block 7 (lgSj - 1) + k - 1, one thread per column
+struct Fr4 {
+  fr v[4];
+};
+__global__ void k_round_table(uint4 *out, const fr *__restrict__ inner, const Fr4 f) {
+  const uint32_t lgSj = blockIdx.x / 7 + 1, k = blockIdx.x % 7 + 1, c = threadIdx.x;
+  if (c >> lgSj) return;
+  const fr w = ldg_fr(inner + ((c * k) << (8 - lgSj)));
+  uint4 *t = out + round_offset(lgSj) + (((k - 1) * 8) << lgSj) + c;
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    const fr v = fr_mul(w, f.v[p]);
+    t[(2 * p) << lgSj] = make_uint4(v.v[0], v.v[1], v.v[2], v.v[3]);
+    t[(2 * p + 1) << lgSj] = make_uint4(v.v[4], v.v[5], v.v[6], v.v[7]);
+  }
+}
+
+// the latency form's layer tables from inner[e] = w_2048^e: layer blockIdx.y,
+// one thread per entry
+__global__ void k_layer_table(uint4 *out, const fr *__restrict__ inner, const Fr4 f) {
+  const uint32_t s = blockIdx.y, j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >> s) return;
+  const fr w = ldg_fr(inner + (j << (10 - s)));
+  uint4 *t = out + layer_offset(s) + j;
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    const fr v = fr_mul(w, f.v[p]);
+    t[(2 * p) << s] = make_uint4(v.v[0], v.v[1], v.v[2], v.v[3]);
+    t[(2 * p + 1) << s] = make_uint4(v.v[4], v.v[5], v.v[6], v.v[7]);
+  }
+}
+
 // ------------------------------------------------------------ host side
 namespace {
 
 std::mutex g_mu;
 
-struct InnerKey {
+struct RoundKey {
   int dev;
-  uint32_t lgR;
   bool inv;
-  bool operator<(const InnerKey &o) const {
-    return std::tie(dev, lgR, inv) < std::tie(o.dev, o.lgR, o.inv);
-  }
+  bool operator<(const RoundKey &o) const { return std::tie(dev, inv) < std::tie(o.dev, o.inv); }
 };
 
 struct Plan {
@@ -643,6 +751,7 @@ struct Plan {
   uint32_t lgR[4] = {0, 0, 0, 0};
   uint32_t lgT[4] = {0, 0, 0, 0};
   const fr *tw_inner[4] = {nullptr, nullptr, nullptr, nullptr};
+  const uint4 *tw_round = nullptr;
   fr *tw_layer[4] = {nullptr, nullptr, nullptr, nullptr};
   // host-pass plans: split layer tables instead of tw_layer
   fr *tw_lo[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -682,7 +791,7 @@ struct PowKey {
   }
 };
 
-std::map<InnerKey, fr *> g_inner;
+std::map<RoundKey, uint4 *> g_round;
 std::map<PlanKey, Plan *> g_plans;
 std::map<PowKey, fr *> g_pows;
 std::map<uint32_t, std::vector<uint32_t>> g_split_override;
@@ -743,17 +852,44 @@ int build_table(fr **out, uint64_t count, const fr &base, uint32_t kind, uint32_
   return PP_OK;
 }
 
-int get_inner(int dev, uint32_t lgR, bool inv, const fr **out) {
-  InnerKey k{dev, lgR, inv};
-  auto it = g_inner.find(k);
-  if (it != g_inner.end()) {
+// the round tables of a direction (kRoundUnits 16-byte units), then the layer
+// tables of the latency form (kLayerUnits)
+int get_round(int dev, bool inv, const uint4 **out) {
+  const RoundKey k{dev, inv};
+  auto it = g_round.find(k);
+  if (it != g_round.end()) {
     *out = it->second;
     return PP_OK;
   }
-  fr *t = nullptr;
-  int st = build_table(&t, 1ull << lgR, host_root_of_unity((int)lgR, inv), 0, 0, nullptr);
+  fr *inner = nullptr;  // w_2048^e, e < 2048
+  const int st = build_table(&inner, 2048, host_root_of_unity(11, inv), 0, 0, nullptr);
   if (st) return st;
-  g_inner[k] = t;
+  // factors that take a Montgomery-form w to w 2^(64 p + 96)
+  Fr4 f;
+  std::memset(&f, 0, sizeof(f));
+  for (int p = 0; p < 3; ++p) f.v[p].v[2 * p + 3] = 1;
+  f.v[3] = host_mont_small(1ull << 32);  // 2^288
+  uint4 *t = nullptr;
+  const size_t bytes = (kRoundUnits + kLayerUnits) * sizeof(uint4);
+  PP_COUNT_ALLOC(bytes);
+  cudaError_t e = cudaMalloc(&t, bytes);
+  if (e != cudaSuccess) {
+    cudaFree(inner);
+    set_error("round twiddle tables: %s", cudaGetErrorString(e));
+    return PP_E_NOMEM;
+  }
+  k_round_table<<<7 * 8, 256>>>(t, inner, f);
+  PP_COUNT_LAUNCH();
+  k_layer_table<<<dim3(2, 10), 256>>>(t + kRoundUnits, inner, f);
+  PP_COUNT_LAUNCH();
+  e = cudaDeviceSynchronize();
+  cudaFree(inner);
+  if (e != cudaSuccess) {
+    cudaFree(t);
+    set_error("table kernel failed: %s", cudaGetErrorString(e));
+    return PP_E_CUDA;
+  }
+  g_round[k] = t;
   *out = t;
   return PP_OK;
 }
@@ -779,6 +915,11 @@ int get_plan(int dev, uint32_t lgN, bool inv, Plan **out, bool small = false, bo
   p->inverse = inv;
   p->P = (uint32_t)bits.size();
   const fr ninv = host_inv(host_mont_small(1ull << lgN));
+  int st = get_round(dev, inv, &p->tw_round);
+  if (st) {
+    delete p;
+    return st;
+  }
   uint32_t acc = 0;
   for (uint32_t j = 0; j < p->P; ++j) {
     p->lgR[j] = bits[j];
@@ -792,12 +933,6 @@ int get_plan(int dev, uint32_t lgN, bool inv, Plan **out, bool small = false, bo
     } else {
       const uint32_t want = 11 - bits[j];
       p->lgT[j] = want < bits[0] ? want : bits[0];
-    }
-    int st = get_inner(dev, bits[j], inv, &p->tw_inner[j]);
-    if (st) {
-      free_plan_tables(p);
-      delete p;
-      return st;
     }
     if (j + 1 < p->P) {
       // w_{R S}^(c k) with R S = 2^(lgN - (acc - bits[j]))
@@ -903,13 +1038,13 @@ const fr *pow_table(const fr &h, uint32_t lg_n, int *status) {
 
 void ntt_release_tables() {
   std::lock_guard<std::mutex> lk(g_mu);
-  for (auto &kv : g_inner) cudaFree(kv.second);
+  for (auto &kv : g_round) cudaFree(kv.second);
   for (auto &kv : g_plans) {
     free_plan_tables(kv.second);
     delete kv.second;
   }
   for (auto &kv : g_pows) cudaFree(kv.second);
-  g_inner.clear();
+  g_round.clear();
   g_plans.clear();
   g_pows.clear();
 }
@@ -950,8 +1085,6 @@ int describe_passes(const fr *d_in, fr *d_out, fr *work, uint32_t lg_m, bool inv
       PP_CUDA_TRY(cudaFuncSetAttribute(k_ntt_batch_level,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        2048 * (int)sizeof(fr)));
-      PP_CUDA_TRY(cudaFuncSetAttribute(k_ntt_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       2048 * (int)sizeof(fr)));
       g_attr_set[dev] = true;
     }
   }
@@ -963,6 +1096,9 @@ int describe_passes(const fr *d_in, fr *d_out, fr *work, uint32_t lg_m, bool inv
   std::memset(&a, 0, sizeof(a));
   a.lgN = lg_m;
   a.P = plan->P;
+  a.inverse = inverse ? 1 : 0;
+  a.tw_round = plan->tw_round;
+  a.tw_dit = plan->tw_round + kRoundUnits;
   for (uint32_t j = 0; j < plan->P; ++j) a.lgRp[j] = plan->lgR[j];
   a.diag = in.diag;
   a.diag_hi = in.diag_hi;
@@ -990,7 +1126,6 @@ int describe_passes(const fr *d_in, fr *d_out, fr *work, uint32_t lg_m, bool inv
     a.unit_out = a.last && in.out_host;
     a.in = j == 0 ? d_in : work;
     a.out = a.last ? d_out : work;
-    a.tw_inner = plan->tw_inner[j];
     a.tw_layer = plan->tw_layer[j];
     a.tw_lo = plan->tw_lo[j];
     a.tw_hi = plan->tw_hi[j];
@@ -1046,21 +1181,25 @@ int ntt_run(const fr *d_in, fr *d_out, uint32_t lg_m, bool inverse, const NttInp
   std::vector<uint64_t> tiles;
   int st = ntt_describe(d_in, d_out, work, lg_m, inverse, in, passes, tiles, small);
   if (st) return st;
-  if (small) {
+  if (small || lg_m <= kSmallOnePass) {
     for (size_t j = 0; j < passes.size(); ++j) {
-      const uint32_t E = 1u << (passes[j].lgR + passes[j].lgT);
-      const uint32_t threads = E / 2 < 32 ? 32 : (E / 2 > 256 ? 256 : E / 2);
-      k_ntt_small_pass<<<(unsigned)tiles[j], threads, E * sizeof(fr), stream>>>(passes[j]);
+      const uint32_t R = 1u << passes[j].lgR;
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3((unsigned)tiles[j]);
+      cfg.blockDim = dim3(R / 2 < 32 ? 32 : R / 2);
+      cfg.dynamicSmemBytes = R * sizeof(fr);
+      cfg.stream = stream;
+      // the second pass's blocks may be placed while the first pass drains;
+      // they wait for it (griddepcontrol.wait) before they read
+      cudaLaunchAttribute attr = {};
+      attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr.val.programmaticStreamSerializationAllowed = 1;
+      cfg.attrs = &attr;
+      cfg.numAttrs = j > 0 ? 1 : 0;
+      PP_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_ntt_small_pass, passes[j]));
       PP_COUNT_LAUNCH();
       PP_LAUNCH_CHECK();
     }
-    return PP_OK;
-  }
-  if (passes.size() == 1 && lg_m <= 11) {
-    const uint32_t threads = (uint32_t)(N / 2 < 32 ? 32 : (N / 2 > 512 ? 512 : N / 2));
-    k_ntt_small<<<1, threads, N * sizeof(fr), stream>>>(passes[0]);
-    PP_COUNT_LAUNCH();
-    PP_LAUNCH_CHECK();
     return PP_OK;
   }
   for (size_t j = 0; j < passes.size(); ++j) {

@@ -13,7 +13,8 @@ namespace pp {
 struct PassArgs {
   const fr *in;
   fr *out;
-  const fr *tw_inner;  // w_R^e, e < R
+  const uint4 *tw_round;  // the direction's round tables (ntt_tile)
+  const uint4 *tw_dit;    // the direction's layer tables (k_ntt_small_pass)
   const fr *tw_layer;  // w_{R S}^(c k) at [k][c], or null
   // split layer twiddles (when tw_layer is null): w_{R S}^e =
   // tw_hi[e >> tw_lgh] * tw_lo[e mod 2^tw_lgh], e = c k, or null
@@ -25,7 +26,7 @@ struct PassArgs {
   fr post_scale;
   uint64_t n_valid;
   uint32_t lgR, lgT, lgS, lgN;
-  uint32_t first, last, has_post_scale, in_kind, spread;
+  uint32_t first, last, inverse, has_post_scale, in_kind, spread;
   uint32_t unit_in, unit_out;  // move 16-byte halves (host-memory input / output)
   uint32_t zero_lg;  // first pass: rows >= R >> zero_lg of every tile are zero (padding)
   uint32_t tw_lgh;   // split layer twiddles: bits of the low table
@@ -91,11 +92,14 @@ int ntt_describe(const fr *d_in, fr *d_out, fr *work, uint32_t lg_m, bool invers
                  const NttInputDesc &in, std::vector<PassArgs> &passes,
                  std::vector<uint64_t> &tiles, bool small = false);
 
-// Single calls of 2^9 .. 2^17 points run the latency form: two passes with
-// one column per tile (k_ntt_small_pass).  Those sizes are bound by latency
-// (a few microseconds of work), and the throughput plan's 2048-element tiles
-// would leave most SMs idle.
-inline bool ntt_small_form(uint32_t lg_m) { return lg_m >= 9 && lg_m <= 17; }
+// Single calls run the latency form (k_ntt_small_pass, one column per block) in
+// one pass up to 2^8 points and in two up to 2^17: those sizes are bound by
+// latency (a few microseconds of work), and the throughput plan's 2048-element
+// tiles would leave most SMs idle.  One pass of 2^9 points instead of two
+// gained nothing (10.2 against 10.9 us on a host-bound call); from 2^18 the
+// tile kernel is as fast or faster.
+constexpr uint32_t kSmallOnePass = 8, kSmallTwoPass = 17;
+inline bool ntt_small_form(uint32_t lg_m) { return lg_m > kSmallOnePass && lg_m <= kSmallTwoPass; }
 // One launch over the tiles of up to kLevelJobs job passes, one block per
 // tile.  The arguments travel as the kernel's parameters (20.5 KB; CUDA
 // allows 32 KB): the tile code then reads them as constant operands, as

@@ -1,8 +1,9 @@
 // Host-side check of the carry-chained field multiplies (csrc/fr.cuh,
 // csrc/fq.cuh): products, squares and lazy products against the row forms,
-// which fr_host_check and g1_host_check hold against the oracle.  Operands are
-// random and built from all-ones and all-zero limbs, so every carry link is
-// exercised.  Built and run by tests/test_cells_host.py.
+// which fr_host_check and g1_host_check hold against the oracle, and the
+// transform's four-part constant multiply against its definition.  Operands are
+// random and built from limbs 0, 1, 2^32 - 1 and 2^32 - 2, which reach the
+// carry links that random limbs meet once in 2^32 products.  Built and run by tests/test_cells_host.py.
 #include <cstdio>
 #include <cstdlib>
 #include <random>
@@ -18,7 +19,8 @@ static T operand(int kind) {
   T a;
   for (int i = 0; i < N; ++i) {
     const uint32_t r = (uint32_t)rng();
-    a.v[i] = kind == 0 ? r : kind == 1 ? (r & 1 ? 0xffffffffu : 0u) : (r & 3 ? r : 0xffffffffu);
+    const uint32_t edge[4] = {0u, 0xffffffffu, 1u, 0xfffffffeu};
+    a.v[i] = kind == 0 ? r : kind == 1 ? edge[r & 3] : (r & 4 ? r : edge[r & 3]);
   }
   return a;
 }
@@ -40,6 +42,23 @@ int main(int argc, char **argv) {
     bad += !fr_eq(fr_sqr(a), fr_mul_row9(a, a));
     fr wc = fr_canon(fr_mul_row9<true>(wide, b));
     bad += !fr_eq(fr_canon(fr_mul_cells<true>(wide, b)), wc);
+
+    // the four-part product: result 2^96 = sum of (64-bit part) w_p (mod r),
+    // and below r + 2^-30 r
+    fr w[4], sum = fr_zero(), p96 = fr_zero();
+    p96.v[3] = 1;
+    for (int p = 0; p < 4; ++p) {
+      w[p] = operand<fr, 8>((it / 9 + p) % 3);
+      w[p].v[7] &= 0x7fffffffu;
+      fr_reduce_once(w[p].v);
+      if (it == 2) w[p] = fr_sub(fr_zero(), fr_one());
+      fr part = fr_zero();
+      part.v[0] = wide.v[2 * p];
+      part.v[1] = wide.v[2 * p + 1];
+      sum = fr_add(sum, fr_mul_row9(fr_mul_row9(part, fr_rr()), w[p]));
+    }
+    const fr four = fr_mul_const4(wide, w);
+    bad += four.v[7] > PP_R7 || !fr_eq(fr_mul_row9(fr_mul_row9(fr_canon(four), fr_rr()), p96), sum);
 
     fq x = operand<fq, 12>(it % 3), y = operand<fq, 12>((it / 3) % 3);
     x.v[11] &= 0x1fffffffu;
