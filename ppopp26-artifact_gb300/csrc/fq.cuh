@@ -320,7 +320,7 @@ PP_HD void fq_sqr_cross(uint32_t *E, uint32_t *O, const uint32_t a[12]) {
 
 // a^2 R^-1 mod q for a < q (same result as fq_mul(a, a)): 66 cross products,
 // doubled, and 12 squares instead of 144 products, then the same reduction
-PP_FQ_MUL fq fq_sqr(fq a) {
+PP_HD fq fq_sqr_cells(const fq &a) {
   uint32_t E[26], O[26], T[24];
 #pragma unroll
   for (int k = 0; k < 26; ++k) E[k] = O[k] = 0;
@@ -343,6 +343,7 @@ PP_FQ_MUL fq fq_sqr(fq a) {
   }
   return fq_redc24_cells(T);
 }
+PP_FQ_MUL fq fq_sqr(fq a) { return fq_sqr_cells(a); }
 
 // ---- binary extended-GCD inverse: shifts and subtractions instead of the
 // ~480 dependent multiplies of a Fermat chain (for single-thread use)

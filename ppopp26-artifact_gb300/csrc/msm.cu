@@ -15,10 +15,13 @@
 //                exact); bucket sizes counted with warp-aggregated atomics
 //   2. scan      exclusive prefix sum of the W * 2^(c-1) bucket sizes (tiled)
 //   3. scatter   (point index, sign) into each bucket's slice: a counting sort
-//   4. buckets   bucket sums in groups of at most K points per thread, then
-//                levels of groups of K partial sums for buckets that had more
-//                (a bucket can hold up to all n points: equal scalars, or the
-//                few-bit top window), so no thread sums more than K values
+//   4. buckets   the sorted list is cut into equal runs of K entries, one thread
+//                each, whatever the bucket sizes: a thread writes the buckets
+//                that lie inside its run and leaves a partial sum for the one
+//                it shares with the run before and the one after.  A second
+//                launch joins each shared bucket's partial sums (one thread
+//                for a few, blocks for many: a bucket can hold up to all n
+//                points: equal scalars, or the few-bit top window)
 //   5. segments  one thread per run of G buckets: running sums T = sum
 //                (j + 1) B and R = sum B over its run
 //   6. windows   sum T + G sum_s s R_s with sum_s s R_s = sum_k 2^k Q_k, Q_k
@@ -301,63 +304,152 @@ __global__ void k_msm_scatter(const uint32_t *__restrict__ digits, uint64_t n, M
 }
 
 constexpr int kPointThreads = 128;
-constexpr uint32_t kGroup = 16;  // values summed by one thread (16 beat 32 and 64 on GB300)
+constexpr int kAccumulateBlocks = 3;       // resident blocks per SM (168 registers)
+constexpr uint32_t kRunMin = 10, kRunMax = 64;
+constexpr uint32_t kJoinMin = 8;           // partial sums one thread adds up
+constexpr uint32_t kJoinChunk = 1024;      // partial sums one block adds up
 
-// Per bucket at one level: m values to sum.  groups = ceil(m / K) threads; a
-// bucket with m <= K is finished by its one group, otherwise its groups leave
-// ceil(m / K) partial sums for the next level (next = that count, else 0).
-__global__ void k_msm_groups(const uint32_t *__restrict__ m, uint64_t nb,
-                             uint32_t *__restrict__ groups, uint32_t *__restrict__ next) {
-  for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nb;
-       b += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t v = m[b];
-    const uint32_t g = (v + kGroup - 1) / kGroup;
-    groups[b] = g;
-    next[b] = v > kGroup ? g : 0;
-  }
-}
-
-// the bucket whose group range [goff[b], goff[b+1]) holds group t
-__device__ __forceinline__ uint32_t bucket_of(const uint32_t *goff, uint32_t nb, uint32_t t) {
-  uint32_t lo = 0, hi = nb;  // goff[lo] <= t < goff[hi]
+// the bucket whose range [off[b], off[b+1]) holds entry t
+__device__ __forceinline__ uint32_t bucket_of(const uint32_t *off, uint32_t nb, uint32_t t) {
+  uint32_t lo = 0, hi = nb;  // off[lo] <= t < off[hi]
   while (hi - lo > 1) {
     const uint32_t mid = (lo + hi) >> 1;
-    if (goff[mid] <= t) lo = mid;
+    if (off[mid] <= t) lo = mid;
     else hi = mid;
   }
   return lo;
 }
 
-// One level of bucket sums.  Level 0 (list != null) adds signed affine points
-// named by the sorted list; later levels add XYZZ partial sums.  Group t of
-// bucket b sums values [off[b] + j K, ...) of that bucket (j = t - goff[b]);
-// a finished bucket is written to buckets[b], else to part_out[noff[b] + j].
-__global__ void __launch_bounds__(kPointThreads, 3)
-    k_msm_level(const g1a *__restrict__ points, const uint32_t *__restrict__ list,
-                const g1x *__restrict__ part_in, const uint32_t *__restrict__ m,
-                const uint32_t *__restrict__ off, const uint32_t *__restrict__ goff,
-                const uint32_t *__restrict__ noff, uint32_t nb, g1x *__restrict__ part_out,
-                g1x *__restrict__ buckets) {
-  const uint32_t total = goff[nb];
-  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
-    const uint32_t b = bucket_of(goff, nb, t);
-    const uint32_t j = t - goff[b];
-    const uint32_t cnt = m[b];
-    const uint32_t lo = off[b] + j * kGroup;
-    const uint32_t hi = lo + kGroup < off[b] + cnt ? lo + kGroup : off[b] + cnt;
-    g1x acc = g1x_inf();
-    if (list) {
-      for (uint32_t k = lo; k < hi; ++k) {
-        const uint32_t e = list[k];
-        g1a pt = ld_g1a(points + (e & 0x7fffffffu));
-        if (e >> 31) pt = g1a_neg(pt);
-        acc = g1x_add_affine(acc, pt);
-      }
-    } else {
-      for (uint32_t k = lo; k < hi; ++k) acc = g1x_add(acc, part_in[k]);
+// Bucket sums.  Thread t adds the signed affine points of entries [t K, (t+1) K)
+// of the sorted list, starting a new sum at each bucket boundary.  Every lane
+// does the same number of additions, so the warps are full whatever the buckets
+// hold; with one thread per 16 entries of a bucket, and a level of partial sums
+// after it, a quarter of the lanes waited.  GB300: 200003 points 3.63 -> 3.13 ms,
+// 2^20 9.84 -> 8.48 ms, fixed-base 2^20 7.65 -> 6.98 ms.  Inlining the ten
+// multiplies instead of calling them: 3.17 -> 3.29 ms.
+// A bucket that lies inside the run goes to buckets[]; the sum shared with the
+// run before goes to part[2 t], the one shared only with the run after to
+// part[2 t + 1].  Bound by the multiply pipe.
+__global__ void __launch_bounds__(kPointThreads, kAccumulateBlocks)
+    k_msm_accumulate(const g1a *__restrict__ points, const uint32_t *__restrict__ list,
+                     const uint32_t *__restrict__ off, uint32_t nb, uint32_t K,
+                     g1x *__restrict__ part, g1x *__restrict__ buckets) {
+  const uint32_t total = off[nb];
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint64_t lo64 = (uint64_t)t * K;
+  if (lo64 >= total) return;
+  const uint32_t lo = (uint32_t)lo64, hi = total - lo < K ? total : lo + K;
+  uint32_t b = bucket_of(off, nb, lo);
+  uint32_t start = off[b], end = off[b + 1];
+  g1x acc = g1x_inf();
+  for (uint32_t k = lo;; ++k) {
+    if (k == end || k == hi) {  // the sum of bucket b ends here
+      g1x *dst = start < lo ? part + 2 * (uint64_t)t : end > hi ? part + 2 * (uint64_t)t + 1 : buckets + b;
+      *dst = acc;
+      if (k == hi) break;
+      do {
+        ++b;
+        start = end;
+        end = off[b + 1];
+      } while (end == k);  // skips empty buckets
+      acc = g1x_inf();
     }
-    if (cnt <= kGroup) buckets[b] = acc;
-    else part_out[noff[b] + j] = acc;
+    const uint32_t e = list[k];
+    g1a pt = ld_g1a(points + (e & 0x7fffffffu));
+    if (e >> 31) pt = g1a_neg(pt);
+    acc = g1x_add_affine(acc, pt);
+  }
+}
+
+// A bucket of entries [start, end) is shared by runs start / K .. (end - 1) / K:
+// the first left its sum in its second slot, the others in their first.
+struct BucketSpan {
+  uint32_t first, m;  // first run, number of partial sums (1: complete, 0: empty)
+};
+__device__ __forceinline__ BucketSpan bucket_span(const uint32_t *off, uint32_t b, uint32_t K) {
+  const uint32_t start = off[b], end = off[b + 1];
+  if (start == end) return {0, 0};
+  return {start / K, (end - 1) / K - start / K + 1};
+}
+__device__ __forceinline__ uint64_t partial_index(const BucketSpan &s, uint32_t j) {
+  return 2 * (uint64_t)(s.first + j) + (j == 0 ? 1 : 0);
+}
+
+// Lists the buckets of more than `few` partial sums: items[i] = (bucket, chunk)
+// for every kJoinChunk of them, multi[] = (bucket, first item) for buckets of
+// several chunks; counts in n_items[0] and n_items[1].
+__global__ void k_msm_spans(const uint32_t *__restrict__ off, uint32_t nb, uint32_t K, uint32_t few,
+                            uint2 *__restrict__ items, uint2 *__restrict__ multi,
+                            uint32_t *__restrict__ n_items) {
+  const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >= nb) return;
+  const BucketSpan sp = bucket_span(off, b, K);
+  if (sp.m <= few) return;
+  const uint32_t chunks = (sp.m + kJoinChunk - 1) / kJoinChunk;
+  const uint32_t first = atomicAdd(n_items, chunks);
+  for (uint32_t c = 0; c < chunks; ++c) items[first + c] = make_uint2(b, c);
+  if (chunks > 1) multi[atomicAdd(n_items + 1, 1u)] = make_uint2(b, first);
+}
+
+// sum of val(j), lo <= j < hi, by a block of kPointThreads (the result in
+// thread 0): strided sums, then a tree in shared memory
+template <typename F>
+__device__ __forceinline__ g1x block_sum(uint32_t lo, uint32_t hi, g1x *red, F val) {
+  g1x acc = g1x_inf();
+  for (uint32_t j = lo + threadIdx.x; j < hi; j += kPointThreads) acc = g1x_add(acc, val(j));
+  red[threadIdx.x] = acc;
+  __syncthreads();
+  for (uint32_t h = kPointThreads / 2; h > 0; h >>= 1) {
+    if (threadIdx.x < h) red[threadIdx.x] = g1x_add(red[threadIdx.x], red[threadIdx.x + h]);
+    __syncthreads();
+  }
+  const g1x r = red[0];
+  __syncthreads();  // red may be used again
+  return r;
+}
+
+// Joins the shared buckets: the first `small_blocks` blocks take one bucket per
+// thread, the others (128 threads each) the listed chunks of the larger ones,
+// whose sums go to buckets[] or, with several chunks, to chunk_sum[item].
+__global__ void __launch_bounds__(kPointThreads)
+    k_msm_join(const g1x *__restrict__ part, const uint32_t *__restrict__ off, uint32_t nb, uint32_t K,
+               uint32_t few, uint32_t small_blocks, const uint2 *__restrict__ items,
+               const uint32_t *__restrict__ n_items, g1x *__restrict__ chunk_sum,
+               g1x *__restrict__ buckets) {
+  __shared__ g1x red[kPointThreads];
+  if (blockIdx.x < small_blocks) {
+    const uint32_t b = blockIdx.x * kPointThreads + threadIdx.x;
+    if (b >= nb) return;
+    const BucketSpan sp = bucket_span(off, b, K);
+    if (sp.m < 2 || sp.m > few) return;
+    g1x acc = part[partial_index(sp, 0)];
+    for (uint32_t j = 1; j < sp.m; ++j) acc = g1x_add(acc, part[partial_index(sp, j)]);
+    buckets[b] = acc;
+    return;
+  }
+  const uint32_t n = n_items[0];
+  for (uint32_t it = blockIdx.x - small_blocks; it < n; it += gridDim.x - small_blocks) {
+    const uint2 item = items[it];
+    const BucketSpan sp = bucket_span(off, item.x, K);
+    const uint32_t lo = item.y * kJoinChunk, hi = sp.m - lo < kJoinChunk ? sp.m : lo + kJoinChunk;
+    const g1x sum = block_sum(lo, hi, red, [&](uint32_t j) { return part[partial_index(sp, j)]; });
+    if (threadIdx.x == 0) (sp.m <= kJoinChunk ? buckets[item.x] : chunk_sum[it]) = sum;
+  }
+}
+
+// the chunks of the buckets that have several
+__global__ void __launch_bounds__(kPointThreads)
+    k_msm_join_chunks(const uint32_t *__restrict__ off, uint32_t K, const uint2 *__restrict__ multi,
+                      const uint32_t *__restrict__ n_items, const g1x *__restrict__ chunk_sum,
+                      g1x *__restrict__ buckets) {
+  __shared__ g1x red[kPointThreads];
+  const uint32_t n = n_items[1];
+  for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
+    const uint2 mb = multi[i];
+    const BucketSpan sp = bucket_span(off, mb.x, K);
+    const uint32_t chunks = (sp.m + kJoinChunk - 1) / kJoinChunk;
+    const g1x sum = block_sum(0, chunks, red, [&](uint32_t j) { return chunk_sum[mb.y + j]; });
+    if (threadIdx.x == 0) buckets[mb.x] = sum;
   }
 }
 
@@ -387,10 +479,11 @@ __global__ void __launch_bounds__(kPointThreads)
 // sum_s T_s, sum j = 1 + k is Q_k) and one short Horner chain; no sum weights
 // a point by more than one doubling at a time.
 //
-// Each sum is cut into chunks of kChunk terms; one thread adds one chunk.
+// Each sum is cut into chunks of kChunk terms; one thread adds one chunk (8
+// instead of 16 terms: 303 -> 118 us of dependent additions).
 // Window w's chunks are part[w ncw + u]: u < nc0 for sum 0, then nc1 chunks
 // for each Q_k in order of k.
-constexpr uint32_t kChunk = 16;
+constexpr uint32_t kChunk = 8;
 
 struct ChunkCounts {
   uint32_t nc0, nc1, ncw;
@@ -432,31 +525,20 @@ __global__ void __launch_bounds__(kPointThreads)
   }
 }
 
-// One block per (window, sum): the sum's chunks, then a tree in shared memory.
-// sums[w (1 + lg S) + j].
-constexpr int kReduceThreads = 128;
-
-__global__ void __launch_bounds__(kReduceThreads)
+// One block per (window, sum): the sum's chunks.  sums[w (1 + lg S) + j].
+__global__ void __launch_bounds__(kPointThreads)
     k_msm_bitreduce(const g1x *__restrict__ part, MsmPlan p, g1x *__restrict__ sums) {
-  __shared__ g1x red[kReduceThreads];
+  __shared__ g1x red[kPointThreads];
   const ChunkCounts cc = chunk_counts(p);
   const uint32_t L = 1 + p.lgS;
   const uint32_t w = blockIdx.x / L, j = blockIdx.x - w * L;
   const uint64_t first = (uint64_t)w * cc.ncw + (j == 0 ? 0 : cc.nc0 + (j - 1) * cc.nc1);
-  const uint32_t cnt = j == 0 ? cc.nc0 : cc.nc1;
-  g1x acc = g1x_inf();
-  for (uint32_t i = threadIdx.x; i < cnt; i += kReduceThreads) acc = g1x_add(acc, part[first + i]);
-  red[threadIdx.x] = acc;
-  __syncthreads();
-  for (uint32_t h = kReduceThreads / 2; h > 0; h >>= 1) {
-    if (threadIdx.x < h) red[threadIdx.x] = g1x_add(red[threadIdx.x], red[threadIdx.x + h]);
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) sums[blockIdx.x] = red[0];
+  const g1x sum = block_sum(0, j == 0 ? cc.nc0 : cc.nc1, red, [&](uint32_t i) { return part[first + i]; });
+  if (threadIdx.x == 0) sums[blockIdx.x] = sum;
 }
 
-// ---- final Horner chain in one warp.  Every lane holds the same point; the
-// independent multiplies of a doubling (3 dependent levels instead of 9
+// ---- Horner chains in one warp.  They are bound by the latency of dependent
+// multiplies, so the independent ones of a doubling (3 levels instead of 9
 // multiplies) or of an addition (4 levels instead of 14) run on different
 // lanes and are exchanged by shuffles.
 __device__ __forceinline__ fq shfl_fq(const fq &a, int src) {
@@ -465,30 +547,50 @@ __device__ __forceinline__ fq shfl_fq(const fq &a, int src) {
   for (int i = 0; i < 12; ++i) r.v[i] = __shfl_sync(0xffffffffu, a.v[i], src);
   return r;
 }
+__device__ __forceinline__ fq sel_fq(bool c, const fq &a, const fq &b) {
+  fq r;
+#pragma unroll
+  for (int i = 0; i < 12; ++i) r.v[i] = c ? a.v[i] : b.v[i];
+  return r;
+}
 
-__device__ g1x dbl_warp(const g1x &p) {
-  if (g1x_is_inf(p) || fq_is_zero(p.y)) return g1x_inf();
+// 2^n p for a point that every lane holds.  During the chain the coordinates
+// live apart, Y in lane 0, X in lane 1, ZZ and ZZZ in lane 3, so a level of
+// multiplies needs one exchange of 12 words, each lane fetching the one operand
+// it lacks (dbl-2008-s-1; ZZ = 0 and Y = 0 need no test: both give ZZ = 0).
+// The multiplies are inlined: the loop is the kernel.  200003 points (247
+// doublings): the final chain took 1.0 ms when every lane held the whole point
+// and each product was broadcast, 0.88 ms so.
+__device__ g1x dbl_chain(const g1x &p, uint32_t n) {
   const int lane = threadIdx.x & 31;
-  const fq u = fq_dbl(p.y);
-  // v = u^2 (lane 0), x2 = x^2 (lane 1): squares on every lane
-  fq a = lane == 0 ? u : p.x;
-  fq r = fq_sqr(a);
-  const fq v = shfl_fq(r, 0), x2 = shfl_fq(r, 1);
-  const fq m = fq_add(fq_dbl(x2), x2);
-  // w = u v (0), s = x v (1), m^2 (2), zz' = v zz (3)
-  a = lane == 0 ? u : lane == 1 ? p.x : lane == 2 ? m : v;
-  fq b = lane == 0 ? v : lane == 1 ? v : lane == 2 ? m : p.zz;
-  r = fq_mul(a, b);
-  const fq w = shfl_fq(r, 0), s = shfl_fq(r, 1), m2 = shfl_fq(r, 2), zz = shfl_fq(r, 3);
+  const int src1 = lane == 2 ? 1 : 0;
+  const int src2 = lane == 1 ? 2 : lane == 2 ? 1 : 0;
+  fq P = sel_fq(lane == 0, p.y, sel_fq(lane == 1, p.x, p.zz)), Z = p.zzz;
+#pragma unroll 1
+  for (uint32_t k = 0; k < n; ++k) {
+    // u = 2Y (0), X (1), ZZ (3); squares V = u^2 (0), X^2 (1)
+    const fq u = sel_fq(lane == 0, fq_dbl(P), P);
+    fq r = fq_sqr_cells(u);
+    fq g = shfl_fq(r, src1);  // V (0, 1, 3), X^2 (2)
+    const fq m = fq_add(fq_dbl(g), g);  // M = 3 X^2 (2)
+    // W = u V (0), S = X V (1), M^2 (2), ZZ' = ZZ V (3)
+    const fq r2 = fq_mul_cells(sel_fq(lane == 2, m, u), sel_fq(lane == 2, m, g));
+    g = shfl_fq(r2, src2);  // M^2 (1), S (2), W (3)
+    const fq s = sel_fq(lane == 2, g, r2), mm = sel_fq(lane == 2, r2, g);
+    const fq x = fq_sub(mm, fq_dbl(s));  // X' (1, 2)
+    // W Y (0), M (S - X') (2), ZZZ' = W ZZZ (3)
+    const fq a = sel_fq(lane == 0, r2, sel_fq(lane == 2, m, g));
+    const fq b = sel_fq(lane == 0, P, sel_fq(lane == 2, fq_sub(s, x), Z));
+    r = fq_mul_cells(a, b);
+    g = shfl_fq(r, 2);
+    P = sel_fq(lane == 0, fq_sub(g, r), sel_fq(lane == 1, x, r2));
+    Z = r;
+  }
   g1x o;
-  o.x = fq_sub(m2, fq_dbl(s));
-  // zzz' = w zzz (0), m (s - x') (1), w y (2)
-  a = lane == 1 ? m : w;
-  b = lane == 0 ? p.zzz : lane == 1 ? fq_sub(s, o.x) : p.y;
-  r = fq_mul(a, b);
-  o.zzz = shfl_fq(r, 0);
-  o.y = fq_sub(shfl_fq(r, 1), shfl_fq(r, 2));
-  o.zz = zz;
+  o.y = shfl_fq(P, 0);
+  o.x = shfl_fq(P, 1);
+  o.zz = shfl_fq(P, 3);
+  o.zzz = shfl_fq(Z, 3);
   return o;
 }
 
@@ -505,7 +607,7 @@ __device__ g1x add_warp(const g1x &p, const g1x &q) {
   const fq u1 = shfl_fq(r, 0), u2 = shfl_fq(r, 1), s1 = shfl_fq(r, 2), s2 = shfl_fq(r, 3);
   const fq zz12 = shfl_fq(r, 4), zzz12 = shfl_fq(r, 5);
   const fq P = fq_sub(u2, u1), R = fq_sub(s2, s1);
-  if (fq_is_zero(P)) return fq_is_zero(R) ? dbl_warp(p) : g1x_inf();
+  if (fq_is_zero(P)) return fq_is_zero(R) ? dbl_chain(p, 1) : g1x_inf();
   // P^2 (0), R^2 (1)
   a = lane == 0 ? P : R;
   r = fq_sqr(a);
@@ -532,9 +634,12 @@ __global__ void __launch_bounds__(32) k_msm_wincombine(const g1x *__restrict__ s
   const uint32_t w = blockIdx.x;
   const g1x *q = sums + (uint64_t)w * (1 + p.lgS);  // q[0] = sum T, q[1 + k] = Q_k
   g1x acc = p.lgS ? q[p.lgS] : g1x_inf();
-  for (int k = (int)p.lgS - 2; k >= 0; --k) acc = add_warp(dbl_warp(acc), q[1 + k]);
-  for (uint32_t i = 0; i < p.lgG; ++i) acc = dbl_warp(acc);
-  acc = add_warp(acc, q[0]);
+#pragma unroll 1
+  for (int k = (int)p.lgS - 2; k >= -1; --k) {
+    // Q_k after one doubling, then (k = -1) sum_s T_s after lg G
+    acc = dbl_chain(acc, k >= 0 ? 1 : p.lgG);
+    acc = add_warp(acc, q[1 + k]);
+  }
   if (threadIdx.x == 0) win[w] = acc;
 }
 
@@ -543,8 +648,9 @@ __global__ void __launch_bounds__(32) k_msm_wincombine(const g1x *__restrict__ s
 __global__ void __launch_bounds__(32) k_msm_final(const g1x *__restrict__ win, MsmPlan p,
                                                   fq *__restrict__ out) {
   g1x acc = win[p.nsets - 1];
+#pragma unroll 1
   for (int w = (int)p.nsets - 2; w >= 0; --w) {
-    for (uint32_t k = 0; k < p.c; ++k) acc = dbl_warp(acc);
+    acc = dbl_chain(acc, p.c);
     acc = add_warp(acc, win[w]);
   }
   if (threadIdx.x != 0) return;
@@ -556,38 +662,45 @@ __global__ void __launch_bounds__(32) k_msm_final(const g1x *__restrict__ win, M
 }
 
 struct MsmLayout {
-  size_t digits, counts, offsets, cursor, list, groups, goff, next[2], noff[2], part[2], buckets,
-      seg_t, seg_r, chunks, sums, win, tiles, total;
-  uint64_t part_cap;  // partial sums one level can leave
-  uint32_t levels;    // group levels: K^levels >= the largest bucket
+  size_t digits, counts, n_items, offsets, cursor, list, part, items, multi, chunk_sum, buckets, seg_t,
+      seg_r, chunks, sums, win, tiles, total;
+  uint32_t K;        // entries per run
+  uint32_t runs;     // ceil(W n / K)
+  uint32_t few;      // partial sums of a bucket that one thread joins
 };
 
+// Entries per run: as many runs as threads are resident at once (3 blocks of 128
+// per SM), or a multiple, so that all waves are full.  Fixed-base 2^20 points
+// (17.8 M entries): 7.85 ms as one wave of 306 entries, 7.33 / 6.98 / 7.05 / 7.03
+// with runs of at most 128 / 64 / 48 / 32: the SMs do not keep step, and shorter
+// waves even that out.  4 blocks per SM (128 registers, spills): no faster.
+// Runs shorter than kRunMin cost more partial sums and workspace than they save.
 MsmLayout msm_layout(uint64_t n, const MsmPlan &p) {
   MsmLayout L{};
   auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
   const uint64_t nb = (uint64_t)p.nsets * p.B;
   const uint64_t entries = (uint64_t)p.W * n;
-  // a bucket of m > K values leaves ceil(m / K) <= 2 m / K partial sums
-  L.part_cap = 2 * entries / kGroup + 1;
-  // a bucket holds at most one entry per point and window: n with a bucket
-  // set per window, W n when all windows share one
-  const uint64_t largest = p.nsets > 1 ? n : entries;
-  L.levels = 1;
-  for (uint64_t span = kGroup; span < largest; span *= kGroup) ++L.levels;
+  const uint64_t resident = (uint64_t)device_sm_count() * kAccumulateBlocks * kPointThreads;
+  const uint64_t waves = (entries + resident * kRunMax - 1) / (resident * kRunMax);
+  const uint64_t K = (entries + resident * waves - 1) / (resident * waves);
+  L.K = (uint32_t)(K < kRunMin ? kRunMin : K);
+  L.runs = (uint32_t)((entries + L.K - 1) / L.K);
+  const uint64_t mean = entries / (nb * L.K) + 1;  // partial sums of an average bucket
+  L.few = (uint32_t)(2 * mean > kJoinMin ? 2 * mean : kJoinMin);
+  // each run leaves at most two partial sums, and a listed bucket has more than
+  // kJoinMin of them: at most 2 runs / 9 buckets, plus one item per full chunk
+  const uint64_t items = L.runs / 4 + 64, multi = 2 * (uint64_t)L.runs / kJoinChunk + 1;
   size_t o = 0;
   L.digits = o, o += up(entries * 4);
-  L.counts = o, o += up(nb * 4);
+  L.counts = o, o += nb * 4;
+  L.n_items = o, o = up(o + 8);  // cleared with the counts
   L.offsets = o, o += up((nb + 1) * 4);
   L.cursor = o, o += up(nb * 4);
   L.list = o, o += up(entries * 4);
-  L.groups = o, o += up(nb * 4);
-  L.goff = o, o += up((nb + 1) * 4);
-  for (int k = 0; k < 2; ++k) {
-    L.next[k] = o, o += up(nb * 4);
-    L.noff[k] = o, o += up((nb + 1) * 4);
-  }
-  L.part[0] = o, o += up(L.part_cap * sizeof(g1x));
-  L.part[1] = o, o += up(L.part_cap * sizeof(g1x));
+  L.part = o, o += up(2 * (size_t)L.runs * sizeof(g1x));
+  L.items = o, o += up(items * sizeof(uint2));
+  L.multi = o, o += up(multi * sizeof(uint2));
+  L.chunk_sum = o, o += up(items * sizeof(g1x));
   L.buckets = o, o += up(nb * sizeof(g1x));
   L.seg_t = o, o += up((size_t)p.nsets * p.S * sizeof(g1x));
   L.seg_r = o, o += up((size_t)p.nsets * p.S * sizeof(g1x));
@@ -680,14 +793,15 @@ int msm_run(const g1a *points, const uint32_t *scalars, uint64_t n, const MsmPla
   auto u32 = [&](size_t off) { return reinterpret_cast<uint32_t *>(ws + off); };
   auto pts = [&](size_t off) { return reinterpret_cast<g1x *>(ws + off); };
   uint32_t *digits = u32(L.digits), *counts = u32(L.counts), *offsets = u32(L.offsets);
-  uint32_t *cursor = u32(L.cursor), *list = u32(L.list), *groups = u32(L.groups);
-  uint32_t *goff = u32(L.goff), *tiles = u32(L.tiles);
+  uint32_t *cursor = u32(L.cursor), *list = u32(L.list), *n_items = u32(L.n_items);
+  uint32_t *tiles = u32(L.tiles);
+  uint2 *items = reinterpret_cast<uint2 *>(ws + L.items), *multi = reinterpret_cast<uint2 *>(ws + L.multi);
   g1x *buckets = pts(L.buckets), *seg_t = pts(L.seg_t), *seg_r = pts(L.seg_r), *win = pts(L.win);
-  g1x *chunks = pts(L.chunks), *sums = pts(L.sums);
+  g1x *chunks = pts(L.chunks), *sums = pts(L.sums), *part = pts(L.part), *chunk_sum = pts(L.chunk_sum);
   const uint64_t nb = (uint64_t)p.nsets * p.B;
 
   // 1-3: signed digits, bucket sizes, counting sort of (point, sign) by bucket
-  PP_CUDA_TRY(cudaMemsetAsync(counts, 0, nb * 4, s));
+  PP_CUDA_TRY(cudaMemsetAsync(counts, 0, nb * 4 + 8, s));  // and n_items
   k_msm_digits<<<grid_for(n, 256), 256, 0, s>>>(scalars, n, p, digits, counts);
   PP_COUNT_LAUNCH();
   PP_LAUNCH_CHECK();
@@ -696,27 +810,24 @@ int msm_run(const g1a *points, const uint32_t *scalars, uint64_t n, const MsmPla
   PP_COUNT_LAUNCH();
   PP_LAUNCH_CHECK();
 
-  // 4: bucket sums, at most K values per thread, over L.levels levels
+  // 4: bucket sums over equal runs of the list, then the shared buckets
   PP_CUDA_TRY(cudaMemsetAsync(buckets, 0, nb * sizeof(g1x), s));  // all zero = infinity
-  const uint32_t *m = counts, *off = offsets;
-  const g1x *part_in = nullptr;
-  for (uint32_t lv = 0; lv < L.levels; ++lv) {
-    uint32_t *next = u32(L.next[lv & 1]), *noff = u32(L.noff[lv & 1]);
-    g1x *part_out = pts(L.part[lv & 1]);
-    k_msm_groups<<<grid_for(nb, 256), 256, 0, s>>>(m, nb, groups, next);
-    PP_COUNT_LAUNCH();
-    PP_LAUNCH_CHECK();
-    if ((st = scan_u32(groups, nb, goff, nullptr, tiles, s))) return st;
-    if ((st = scan_u32(next, nb, noff, nullptr, tiles, s))) return st;
-    k_msm_level<<<grid_for((uint64_t)p.W * n / 4 + nb, kPointThreads), kPointThreads, 0, s>>>(
-        points, lv == 0 ? list : nullptr, part_in, m, off, goff, noff,
-        (uint32_t)nb, part_out, buckets);
-    PP_COUNT_LAUNCH();
-    PP_LAUNCH_CHECK();
-    m = next;
-    off = noff;
-    part_in = part_out;
-  }
+  k_msm_accumulate<<<grid_for(L.runs, kPointThreads), kPointThreads, 0, s>>>(
+      points, list, offsets, (uint32_t)nb, L.K, part, buckets);
+  PP_COUNT_LAUNCH();
+  PP_LAUNCH_CHECK();
+  k_msm_spans<<<grid_for(nb, 256), 256, 0, s>>>(offsets, (uint32_t)nb, L.K, L.few, items, multi, n_items);
+  PP_COUNT_LAUNCH();
+  PP_LAUNCH_CHECK();
+  const unsigned small_blocks = grid_for(nb, kPointThreads), big_blocks = 2 * (unsigned)device_sm_count();
+  k_msm_join<<<small_blocks + big_blocks, kPointThreads, 0, s>>>(
+      part, offsets, (uint32_t)nb, L.K, L.few, small_blocks, items, n_items, chunk_sum, buckets);
+  PP_COUNT_LAUNCH();
+  PP_LAUNCH_CHECK();
+  k_msm_join_chunks<<<(unsigned)device_sm_count(), kPointThreads, 0, s>>>(offsets, L.K, multi, n_items,
+                                                                         chunk_sum, buckets);
+  PP_COUNT_LAUNCH();
+  PP_LAUNCH_CHECK();
 
   // 5-7: weighted bucket sums per bucket set, sets combined, affine result
   k_msm_segments<<<grid_for((uint64_t)p.nsets * p.S, kPointThreads), kPointThreads, 0, s>>>(
@@ -727,7 +838,7 @@ int msm_run(const g1a *points, const uint32_t *scalars, uint64_t n, const MsmPla
                   0, s>>>(seg_t, seg_r, p, chunks);
   PP_COUNT_LAUNCH();
   PP_LAUNCH_CHECK();
-  k_msm_bitreduce<<<p.nsets * (1 + p.lgS), kReduceThreads, 0, s>>>(chunks, p, sums);
+  k_msm_bitreduce<<<p.nsets * (1 + p.lgS), kPointThreads, 0, s>>>(chunks, p, sums);
   PP_COUNT_LAUNCH();
   PP_LAUNCH_CHECK();
   k_msm_wincombine<<<p.nsets, 32, 0, s>>>(sums, p, win);
