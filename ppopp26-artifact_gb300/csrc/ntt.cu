@@ -1181,7 +1181,7 @@ int ntt_run(const fr *d_in, fr *d_out, uint32_t lg_m, bool inverse, const NttInp
   std::vector<uint64_t> tiles;
   int st = ntt_describe(d_in, d_out, work, lg_m, inverse, in, passes, tiles, small);
   if (st) return st;
-  if (small || lg_m <= kSmallOnePass) {
+  if (small || (passes.size() == 1 && lg_m <= kSmallOnePass)) {
     for (size_t j = 0; j < passes.size(); ++j) {
       const uint32_t R = 1u << passes[j].lgR;
       cudaLaunchConfig_t cfg = {};

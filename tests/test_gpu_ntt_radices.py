@@ -43,3 +43,15 @@ def test_radices(pp, cuda, expected, split):
             assert (got == want["lde", lam]).all(), lam
     finally:
         pp.ppfr.set_split(LG, [9, 9])
+
+
+@pytest.mark.parametrize("lg,split", [(6, (3, 3)), (7, (4, 3)), (8, (3, 5)), (9, (9,)), (10, (5, 5)), (11, (4, 7))])
+def test_splits_of_small_sizes(pp, O, cuda, lg, split):
+    """Single calls below 2^9 points follow a split that is set for them."""
+    x = pp.random_fr(1 << lg, 5)
+    try:
+        pp.ppfr.set_split(lg, split)
+        for inverse in (False, True):
+            assert O.first_diff(host(pp.ntt(x, inverse)), O.ntt(host(x), inverse=inverse)) == -1
+    finally:
+        pp.ppfr.set_split(lg)
