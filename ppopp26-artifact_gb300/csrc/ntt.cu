@@ -775,8 +775,10 @@ struct PlanKey {
   bool inv;
   bool small;  // the latency form for single calls of 2^9 .. 2^17 points
   bool split;  // split layer tables (host-pass transforms)
+  bool host;   // host endpoints that the size's own split serves badly
   bool operator<(const PlanKey &o) const {
-    return std::tie(dev, lgN, inv, small, split) < std::tie(o.dev, o.lgN, o.inv, o.small, o.split);
+    return std::tie(dev, lgN, inv, small, split, host) <
+           std::tie(o.dev, o.lgN, o.inv, o.small, o.split, o.host);
   }
 };
 
@@ -805,6 +807,16 @@ std::vector<uint32_t> default_split(uint32_t lgN) {
   const uint32_t P = (lgN + 8) / 9;
   for (uint32_t p = 0; p < P; ++p) b.push_back(lgN / P + (p < lgN % P ? 1 : 0));
   return b;
+}
+
+// The split for host endpoints (host_split_differs): the passes that touch host
+// memory are bound by the link and do their multiplies beside it, so they take
+// as many bits as whole 128-byte lines allow (9) and the middle pass the rest.
+// 2^22 points: 9, 4, 9 bits 1626 us, 8, 7, 7 bits 1696 us.
+std::vector<uint32_t> host_split(uint32_t lgN) {
+  if (lgN < 19 || lgN > 27) return default_split(lgN);
+  const uint32_t mid = lgN > 21 ? lgN - 18 : 3, ends = lgN - mid;
+  return {ends - ends / 2, mid, ends / 2};
 }
 
 int build_windows(const fr &base, fr **d_win) {
@@ -900,15 +912,18 @@ int get_round(int dev, bool inv, const uint4 **out) {
 // split: layer twiddles as two tables of about 2^(lgRS / 2) entries each
 // (w^i and w^(i 2^h)) instead of one of 2^lgRS, for transforms whose data
 // never sits in device memory
-int get_plan(int dev, uint32_t lgN, bool inv, Plan **out, bool small = false, bool split = false) {
-  PlanKey key{dev, lgN, inv, small, split};
+// host: host_split instead of the size's own split (host_split_differs)
+int get_plan(int dev, uint32_t lgN, bool inv, Plan **out, bool small = false, bool split = false,
+             bool host = false) {
+  PlanKey key{dev, lgN, inv, small, split, host};
   auto it = g_plans.find(key);
   if (it != g_plans.end()) {
     *out = it->second;
     return PP_OK;
   }
   auto ov = g_split_override.find(lgN);
-  std::vector<uint32_t> bits = ov != g_split_override.end() ? ov->second : default_split(lgN);
+  std::vector<uint32_t> bits =
+      host ? host_split(lgN) : ov != g_split_override.end() ? ov->second : default_split(lgN);
   if (small) bits = {lgN - lgN / 2, lgN / 2};
   Plan *p = new Plan();
   p->lgN = lgN;
@@ -961,6 +976,20 @@ int get_plan(int dev, uint32_t lgN, bool inv, Plan **out, bool small = false, bo
   g_plans[key] = p;
   *out = p;
   return PP_OK;
+}
+
+// Whether a transform with host endpoints should leave the size's own split:
+// passes of 10 or 11 bits take one or two columns per tile, so the first
+// pass's reads and the last one's writes are 32- or 64-byte pieces of host
+// memory.  host_split's passes move whole 128-byte lines (2^22 points: 2042 us
+// with 11 + 11 bits, 1626 with 9 + 4 + 9; the link alone takes 640 in and 700
+// out).  Not while the stream is being captured
+// unless its tables exist: building them allocates.
+bool host_split_differs(uint32_t lgN, const NttInputDesc &in) {
+  if (!in.in_host && !in.out_host) return false;
+  const auto ov = g_split_override.find(lgN);
+  if (ov == g_split_override.end() || ov->second.size() < 2) return false;
+  return (in.in_host && ov->second.front() > 9) || (in.out_host && ov->second.back() > 9);
 }
 
 bool g_attr_set[64] = {false};
@@ -1052,19 +1081,19 @@ void ntt_release_tables() {
 namespace {
 int describe_passes(const fr *d_in, fr *d_out, fr *work, uint32_t lg_m, bool inverse,
                     const NttInputDesc &in, std::vector<PassArgs> &passes,
-                    std::vector<uint64_t> &tiles, bool small, bool split);
+                    std::vector<uint64_t> &tiles, bool small, bool split, bool host);
 }  // namespace
 
 int ntt_describe(const fr *d_in, fr *d_out, fr *work, uint32_t lg_m, bool inverse,
                  const NttInputDesc &in, std::vector<PassArgs> &passes,
-                 std::vector<uint64_t> &tiles, bool small) {
-  return describe_passes(d_in, d_out, work, lg_m, inverse, in, passes, tiles, small, false);
+                 std::vector<uint64_t> &tiles, bool small, bool host) {
+  return describe_passes(d_in, d_out, work, lg_m, inverse, in, passes, tiles, small, false, host);
 }
 
 namespace {
 int describe_passes(const fr *d_in, fr *d_out, fr *work, uint32_t lg_m, bool inverse,
                     const NttInputDesc &in, std::vector<PassArgs> &passes,
-                    std::vector<uint64_t> &tiles, bool small, bool split) {
+                    std::vector<uint64_t> &tiles, bool small, bool split, bool host) {
   if (lg_m > PP_MAX_LG_N || lg_m < 3) {
     set_error("batched transform of 2^%u points: supported sizes are 2^3 .. 2^%d", lg_m, PP_MAX_LG_N);
     return PP_E_UNSUPPORTED;
@@ -1075,7 +1104,7 @@ int describe_passes(const fr *d_in, fr *d_out, fr *work, uint32_t lg_m, bool inv
   Plan *plan = nullptr;
   {
     std::lock_guard<std::mutex> lk(g_mu);
-    int st = get_plan(dev, lg_m, inverse, &plan, small, split);
+    int st = get_plan(dev, lg_m, inverse, &plan, small, split, host);
     if (st) return st;
     if (dev < 64 && !g_attr_set[dev]) {
       PP_CUDA_TRY(cudaFuncSetAttribute(k_ntt_pass<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1169,6 +1198,17 @@ int ntt_run(const fr *d_in, fr *d_out, uint32_t lg_m, bool inverse, const NttInp
     return PP_OK;
   }
   const bool small = ntt_small_form(lg_m);
+  bool host = false;
+  if (!small && (in.in_host || in.out_host)) {
+    int dev = 0;
+    PP_CUDA_TRY(cudaGetDevice(&dev));
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    PP_CUDA_TRY(cudaStreamIsCapturing(stream, &cap));
+    std::lock_guard<std::mutex> lk(g_mu);
+    host = host_split_differs(lg_m, in) &&
+           (cap == cudaStreamCaptureStatusNone ||
+            g_plans.count(PlanKey{dev, lg_m, inverse, false, false, true}));
+  }
   uint32_t bits[4], np = 2;
   if (!small) ntt_get_split(lg_m, bits, &np);
   fr *work = nullptr;
@@ -1179,7 +1219,7 @@ int ntt_run(const fr *d_in, fr *d_out, uint32_t lg_m, bool inverse, const NttInp
   }
   std::vector<PassArgs> passes;
   std::vector<uint64_t> tiles;
-  int st = ntt_describe(d_in, d_out, work, lg_m, inverse, in, passes, tiles, small);
+  int st = ntt_describe(d_in, d_out, work, lg_m, inverse, in, passes, tiles, small, host);
   if (st) return st;
   if (small || (passes.size() == 1 && lg_m <= kSmallOnePass)) {
     for (size_t j = 0; j < passes.size(); ++j) {
@@ -1257,7 +1297,7 @@ int ntt_run_host_passes(const fr *h_in, fr *h_out, fr *h_scratch, uint32_t lg_m,
   }
   std::vector<PassArgs> passes;
   std::vector<uint64_t> tiles;
-  int st = describe_passes(h_in, h_out, h_scratch, lg_m, inverse, in, passes, tiles, false, true);
+  int st = describe_passes(h_in, h_out, h_scratch, lg_m, inverse, in, passes, tiles, false, true, false);
   if (st) return st;
   // pass j reads X_j and writes X_(j+1): X_0 = h_in, X_P = h_out, and the
   // intermediates alternate so that X_(P-1) = h_scratch

@@ -87,10 +87,11 @@ int ntt_run(const fr *d_in, fr *d_out, uint32_t lg_m, bool inverse, const NttInp
 // Per-pass descriptors (and tile counts) of one transform whose passes use
 // `work` (2^lg_m elements) between them; for batch plans.  lg_m >= 3.
 // small = the latency form of single calls (ntt_small_form); batch plans use
-// the throughput form.
+// the throughput form.  host = the split for host endpoints where the size's
+// own serves them badly.
 int ntt_describe(const fr *d_in, fr *d_out, fr *work, uint32_t lg_m, bool inverse,
                  const NttInputDesc &in, std::vector<PassArgs> &passes,
-                 std::vector<uint64_t> &tiles, bool small = false);
+                 std::vector<uint64_t> &tiles, bool small = false, bool host = false);
 
 // Single calls run the latency form (k_ntt_small_pass, one column per block) in
 // one pass up to 2^8 points and in two up to 2^17: those sizes are bound by

@@ -55,3 +55,22 @@ def test_splits_of_small_sizes(pp, O, cuda, lg, split):
             assert O.first_diff(host(pp.ntt(x, inverse)), O.ntt(host(x), inverse=inverse)) == -1
     finally:
         pp.ppfr.set_split(lg)
+
+
+@pytest.mark.parametrize("split", [(11, 7), (7, 11), (8, 10), (9, 9)])
+def test_host_endpoints_under_any_split(pp, cuda, expected, split):
+    """Host endpoints leave splits with short row segments for the default one."""
+    x, want = expected
+    hx, ho = pp.ppfr.empty_pinned(1 << LG), pp.ppfr.empty_pinned(1 << LG)
+    hx.copy_(x)
+    try:
+        pp.ppfr.set_split(LG, split)
+        for key, inverse in (("ntt", False), ("intt", True)):
+            pp.ppfr.ntt_host(hx, inverse, out=ho)
+            cuda.cuda.synchronize()
+            assert (ho == want[key].cpu()).all()
+        lo = pp.ppfr.lde_host(hx[:1 << (LG - 2)].contiguous().pin_memory(), 2, pp.LDE_COEFFS)
+        cuda.cuda.synchronize()
+        assert (lo == want["lde", 2].cpu()).all()
+    finally:
+        pp.ppfr.set_split(LG, [9, 9])
