@@ -309,6 +309,27 @@ constexpr uint32_t kRunMin = 10, kRunMax = 64;
 constexpr uint32_t kJoinMin = 8;           // partial sums one thread adds up
 constexpr uint32_t kJoinChunk = 1024;      // partial sums one block adds up
 
+// Entries per run for a list of that many: as many runs as threads are resident
+// at once (3 blocks of 128 per SM), or a multiple, so that all waves are full.
+// Fixed-base 2^20 points (17.8 M entries): 7.85 ms as one wave of 306 entries,
+// 7.33 / 6.98 / 7.05 / 7.03 with runs of at most 128 / 64 / 48 / 32: the SMs do
+// not keep step, and shorter waves even that out.  4 blocks per SM (128
+// registers, spills): no faster.  Runs shorter than kRunMin cost more partial
+// sums and workspace than they save.  The kernels take it from the list's real
+// length (zero digits have no entry): half of 2^18 scalars zero and the rest one
+// took 1638 us with runs sized for a full list.
+__host__ __device__ __forceinline__ uint32_t run_length(uint64_t entries, uint32_t resident) {
+  const uint64_t span = (uint64_t)resident * kRunMax;
+  const uint64_t waves = entries ? (entries + span - 1) / span : 1;
+  const uint64_t K = (entries + resident * waves - 1) / (resident * waves);
+  return (uint32_t)(K < kRunMin ? kRunMin : K);
+}
+// partial sums of a bucket that one thread joins: twice an average bucket's
+__device__ __forceinline__ uint32_t join_few(uint32_t entries, uint32_t nb, uint32_t K) {
+  const uint32_t twice = 2 * (entries / ((uint64_t)nb * K) + 1);
+  return twice > kJoinMin ? twice : kJoinMin;
+}
+
 // the bucket whose range [off[b], off[b+1]) holds entry t
 __device__ __forceinline__ uint32_t bucket_of(const uint32_t *off, uint32_t nb, uint32_t t) {
   uint32_t lo = 0, hi = nb;  // off[lo] <= t < off[hi]
@@ -332,9 +353,9 @@ __device__ __forceinline__ uint32_t bucket_of(const uint32_t *off, uint32_t nb, 
 // part[2 t + 1].  Bound by the multiply pipe.
 __global__ void __launch_bounds__(kPointThreads, kAccumulateBlocks)
     k_msm_accumulate(const g1a *__restrict__ points, const uint32_t *__restrict__ list,
-                     const uint32_t *__restrict__ off, uint32_t nb, uint32_t K,
+                     const uint32_t *__restrict__ off, uint32_t nb, uint32_t resident,
                      g1x *__restrict__ part, g1x *__restrict__ buckets) {
-  const uint32_t total = off[nb];
+  const uint32_t total = off[nb], K = run_length(total, resident);
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   const uint64_t lo64 = (uint64_t)t * K;
   if (lo64 >= total) return;
@@ -375,16 +396,16 @@ __device__ __forceinline__ uint64_t partial_index(const BucketSpan &s, uint32_t 
   return 2 * (uint64_t)(s.first + j) + (j == 0 ? 1 : 0);
 }
 
-// Lists the buckets of more than `few` partial sums: items[i] = (bucket, chunk)
+// Lists the buckets of more partial sums than one thread joins: items[i] = (bucket, chunk)
 // for every kJoinChunk of them, multi[] = (bucket, first item) for buckets of
 // several chunks; counts in n_items[0] and n_items[1].
-__global__ void k_msm_spans(const uint32_t *__restrict__ off, uint32_t nb, uint32_t K, uint32_t few,
-                            uint2 *__restrict__ items, uint2 *__restrict__ multi,
+__global__ void k_msm_spans(const uint32_t *__restrict__ off, uint32_t nb, uint32_t resident, uint2 *__restrict__ items, uint2 *__restrict__ multi,
                             uint32_t *__restrict__ n_items) {
   const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= nb) return;
+  const uint32_t K = run_length(off[nb], resident);
   const BucketSpan sp = bucket_span(off, b, K);
-  if (sp.m <= few) return;
+  if (sp.m <= join_few(off[nb], nb, K)) return;
   const uint32_t chunks = (sp.m + kJoinChunk - 1) / kJoinChunk;
   const uint32_t first = atomicAdd(n_items, chunks);
   for (uint32_t c = 0; c < chunks; ++c) items[first + c] = make_uint2(b, c);
@@ -412,12 +433,14 @@ __device__ __forceinline__ g1x block_sum(uint32_t lo, uint32_t hi, g1x *red, F v
 // thread, the others (128 threads each) the listed chunks of the larger ones,
 // whose sums go to buckets[] or, with several chunks, to chunk_sum[item].
 __global__ void __launch_bounds__(kPointThreads)
-    k_msm_join(const g1x *__restrict__ part, const uint32_t *__restrict__ off, uint32_t nb, uint32_t K,
-               uint32_t few, uint32_t small_blocks, const uint2 *__restrict__ items,
+    k_msm_join(const g1x *__restrict__ part, const uint32_t *__restrict__ off, uint32_t nb,
+               uint32_t resident, uint32_t small_blocks, const uint2 *__restrict__ items,
                const uint32_t *__restrict__ n_items, g1x *__restrict__ chunk_sum,
                g1x *__restrict__ buckets) {
   __shared__ g1x red[kPointThreads];
+  const uint32_t K = run_length(off[nb], resident);
   if (blockIdx.x < small_blocks) {
+    const uint32_t few = join_few(off[nb], nb, K);
     const uint32_t b = blockIdx.x * kPointThreads + threadIdx.x;
     if (b >= nb) return;
     const BucketSpan sp = bucket_span(off, b, K);
@@ -439,11 +462,12 @@ __global__ void __launch_bounds__(kPointThreads)
 
 // the chunks of the buckets that have several
 __global__ void __launch_bounds__(kPointThreads)
-    k_msm_join_chunks(const uint32_t *__restrict__ off, uint32_t K, const uint2 *__restrict__ multi,
+    k_msm_join_chunks(const uint32_t *__restrict__ off, uint32_t nb, uint32_t resident,
+                      const uint2 *__restrict__ multi,
                       const uint32_t *__restrict__ n_items, const g1x *__restrict__ chunk_sum,
                       g1x *__restrict__ buckets) {
   __shared__ g1x red[kPointThreads];
-  const uint32_t n = n_items[1];
+  const uint32_t n = n_items[1], K = run_length(off[nb], resident);
   for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
     const uint2 mb = multi[i];
     const BucketSpan sp = bucket_span(off, mb.x, K);
@@ -557,11 +581,12 @@ __device__ __forceinline__ fq sel_fq(bool c, const fq &a, const fq &b) {
 // 2^n p for a point that every lane holds.  During the chain the coordinates
 // live apart, Y in lane 0, X in lane 1, ZZ and ZZZ in lane 3, so a level of
 // multiplies needs one exchange of 12 words, each lane fetching the one operand
-// it lacks (dbl-2008-s-1; ZZ = 0 and Y = 0 need no test: both give ZZ = 0).
+// it lacks (dbl-2008-s-1; Y = 0 needs no test: it gives ZZ = 0).
 // The multiplies are inlined: the loop is the kernel.  200003 points (247
 // doublings): the final chain took 1.0 ms when every lane held the whole point
 // and each product was broadcast, 0.88 ms so.
 __device__ g1x dbl_chain(const g1x &p, uint32_t n) {
+  if (g1x_is_inf(p)) return p;  // the upper windows of short scalars are empty
   const int lane = threadIdx.x & 31;
   const int src1 = lane == 2 ? 1 : 0;
   const int src2 = lane == 1 ? 2 : lane == 2 ? 1 : 0;
@@ -664,29 +689,22 @@ __global__ void __launch_bounds__(32) k_msm_final(const g1x *__restrict__ win, M
 struct MsmLayout {
   size_t digits, counts, n_items, offsets, cursor, list, part, items, multi, chunk_sum, buckets, seg_t,
       seg_r, chunks, sums, win, tiles, total;
-  uint32_t K;        // entries per run
-  uint32_t runs;     // ceil(W n / K)
-  uint32_t few;      // partial sums of a bucket that one thread joins
+  uint32_t resident; // threads of k_msm_accumulate resident at once
+  uint32_t runs;     // runs of the list at most
 };
 
-// Entries per run: as many runs as threads are resident at once (3 blocks of 128
-// per SM), or a multiple, so that all waves are full.  Fixed-base 2^20 points
-// (17.8 M entries): 7.85 ms as one wave of 306 entries, 7.33 / 6.98 / 7.05 / 7.03
-// with runs of at most 128 / 64 / 48 / 32: the SMs do not keep step, and shorter
-// waves even that out.  4 blocks per SM (128 registers, spills): no faster.
-// Runs shorter than kRunMin cost more partial sums and workspace than they save.
 MsmLayout msm_layout(uint64_t n, const MsmPlan &p) {
   MsmLayout L{};
   auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
   const uint64_t nb = (uint64_t)p.nsets * p.B;
   const uint64_t entries = (uint64_t)p.W * n;
-  const uint64_t resident = (uint64_t)device_sm_count() * kAccumulateBlocks * kPointThreads;
-  const uint64_t waves = (entries + resident * kRunMax - 1) / (resident * kRunMax);
-  const uint64_t K = (entries + resident * waves - 1) / (resident * waves);
-  L.K = (uint32_t)(K < kRunMin ? kRunMin : K);
-  L.runs = (uint32_t)((entries + L.K - 1) / L.K);
-  const uint64_t mean = entries / (nb * L.K) + 1;  // partial sums of an average bucket
-  L.few = (uint32_t)(2 * mean > kJoinMin ? 2 * mean : kJoinMin);
+  L.resident = (uint32_t)device_sm_count() * kAccumulateBlocks * kPointThreads;
+  // run_length gives at most entries / kRunMin + 1 runs, and at most a full
+  // list's number of waves
+  const uint64_t span = (uint64_t)L.resident * kRunMax;
+  const uint64_t by_waves = (uint64_t)L.resident * ((entries + span - 1) / span);
+  const uint64_t by_min = entries / kRunMin + 1;
+  L.runs = (uint32_t)(by_min < by_waves ? by_min : by_waves);
   // each run leaves at most two partial sums, and a listed bucket has more than
   // kJoinMin of them: at most 2 runs / 9 buckets, plus one item per full chunk
   const uint64_t items = L.runs / 4 + 64, multi = 2 * (uint64_t)L.runs / kJoinChunk + 1;
@@ -813,19 +831,20 @@ int msm_run(const g1a *points, const uint32_t *scalars, uint64_t n, const MsmPla
   // 4: bucket sums over equal runs of the list, then the shared buckets
   PP_CUDA_TRY(cudaMemsetAsync(buckets, 0, nb * sizeof(g1x), s));  // all zero = infinity
   k_msm_accumulate<<<grid_for(L.runs, kPointThreads), kPointThreads, 0, s>>>(
-      points, list, offsets, (uint32_t)nb, L.K, part, buckets);
+      points, list, offsets, (uint32_t)nb, L.resident, part, buckets);
   PP_COUNT_LAUNCH();
   PP_LAUNCH_CHECK();
-  k_msm_spans<<<grid_for(nb, 256), 256, 0, s>>>(offsets, (uint32_t)nb, L.K, L.few, items, multi, n_items);
+  k_msm_spans<<<grid_for(nb, 256), 256, 0, s>>>(offsets, (uint32_t)nb, L.resident, items, multi,
+                                                   n_items);
   PP_COUNT_LAUNCH();
   PP_LAUNCH_CHECK();
   const unsigned small_blocks = grid_for(nb, kPointThreads), big_blocks = 2 * (unsigned)device_sm_count();
   k_msm_join<<<small_blocks + big_blocks, kPointThreads, 0, s>>>(
-      part, offsets, (uint32_t)nb, L.K, L.few, small_blocks, items, n_items, chunk_sum, buckets);
+      part, offsets, (uint32_t)nb, L.resident, small_blocks, items, n_items, chunk_sum, buckets);
   PP_COUNT_LAUNCH();
   PP_LAUNCH_CHECK();
-  k_msm_join_chunks<<<(unsigned)device_sm_count(), kPointThreads, 0, s>>>(offsets, L.K, multi, n_items,
-                                                                         chunk_sum, buckets);
+  k_msm_join_chunks<<<(unsigned)device_sm_count(), kPointThreads, 0, s>>>(
+      offsets, (uint32_t)nb, L.resident, multi, n_items, chunk_sum, buckets);
   PP_COUNT_LAUNCH();
   PP_LAUNCH_CHECK();
 
