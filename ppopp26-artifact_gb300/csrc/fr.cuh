@@ -1236,6 +1236,20 @@ PP_HD fr fr_mul_const4(const fr &a, const fr w[4]) {
   return o;
 }
 
+// The factor that takes a Montgomery-form constant k to part p of fr_mul_const4:
+// fr_mul(k, fr_const4_factor(p)) = k 2^(64 p + 96), plain.  2^96, 2^160, 2^224
+// and 2^288 mod r.
+PP_HD fr fr_const4_factor(uint32_t p) {
+  if (p == 3)
+    return fr{{0xcaaf6b13u, 0x355094eau, 0x69a568efu, 0xf6b10cb3u,
+               0x40cc3869u, 0xe2c926a6u, 0xed269aadu, 0x736a6d3bu}};
+  fr f = fr_zero();
+  f.v[3] = p == 0;
+  f.v[5] = p == 1;
+  f.v[7] = p == 2;
+  return f;
+}
+
 // 2r, least significant limb first
 #define PP_2R0 0x00000002u
 #define PP_2R1 0xfffffffeu

@@ -28,12 +28,9 @@ namespace pp {
 // Blocks per SM each operator's geometry aims for (scan_geom): longer chunks
 // cut the summaries to scan, more blocks hide more latency.  Swept over 1, 2,
 // 3 and 4 on GB300 (us at 2^20 / 2^22 / 2^24): division 2 (77 / 170 / 529;
-// 1: 72 / 171 / 559, 4: 115 / 207 / 546); permutation product 8 at 2^20 / 2^22
-// (424 / 1702; 4: 425 / 1632, 6: 451 / 1721; its local pass runs 2 blocks per
-// SM, so it needs more of them to hide latency).  Evaluation has its own
-// geometry (k_eval_tree).
-constexpr uint32_t kGpBlocksPerSm = 2, kDivBlocksPerSm = 2,
-                   kPermBlocksPerSm = 8;
+// 1: 72 / 171 / 559, 4: 115 / 207 / 546).  Evaluation has its own geometry
+// (k_eval_tree), and so has the permutation product (k_perm_local).
+constexpr uint32_t kGpBlocksPerSm = 2, kDivBlocksPerSm = 2;
 // The grand product's chains grow with n while its block trees do not: us with
 // 2 / 3 / 4 blocks per SM at 2^20 57.4 / 57.4 / 65.6, at 2^22 159.5 / 156.1 /
 // 162.0, at 2^24 563 / 547 / 545.
@@ -227,118 +224,99 @@ __device__ __forceinline__ void warp_power_table17(const fr &x, fr *pw) {
   if (lane <= 16) sts_fr(pw + lane, v);
 }
 
-// inclusive prefix product over a block of 256 threads (commutative);
-// afterwards s[t] holds thread t's inclusive product, which is also returned.
-// A work-efficient up-sweep over the lowest three tree levels leaves the
-// products of the 32 runs of 8; one warp scans those with shuffles (5 steps),
-// and a three-level down-sweep hands the run prefixes back down.  12
+// Exclusive prefix product over a block of 256 threads (commutative): returns
+// the product of the v of the threads before this one; *total receives the
+// product of all.  A work-efficient up-sweep over the lowest three tree levels
+// leaves the products of the 32 runs of 8; one warp scans those with shuffles
+// (5 steps), and a three-level down-sweep hands the run prefixes back down.  11
 // dependent multiplies against 17 for the full up- and down-sweep: the block
 // scan is latency-bound (few threads multiply at each level).
-__device__ __forceinline__ fr shfl_up_fr(const fr &v, int o);
-
-__device__ fr block_prefix_product(fr v, fr *s) {
-  const int t = threadIdx.x;
-  constexpr int n = kScanThreads;
-  static_assert(kScanThreads == 256, "32 runs of 8");
-  sts_fr(s + t, v);
-  __syncthreads();
-  for (int d = 1; d < 8; d <<= 1) {
-    const int idx = (t + 1) * 2 * d - 1;
-    if (idx < n) sts_fr(s + idx, fr_mul(lds_fr(s + idx - d), lds_fr(s + idx)));
-    __syncthreads();
-  }
-  if (t < 32) {
-    fr inc = lds_fr(s + 8 * t + 7);
-    for (int o = 1; o < 32; o <<= 1) {
-      const fr u = shfl_up_fr(inc, o);
-      if (t >= o) inc = fr_mul(u, inc);
-    }
-    const fr ex = shfl_up_fr(inc, 1);
-    sts_fr(s + 8 * t + 7, t ? ex : fr_one());
-  }
-  __syncthreads();
-  for (int d = 4; d >= 1; d >>= 1) {
-    const int idx = (t + 1) * 2 * d - 1;
-    if (idx < n) {
-      const fr left = lds_fr(s + idx - d);
-      sts_fr(s + idx - d, lds_fr(s + idx));
-      sts_fr(s + idx, fr_mul(lds_fr(s + idx), left));
-    }
-    __syncthreads();
-  }
-  const fr incl = fr_mul(lds_fr(s + t), v);
-  __syncthreads();
-  sts_fr(s + t, incl);
-  __syncthreads();
-  return incl;
-}
-
-// Warp-shuffle (Kogge-Stone) forms: each warp scans its 32 values in 5
-// steps, then warp 0 scans the warp totals -- 9 dependent multiplies and 3
-// barriers against 16 of each, for about 2.5 times the multiplies.  They win
-// where latency, not multiply throughput, bounds the block: the permutation
-// product's local pass (2 blocks per SM) and its single-block carry pass
-// (2^20: 0.607 -> 0.588 ms).  Afterwards s[t] holds thread t's inclusive
-// prefix (or suffix) product, which is also returned.
 __device__ __forceinline__ fr shfl_up_fr(const fr &v, int o) {
   fr r;
 #pragma unroll
   for (int i = 0; i < 8; ++i) r.v[i] = __shfl_up_sync(0xffffffffu, v.v[i], o);
   return r;
 }
-__device__ __forceinline__ fr shfl_down_fr(const fr &v, int o) {
-  fr r;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) r.v[i] = __shfl_down_sync(0xffffffffu, v.v[i], o);
-  return r;
-}
 
-__device__ fr warp_block_prefix_product(fr v, fr *s) {
-  const int t = threadIdx.x, lane = t & 31, w = t >> 5, nw = blockDim.x >> 5;
-  for (int o = 1; o < 32; o <<= 1) {
-    const fr u = shfl_up_fr(v, o);
-    if (lane >= o) v = fr_mul(u, v);
-  }
-  if (lane == 31) sts_fr(s + w, v);  // warp totals
-  __syncthreads();
-  if (w == 0) {
-    fr x = lane < nw ? lds_fr(s + lane) : fr_one();
-    for (int o = 1; o < nw; o <<= 1) {
-      const fr u = shfl_up_fr(x, o);
-      if (lane >= o) x = fr_mul(u, x);
-    }
-    if (lane < nw) sts_fr(s + lane, x);  // warps 0 .. lane
-  }
-  __syncthreads();
-  if (w > 0) v = fr_mul(lds_fr(s + w - 1), v);
-  __syncthreads();
+__device__ fr block_exclusive_product(const fr &v, fr *s, fr *total) {
+  const uint32_t t = threadIdx.x;
+  static_assert(kScanThreads == 256, "32 runs of 8");
   sts_fr(s + t, v);
   __syncthreads();
-  return v;
+#pragma unroll 1
+  for (uint32_t d = 1; d < 8; d <<= 1) {
+    const uint32_t idx = (t + 1) * 2 * d - 1;
+    if (idx < 256) sts_fr(s + idx, fr_mul(lds_fr(s + idx - d), lds_fr(s + idx)));
+    __syncthreads();
+  }
+  if (t < 32) {
+    fr inc = lds_fr(s + 8 * t + 7);
+#pragma unroll 1
+    for (int o = 1; o < 32; o <<= 1) {
+      const fr u = shfl_up_fr(inc, o);
+      if ((int)t >= o) inc = fr_mul(u, inc);
+    }
+    const fr ex = shfl_up_fr(inc, 1);
+    sts_fr(s + 8 * t + 7, t ? ex : fr_one());
+    if (t == 31) sts_fr(total, inc);
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (uint32_t d = 4; d >= 1; d >>= 1) {
+    const uint32_t idx = (t + 1) * 2 * d - 1;
+    if (idx < 256) {
+      const fr left = lds_fr(s + idx - d), before = lds_fr(s + idx);
+      sts_fr(s + idx - d, before);
+      sts_fr(s + idx, fr_mul(before, left));
+    }
+    __syncthreads();
+  }
+  return lds_fr(s + t);
 }
 
-__device__ fr warp_block_suffix_product(fr v, fr *s) {
-  const int t = threadIdx.x, lane = t & 31, w = t >> 5, nw = blockDim.x >> 5;
-  for (int o = 1; o < 32; o <<= 1) {
-    const fr u = shfl_down_fr(v, o);
-    if (lane + o < 32) v = fr_mul(v, u);
-  }
-  if (lane == 0) sts_fr(s + w, v);  // warp totals
+// Two scans over a block of 256 threads at once: afterwards s1[t] is the product
+// of the a of the threads before t and s2[255 - t] the product of the b of the
+// threads after t; total[0] and total[1] hold the products of all a and all b.
+// Half of the threads work on each array: three up-sweep levels, one warp
+// scanning the 32 run products, three down-sweep levels, as
+// block_exclusive_product: 38 warp-wide multiplies for both scans, 11 deep.  Two
+// warp-shuffle (Kogge-Stone) scans took 100, 9 deep, a quarter of the
+// permutation product's multiplies.
+__device__ void block_scan_pair(const fr &a, const fr &b, fr *s1, fr *s2, fr *total) {
+  static_assert(kScanThreads == 256, "32 runs of 8");
+  const uint32_t t = threadIdx.x, h = t & 127;
+  fr *s = t < 128 ? s1 : s2;
+  sts_fr(s1 + t, a);
+  sts_fr(s2 + 255 - t, b);
   __syncthreads();
-  if (w == 0) {
-    fr x = lane < nw ? lds_fr(s + lane) : fr_one();
-    for (int o = 1; o < nw; o <<= 1) {
-      const fr u = shfl_down_fr(x, o);
-      if (lane + o < nw) x = fr_mul(x, u);
+#pragma unroll 1
+  for (uint32_t d = 1; d < 8; d <<= 1) {
+    const uint32_t idx = (h + 1) * 2 * d - 1;
+    if (idx < 256) sts_fr(s + idx, fr_mul(lds_fr(s + idx - d), lds_fr(s + idx)));
+    __syncthreads();
+  }
+  if (h < 32) {
+    fr inc = lds_fr(s + 8 * h + 7);
+#pragma unroll 1
+    for (uint32_t o = 1; o < 32; o <<= 1) {
+      const fr u = shfl_up_fr(inc, o);
+      if (h >= o) inc = fr_mul(u, inc);
     }
-    if (lane < nw) sts_fr(s + lane, x);  // warps lane .. nw-1
+    const fr ex = shfl_up_fr(inc, 1);
+    sts_fr(s + 8 * h + 7, h ? ex : fr_one());
+    if (h == 31) sts_fr(total + (t >> 7), inc);
   }
   __syncthreads();
-  if (w + 1 < nw) v = fr_mul(v, lds_fr(s + w + 1));
-  __syncthreads();
-  sts_fr(s + t, v);
-  __syncthreads();
-  return v;
+#pragma unroll 1
+  for (uint32_t d = 4; d >= 1; d >>= 1) {
+    const uint32_t idx = (h + 1) * 2 * d - 1;
+    if (idx < 256) {
+      const fr left = lds_fr(s + idx - d), before = lds_fr(s + idx);
+      sts_fr(s + idx - d, before);
+      sts_fr(s + idx, fr_mul(before, left));
+    }
+    __syncthreads();
+  }
 }
 
 // Suffix composition of affine maps f_t(x) = a_t + b_t x over the block.
@@ -362,7 +340,7 @@ __device__ void block_affine_suffix(fr &a, fr &b, fr *sa, fr *sb, bool all = tru
   sts_fr(sa + u, a);
   sts_fr(sb + u, b);
   scan_sync<NAMED>();
-  // The full scan of 256 maps takes the hybrid form of block_prefix_product:
+  // The full scan of 256 maps takes the hybrid form of block_exclusive_product:
   // three up-sweep levels, one warp scanning the 32 run maps, three
   // down-sweep levels.
   const bool hybrid = all && n == 256;
@@ -445,11 +423,11 @@ __device__ __forceinline__ void gp_local_body(const fr *__restrict__ in, const S
       if (e == 0 || t * kTileElems + e < g.k) p = t + e ? fr_mul(p, ct.get(slot, e)) : ct.get(slot, e);
   });
   __syncthreads();
-  const fr incl = block_prefix_product(p, s);
-  // exclusive = inclusive of the previous thread
-  const fr excl = threadIdx.x ? lds_fr(s + threadIdx.x - 1) : fr_one();
+  // the tiles are free: the scan takes their first 8 KiB, the total what follows
+  fr *total = s + kScanThreads;
+  const fr excl = block_exclusive_product(p, s, total);
   if (gt < g.threads) st_fr(thread_excl + gt, excl);
-  if (threadIdx.x == blockDim.x - 1) st_fr(block_total + blk, incl);
+  if (threadIdx.x == 0) st_fr(block_total + blk, lds_fr(total));
 }
 
 __global__ void __launch_bounds__(kScanThreads) k_gp_local(const fr *__restrict__ in, ScanGeom g,
@@ -556,8 +534,7 @@ struct PermArgs {
   const fr *sigma[3];
   const fr *params;     // beta, gamma, k1, k2, k3
   const fr *omega_pow;  // w^i, i < n
-  fr *z;                // output; holds the numerators until the last pass
-  fr *den;              // scratch: denominators
+  fr *z;                // output; holds the in-block terms until the last pass
 };
 
 // Copy-constraint grand product z_i = prod_{j<i} num_j / den_j, computed as
@@ -567,103 +544,175 @@ struct PermArgs {
 // vector instead of one per block.  A zero denominator makes its ratio 0
 // (num := 0, den := 1), the field-inverse-of-zero-is-zero convention.
 //
-// Pass 1: numerators and denominators; each thread's chunk products; their
-// in-block exclusive prefix (numerators) and exclusive suffix (denominators);
-// the block totals.
+// A block takes 1024 rows, 4 consecutive ones per thread.  Inside a block the
+// term is q_i = (numerators of the block before i) (denominators of the block
+// from i on), and z_i = q_i c_b with one factor c_b per block: the numerators
+// of the earlier blocks times the denominators of the later ones over all of
+// them.  So the first pass leaves one vector of terms (in z) and the last one
+// multiplies it by a per-block constant; the vectors of numerators and
+// denominators, and the two replays over them, are gone.
+//
+// Values are below 2r throughout (fr_mul of two such values is below 1.82 r,
+// since 4 r^2 / 2^256 < 1.82 r); the last pass stores them canonical.  The
+// products by beta and beta k_j take the four-part constant form.
+//
+// GB300, 2^20 rows, us: first pass / carry / last pass 257 / 55 / 110 with
+// numerators and denominators kept in memory, 221 / 48 / 21 so (561 -> 292 per
+// call with the general multiply's rows counted in; 3, 4 and 5 rows per thread:
+// 293, 292 and 308; at 2^22 1029, 1002 and 1005).
+constexpr uint32_t kPermRows = 4, kPermBlockRows = kPermRows * kScanThreads;
+constexpr uint32_t kPermSlots = 2 * kPermRows * 2 * kScanThreads;  // 16-byte units: 64 KiB
+
+// x times the constant whose four parts lie at k in shared memory
+__device__ __forceinline__ fr mul_shared_const(const fr &x, const fr *k) {
+  fr w[4];
+#pragma unroll
+  for (int p = 0; p < 4; ++p) w[p] = lds_fr(k + p);
+  return fr_mul_const4(x, w);
+}
+
+// x k + w + gamma below 2r, from canonical w and gamma
+__device__ __forceinline__ fr perm_factor(const fr &xk, const fr &w, const fr &gamma) {
+  fr u;
+  u.v[0] = add_cc(w.v[0], gamma.v[0]);
+#pragma unroll
+  for (int i = 1; i < 7; ++i) u.v[i] = addc_cc(w.v[i], gamma.v[i]);
+  u.v[7] = addc(w.v[7], gamma.v[7]);  // below 2r < 2^256
+  return fr_add_lazy(xk, u);
+}
+
+// Pass 1: the block's terms q_i into z, the block's products of numerators and
+// of denominators.
 __global__ void __launch_bounds__(kScanThreads, 2)
-    k_perm_local(const PermArgs a, ScanGeom g, fr *__restrict__ thread_num,
-                 fr *__restrict__ thread_den, fr *__restrict__ block_num,
-                 fr *__restrict__ block_den) {
+    k_perm_local(const PermArgs a, uint64_t n, fr *__restrict__ block_num, fr *__restrict__ block_den) {
+  extern __shared__ uint4 slots[];
   __shared__ __align__(16) fr s1[kScanThreads], s2[kScanThreads];
-  const fr beta = ld_fr(a.params), gamma = ld_fr(a.params + 1);
-  const fr bk0 = fr_mul(beta, ld_fr(a.params + 2));
-  const fr bk1 = fr_mul(beta, ld_fr(a.params + 3));
-  const fr bk2 = fr_mul(beta, ld_fr(a.params + 4));
-  const uint64_t gt = blockIdx.x * (uint64_t)kScanThreads + threadIdx.x;
-  const uint64_t lo = gt * g.k < g.n ? gt * g.k : g.n;
-  const uint64_t hi = lo + g.k < g.n ? lo + g.k : g.n;
-  fr N = fr_one(), D = fr_one();
-  for (uint64_t i = lo; i < hi; ++i) {
-    const fr wi = ld_fr(a.omega_pow + i);
-    const fr x0 = ld_fr(a.w[0] + i), x1 = ld_fr(a.w[1] + i), x2 = ld_fr(a.w[2] + i);
-    fr num = fr_add(fr_add(x0, fr_mul(bk0, wi)), gamma);
-    num = fr_mul(num, fr_add(fr_add(x1, fr_mul(bk1, wi)), gamma));
-    num = fr_mul(num, fr_add(fr_add(x2, fr_mul(bk2, wi)), gamma));
-    fr den = fr_add(fr_add(x0, fr_mul(beta, ld_fr(a.sigma[0] + i))), gamma);
-    den = fr_mul(den, fr_add(fr_add(x1, fr_mul(beta, ld_fr(a.sigma[1] + i))), gamma));
-    den = fr_mul(den, fr_add(fr_add(x2, fr_mul(beta, ld_fr(a.sigma[2] + i))), gamma));
-    if (fr_is_zero(den)) {
-      num = fr_zero();
-      den = fr_one();
-    }
-    st_fr(a.z + i, num);
-    st_fr(a.den + i, den);
-    N = fr_mul(N, num);
-    D = fr_mul(D, den);
+  __shared__ __align__(16) fr s_total[2];
+  __shared__ __align__(16) fr s_k[16];  // beta, beta k1, beta k2, beta k3 in four parts each
+  const uint32_t t = threadIdx.x;
+  if (t < 16) {
+    fr k = ld_fr(a.params);
+    if (t >> 2) k = fr_mul(k, ld_fr(a.params + 1 + (t >> 2)));
+    sts_fr(s_k + t, fr_mul(k, fr_const4_factor(t & 3)));
   }
-  const fr incl_n = warp_block_prefix_product(N, s1);  // s1[t] = N_0 .. N_t
-  const fr incl_d = warp_block_suffix_product(D, s2);  // s2[t] = D_t .. D_last
-  if (gt < g.threads) {
-    st_fr(thread_num + gt, threadIdx.x ? lds_fr(s1 + threadIdx.x - 1) : fr_one());
-    st_fr(thread_den + gt, threadIdx.x + 1 < blockDim.x ? lds_fr(s2 + threadIdx.x + 1) : fr_one());
-  }
-  if (threadIdx.x == blockDim.x - 1) st_fr(block_num + blockIdx.x, incl_n);
-  if (threadIdx.x == 0) st_fr(block_den + blockIdx.x, incl_d);
-}
-
-// Pass 2, one block: in place, block_num[b] := the product of the numerator
-// totals of the blocks before b, block_den[b] := the product of the
-// denominator totals of the blocks after b, divided by all denominators.
-__global__ void __launch_bounds__(kScanThreads) k_perm_carry(fr *block_num, fr *block_den,
-                                                              uint32_t nb) {
-  __shared__ __align__(16) fr s1[kScanThreads], s2[kScanThreads];
-  __shared__ fr s_inv;
-  const uint32_t per = (nb + blockDim.x - 1) / blockDim.x;
-  const uint32_t lo = threadIdx.x * per < nb ? threadIdx.x * per : nb;
-  const uint32_t hi = lo + per < nb ? lo + per : nb;
-  fr N = fr_one(), D = fr_one();
-  for (uint32_t b = lo; b < hi; ++b) {
-    N = fr_mul(N, ld_fr(block_num + b));
-    D = fr_mul(D, ld_fr(block_den + b));
-  }
-  warp_block_prefix_product(N, s1);
-  warp_block_suffix_product(D, s2);  // s2[0]: every denominator (none is zero)
-  if (threadIdx.x == 0) s_inv = fr_inv_fast(lds_fr(s2));
   __syncthreads();
-  fr run_n = threadIdx.x ? lds_fr(s1 + threadIdx.x - 1) : fr_one();
-  fr run_d = fr_mul(s_inv, threadIdx.x + 1 < blockDim.x ? lds_fr(s2 + threadIdx.x + 1) : fr_one());
-  for (uint32_t b = lo; b < hi; ++b) {
-    const fr v = ld_fr(block_num + b);
-    st_fr(block_num + b, run_n);
-    run_n = fr_mul(run_n, v);
+  const auto slot = [&](uint32_t j) { return slots + j * 2 * kScanThreads + t; };
+  const auto put = [&](uint32_t j, const fr &v) {
+    slot(j)[0] = make_uint4(v.v[0], v.v[1], v.v[2], v.v[3]);
+    slot(j)[kScanThreads] = make_uint4(v.v[4], v.v[5], v.v[6], v.v[7]);
+  };
+  const auto get = [&](uint32_t j) {
+    const uint4 u = slot(j)[0], v = slot(j)[kScanThreads];
+    return fr{{u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w}};
+  };
+  const uint64_t row0 = (blockIdx.x * (uint64_t)kScanThreads + t) * kPermRows;
+  fr N = fr_one(), D = fr_one();
+#pragma unroll 1
+  for (uint32_t j = 0; j < kPermRows; ++j) {
+    const uint64_t i = row0 + j;
+    put(j, N);  // numerators of this thread before row j
+    fr den = fr_one();
+    if (i < n) {
+      const fr gamma = ld_fr(a.params + 1);
+      const fr wi = ldcs_fr(a.omega_pow + i);
+      fr x = ldcs_fr(a.w[0] + i);
+      fr num = perm_factor(mul_shared_const(wi, s_k + 4), x, gamma);
+      den = perm_factor(mul_shared_const(ldcs_fr(a.sigma[0] + i), s_k), x, gamma);
+#pragma unroll 1
+      for (uint32_t c = 1; c < 3; ++c) {
+        x = ldcs_fr(a.w[c] + i);
+        num = fr_mul(num, perm_factor(mul_shared_const(wi, s_k + 4 + 4 * c), x, gamma));
+        den = fr_mul(den, perm_factor(mul_shared_const(ldcs_fr(a.sigma[c] + i), s_k), x, gamma));
+      }
+      if (fr_is_zero(fr_canon(den))) {
+        num = fr_zero();
+        den = fr_one();
+      }
+      N = j ? fr_mul(N, num) : num;
+    }
+    put(kPermRows + j, den);
   }
-  for (uint32_t b = hi; b > lo; --b) {
-    const fr v = ld_fr(block_den + b - 1);
-    st_fr(block_den + b - 1, run_d);
-    run_d = fr_mul(run_d, v);
+#pragma unroll 1
+  for (uint32_t j = kPermRows; j-- > 0;) {
+    D = j + 1 < kPermRows ? fr_mul(D, get(kPermRows + j)) : get(kPermRows + j);
+    put(j, j ? fr_mul(get(j), D) : D);
+  }
+  block_scan_pair(N, D, s1, s2, s_total);
+  const fr T = fr_mul(lds_fr(s1 + t), lds_fr(s2 + kScanThreads - 1 - t));
+#pragma unroll 1
+  for (uint32_t j = 0; j < kPermRows && row0 + j < n; ++j) st_fr(a.z + row0 + j, fr_mul(get(j), T));
+  if (t == 0) {
+    st_fr(block_num + blockIdx.x, lds_fr(s_total));
+    st_fr(block_den + blockIdx.x, lds_fr(s_total + 1));
   }
 }
 
-// Pass 3: z_i = (numerators before i) * (denominators from i on) / (all):
-// forward over the chunk for the first factor (kept in z), backward for the
-// second.
-__global__ void __launch_bounds__(kScanThreads)
-    k_perm_apply(const PermArgs a, ScanGeom g, const fr *__restrict__ thread_num,
-                 const fr *__restrict__ thread_den, const fr *__restrict__ block_num,
-                 const fr *__restrict__ block_den) {
-  const uint64_t gt = blockIdx.x * (uint64_t)kScanThreads + threadIdx.x;
-  if (gt >= g.threads) return;
-  const uint64_t lo = gt * g.k, hi = lo + g.k < g.n ? lo + g.k : g.n;
-  fr run = fr_mul(ld_fr(block_num + blockIdx.x), ld_fr(thread_num + gt));
-  for (uint64_t i = lo; i < hi; ++i) {
-    const fr v = ld_fr(a.z + i);
-    st_fr(a.z + i, run);
-    run = fr_mul(run, v);
+// Pass 2, one block of two halves: in place, block_num[b] := the product of the
+// numerators of the blocks before b (first half of the threads), block_den[b]
+// := the product of the denominators of the blocks after b, divided by all
+// denominators (second half, over the blocks in reverse).
+__global__ void __launch_bounds__(2 * kScanThreads) k_perm_carry(fr *block_num, fr *block_den, uint32_t nb) {
+  __shared__ __align__(16) fr sw[2][kScanThreads / 32];
+  __shared__ __align__(16) fr s_inv;
+  const uint32_t half = threadIdx.x / kScanThreads, t = threadIdx.x % kScanThreads;
+  const uint32_t lane = t & 31, w = t >> 5;
+  constexpr uint32_t nw = kScanThreads / 32;
+  fr *v = half ? block_den : block_num;
+  const auto at = [&](uint32_t l) { return half ? nb - 1 - l : l; };
+  const uint32_t per = (nb + kScanThreads - 1) / kScanThreads;
+  const uint32_t lo = t * per < nb ? t * per : nb, hi = lo + per < nb ? lo + per : nb;
+  fr P = fr_one();
+  for (uint32_t l = lo; l < hi; ++l) P = l > lo ? fr_mul(P, ld_fr(v + at(l))) : ld_fr(v + at(l));
+  // inclusive scan of the half's 256 products
+  for (uint32_t o = 1; o < 32; o <<= 1) {
+    const fr u = shfl_up_fr(P, o);
+    if (lane >= o) P = fr_mul(u, P);
   }
-  run = fr_mul(ld_fr(block_den + blockIdx.x), ld_fr(thread_den + gt));
-  for (uint64_t i = hi; i > lo; --i) {
-    run = fr_mul(run, ld_fr(a.den + i - 1));
-    st_fr(a.z + i - 1, fr_mul(ld_fr(a.z + i - 1), run));
+  if (lane == 31) sts_fr(&sw[half][w], P);
+  __syncthreads();
+  if (w == 0) {
+    fr x = lane < nw ? lds_fr(&sw[half][lane]) : fr_one();
+    for (uint32_t o = 1; o < nw; o <<= 1) {
+      const fr u = shfl_up_fr(x, o);
+      if (lane >= o) x = fr_mul(u, x);
+    }
+    if (lane < nw) sts_fr(&sw[half][lane], x);
+  }
+  __syncthreads();
+  // one inversion for the vector (no denominator is zero), beside the
+  // numerators' half, which does not need it
+  if (threadIdx.x == kScanThreads) sts_fr(&s_inv, fr_inv_fast(fr_canon(lds_fr(&sw[1][nw - 1]))));
+  fr run = shfl_up_fr(P, 1);
+  if (lane == 0) run = w ? lds_fr(&sw[half][w - 1]) : fr_one();
+  else if (w) run = fr_mul(run, lds_fr(&sw[half][w - 1]));
+  if (half) {
+    asm volatile("bar.sync 1, 256;" ::: "memory");  // the second half: s_inv is there
+    run = fr_mul(run, lds_fr(&s_inv));
+  }
+  for (uint32_t l = lo; l < hi; ++l) {
+    const fr x = ld_fr(v + at(l));
+    st_fr(v + at(l), run);
+    if (l + 1 < hi) run = fr_mul(run, x);
+  }
+}
+
+// Pass 3: z_i = q_i c_b
+__global__ void __launch_bounds__(kScanThreads)
+    k_perm_apply(fr *z, uint64_t n, const fr *__restrict__ block_num, const fr *__restrict__ block_den) {
+  __shared__ __align__(16) fr s_c[4];
+  if (threadIdx.x < 4) {
+    const fr c = fr_mul(ld_fr(block_num + blockIdx.x), ld_fr(block_den + blockIdx.x));
+    sts_fr(s_c + threadIdx.x, fr_mul(c, fr_const4_factor(threadIdx.x)));
+  }
+  __syncthreads();
+  fr w[4];
+#pragma unroll
+  for (int p = 0; p < 4; ++p) w[p] = lds_fr(s_c + p);
+  const uint64_t i0 = blockIdx.x * (uint64_t)kPermBlockRows + threadIdx.x;
+#pragma unroll 1
+  for (uint32_t j = 0; j < kPermRows; ++j) {
+    const uint64_t i = i0 + j * kScanThreads;
+    if (i < n) st_fr(z + i, fr_canon(fr_mul_const4(ld_fr(z + i), w)));
   }
 }
 
@@ -1025,12 +1074,13 @@ extern "C" int pp_gp_perm(const void *const *d_w, const void *const *d_sigma, co
   }
   cudaStream_t s = (cudaStream_t)stream;
   const uint64_t n = 1ull << lg_n;
-  const pp::ScanGeom g = pp::scan_geom(n, pp::kPermBlocksPerSm);
+  const uint64_t nb64 = (n + pp::kPermBlockRows - 1) / pp::kPermBlockRows;
+  const uint32_t nb = (uint32_t)nb64;
   int st = PP_OK;
   const fr *omega_pow = pp::pow_table(pp::host_root_of_unity((int)lg_n, false), lg_n, &st);
   if (st) return st;
   fr *ws = static_cast<fr *>(
-      pp::workspace_get((n + 2 * g.threads + 2 * g.blocks) * sizeof(fr), s, 1, &st));
+      pp::workspace_get(2 * (size_t)nb * sizeof(fr), s, 1, &st));
   if (st) return st;
   pp::PermArgs a;
   for (int j = 0; j < 3; ++j) {
@@ -1040,18 +1090,16 @@ extern "C" int pp_gp_perm(const void *const *d_w, const void *const *d_sigma, co
   a.params = static_cast<const fr *>(d_params);
   a.omega_pow = omega_pow;
   a.z = static_cast<fr *>(d_z);
-  a.den = ws;
-  fr *thread_num = ws + n, *thread_den = thread_num + g.threads;
-  fr *block_num = thread_den + g.threads, *block_den = block_num + g.blocks;
-  pp::k_perm_local<<<g.blocks, pp::kScanThreads, 0, s>>>(a, g, thread_num, thread_den, block_num,
-                                                         block_den);
+  fr *block_num = ws, *block_den = ws + nb;
+  constexpr size_t smem = pp::kPermSlots * sizeof(uint4);
+  PP_CUDA_TRY(cudaFuncSetAttribute(pp::k_perm_local, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  pp::k_perm_local<<<nb, pp::kScanThreads, smem, s>>>(a, n, block_num, block_den);
   PP_COUNT_LAUNCH();
   PP_LAUNCH_CHECK();
-  pp::k_perm_carry<<<1, pp::kScanThreads, 0, s>>>(block_num, block_den, g.blocks);
+  pp::k_perm_carry<<<1, 2 * pp::kScanThreads, 0, s>>>(block_num, block_den, nb);
   PP_COUNT_LAUNCH();
   PP_LAUNCH_CHECK();
-  pp::k_perm_apply<<<g.blocks, pp::kScanThreads, 0, s>>>(a, g, thread_num, thread_den, block_num,
-                                                         block_den);
+  pp::k_perm_apply<<<nb, pp::kScanThreads, 0, s>>>(a.z, n, block_num, block_den);
   PP_COUNT_LAUNCH();
   PP_LAUNCH_CHECK();
   return PP_OK;
