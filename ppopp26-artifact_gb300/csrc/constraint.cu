@@ -1,10 +1,18 @@
 // constraint.cu -- PLONK quotient-constraint operators: element-wise terms
 // over the points of the extended domain, computed from the LDE outputs.
 //
-// Each output point costs 18 (permutation, fused) to ~105 (gate) Montgomery
-// multiplies against 448 / 736 bytes of HBM traffic, so both kernels are
-// integer-multiply bound by a factor of 5-40 over HBM.  They are plain
-// element-wise loops: one thread per point, scalars staged once per block.
+// Each output point costs 18 (permutation, fused) to ~80 (gate) multiplies
+// against 448 / 736 bytes of HBM traffic, so both kernels are integer-multiply
+// bound by a factor of 5-40 over HBM.  They are plain element-wise loops: one
+// thread per point, scalars staged once per block.
+//
+// Multiplies by a scalar of the call take the four-part constant form
+// (fr_mul_const4, 82 wide products against 112; the parts are prepared once per
+// block or call), squares the squaring (84), sums of products one reduction for
+// all (fr_mac17), small integers fr_mul_small.  Values are lazy (below 2r)
+// between loads and the store: fr_mul and fr_sqr of lazy values are below 1.82 r
+// (4 r^2 / 2^256), and canonical again when one factor is below r and the other
+// below 2r.
 #include "common.cuh"
 
 namespace pp {
@@ -19,53 +27,70 @@ struct PermArgs {
 
 enum : int { kIdentity = 1, kCopy = 2, kTermOne = 4, kAll = 7 };
 
-// prod_j (u_j * beta * c_j + w_j + gamma): the identity product uses u_j = x
-// and c = (1, k1, k2, k3); the copy product u_j = sigma_j and c_j = 1
-__device__ __forceinline__ fr identity_product(const PermArgs &a, uint64_t i, const fr &beta,
-                                               const fr &gamma, const fr k[3]) {
-  const fr xb = fr_mul(ldcs_fr(a.x + i), beta);
-  fr acc = fr_add(fr_add(xb, ldcs_fr(a.w[0] + i)), gamma);
+// The scalars as shared constants, four parts each: alpha, beta, beta k_1..3.
+enum : int { kCAlpha, kCBeta, kCBetaK, kPermConsts = kCBetaK + 3 };
+
+__device__ __forceinline__ void stage_perm_constants(const PermArgs &a, fr *sc, int terms) {
+  if (threadIdx.x < 4 * kPermConsts) {
+    const int c = threadIdx.x >> 2;
+    const bool used = c == kCAlpha || c == kCBeta ? (terms & (kIdentity | kCopy)) != 0 : (terms & kIdentity) != 0;
+    if (used) {
+      fr k = ld_fr(c == kCAlpha ? a.alpha : a.beta);
+      if (c >= kCBetaK) k = fr_mul(k, ld_fr(a.k[c - kCBetaK]));
+      st_fr(sc + threadIdx.x, fr_mul(k, fr_const4_factor(threadIdx.x & 3)));
+    }
+  }
+  __syncthreads();
+}
+
+// prod_j (u_j * beta * c_j + w_j + gamma) below 2r: the identity product uses
+// u_j = x and c = (1, k1, k2, k3); the copy product u_j = sigma_j and c_j = 1.
+// wg[j] = w_j + gamma, unreduced.
+__device__ __forceinline__ fr identity_product(const fr &x, const fr wg[4], const fr *sc) {
+  fr acc = fr_add_lazy(mul_shared_const(x, sc + 4 * kCBeta), wg[0]);
 #pragma unroll
   for (int j = 1; j < 4; ++j)
-    acc = fr_mul(acc, fr_add(fr_add(fr_mul(xb, k[j - 1]), ldcs_fr(a.w[j] + i)), gamma));
+    acc = fr_mul(acc, fr_add_lazy(mul_shared_const(x, sc + 4 * (kCBetaK + j - 1)), wg[j]));
   return acc;
 }
 
-__device__ __forceinline__ fr copy_product(const PermArgs &a, uint64_t i, const fr &beta,
-                                           const fr &gamma) {
-  fr acc = fr_add(fr_add(fr_mul(ldcs_fr(a.sigma[0] + i), beta), ldcs_fr(a.w[0] + i)), gamma);
+__device__ __forceinline__ fr copy_product(const PermArgs &a, uint64_t i, const fr wg[4], const fr *sc) {
+  fr acc = fr_add_lazy(mul_shared_const(ldcs_fr(a.sigma[0] + i), sc + 4 * kCBeta), wg[0]);
 #pragma unroll
   for (int j = 1; j < 4; ++j)
-    acc = fr_mul(acc, fr_add(fr_add(fr_mul(ldcs_fr(a.sigma[j] + i), beta), ldcs_fr(a.w[j] + i)),
-                             gamma));
+    acc = fr_mul(acc, fr_add_lazy(mul_shared_const(ldcs_fr(a.sigma[j] + i), sc + 4 * kCBeta), wg[j]));
   return acc;
 }
 
 template <int TERMS>
-__global__ void __launch_bounds__(kThreads) k_perm_quotient(const PermArgs a, fr *result,
-                                                            uint64_t n) {
-  const fr alpha = ldg_fr(a.alpha), beta = ldg_fr(a.beta), gamma = ldg_fr(a.gamma);
-  fr k[3];
-  if (TERMS & kIdentity) {
-#pragma unroll
-    for (int j = 0; j < 3; ++j) k[j] = ldg_fr(a.k[j]);
-  }
-  const fr one = (TERMS & kTermOne) ? ldg_fr(a.one) : fr_zero();
+__global__ void __launch_bounds__(kThreads, 2) k_perm_quotient(const PermArgs a, fr *result,
+                                                               uint64_t n) {
+  __shared__ __align__(16) fr sc[4 * kPermConsts];
+  stage_perm_constants(a, sc, TERMS);
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+    fr wg[4];
+    if (TERMS & (kIdentity | kCopy)) {
+      const fr gamma = ldg_fr(a.gamma);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) wg[j] = fr_add_raw(ldcs_fr(a.w[j] + i), gamma);
+    }
+    const fr one = (TERMS & kTermOne) ? ldg_fr(a.one) : fr_zero();
     fr r;
     if (TERMS == kAll) {
       // (id * z - cp * z_next) * alpha + mod + (z - one) * l1: alpha once
       const fr z = ldcs_fr(a.z + i);
-      const fr id = fr_mul(identity_product(a, i, beta, gamma, k), z);
-      const fr cp = fr_mul(copy_product(a, i, beta, gamma), ldcs_fr(a.z_next + i));
-      r = fr_add(fr_mul(fr_sub(id, cp), alpha), ldcs_fr(a.mod + i));
-      r = fr_add(r, fr_mul(fr_sub(z, one), ldcs_fr(a.l1 + i)));
+      const fr id = fr_mul(identity_product(ldcs_fr(a.x + i), wg, sc), z);
+      const fr cp = fr_mul(copy_product(a, i, wg, sc), ldcs_fr(a.z_next + i));
+      r = fr_add_lazy(mul_shared_const(fr_sub_lazy(id, cp), sc + 4 * kCAlpha), ldcs_fr(a.mod + i));
+      r = fr_canon(fr_add_lazy(r, fr_mul(fr_sub_lazy(z, one), ldcs_fr(a.l1 + i))));
     } else if (TERMS == kIdentity) {
-      r = fr_mul(fr_mul(identity_product(a, i, beta, gamma, k), ldcs_fr(a.z + i)), alpha);
+      r = fr_mul(identity_product(ldcs_fr(a.x + i), wg, sc), ldcs_fr(a.z + i));
+      r = fr_canon(mul_shared_const(r, sc + 4 * kCAlpha));
     } else if (TERMS == kCopy) {
-      const fr cp = fr_mul(fr_mul(copy_product(a, i, beta, gamma), ldcs_fr(a.z_next + i)), alpha);
-      r = fr_sub(fr_add(ld_fr(result + i), ldcs_fr(a.mod + i)), cp);
+      const fr cp = fr_mul(copy_product(a, i, wg, sc), ldcs_fr(a.z_next + i));
+      r = fr_add_raw(ld_fr(result + i), ldcs_fr(a.mod + i));
+      r = fr_canon(fr_sub_lazy(r, mul_shared_const(cp, sc + 4 * kCAlpha)));
     } else {
       r = fr_add(ld_fr(result + i), fr_mul(fr_sub(ldcs_fr(a.z + i), one), ldcs_fr(a.l1 + i)));
     }
@@ -80,78 +105,111 @@ struct GateArgs {
   uint32_t sbox_alpha;  // 2 <= sbox_alpha < 2^31
 };
 
-// x^e for 2 <= e < 2^31, square and multiply from the top set bit
+// x^e below 2r for 2 <= e < 2^31, square and multiply from the top set bit
 __device__ __forceinline__ fr pow_small(const fr &x, uint32_t e) {
   fr r = x;
   for (int b = 30 - __clz(e); b >= 0; --b) {
-    r = fr_mul(r, r);
+    r = fr_sqr(r);
     if ((e >> b) & 1) r = fr_mul(r, x);
   }
   return r;
 }
 
-// x^4 * three * one * two: the reference's x (x three)((x one)(x two))
-__device__ __forceinline__ fr delta4(const fr &x, const fr &k312) {
-  const fr x2 = fr_mul(x, x);
-  return fr_mul(fr_mul(x2, x2), k312);
-}
-
-// small multiples by additions (exact, like any field identity)
+// small multiples by additions, canonical (k_gate_prepare's comparison)
 __device__ __forceinline__ fr dbl(const fr &x) { return fr_add(x, x); }
 __device__ __forceinline__ fr mul3(const fr &x) { return fr_add(dbl(x), x); }
 __device__ __forceinline__ fr mul4(const fr &x) { return dbl(dbl(x)); }
-__device__ __forceinline__ fr mul6(const fr &x) { return dbl(mul3(x)); }
 __device__ __forceinline__ fr mul9(const fr &x) { return fr_add(dbl(mul4(x)), x); }
 __device__ __forceinline__ fr mul18(const fr &x) { return dbl(mul9(x)); }
-__device__ __forceinline__ fr mul36(const fr &x) { return dbl(mul18(x)); }
 __device__ __forceinline__ fr mul81(const fr &x) { return mul9(mul9(x)); }
 __device__ __forceinline__ fr mul83(const fr &x) { return fr_add(mul81(x), dbl(x)); }
-
-// 6 x^4 (delta4 with three one two = 6)
-__device__ __forceinline__ fr delta4_6(const fr &x) {
-  const fr x2 = fr_mul(x, x);
-  return mul6(fr_mul(x2, x2));
-}
 
 // The gate runs as three launches so that each keeps its live values in
 // fewer registers (more resident warps): the range and logic terms are
 // written first, then the arithmetic and public-input terms and the fixed-
 // and variable-base group additions are added.
 
-// The scalars as the gate kernels use them, prepared once per call by
-// k_gate_prepare: the PP_GATE_NS scalars, then three one two, then whether
-// four, one, two, three, nine, eighteen, eightyone and eightythree hold
-// those integers, as the prover passes them.  Then the kernels take
-// SMALL = true: multiplies by them become additions and one one / three one
-// two drop out, with the same field values (range and logic 47 -> 27
-// multiplies per point, groups 38 -> 35).  Any other values take SMALL =
-// false, the expression as written.
+// The constants of the gate kernels, prepared once per call by k_gate_prepare
+// in the four-part form: products of the call's scalars, with each gate's
+// challenge multiplied in (Kxx below: the reference's kappa names), so that a
+// sum of terms needs no further multiply by it.  `small` says whether four, one,
+// two, three, nine, eighteen, eightyone and eightythree hold those integers, as
+// the prover passes them.  Then the kernels take SMALL = true: multiplies by
+// them become fr_mul_small.  Any other values take SMALL = false, the
+// expression as written.
+enum : int {
+  kRangeCu, kRangeSq, kRangeOne, kRangeK,  // three one two kappa.. range_challenge
+  kLogicQu, kLogicCu, kLogicQuad,          // the last: three one two logic_challenge
+  kFbK, kFbCu, kFbOne, kFbSq, kPd, kPa, kVbSq, kVbOne, kVbK,
+  kOneSq, kFour, kEighteen, kEightyone, kTwo83, kThree, kNine,  // SMALL = false only
+  kGateConsts
+};
 struct GateScalars {
-  fr s[PP_GATE_NS + 1];
+  fr c[4 * kGateConsts];
   int small;
 };
 
-__global__ void k_gate_prepare(const GateArgs a, GateScalars *out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  fr sc[PP_GATE_NS + 1];
-  for (int j = 0; j < PP_GATE_NS; ++j) sc[j] = ldg_fr(a.s[j]);
-  sc[PP_GATE_NS] = fr_mul(fr_mul(sc[PP_GATE_S_THREE], sc[PP_GATE_S_ONE]), sc[PP_GATE_S_TWO]);
-  const fr one = fr_one();
-  out->small = fr_eq(sc[PP_GATE_S_ONE], one) && fr_eq(sc[PP_GATE_S_TWO], dbl(one)) &&
-               fr_eq(sc[PP_GATE_S_THREE], mul3(one)) && fr_eq(sc[PP_GATE_S_FOUR], mul4(one)) &&
-               fr_eq(sc[PP_GATE_S_NINE], mul9(one)) && fr_eq(sc[PP_GATE_S_EIGHTEEN], mul18(one)) &&
-               fr_eq(sc[PP_GATE_S_EIGHTYONE], mul81(one)) &&
-               fr_eq(sc[PP_GATE_S_EIGHTYTHREE], mul83(one));
-  for (int j = 0; j <= PP_GATE_NS; ++j) st_fr(out->s + j, sc[j]);
-}
+// constant c is the product of these scalars (PP_GATE_NS: the factor 1)
+#define GS(name) PP_GATE_S_##name
+constexpr int kNone = PP_GATE_NS, kGateFactors = 5;
+__constant__ unsigned char c_gate_factors[kGateConsts][kGateFactors] = {
+    {GS(THREE), GS(ONE), GS(TWO), GS(KAPPA_CU_RANGE), GS(RANGE_CHALLENGE)},
+    {GS(THREE), GS(ONE), GS(TWO), GS(KAPPA_SQ_RANGE), GS(RANGE_CHALLENGE)},
+    {GS(THREE), GS(ONE), GS(TWO), GS(RANGE_CHALLENGE), kNone},
+    {GS(THREE), GS(ONE), GS(TWO), GS(KAPPA_RANGE), GS(RANGE_CHALLENGE)},
+    {GS(KAPPA_QU_LOGIC), GS(LOGIC_CHALLENGE), kNone, kNone, kNone},
+    {GS(KAPPA_CU_LOGIC), GS(LOGIC_CHALLENGE), kNone, kNone, kNone},
+    {GS(THREE), GS(ONE), GS(TWO), GS(LOGIC_CHALLENGE), kNone},
+    {GS(KAPPA_FB), GS(FB_CHALLENGE), kNone, kNone, kNone},
+    {GS(KAPPA_CU_FB), GS(FB_CHALLENGE), kNone, kNone, kNone},
+    {GS(ONE), GS(ONE), GS(FB_CHALLENGE), kNone, kNone},
+    {GS(KAPPA_SQ_FB), GS(FB_CHALLENGE), kNone, kNone, kNone},
+    {GS(P_D), kNone, kNone, kNone, kNone},
+    {GS(P_A), kNone, kNone, kNone, kNone},
+    {GS(KAPPA_SQ_VB), GS(VB_CHALLENGE), kNone, kNone, kNone},
+    {GS(VB_CHALLENGE), kNone, kNone, kNone, kNone},
+    {GS(KAPPA_VB), GS(VB_CHALLENGE), kNone, kNone, kNone},
+    {GS(ONE), GS(ONE), kNone, kNone, kNone},
+    {GS(FOUR), kNone, kNone, kNone, kNone},
+    {GS(EIGHTEEN), kNone, kNone, kNone, kNone},
+    {GS(EIGHTYONE), kNone, kNone, kNone, kNone},
+    {GS(TWO), GS(EIGHTYTHREE), kNone, kNone, kNone},
+    {GS(THREE), kNone, kNone, kNone, kNone},
+    {GS(NINE), kNone, kNone, kNone, kNone},
+};
+#undef GS
 
-// copies the prepared scalars to shared memory
-__device__ __forceinline__ void stage_scalars(const GateScalars *g, fr *sc) {
-  if (threadIdx.x <= PP_GATE_NS) sc[threadIdx.x] = ldg_fr(g->s + threadIdx.x);
+// one thread per part of a constant
+__global__ void __launch_bounds__(128) k_gate_prepare(const GateArgs a, GateScalars *out) {
+  __shared__ __align__(16) fr sc[PP_GATE_NS + 1];
+  const uint32_t t = threadIdx.x;
+  if (t < PP_GATE_NS) st_fr(sc + t, ldg_fr(a.s[t]));
+  if (t == PP_GATE_NS) st_fr(sc + t, fr_one());
+  __syncthreads();
+  if (t < 4 * kGateConsts) {
+    fr k = lds_fr(sc + c_gate_factors[t >> 2][0]);
+#pragma unroll 1
+    for (int f = 1; f < kGateFactors; ++f) k = fr_mul(k, lds_fr(sc + c_gate_factors[t >> 2][f]));
+    st_fr(out->c + t, fr_mul(k, fr_const4_factor(t & 3)));
+  }
+  if (t == 127) {
+    const fr one = fr_one();
+    auto is = [&](int s, const fr &v) { return fr_eq(lds_fr(sc + s), v); };
+    out->small = is(PP_GATE_S_ONE, one) && is(PP_GATE_S_TWO, dbl(one)) && is(PP_GATE_S_THREE, mul3(one)) &&
+                 is(PP_GATE_S_FOUR, mul4(one)) && is(PP_GATE_S_NINE, mul9(one)) &&
+                 is(PP_GATE_S_EIGHTEEN, mul18(one)) && is(PP_GATE_S_EIGHTYONE, mul81(one)) &&
+                 is(PP_GATE_S_EIGHTYTHREE, mul83(one));
+  }
+}
+static_assert(4 * kGateConsts < 127, "k_gate_prepare: one thread per part, the last compares");
+
+// copies the prepared constants to shared memory
+__device__ __forceinline__ void stage_constants(const GateScalars *g, fr *sc) {
+  if (threadIdx.x < 4 * kGateConsts) st_fr(sc + threadIdx.x, ldg_fr(g->c + threadIdx.x));
   __syncthreads();
 }
 
-#define S(name) sc[PP_GATE_S_##name]
+#define MC(x, c) mul_shared_const(x, sc + 4 * (c))
 #define V(name) ldcs_fr(a.v[PP_GATE_V_##name] + i)
 
 // The host launches both forms; the one whose SMALL does not match the
@@ -161,73 +219,61 @@ __global__ void __launch_bounds__(kThreads, 2) k_gate_range_logic(const GateArgs
                                                                const GateScalars *gs, fr *out,
                                                                uint64_t n) {
   if ((__ldg(&gs->small) != 0) != SMALL) return;
-  __shared__ __align__(16) fr sc[PP_GATE_NS + 1];
-  stage_scalars(gs, sc);
+  __shared__ __align__(16) fr sc[4 * kGateConsts];
+  stage_constants(gs, sc);
+  // x times one of the gate's integers, below 2r
+  const auto times = [&](const fr &x, uint32_t k, int c) { return SMALL ? fr_mul_small(x, k) : MC(x, c); };
+  const auto pow4 = [](const fr &x) { return fr_sqr(fr_sqr(x)); };
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-    const fr k312 = sc[PP_GATE_NS];
     const fr a_ = V(A), b = V(B), c = V(C), d = V(D), dn = V(D_NEXT);
-    fr a4, b4, c4, d4;
-    if constexpr (SMALL) {
-      a4 = mul4(a_), b4 = mul4(b), c4 = mul4(c), d4 = mul4(d);
-    } else {
-      const fr four = S(FOUR);
-      a4 = fr_mul(a_, four), b4 = fr_mul(b, four), c4 = fr_mul(c, four), d4 = fr_mul(d, four);
-    }
-    auto quad = [&](const fr &x) { return SMALL ? delta4_6(x) : delta4(x, k312); };
+    const fr a4 = times(a_, 4, kFour), b4 = times(b, 4, kFour);
+    const fr c4 = times(c, 4, kFour), d4 = times(d, 4, kFour);
 
-    // range gate: four 2-bit quads
-    fr t = fr_mul(quad(fr_sub(a4, dn)), S(KAPPA_CU_RANGE));
-    t = fr_add(t, fr_mul(quad(fr_sub(a_, b4)), S(KAPPA_SQ_RANGE)));
-    t = fr_add(t, quad(fr_sub(c, d4)));
-    t = fr_add(t, fr_mul(quad(fr_sub(b, c4)), S(KAPPA_RANGE)));
-    fr acc = fr_mul(fr_mul(t, S(RANGE_CHALLENGE)), V(RANGE));
+    // range gate: four 2-bit quads, quad(x) = x^4 three one two
+    fr t = MC(pow4(fr_sub_lazy(a4, dn)), kRangeCu);
+    t = fr_add_lazy(t, MC(pow4(fr_sub_lazy(a_, b4)), kRangeSq));
+    t = fr_add_lazy(t, MC(pow4(fr_sub_lazy(c, d4)), kRangeOne));
+    t = fr_add_lazy(t, MC(pow4(fr_sub_lazy(b, c4)), kRangeK));
+    fr acc = fr_mul(t, V(RANGE));
 
     // logic gate
-    const fr da = fr_sub(a4, V(A_NEXT)), db = fr_sub(b4, V(B_NEXT));
-    const fr w = fr_add(da, db), e = fr_sub(dn, d4);
-    const fr da2 = fr_mul(da, da);
-    fr inner, A, B, da4;
-    if constexpr (SMALL) {
-      inner = fr_sub(mul81(w), fr_add(fr_mul(c, mul81(fr_sub(c4, mul18(w)))), mul36(da2)));
-      A = fr_sub(mul3(fr_add(e, w)), dbl(fr_mul(c, mul83(inner))));
-      B = fr_mul(V(Q_C), fr_sub(mul9(e), mul3(w)));
-      da4 = mul6(fr_mul(da2, da2));
-    } else {
-      inner = fr_sub(fr_mul(w, S(EIGHTYONE)),
-                     fr_add(fr_mul(c, fr_mul(fr_sub(c4, fr_mul(w, S(EIGHTEEN))), S(EIGHTYONE))),
-                            fr_mul(fr_add(da2, da2), S(EIGHTEEN))));
-      A = fr_sub(fr_mul(fr_add(e, w), S(THREE)),
-                 fr_mul(fr_mul(c, fr_mul(inner, S(EIGHTYTHREE))), S(TWO)));
-      B = fr_mul(V(Q_C), fr_sub(fr_mul(e, S(NINE)), fr_mul(w, S(THREE))));
-      da4 = fr_mul(fr_mul(da2, da2), k312);
-    }
-    fr l = fr_mul(fr_add(A, B), S(KAPPA_QU_LOGIC));
-    l = fr_add(l, fr_mul(fr_sub(c, fr_mul(da, db)), S(KAPPA_CU_LOGIC)));
-    l = fr_add(l, quad(e));
-    l = fr_add(l, da4);
-    l = fr_add(l, quad(db));
-    acc = fr_add(acc, fr_mul(fr_mul(l, S(LOGIC_CHALLENGE)), V(LOGIC)));
-    st_fr(out + i, acc);
+    const fr da = fr_sub_lazy(a4, V(A_NEXT)), db = fr_sub_lazy(b4, V(B_NEXT));
+    const fr w = fr_add_lazy(da, db), e = fr_sub_lazy(dn, d4);
+    const fr da2 = fr_sqr(da);
+    const fr u = fr_mul(times(fr_sub_lazy(c4, times(w, 18, kEighteen)), 81, kEightyone), c);
+    const fr inner = fr_sub_lazy(times(w, 81, kEightyone),
+                                 fr_add_lazy(u, times(fr_add_lazy(da2, da2), 18, kEighteen)));
+    const fr A = fr_sub_lazy(times(fr_add_lazy(e, w), 3, kThree), times(fr_mul(inner, c), 166, kTwo83));
+    const fr B = fr_mul(fr_sub_lazy(times(e, 9, kNine), times(w, 3, kThree)), V(Q_C));
+    fr l = MC(fr_add_lazy(A, B), kLogicQu);
+    l = fr_add_lazy(l, MC(fr_sub_lazy(c, fr_mul(da, db)), kLogicCu));
+    l = fr_add_lazy(l, MC(fr_add_lazy(fr_add_lazy(pow4(e), fr_sqr(da2)), pow4(db)), kLogicQuad));
+    st_fr(out + i, fr_add(acc, fr_mul(l, V(LOGIC))));
   }
 }
 
 __global__ void __launch_bounds__(kThreads, 2) k_gate_arith(const GateArgs a, fr *out, uint64_t n) {
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-    const fr a_ = V(A), b = V(B), c = V(C), d = V(D);
-    // arithmetic gate (with the x^alpha S-box terms) and public inputs
-    fr ar = fr_mul(pow_small(d, a.sbox_alpha), V(Q_H4));
-    ar = fr_add(ar, fr_mul(pow_small(b, a.sbox_alpha), V(Q_HR)));
-    ar = fr_add(ar, fr_mul(pow_small(a_, a.sbox_alpha), V(Q_HL)));
-    ar = fr_add(ar, fr_mul(d, V(Q_4)));
-    ar = fr_add(ar, fr_mul(c, V(Q_O)));
-    ar = fr_add(ar, fr_mul(b, V(Q_R)));
-    ar = fr_add(ar, fr_mul(fr_mul(a_, b), V(Q_M)));
-    ar = fr_add(ar, fr_mul(a_, V(Q_L)));
-    ar = fr_add(ar, V(Q_C));
-    const fr acc = fr_add(fr_add(ld_fr(out + i), fr_mul(ar, V(Q_ARITH))), V(PI));
-    st_fr(out + i, acc);
+    // arithmetic gate (with the x^alpha S-box terms) and public inputs: eight
+    // products of a value below 2r and a canonical one, one reduction (their
+    // sum is below 16 r^2, as fr_redc17 allows)
+    uint32_t s[17];
+#pragma unroll
+    for (int k = 0; k < 17; ++k) s[k] = 0;
+    const fr a_ = V(A), b = V(B);
+    fr_mac17(s, pow_small(a_, a.sbox_alpha), V(Q_HL));
+    fr_mac17(s, a_, V(Q_L));
+    fr_mac17(s, pow_small(b, a.sbox_alpha), V(Q_HR));
+    fr_mac17(s, b, V(Q_R));
+    fr_mac17(s, fr_mul(a_, b), V(Q_M));
+    const fr d = V(D);
+    fr_mac17(s, pow_small(d, a.sbox_alpha), V(Q_H4));
+    fr_mac17(s, d, V(Q_4));
+    fr_mac17(s, V(C), V(Q_O));
+    const fr ar = fr_add_raw(fr_redc17(s), V(Q_C));
+    st_fr(out + i, fr_add(fr_add(ld_fr(out + i), fr_mul(ar, V(Q_ARITH))), V(PI)));
   }
 }
 
@@ -236,44 +282,44 @@ __global__ void __launch_bounds__(kThreads, 2) k_gate_groups(const GateArgs a,
                                                           const GateScalars *gs, fr *out,
                                                           uint64_t n) {
   if ((__ldg(&gs->small) != 0) != SMALL) return;
-  __shared__ __align__(16) fr sc[PP_GATE_NS + 1];
-  stage_scalars(gs, sc);
+  __shared__ __align__(16) fr sc[4 * kGateConsts];
+  stage_constants(gs, sc);
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-    const fr a_ = V(A), b = V(B), c = V(C), d = V(D);
+    const fr a_ = V(A), b = V(B), c = V(C);
     const fr an = V(A_NEXT), bn = V(B_NEXT), dn = V(D_NEXT);
-    const fr pd = S(P_D);
     const fr bc = fr_mul(b, c);
-    // fixed-base group addition
-    fr f;
+    fr f, g;
     {
-      const fr abc = fr_mul(a_, bc);
-      const fr dn2 = fr_mul(dn, dn);
-      // one one = 1 when SMALL
-      const fr one2 = SMALL ? fr_one() : fr_mul(S(ONE), S(ONE));
-      const fr qr2 = SMALL ? fr_mul(V(Q_R), dn2) : fr_mul(fr_mul(V(Q_R), dn2), one2);
-      const fr qldn = fr_mul(V(Q_L), dn);
-      f = fr_mul(fr_sub(c, fr_mul(V(Q_C), dn)), S(KAPPA_FB));
-      f = fr_add(f, fr_mul(fr_sub(fr_sub(bn, fr_mul(fr_mul(abc, bn), pd)),
-                                  fr_sub(fr_mul(b, qr2), fr_mul(a_, fr_mul(qldn, S(P_A))))),
-                           S(KAPPA_CU_FB)));
-      f = fr_add(f, SMALL ? fr_mul(dn2, dn) : fr_mul(fr_mul(dn2, dn), one2));
-      f = fr_add(f, fr_mul(fr_sub(fr_add(an, fr_mul(fr_mul(abc, an), pd)),
-                                  fr_add(fr_mul(b, qldn), fr_mul(a_, qr2))),
-                           S(KAPPA_SQ_FB)));
-      f = fr_mul(fr_mul(f, S(FB_CHALLENGE)), V(FIXED_GROUP_ADD));
+      // fixed-base group addition
+      const fr dn2 = fr_sqr(dn), qldn = fr_mul(V(Q_L), dn);
+      fr qr2 = fr_mul(dn2, V(Q_R));
+      if (!SMALL) qr2 = MC(qr2, kOneSq);  // one one = 1 when SMALL
+      const fr abc_pd = MC(fr_mul(a_, bc), kPd);
+      fr u = fr_sub_lazy(fr_sub_lazy(bn, fr_mul(abc_pd, bn)),
+                         fr_sub_lazy(fr_mul(qr2, b), fr_mul(MC(qldn, kPa), a_)));
+      f = MC(u, kFbCu);
+      u = fr_sub_lazy(fr_add_lazy(an, fr_mul(abc_pd, an)), fr_add_lazy(fr_mul(qldn, b), fr_mul(qr2, a_)));
+      f = fr_add_lazy(f, MC(u, kFbSq));
+      f = fr_add_lazy(f, MC(fr_mul(dn2, dn), kFbOne));
+      f = fr_add_lazy(f, MC(fr_sub_lazy(c, fr_mul(V(Q_C), dn)), kFbK));
+      f = fr_mul(f, V(FIXED_GROUP_ADD));
     }
-    // variable-base group addition
-    fr v1 = fr_sub(fr_sub(fr_mul(b, d), fr_mul(fr_mul(a_, c), S(P_A))),
-                   fr_sub(bn, fr_mul(bc, fr_mul(dn, fr_mul(bn, pd)))));
-    v1 = fr_mul(v1, S(KAPPA_SQ_VB));
-    fr v2 = fr_sub(fr_add(dn, bc), fr_add(an, fr_mul(bc, fr_mul(dn, fr_mul(an, pd)))));
-    v2 = fr_add(fr_sub(dn, fr_mul(a_, d)), fr_mul(v2, S(KAPPA_VB)));
-    const fr vb = fr_mul(fr_mul(fr_add(v1, v2), S(VB_CHALLENGE)), V(VARIABLE_GROUP_ADD));
-    st_fr(out + i, fr_add(fr_add(ld_fr(out + i), f), vb));
+    {
+      // variable-base group addition
+      const fr d = V(D);
+      const fr h = MC(fr_mul(bc, dn), kPd);
+      fr u = fr_sub_lazy(fr_sub_lazy(fr_mul(b, d), MC(fr_mul(a_, c), kPa)), fr_sub_lazy(bn, fr_mul(h, bn)));
+      g = MC(u, kVbSq);
+      u = fr_sub_lazy(fr_add_raw(dn, bc), fr_add_lazy(an, fr_mul(h, an)));
+      g = fr_add_lazy(g, MC(u, kVbK));
+      g = fr_add_lazy(g, MC(fr_sub_lazy(dn, fr_mul(a_, d)), kVbOne));
+      g = fr_mul(g, V(VARIABLE_GROUP_ADD));
+    }
+    st_fr(out + i, fr_add(fr_add(ld_fr(out + i), f), g));
   }
 }
-#undef S
+#undef MC
 #undef V
 
 bool aligned16(const void *p) { return p && (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -394,7 +440,7 @@ extern "C" int pp_gate_constraint(const pp_gate_args *a, void *d_out, uint64_t n
   int st = PP_OK;
   auto *gs = static_cast<pp::GateScalars *>(pp::workspace_get(sizeof(pp::GateScalars), s, 8, &st));
   if (st) return st;
-  pp::k_gate_prepare<<<1, 32, 0, s>>>(g, gs);
+  pp::k_gate_prepare<<<1, 128, 0, s>>>(g, gs);
   PP_COUNT_LAUNCH();
   PP_LAUNCH_CHECK();
   // one thread per point; of each pair, the form that does not match the

@@ -986,7 +986,7 @@ PP_HD void fr_add_r_masked(uint32_t o[8], uint32_t mask) {
 
 // a b 2^-256 mod r.  The value before the last step is (a b - M r) / 2^256
 // with 0 <= M < 2^256: above -r, and below r when a b < r 2^256 (b < r and
-// any 256-bit a).  Canonical form adds r to a negative value; LAZY always
+// any 256-bit a; for a, b < 2r it is below 4 r^2 / 2^256 < 1.82 r).  Canonical form adds r to a negative value; LAZY always
 // adds it, leaving 0 < result < 2r.
 template <bool LAZY = false>
 PP_HD fr fr_mul_cells(const fr &a, const fr &b) {
@@ -1118,7 +1118,7 @@ PP_HD void sqr8_cross(uint32_t *E, uint32_t *O, const uint32_t a[8]) {
   if constexpr (I < 6) sqr8_cross<I + 1>(E, O, a);
 }
 
-// r[0..16) = a^2 for a < 2^255: the 28 cross products, doubled, plus the 8
+// r[0..16) = a^2 for any a: the 28 cross products, doubled, plus the 8
 // squares a_i^2 in one carry chain: 36 wide products where a general product
 // needs 64.
 PP_HD void sqr8_cells(uint32_t r[16], const uint32_t a[8]) {
@@ -1132,7 +1132,7 @@ PP_HD void sqr8_cells(uint32_t r[16], const uint32_t a[8]) {
 #pragma unroll
   for (int k = 3; k < 15; ++k) r[k] = addc_cc(E[k], O[k - 1]);
   r[15] = addc(E[15], O[14]);
-  // 2 x (the cross products) < a^2 < 2^510: the shift loses no bit
+  // 2 x (the cross products) < a^2 < 2^512: the shift loses no bit
 #pragma unroll
   for (int k = 15; k > 0; --k) r[k] = (r[k] << 1) | (r[k - 1] >> 31);
   r[0] = madlo_cc(a[0], a[0], r[0]);
@@ -1144,8 +1144,9 @@ PP_HD void sqr8_cells(uint32_t r[16], const uint32_t a[8]) {
   }
 }
 
-// a^2 2^-256 mod r for canonical a (a^2 < r 2^256): the square's 36 wide
-// products, then the reduction's 48
+// a^2 2^-256 mod r: the square's 36 wide products, then the reduction's 48.
+// Canonical for canonical a (a^2 < r 2^256); for a below 2r the result is below
+// 4 r^2 / 2^256 < 1.82 r, as fr_mul's is for two such factors.
 PP_HD fr fr_sqr(const fr &a) {
   uint32_t t[16];
   sqr8_cells(t, a.v);
@@ -1312,6 +1313,45 @@ PP_HD fr fr_sub_lazy(const fr &a, const fr &b) {
   d.v[7] = addc(d.v[7], PP_2R7 & mask);
 #endif
   return d;
+}
+
+// k x mod r below 2r for a lazy x (< 2r) and a small integer k (2 <= k <= 256):
+// y = k x has 264 bits; q = floor(y / r) or one less from its top 32 bits
+// (r 2^-232 rounded up, by a reciprocal), and y - q r = y + q (2^256 - r)
+// modulo 2^256.  16 wide products and about 20 additions, where 9 x by doublings
+// takes 4 lazy additions (112).  The quotient's estimate is short by less than
+// 2^-12 before the floor, so 0 <= y - q r < 1.001 r.
+PP_HD fr fr_mul_small(const fr &x, uint32_t k) {
+  // 2^256 - r
+  const uint32_t nr[8] = {0xffffffffu, 0x00000000u, 0x0001a401u, 0xac425bfdu,
+                          0xf65e27fau, 0xccc627f7u, 0xd66282b7u, 0x8c1258acu};
+  uint32_t E[9], O[9];
+  mul_cells<4>(E, k, x.v);      // words 0 .. 7
+  mul_cells<4>(O, k, x.v + 1);  // words 1 .. 8
+  // y >> 232 up to the carry into word 7: words 7 (O[6] + E[7]) and 8 (O[7])
+  const uint32_t w7 = add_cc(O[6], E[7]);
+  const uint32_t w8 = addc(O[7], 0);
+  const uint32_t t = (w8 << 24) | (w7 >> 8);
+  const uint32_t q = mulhi(t, 2371101800u) >> 22;  // t / (r 2^-232)
+  mad_chain<4>(E, q, nr);
+  mad_chain<4>(O, q, nr + 1);
+  fr o;
+  o.v[0] = E[0];
+  o.v[1] = add_cc(E[1], O[0]);
+#pragma unroll
+  for (int i = 2; i < 7; ++i) o.v[i] = addc_cc(E[i], O[i - 1]);
+  o.v[7] = addc(E[7], O[6]);
+  return o;
+}
+
+// a + b without reduction, for a + b < 2^256
+PP_HD fr fr_add_raw(const fr &a, const fr &b) {
+  fr o;
+  o.v[0] = add_cc(a.v[0], b.v[0]);
+#pragma unroll
+  for (int i = 1; i < 7; ++i) o.v[i] = addc_cc(a.v[i], b.v[i]);
+  o.v[7] = addc(a.v[7], b.v[7]);
+  return o;
 }
 
 // canonical form of a value < 2r

@@ -39,24 +39,6 @@ inline uint32_t gp_blocks_per_sm(uint64_t n) {
 }
 
 // ---------------------------------------------------------------- helpers
-// A field element in shared memory as two 16-byte accesses (p 16-byte
-// aligned).  Read through a plain fr lvalue the compiler issues eight 4-byte
-// loads, and where the address is the same for the whole warp it keeps the
-// words in uniform registers, from which a wide multiply-add runs slower: the
-// dot products' 64-product term took 471 cycles per warp that way, 318 so.
-__device__ __forceinline__ fr lds_fr(const fr *p) {
-  const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
-  fr r;
-  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3])
-               : "r"(a)
-               : "memory");
-  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r.v[4]), "=r"(r.v[5]), "=r"(r.v[6]), "=r"(r.v[7])
-               : "r"(a + 16)
-               : "memory");
-  return r;
-}
 __device__ __forceinline__ void sts_fr(fr *p, const fr &v) { st_fr(p, v); }
 
 // Block scans are work-efficient (Blelloch, "Prefix sums and their
@@ -563,22 +545,9 @@ struct PermArgs {
 constexpr uint32_t kPermRows = 4, kPermBlockRows = kPermRows * kScanThreads;
 constexpr uint32_t kPermSlots = 2 * kPermRows * 2 * kScanThreads;  // 16-byte units: 64 KiB
 
-// x times the constant whose four parts lie at k in shared memory
-__device__ __forceinline__ fr mul_shared_const(const fr &x, const fr *k) {
-  fr w[4];
-#pragma unroll
-  for (int p = 0; p < 4; ++p) w[p] = lds_fr(k + p);
-  return fr_mul_const4(x, w);
-}
-
 // x k + w + gamma below 2r, from canonical w and gamma
 __device__ __forceinline__ fr perm_factor(const fr &xk, const fr &w, const fr &gamma) {
-  fr u;
-  u.v[0] = add_cc(w.v[0], gamma.v[0]);
-#pragma unroll
-  for (int i = 1; i < 7; ++i) u.v[i] = addc_cc(w.v[i], gamma.v[i]);
-  u.v[7] = addc(w.v[7], gamma.v[7]);  // below 2r < 2^256
-  return fr_add_lazy(xk, u);
+  return fr_add_lazy(xk, fr_add_raw(w, gamma));
 }
 
 // Pass 1: the block's terms q_i into z, the block's products of numerators and

@@ -1,7 +1,7 @@
 // Host-side check of the carry-chained field multiplies (csrc/fr.cuh,
 // csrc/fq.cuh): products, squares and lazy products against the row forms,
 // which fr_host_check and g1_host_check hold against the oracle, and the
-// transform's four-part constant multiply against its definition.  Operands are
+// four-part constant multiply and the small multiples against their definitions.  Operands are
 // random and built from limbs 0, 1, 2^32 - 1 and 2^32 - 2, which reach the
 // carry links that random limbs meet once in 2^32 products.  Built and run by tests/test_cells_host.py.
 #include <cstdio>
@@ -59,6 +59,23 @@ int main(int argc, char **argv) {
     }
     const fr four = fr_mul_const4(wide, w);
     bad += four.v[7] > PP_R7 || !fr_eq(fr_mul_row9(fr_mul_row9(fr_canon(four), fr_rr()), p96), sum);
+
+    // small multiples of a lazy value (below 2r): k x (mod r), below 1.002 r
+    fr lazy = wide;
+    lazy.v[7] %= 0xe7db4ea6u;
+    if (it == 3) lazy = fr{{0x00000001u, 0xfffffffeu, 0xfffcb7fdu, 0xa77b4805u, 0x1343b00au, 0x6673b010u,
+                            0x533afa90u, 0xe7db4ea6u}};  // 2r - 1
+    const uint32_t k = it % 2 ? 2 + (uint32_t)(rng() % 255) : 256 - (uint32_t)(it % 7);
+    const fr small = fr_mul_small(lazy, k);
+    fr multiple = fr_zero();
+    for (int bit = 8; bit >= 0; --bit) {
+      multiple = fr_add(multiple, multiple);
+      if ((k >> bit) & 1) multiple = fr_add(multiple, fr_canon(lazy));
+    }
+    bad += small.v[7] >= 0x74100000u || !fr_eq(fr_canon(small), multiple);
+    // squares and products of lazy values stay lazy
+    bad += !fr_eq(fr_canon(fr_sqr(lazy)), fr_mul_row9(fr_canon(lazy), fr_canon(lazy)));
+    bad += !fr_eq(fr_canon(fr_mul_cells(lazy, lazy)), fr_mul_row9(fr_canon(lazy), fr_canon(lazy)));
 
     fq x = operand<fq, 12>(it % 3), y = operand<fq, 12>((it / 3) % 3);
     x.v[11] &= 0x1fffffffu;
