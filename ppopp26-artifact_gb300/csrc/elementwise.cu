@@ -34,16 +34,19 @@ unsigned grid_for(uint64_t work) {
 
 bool aligned16(const void *p) { return p && (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-// c = a op b, or a op b[0] when b_scalar
+// c = a OP b, or a OP b[0] when b_scalar.  One kernel per operation: with the
+// multiply's registers (one kernel for all three) an addition of 2^24 elements
+// takes 6 % longer (HBM bounds it: 227 us, 1.6 GB).
+template <uint32_t OP>
 __global__ void __launch_bounds__(kThreads)
-    k_fr_binary(uint32_t op, const fr *a, const fr *b, fr *c, uint64_t n, int b_scalar) {
+    k_fr_binary(const fr *a, const fr *b, fr *c, uint64_t n, int b_scalar) {
   const fr s = b_scalar ? ld_fr(b) : fr_zero();
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (uint64_t)gridDim.x * blockDim.x) {
     const fr x = ld_fr(a + i), y = b_scalar ? s : ld_fr(b + i);
     fr r;
-    if (op == PP_FR_ADD) r = fr_add(x, y);
-    else if (op == PP_FR_SUB) r = fr_sub(x, y);
+    if (OP == PP_FR_ADD) r = fr_add(x, y);
+    else if (OP == PP_FR_SUB) r = fr_sub(x, y);
     else r = fr_mul(x, y);
     st_fr(c + i, r);
   }
@@ -217,7 +220,10 @@ extern "C" int pp_fr_binary(uint32_t op, const void *d_a, const void *d_b, void 
     b = inv;
     op = PP_FR_MUL;
   }
-  pp::k_fr_binary<<<pp::grid_for(n), pp::kThreads, 0, s>>>(op, a, b, c, n, b_is_scalar);
+  const auto kernel = op == PP_FR_ADD   ? pp::k_fr_binary<PP_FR_ADD>
+                      : op == PP_FR_SUB ? pp::k_fr_binary<PP_FR_SUB>
+                                        : pp::k_fr_binary<PP_FR_MUL>;
+  kernel<<<pp::grid_for(n), pp::kThreads, 0, s>>>(a, b, c, n, b_is_scalar);
   PP_COUNT_LAUNCH();
   PP_LAUNCH_CHECK();
   return PP_OK;
