@@ -90,6 +90,9 @@ __device__ __forceinline__ fr mul_shared_const(const fr &x, const fr *k) {
 // One buffer per (device, stream, slot): work queued on one stream is ordered,
 // so calls on that stream may reuse it; different streams never share one.
 void *workspace_get(size_t bytes, cudaStream_t stream, int slot, int *status);
+// The same, of `most` bytes if the device has them beside the slot's present
+// buffer, else of `least` (kept, or grown as above); *got is which.
+void *workspace_get_most(size_t most, size_t least, cudaStream_t stream, int slot, size_t *got, int *status);
 // frees every workspace of `stream` (call before destroying the stream)
 void workspace_release_stream(cudaStream_t stream);
 // destroys pp_ntt_host_many's cached copy streams and events (pp_release)

@@ -15,20 +15,22 @@
 //                exact); bucket sizes counted with warp-aggregated atomics
 //   2. scan      exclusive prefix sum of the W * 2^(c-1) bucket sizes (tiled)
 //   3. scatter   (point index, sign) into each bucket's slice: a counting sort
-//   4. buckets   the sorted list is cut into equal runs of K entries, one thread
+//   4. pairs     while buckets are large, rounds of affine pair sums with shared
+//                inversions (k_msm_pairs) halve every bucket's entries
+//   5. buckets   the sorted list is cut into equal runs of K entries, one thread
 //                each, whatever the bucket sizes: a thread writes the buckets
 //                that lie inside its run and leaves a partial sum for the one
 //                it shares with the run before and the one after.  A second
 //                launch joins each shared bucket's partial sums (one thread
 //                for a few, blocks for many: a bucket can hold up to all n
 //                points: equal scalars, or the few-bit top window)
-//   5. segments  one thread per run of G buckets: running sums T = sum
+//   6. segments  one thread per run of G buckets: running sums T = sum
 //                (j + 1) B and R = sum B over its run
-//   6. windows   sum T + G sum_s s R_s with sum_s s R_s = sum_k 2^k Q_k, Q_k
+//   7. windows   sum T + G sum_s s R_s with sum_s s R_s = sum_k 2^k Q_k, Q_k
 //                the R_s whose index has bit k set: plain sums in chunks, a
 //                block tree per sum, then one warp per window for the Horner
 //                chain over k
-//   7. final     one warp: Horner over the windows (c doublings each, the
+//   8. final     one warp: Horner over the windows (c doublings each, the
 //                independent multiplies of each step on different lanes), one
 //                inversion to affine
 // Every step is integer-multiply bound (an Fq multiply is ~300 32-bit wide
@@ -188,7 +190,8 @@ __global__ void k_msm_digits(const uint32_t *__restrict__ scalars, uint64_t n, M
 
 // Exclusive prefix sum of len counts into out (len + 1 entries: the last is
 // the total) and, when cursor is not null, a copy of it.  Three launches over
-// tiles of 4096 entries: tile sums, a scan of the tile sums, tile scans.
+// tiles of 4096 entries: tile sums, a scan of the tile sums, tile scans.  With
+// HALVE the counts are those of the offsets in[0 .. len], halved and rounded up.
 constexpr int kScanThreads = 256, kScanItems = 16;
 constexpr uint32_t kScanTile = kScanThreads * kScanItems;
 
@@ -219,6 +222,12 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t *total)
   return before;
 }
 
+template <bool HALVE>
+__device__ __forceinline__ uint32_t scan_count(const uint32_t *in, uint64_t i) {
+  return HALVE ? (in[i + 1] - in[i] + 1) >> 1 : in[i];
+}
+
+template <bool HALVE>
 __global__ void __launch_bounds__(kScanThreads)
     k_scan_tiles(const uint32_t *__restrict__ in, uint64_t len, uint32_t *__restrict__ tile_sum) {
   const uint64_t base = (uint64_t)blockIdx.x * kScanTile;
@@ -226,7 +235,7 @@ __global__ void __launch_bounds__(kScanThreads)
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k) {
     const uint64_t i = base + (uint64_t)k * kScanThreads + threadIdx.x;
-    if (i < len) v += in[i];
+    if (i < len) v += scan_count<HALVE>(in, i);
   }
   uint32_t total;
   block_excl_scan(v, &total);
@@ -249,6 +258,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_top(uint32_t *tile_sum, u
   if (threadIdx.x == 0) tile_sum[ntiles] = total;
 }
 
+template <bool HALVE>
 __global__ void __launch_bounds__(kScanThreads)
     k_scan_down(const uint32_t *__restrict__ in, uint64_t len, const uint32_t *__restrict__ tile_off,
                 uint32_t ntiles, uint32_t *__restrict__ out, uint32_t *__restrict__ cursor) {
@@ -256,7 +266,7 @@ __global__ void __launch_bounds__(kScanThreads)
   uint32_t v[kScanItems], sum = 0;
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k) {
-    v[k] = base + k < len ? in[base + k] : 0;
+    v[k] = base + k < len ? scan_count<HALVE>(in, base + k) : 0;
     sum += v[k];
   }
   uint32_t total;
@@ -272,16 +282,17 @@ __global__ void __launch_bounds__(kScanThreads)
   if (blockIdx.x == 0 && threadIdx.x == 0) out[len] = tile_off[ntiles];
 }
 
+template <bool HALVE>
 int scan_u32(const uint32_t *in, uint64_t len, uint32_t *out, uint32_t *cursor, uint32_t *tiles,
              cudaStream_t s) {
   const uint32_t ntiles = (uint32_t)((len + kScanTile - 1) / kScanTile);
-  k_scan_tiles<<<ntiles, kScanThreads, 0, s>>>(in, len, tiles);
+  k_scan_tiles<HALVE><<<ntiles, kScanThreads, 0, s>>>(in, len, tiles);
   PP_COUNT_LAUNCH();
   PP_LAUNCH_CHECK();
   k_scan_top<<<1, kScanThreads, 0, s>>>(tiles, ntiles);
   PP_COUNT_LAUNCH();
   PP_LAUNCH_CHECK();
-  k_scan_down<<<ntiles, kScanThreads, 0, s>>>(in, len, tiles, ntiles, out, cursor);
+  k_scan_down<HALVE><<<ntiles, kScanThreads, 0, s>>>(in, len, tiles, ntiles, out, cursor);
   PP_COUNT_LAUNCH();
   PP_LAUNCH_CHECK();
   return PP_OK;
@@ -318,11 +329,31 @@ constexpr uint32_t kJoinChunk = 1024;      // partial sums one block adds up
 // sums and workspace than they save.  The kernels take it from the list's real
 // length (zero digits have no entry): half of 2^18 scalars zero and the rest one
 // took 1638 us with runs sized for a full list.
+__host__ __device__ __forceinline__ uint32_t equal_run(uint64_t items, uint32_t resident, uint32_t least,
+                                                       uint32_t most) {
+  const uint64_t span = (uint64_t)resident * most;
+  const uint64_t waves = items ? (items + span - 1) / span : 1;
+  const uint64_t K = (items + resident * waves - 1) / (resident * waves);
+  return (uint32_t)(K < least ? least : K);
+}
 __host__ __device__ __forceinline__ uint32_t run_length(uint64_t entries, uint32_t resident) {
-  const uint64_t span = (uint64_t)resident * kRunMax;
-  const uint64_t waves = entries ? (entries + span - 1) / span : 1;
-  const uint64_t K = (entries + resident * waves - 1) / (resident * waves);
-  return (uint32_t)(K < kRunMin ? kRunMin : K);
+  return equal_run(entries, resident, kRunMin, kRunMax);
+}
+// Outputs per thread of a round of pair sums: longer runs spread the inversion
+// over more sums, shorter ones even out the SMs.  Fixed-base 2^20 points, three
+// rounds, with at most 80 / 160 / 320: 6.27 / 6.23 / 6.23 ms; 2^22 points 23.6 /
+// 23.3 / 23.4 ms.
+constexpr uint32_t kPairMin = 16, kPairMax = 160;
+__host__ __device__ __forceinline__ uint32_t pair_run(uint64_t outputs, uint32_t resident) {
+  return equal_run(outputs, resident, kPairMin, kPairMax);
+}
+// runs of a list of at most that many items, at most: their length is least or
+// more, and a shorter list makes no more waves
+inline uint32_t most_runs(uint64_t items, uint32_t resident, uint32_t least, uint32_t most) {
+  const uint64_t span = (uint64_t)resident * most;
+  const uint64_t by_waves = (uint64_t)resident * ((items + span - 1) / span);
+  const uint64_t by_least = items / least + 1;
+  return (uint32_t)(by_least < by_waves ? by_least : by_waves);
 }
 // partial sums of a bucket that one thread joins: twice an average bucket's
 __device__ __forceinline__ uint32_t join_few(uint32_t entries, uint32_t nb, uint32_t K) {
@@ -341,6 +372,241 @@ __device__ __forceinline__ uint32_t bucket_of(const uint32_t *off, uint32_t nb, 
   return lo;
 }
 
+__device__ __forceinline__ fq ld_fq(const fq *p) {
+  const uint4 *q = reinterpret_cast<const uint4 *>(p);
+  fq r;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const uint4 u = q[k];
+    r.v[4 * k] = u.x, r.v[4 * k + 1] = u.y, r.v[4 * k + 2] = u.z, r.v[4 * k + 3] = u.w;
+  }
+  return r;
+}
+__device__ __forceinline__ void st_fq(fq *p, const fq &a) {
+  uint4 *q = reinterpret_cast<uint4 *>(p);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) q[k] = make_uint4(a.v[4 * k], a.v[4 * k + 1], a.v[4 * k + 2], a.v[4 * k + 3]);
+}
+
+// Entry k of a sorted list: point list[k] & 0x7fffffff, negated when bit 31 is
+// set, or (without a list) points[k].
+struct EntryPoints {
+  const g1a *points;
+  const uint32_t *list;
+  __device__ __forceinline__ uint32_t key(uint32_t k) const { return list ? list[k] : k; }
+  __device__ __forceinline__ fq x(uint32_t key) const { return ld_fq(&points[key & 0x7fffffffu].x); }
+  __device__ __forceinline__ fq y(uint32_t key) const {
+    const fq v = ld_fq(&points[key & 0x7fffffffu].y);
+    return list && key >> 31 ? fq_neg(v) : v;  // fq_neg(0) = 0: infinity stays all zero
+  }
+};
+
+// What an output of a round of pair sums is: a copy of the point with key k1, the
+// point at infinity, or a sum that takes a division.
+enum PairKind : uint32_t { kPairCopy, kPairNone, kPairDouble, kPairAdd };
+
+// 16-byte units of a thread's operands in shared memory, [unit][thread]: two
+// slots of x1, x2, y1, y2 and the parked product
+constexpr uint32_t kPairUnits = 15, kPairSmem = 2 * kPairUnits * kPointThreads * 16;
+__device__ __forceinline__ void fetch_fq(uint4 *dst, const fq *p) {
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst + k * kPointThreads);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(d),
+                 "l"(reinterpret_cast<const uint4 *>(p) + k)
+                 : "memory");
+  }
+}
+__device__ __forceinline__ fq take_fq(const uint4 *src) {
+  fq r;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const uint4 u = src[k * kPointThreads];
+    r.v[4 * k] = u.x, r.v[4 * k + 1] = u.y, r.v[4 * k + 2] = u.z, r.v[4 * k + 3] = u.w;
+  }
+  return r;
+}
+
+// One round of pair sums: the entries off[b] .. off[b+1] of each bucket become
+// half as many, out[next[b] + j] = entry 2j + entry 2j + 1 in affine form.  An
+// affine sum costs a division, y' = l (x1 - x') - y1 with l = (y2 - y1) / (x2 - x1),
+// and a thread's divisions share one inversion (Montgomery's simultaneous
+// inversion): five multiplies and a square a sum, plus the share of the
+// inversion, against eight and two squares of a sum into an XYZZ accumulator.
+// A warp takes 32 K outputs in a row, neighbouring lanes neighbouring ones.  The
+// forward pass leaves each output's keys and kind in its y and the product of
+// the divisors before it in its x, for the backward pass.  Operands are copied
+// to shared memory one step ahead, keys loaded two steps ahead (with plain loads
+// the gathers' latency took the whole gain: 1.55 against 1.27 ms for 4.5 M sums).
+// All lanes make K steps and meet at each multiply: left to themselves, the
+// lanes of a warp drift apart at the branches and 18 of 32 work.  One warp
+// inverts for its block, an inversion for 128 K sums: each thread inverting for
+// itself took 6.35 instead of 6.23 ms.  Bound by the multiply pipe (69 % busy)
+// and by the one inversion's latency, per round.  Bucket sums in all, fixed-base
+// 2^20 points: 6.98 -> 6.23 ms; 2^20 points 8.42 -> 7.87 ms, 2^22 26.7 -> 22.5.
+__global__ void __launch_bounds__(kPointThreads, kAccumulateBlocks)
+    k_msm_pairs(EntryPoints in, const uint32_t *__restrict__ off, const uint32_t *__restrict__ next,
+                uint32_t nb, uint32_t resident, g1a *out) {
+  extern __shared__ uint4 pair_sm[];
+  const uint32_t total = next[nb], K = pair_run(total, resident);
+  const uint64_t block0 = (uint64_t)blockIdx.x * kPointThreads * K;
+  if (block0 >= total) return;
+  // this lane's outputs: lo + 32 i, i < m
+  const uint64_t lo64 = block0 + (uint64_t)(threadIdx.x & ~31u) * K + (threadIdx.x & 31);
+  const uint32_t lo = lo64 < total ? (uint32_t)lo64 : total;
+  const uint32_t left = (total - lo + 31) / 32, m = left < K ? left : K;
+  uint4 *const sm = pair_sm + threadIdx.x;
+  const auto slot = [&](uint32_t i) { return sm + (i & 1) * kPairUnits * kPointThreads; };
+  constexpr uint32_t U = 3 * kPointThreads;  // x1, x2, y1, y2, product: U apart
+
+  uint32_t b = m ? bucket_of(next, nb, lo) : 0, begin = next[b], end = next[b + 1];
+  // keys of output i of this lane; k2 = k1 for a bucket's odd entry
+  const auto keys = [&](uint32_t i, uint32_t &k1, uint32_t &k2) {
+    k1 = k2 = 0;
+    if (i >= m) return;
+    const uint32_t o = lo + 32 * i;
+    for (int k = 0; o >= end && k < 8; ++k) ++b, begin = end, end = next[b + 1];
+    if (o >= end) b = bucket_of(next, nb, o), begin = next[b], end = next[b + 1];
+    const uint32_t src = off[b] + 2 * (o - begin);
+    const bool two = src + 1 < off[b + 1];
+    k1 = in.key(src);
+    k2 = two ? in.key(src + 1) : kNone;
+  };
+  const auto fetch_x = [&](uint32_t i, uint32_t k1, uint32_t k2) {
+    if (i < m && k2 != kNone) {
+      fetch_fq(slot(i), &in.points[k1 & 0x7fffffffu].x);
+      fetch_fq(slot(i) + U, &in.points[k2 & 0x7fffffffu].x);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  uint32_t a1, a2, b1, b2;  // keys of steps i and i + 1
+  keys(0, a1, a2);
+  keys(1, b1, b2);
+  fetch_x(0, a1, a2);
+  fq prod = fq_one();
+#pragma unroll 1
+  for (uint32_t i = 0; i < K; ++i) {
+    fetch_x(i + 1, b1, b2);
+    uint32_t c1, c2;
+    keys(i + 2, c1, c2);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    fq d = fq_one();
+    if (i < m) {
+      g1a *dst = out + lo + 32 * (uint64_t)i;
+      PairKind kind = kPairCopy;
+      if (a2 != kNone) {
+        const fq x1 = take_fq(slot(i)), x2 = take_fq(slot(i) + U);
+        d = fq_sub(x2, x1);
+        const bool z1 = fq_is_zero(x1), z2 = fq_is_zero(x2), same = fq_is_zero(d);
+        kind = kPairAdd;
+        if (z1 | z2 | same) {  // infinity, or equal abscissae: the ordinates decide
+          const fq y1 = in.y(a1), y2 = in.y(a2);
+          if (z2 && fq_is_zero(y2)) {
+            kind = kPairCopy;
+          } else if (z1 && fq_is_zero(y1)) {
+            kind = kPairCopy, a1 = a2;
+          } else if (same) {
+            kind = fq_is_zero(fq_sub(y1, y2)) && !fq_is_zero(y1) ? kPairDouble : kPairNone;
+          }
+          if (kind == kPairDouble) d = fq_dbl(y1);
+          else if (kind != kPairAdd) d = fq_one();
+        }
+        if (kind >= kPairDouble) st_fq(&dst->x, prod);
+      }
+      *reinterpret_cast<uint4 *>(&dst->y) = make_uint4(a1, a2, kind, 0);
+    }
+    a1 = b1, a2 = b2, b1 = c1, b2 = c2;
+    __syncwarp();
+    prod = fq_mul(prod, d);
+  }
+  // 1 / prod (a product of non-zero values): the first warp inverts for the
+  // block, lane l the product of threads l, l + 32, l + 64 and l + 96
+  fq *const shared = reinterpret_cast<fq *>(pair_sm);
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  st_fq(shared + threadIdx.x, prod);
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    fq *q = shared + threadIdx.x;
+    fq before[kPointThreads / 32 - 1];  // products of the first 1, 2, 3
+    fq all = ld_fq(q);
+#pragma unroll
+    for (int k = 1; k < kPointThreads / 32; ++k) {
+      before[k - 1] = all;
+      all = fq_mul(all, ld_fq(q + 32 * k));
+    }
+    all = fq_inv_fast(all);
+#pragma unroll
+    for (int k = kPointThreads / 32 - 1; k > 0; --k) {
+      const fq p = ld_fq(q + 32 * k);
+      st_fq(q + 32 * k, fq_mul(all, before[k - 1]));
+      all = fq_mul(all, p);
+    }
+    st_fq(q, all);
+  }
+  __syncthreads();
+  fq inv = ld_fq(shared + threadIdx.x);
+  __syncthreads();
+
+  const auto load_info = [&](uint32_t i) {  // i may have wrapped below zero
+    uint4 r = make_uint4(0, 0, kPairNone, 0);
+    if (i < m) r = *reinterpret_cast<const uint4 *>(&out[lo + 32 * (uint64_t)i].y);
+    return r;
+  };
+  const auto fetch_all = [&](uint32_t i, const uint4 &f) {
+    if (f.z != kPairNone) {
+      const g1a *p1 = in.points + (f.x & 0x7fffffffu), *p2 = in.points + (f.y & 0x7fffffffu);
+      fetch_fq(slot(i), &p1->x);
+      fetch_fq(slot(i) + 2 * U, &p1->y);
+      if (f.z == kPairAdd) {
+        fetch_fq(slot(i) + U, &p2->x);
+        fetch_fq(slot(i) + 3 * U, &p2->y);
+      }
+      if (f.z >= kPairDouble) fetch_fq(slot(i) + 4 * U, &out[lo + 32 * (uint64_t)i].x);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  uint4 f0 = load_info(K - 1), f1 = load_info(K - 2);
+  fetch_all(K - 1, f0);
+#pragma unroll 1
+  for (uint32_t i = K; i-- > 0;) {
+    fetch_all(i - 1, f1);
+    const uint4 f2 = load_info(i - 2);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    fq x = fq_zero(), y = x, x2 = x, num = x, before = x, d = fq_one();
+    if (f0.z != kPairNone) {
+      x = take_fq(slot(i));
+      y = take_fq(slot(i) + 2 * U);
+      if (in.list && f0.x >> 31) y = fq_neg(y);
+      if (f0.z >= kPairDouble) before = take_fq(slot(i) + 4 * U);
+      if (f0.z == kPairAdd) {
+        x2 = take_fq(slot(i) + U);
+        num = take_fq(slot(i) + 3 * U);
+        if (in.list && f0.y >> 31) num = fq_neg(num);
+        num = fq_sub(num, y);
+        d = fq_sub(x2, x);
+      } else if (f0.z == kPairDouble) {
+        const fq xx = fq_sqr(x);
+        num = fq_add(fq_dbl(xx), xx);
+        x2 = x;
+        d = fq_dbl(y);
+      }
+    }
+    __syncwarp();
+    const fq l = fq_mul(num, fq_mul(inv, before));
+    inv = fq_mul(inv, d);
+    const fq x3 = fq_sub(fq_sub(fq_sqr(l), x), x2);
+    const fq y3 = fq_sub(fq_mul(l, fq_sub(x, x3)), y);
+    if (i < m) {
+      g1a *dst = out + lo + 32 * (uint64_t)i;
+      st_fq(&dst->x, f0.z >= kPairDouble ? x3 : x);
+      st_fq(&dst->y, f0.z >= kPairDouble ? y3 : y);
+    }
+    f0 = f1, f1 = f2;
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
 // Bucket sums.  Thread t adds the signed affine points of entries [t K, (t+1) K)
 // of the sorted list, starting a new sum at each bucket boundary.  Every lane
 // does the same number of additions, so the warps are full whatever the buckets
@@ -352,8 +618,7 @@ __device__ __forceinline__ uint32_t bucket_of(const uint32_t *off, uint32_t nb, 
 // run before goes to part[2 t], the one shared only with the run after to
 // part[2 t + 1].  Bound by the multiply pipe.
 __global__ void __launch_bounds__(kPointThreads, kAccumulateBlocks)
-    k_msm_accumulate(const g1a *__restrict__ points, const uint32_t *__restrict__ list,
-                     const uint32_t *__restrict__ off, uint32_t nb, uint32_t resident,
+    k_msm_accumulate(EntryPoints in, const uint32_t *__restrict__ off, uint32_t nb, uint32_t resident,
                      g1x *__restrict__ part, g1x *__restrict__ buckets) {
   const uint32_t total = off[nb], K = run_length(total, resident);
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -375,10 +640,8 @@ __global__ void __launch_bounds__(kPointThreads, kAccumulateBlocks)
       } while (end == k);  // skips empty buckets
       acc = g1x_inf();
     }
-    const uint32_t e = list[k];
-    g1a pt = ld_g1a(points + (e & 0x7fffffffu));
-    if (e >> 31) pt = g1a_neg(pt);
-    acc = g1x_add_affine(acc, pt);
+    const uint32_t e = in.key(k);
+    acc = g1x_add_affine(acc, g1a{in.x(e), in.y(e)});
   }
 }
 
@@ -688,23 +951,38 @@ __global__ void __launch_bounds__(32) k_msm_final(const g1x *__restrict__ win, M
 
 struct MsmLayout {
   size_t digits, counts, n_items, offsets, cursor, list, part, items, multi, chunk_sum, buckets, seg_t,
-      seg_r, chunks, sums, win, tiles, total;
+      seg_r, chunks, sums, win, tiles, pairs[2], pair_off, total;
   uint32_t resident; // threads of k_msm_accumulate resident at once
   uint32_t runs;     // runs of the list at most
 };
 
-MsmLayout msm_layout(uint64_t n, const MsmPlan &p) {
+// Rounds of pair sums before the buckets are accumulated: while a round has 28
+// outputs per resident thread, over which an inversion and the round's launches
+// spread, and 8 per bucket, below which unpaired entries and steps between buckets
+// take the gain.  Milliseconds with 0, 1, 2, 3 and 4 rounds (rule's choice marked):
+//   200003 points  3.13 3.08* 3.12 3.30 3.55   window tables 2.03 2.00* 2.07 2.25
+//   2^20 points    8.42 7.97 7.87* 7.94 8.10   window tables 6.97 6.46 6.29 6.23* 6.26
+//   2^22 points    26.7 24.4 23.1 22.6 22.5*
+//   2^16 points    2.05* 2.18 2.47             window tables 1.16* 1.35 1.53
+// The bound on the entries keeps the rounds' buffers below 20 GB.
+uint32_t pair_rounds(uint64_t n, const MsmPlan &p) {
+  const uint64_t entries = (uint64_t)p.W * n, nb = (uint64_t)p.nsets * p.B;
+  const uint64_t resident = (uint64_t)device_sm_count() * kAccumulateBlocks * kPointThreads;
+  uint32_t r = 0;
+  if (entries <= 1ull << 28)
+    while ((entries >> (r + 1)) >= 28 * resident && (entries >> (r + 1)) >= 8 * nb) ++r;
+  return r;
+}
+// outputs of a round over that many inputs, at most: every bucket rounds up
+inline uint64_t pair_outputs(uint64_t inputs, uint64_t nb) { return (inputs + nb) / 2; }
+
+MsmLayout msm_layout(uint64_t n, const MsmPlan &p, uint32_t rounds) {
   MsmLayout L{};
   auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
   const uint64_t nb = (uint64_t)p.nsets * p.B;
   const uint64_t entries = (uint64_t)p.W * n;
   L.resident = (uint32_t)device_sm_count() * kAccumulateBlocks * kPointThreads;
-  // run_length gives at most entries / kRunMin + 1 runs, and at most a full
-  // list's number of waves
-  const uint64_t span = (uint64_t)L.resident * kRunMax;
-  const uint64_t by_waves = (uint64_t)L.resident * ((entries + span - 1) / span);
-  const uint64_t by_min = entries / kRunMin + 1;
-  L.runs = (uint32_t)(by_min < by_waves ? by_min : by_waves);
+  L.runs = most_runs(entries, L.resident, kRunMin, kRunMax);
   // each run leaves at most two partial sums, and a listed bucket has more than
   // kJoinMin of them: at most 2 runs / 9 buckets, plus one item per full chunk
   const uint64_t items = L.runs / 4 + 64, multi = 2 * (uint64_t)L.runs / kJoinChunk + 1;
@@ -726,6 +1004,12 @@ MsmLayout msm_layout(uint64_t n, const MsmPlan &p) {
   L.sums = o, o += up((size_t)p.nsets * (1 + p.lgS) * sizeof(g1x));
   L.win = o, o += up((size_t)p.nsets * sizeof(g1x));
   L.tiles = o, o += up(((nb + kScanTile - 1) / kScanTile + 1) * 4);
+  if (rounds > 0) {  // the rounds write two buffers in turn
+    const uint64_t first = pair_outputs(entries, nb);
+    L.pairs[0] = o, o += up(first * sizeof(g1a));
+    if (rounds > 1) L.pairs[1] = o, o += up(pair_outputs(first, nb) * sizeof(g1a));
+  }
+  L.pair_off = o, o += rounds ? up((nb + 1) * 4) : 0;
   L.total = o;
   return L;
 }
@@ -804,10 +1088,14 @@ uint32_t fixed_window_bits(uint64_t n) {
 // scalars n plain 256-bit integers; out receives (x, y, 1), or zeros.
 int msm_run(const g1a *points, const uint32_t *scalars, uint64_t n, const MsmPlan &p, fq *out,
             cudaStream_t s) {
-  const MsmLayout L = msm_layout(n, p);
+  uint32_t rounds = pair_rounds(n, p);
+  MsmLayout L = msm_layout(n, p, rounds);
+  const MsmLayout least = msm_layout(n, p, 0);
+  size_t got = 0;
   int st = PP_OK;
-  char *ws = static_cast<char *>(workspace_get(L.total, s, 3, &st));
+  char *ws = static_cast<char *>(workspace_get_most(L.total, least.total, s, 3, &got, &st));
   if (st) return st;
+  if (got < L.total) L = least, rounds = 0;  // no room for the rounds' buffers
   auto u32 = [&](size_t off) { return reinterpret_cast<uint32_t *>(ws + off); };
   auto pts = [&](size_t off) { return reinterpret_cast<g1x *>(ws + off); };
   uint32_t *digits = u32(L.digits), *counts = u32(L.counts), *offsets = u32(L.offsets);
@@ -823,15 +1111,35 @@ int msm_run(const g1a *points, const uint32_t *scalars, uint64_t n, const MsmPla
   k_msm_digits<<<grid_for(n, 256), 256, 0, s>>>(scalars, n, p, digits, counts);
   PP_COUNT_LAUNCH();
   PP_LAUNCH_CHECK();
-  if ((st = scan_u32(counts, nb, offsets, cursor, tiles, s))) return st;
+  if ((st = scan_u32<false>(counts, nb, offsets, cursor, tiles, s))) return st;
   k_msm_scatter<<<grid_for((uint64_t)p.W * n, 256), 256, 0, s>>>(digits, n, p, cursor, list);
   PP_COUNT_LAUNCH();
   PP_LAUNCH_CHECK();
 
-  // 4: bucket sums over equal runs of the list, then the shared buckets
+  // 4: rounds of pair sums, each halving every bucket's entries
+  EntryPoints in{points, list};
+  uint32_t *spare = u32(L.pair_off);
+  if (rounds)
+    PP_CUDA_TRY(cudaFuncSetAttribute(k_msm_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmem));
+  uint64_t left = (uint64_t)p.W * n;
+  for (uint32_t r = 0; r < rounds; ++r) {
+    if ((st = scan_u32<true>(offsets, nb, spare, nullptr, tiles, s))) return st;
+    left = pair_outputs(left, nb);
+    g1a *pair_sums = reinterpret_cast<g1a *>(ws + L.pairs[r & 1]);
+    k_msm_pairs<<<grid_for(most_runs(left, L.resident, kPairMin, kPairMax), kPointThreads),
+                  kPointThreads, kPairSmem, s>>>(in, offsets, spare, (uint32_t)nb, L.resident, pair_sums);
+    PP_COUNT_LAUNCH();
+    PP_LAUNCH_CHECK();
+    in = EntryPoints{pair_sums, nullptr};
+    uint32_t *const t = offsets;
+    offsets = spare;
+    spare = t;
+  }
+
+  // 5: bucket sums over equal runs of the list, then the shared buckets
   PP_CUDA_TRY(cudaMemsetAsync(buckets, 0, nb * sizeof(g1x), s));  // all zero = infinity
   k_msm_accumulate<<<grid_for(L.runs, kPointThreads), kPointThreads, 0, s>>>(
-      points, list, offsets, (uint32_t)nb, L.resident, part, buckets);
+      in, offsets, (uint32_t)nb, L.resident, part, buckets);
   PP_COUNT_LAUNCH();
   PP_LAUNCH_CHECK();
   k_msm_spans<<<grid_for(nb, 256), 256, 0, s>>>(offsets, (uint32_t)nb, L.resident, items, multi,
@@ -848,7 +1156,7 @@ int msm_run(const g1a *points, const uint32_t *scalars, uint64_t n, const MsmPla
   PP_COUNT_LAUNCH();
   PP_LAUNCH_CHECK();
 
-  // 5-7: weighted bucket sums per bucket set, sets combined, affine result
+  // 6-8: weighted bucket sums per bucket set, sets combined, affine result
   k_msm_segments<<<grid_for((uint64_t)p.nsets * p.S, kPointThreads), kPointThreads, 0, s>>>(
       buckets, p, seg_t, seg_r);
   PP_COUNT_LAUNCH();

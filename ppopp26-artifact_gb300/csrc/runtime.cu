@@ -94,6 +94,46 @@ void *workspace_get(size_t bytes, cudaStream_t stream, int slot, int *status) {
   return b.ptr;
 }
 
+void *workspace_get_most(size_t most, size_t least, cudaStream_t stream, int slot, size_t *got, int *status) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) {
+    *status = PP_E_CUDA;
+    set_error("cudaGetDevice failed");
+    return nullptr;
+  }
+  {
+    std::lock_guard<std::mutex> lk(g_ws_mu);
+    WsBuf &b = g_ws[WsKey{dev, stream, slot}];
+    void *larger = nullptr;
+    // a capture must not allocate: the buffer at hand does
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (b.bytes < most && b.bytes >= least) cudaStreamIsCapturing(stream, &capture);
+    if (b.bytes < most && capture == cudaStreamCaptureStatusNone) {
+      PP_COUNT_ALLOC(most);
+      if (cudaMalloc(&larger, most) != cudaSuccess) {
+        cudaGetLastError();
+        larger = nullptr;
+      }
+    }
+    if (larger) {
+      if (b.ptr) {
+        // the old buffer may still be in use by queued work on this stream
+        cudaStreamSynchronize(stream);
+        cudaFree(b.ptr);
+      }
+      b.ptr = larger;
+      b.bytes = most;
+    }
+    if (b.bytes >= most) {
+      *got = most;
+      *status = PP_OK;
+      return b.ptr;
+    }
+  }
+  *got = least;
+  return workspace_get(least, stream, slot, status);
+}
+
 // frees the workspaces of one stream (before the stream is destroyed); a
 // later stream may reuse the handle value, so stale entries must not stay
 void workspace_release_stream(cudaStream_t stream) {
