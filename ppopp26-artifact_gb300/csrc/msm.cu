@@ -39,6 +39,7 @@
 #include <cstring>
 
 #include "common.cuh"
+#include "fq_lanes.cuh"
 #include "g1.cuh"
 
 namespace pp {
@@ -54,6 +55,7 @@ struct MsmPlan {
   uint32_t S;      // segments per bucket set, B / G
   uint32_t lgG;    // log2 G
   uint32_t lgS;    // log2 S
+  uint32_t chunk;  // terms per thread of the window sums (k_msm_bitsums)
   uint32_t nsets;  // bucket sets: W (one per window), or 1 with window tables
 };
 
@@ -61,6 +63,12 @@ struct MsmPlan {
 // gives 2^15 segment threads.  On GB300 this beat fixed 4, 8 and 16 (2^16
 // points: 16 -> 4.65 ms, 4 -> 3.92 ms; 2^22: 4 -> 53.2 ms, 16 -> 51.3 ms).
 constexpr uint32_t kSegmentMax = 16, kSegmentMin = 4, kSegmentThreads = 1u << 15;
+
+// Terms per thread of the window sums: 8, and 4 where that leaves the chip less
+// than full and a block of k_msm_bitreduce at most two chunks per thread.  8 / 4:
+// 200003 points 2.575 / 2.551 ms, 2^14 1.189 / 1.165; but with one bucket set 2^16
+// points (8192 segments) 1.059 / 1.117, and 2^20 points 7.37 / 7.39.
+constexpr uint32_t kChunkMax = 8, kChunkThreads = 1u << 14, kChunkSum = 2048;
 
 // the rest of a plan once c and the number of bucket sets are fixed
 MsmPlan msm_plan_for(uint32_t c, uint32_t nsets) {
@@ -74,6 +82,8 @@ MsmPlan msm_plan_for(uint32_t c, uint32_t nsets) {
   p.S = p.B / p.G;
   while ((1u << p.lgG) < p.G) ++p.lgG;
   while ((1u << p.lgS) < p.S) ++p.lgS;
+  p.chunk = kChunkMax;
+  if ((uint64_t)nsets * (2 + p.lgS) * p.S / (2 * kChunkMax) <= kChunkThreads && p.S <= kChunkSum) p.chunk /= 2;
   return p;
 }
 
@@ -143,21 +153,29 @@ __device__ __forceinline__ uint32_t window_bits(const uint32_t s[8], uint32_t of
   return (uint32_t)(x >> sh) & ((1u << c) - 1);
 }
 
-// atomicAdd(base + key, 1) for every active lane, one atomic per distinct key
-// in the warp; returns the old value plus the lane's rank among equal keys
+// atomicAdd(base + key, 1) for every active lane; returns the old value plus the
+// lane's rank among its group.  Lanes with the first active lane's key, or that of the
+// first of the others, make one atomic together (equal or few scalars: up to all n
+// entries fall into a bucket); the rest one each (random ones hardly ever meet).
+// With __match_any_sync the digits of 200003 points took 100 us without the
+// returned place, 82 so.
 __device__ __forceinline__ uint32_t warp_increment(uint32_t *base, uint32_t key) {
   const uint32_t mask = __activemask();
-  const uint32_t same = __match_any_sync(mask, key);
-  const int lane = threadIdx.x & 31;
-  const int leader = __ffs(same) - 1;
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t g0 = __ballot_sync(mask, key == __shfl_sync(mask, key, __ffs(mask) - 1));
+  const uint32_t rest = mask & ~g0;
+  const uint32_t g1 = __ballot_sync(mask, key == __shfl_sync(mask, key, __ffs(rest ? rest : mask) - 1)) & rest;
+  const uint32_t same = g0 >> lane & 1 ? g0 : g1 >> lane & 1 ? g1 : 1u << lane;
+  const uint32_t leader = __ffs(same) - 1;
   uint32_t old = 0;
   if (lane == leader) old = atomicAdd(base + key, (uint32_t)__popc(same));
-  old = __shfl_sync(same, old, leader);
+  old = __shfl_sync(mask, old, leader);
   return old + __popc(same & ((1u << lane) - 1));
 }
 
 __global__ void k_msm_digits(const uint32_t *__restrict__ scalars, uint64_t n, MsmPlan p,
-                             uint32_t *__restrict__ digits, uint32_t *__restrict__ counts) {
+                             uint32_t *__restrict__ digits, uint32_t *__restrict__ rank,
+                             uint32_t *__restrict__ counts) {
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (uint64_t)gridDim.x * blockDim.x) {
     uint32_t s[8];
@@ -181,7 +199,7 @@ __global__ void k_msm_digits(const uint32_t *__restrict__ scalars, uint64_t n, M
       if (mag) {
         const uint32_t bucket = mag - 1;
         e = (bucket << 1) | sign;
-        warp_increment(counts, (p.nsets > 1 ? w * p.B : 0) + bucket);
+        rank[(uint64_t)w * n + i] = warp_increment(counts, (p.nsets > 1 ? w * p.B : 0) + bucket);
       }
       digits[(uint64_t)w * n + i] = e;
     }
@@ -189,7 +207,7 @@ __global__ void k_msm_digits(const uint32_t *__restrict__ scalars, uint64_t n, M
 }
 
 // Exclusive prefix sum of len counts into out (len + 1 entries: the last is
-// the total) and, when cursor is not null, a copy of it.  Three launches over
+// the total).  Three launches over
 // tiles of 4096 entries: tile sums, a scan of the tile sums, tile scans.  With
 // HALVE the counts are those of the offsets in[0 .. len], halved and rounded up.
 constexpr int kScanThreads = 256, kScanItems = 16;
@@ -261,7 +279,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_top(uint32_t *tile_sum, u
 template <bool HALVE>
 __global__ void __launch_bounds__(kScanThreads)
     k_scan_down(const uint32_t *__restrict__ in, uint64_t len, const uint32_t *__restrict__ tile_off,
-                uint32_t ntiles, uint32_t *__restrict__ out, uint32_t *__restrict__ cursor) {
+                uint32_t ntiles, uint32_t *__restrict__ out) {
   const uint64_t base = (uint64_t)blockIdx.x * kScanTile + (uint64_t)threadIdx.x * kScanItems;
   uint32_t v[kScanItems], sum = 0;
 #pragma unroll
@@ -275,7 +293,6 @@ __global__ void __launch_bounds__(kScanThreads)
   for (int k = 0; k < kScanItems; ++k) {
     if (base + k < len) {
       out[base + k] = run;
-      if (cursor) cursor[base + k] = run;
     }
     run += v[k];
   }
@@ -283,8 +300,7 @@ __global__ void __launch_bounds__(kScanThreads)
 }
 
 template <bool HALVE>
-int scan_u32(const uint32_t *in, uint64_t len, uint32_t *out, uint32_t *cursor, uint32_t *tiles,
-             cudaStream_t s) {
+int scan_u32(const uint32_t *in, uint64_t len, uint32_t *out, uint32_t *tiles, cudaStream_t s) {
   const uint32_t ntiles = (uint32_t)((len + kScanTile - 1) / kScanTile);
   k_scan_tiles<HALVE><<<ntiles, kScanThreads, 0, s>>>(in, len, tiles);
   PP_COUNT_LAUNCH();
@@ -292,16 +308,19 @@ int scan_u32(const uint32_t *in, uint64_t len, uint32_t *out, uint32_t *cursor, 
   k_scan_top<<<1, kScanThreads, 0, s>>>(tiles, ntiles);
   PP_COUNT_LAUNCH();
   PP_LAUNCH_CHECK();
-  k_scan_down<HALVE><<<ntiles, kScanThreads, 0, s>>>(in, len, tiles, ntiles, out, cursor);
+  k_scan_down<HALVE><<<ntiles, kScanThreads, 0, s>>>(in, len, tiles, ntiles, out);
   PP_COUNT_LAUNCH();
   PP_LAUNCH_CHECK();
   return PP_OK;
 }
 
+// The digits kernel left each entry's place in its bucket (its atomic's result), so
+// this one needs no atomics: 200003 points 113 -> 33 us.
 // With one bucket set per window an entry names its point i; with window
 // tables (one bucket set) it names the table entry w n + i = 2^(c w) P_i.
 __global__ void k_msm_scatter(const uint32_t *__restrict__ digits, uint64_t n, MsmPlan p,
-                              uint32_t *__restrict__ cursor, uint32_t *__restrict__ list) {
+                              const uint32_t *__restrict__ rank, const uint32_t *__restrict__ off,
+                              uint32_t *__restrict__ list) {
   const uint64_t total = (uint64_t)p.W * n;
   for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total;
        t += (uint64_t)gridDim.x * blockDim.x) {
@@ -309,15 +328,15 @@ __global__ void k_msm_scatter(const uint32_t *__restrict__ digits, uint64_t n, M
     if (e == kNone) continue;
     const uint64_t w = t / n, i = t - w * n;
     const bool per_window = p.nsets > 1;
-    const uint32_t pos = warp_increment(cursor, (per_window ? (uint32_t)(w * p.B) : 0u) + (e >> 1));
-    list[pos] = (uint32_t)(per_window ? i : t) | ((e & 1u) << 31);
+    list[off[(per_window ? (uint32_t)(w * p.B) : 0u) + (e >> 1)] + rank[t]] = (uint32_t)(per_window ? i : t) | ((e & 1u) << 31);
   }
 }
 
 constexpr int kPointThreads = 128;
 constexpr int kAccumulateBlocks = 3;       // resident blocks per SM (168 registers)
 constexpr uint32_t kRunMin = 10, kRunMax = 64;
-constexpr uint32_t kJoinMin = 8;           // partial sums one thread adds up
+constexpr uint32_t kJoinMin = 3;           // partial sums one thread adds up (3 / 5 / 8:
+                                           // 200003 points 2.42 / 2.45 / 2.47 ms)
 constexpr uint32_t kJoinChunk = 1024;      // partial sums one block adds up
 
 // Entries per run for a list of that many: as many runs as threads are resident
@@ -675,18 +694,132 @@ __global__ void k_msm_spans(const uint32_t *__restrict__ off, uint32_t nb, uint3
   if (chunks > 1) multi[atomicAdd(n_items + 1, 1u)] = make_uint2(b, first);
 }
 
+// ---- Points spread over a warp (fq_lanes.cuh): Y with element 0, X with 1, ZZ with
+// 3, ZZZ with 4; element 2 is scratch.  X and Y are below 1.04 q, ZZ below 1.9 q and
+// ZZZ below 1.5 q; ZZ = 0 or q is infinity.  For chains and trees that are
+// bound by the latency of dependent additions: a doubling 1.46 us, an addition 2.2 us, against
+// 3.56 (its multiplies on four lanes) and 13 us (one lane).
+__device__ __forceinline__ digit point_load(const Spread &S, const g1x *p) {
+  const uint32_t c = S.el == 0 ? 12 : S.el == 3 ? 24 : S.el == 4 ? 36 : 0;
+  const uint2 w = *reinterpret_cast<const uint2 *>(reinterpret_cast<const uint32_t *>(p) + c + 2 * S.k);
+  return {w.x, w.y, 0};
+}
+// as it is
+__device__ __forceinline__ void point_park(const Spread &S, const digit &P, g1x *p) {
+  const uint32_t c = S.el == 0 ? 12 : S.el == 1 ? 0 : S.el == 3 ? 24 : 36;
+  if (S.el < 5 && S.el != 2)
+    *reinterpret_cast<uint2 *>(reinterpret_cast<uint32_t *>(p) + c + 2 * S.k) = make_uint2(P.l, P.h);
+}
+// with reduced coordinates
+__device__ __forceinline__ void point_store(const Spread &S, const digit &P, g1x *p) {
+  const uint32_t c = S.lane & 3;  // X, Y, ZZ, ZZZ
+  const uint32_t from = c == 0 ? 1 : c == 1 ? 0 : c + 1;
+  fq v;
+#pragma unroll
+  for (uint32_t k = 0; k < kSpread; ++k) {
+    v.v[2 * k] = __shfl_sync(0xffffffffu, P.l, from * kSpread + k);
+    v.v[2 * k + 1] = __shfl_sync(0xffffffffu, P.h, from * kSpread + k);
+  }
+  v = fq_mul(v, fq_one());
+  if (S.lane < 4) st_fq(&p->x + c, v);
+}
+// (the same for all lanes)
+__device__ __forceinline__ bool point_is_inf(const Spread &S, const digit &P) {
+  return element_all(__ballot_sync(0xffffffffu, (P.l | P.h) == 0), 3) ||
+         element_all(__ballot_sync(0xffffffffu, P.l == S.q[0][0] && P.h == S.q[0][1]), 3);
+}
+
+// dbl-2008-s-1; Y = 0 gives ZZ = 0.  Bounds in units of q: V < 4.5, M < 3.4, S < 1.5,
+// W < 3, M (S - X') < 2.3.
+__device__ __forceinline__ digit point_dbl(const Spread &S, const digit &P) {
+  const uint32_t el = S.el;
+  digit r = S.mul(P, P);                    // Y^2 (0), X^2 (1)
+  digit g = S.from(r, el == 2 ? 1 : 0);     // Y^2 (0, 1, 3), X^2 (2)
+  const digit g2 = Spread::add(g, g);
+  const digit m = S.norm(Spread::add(g2, sel_digit(el == 2, g, g2)));  // V = 4 Y^2, M = 3 X^2 (2)
+  // W / 2 = Y V (0), S = X V (1), M^2 (2), ZZ' = ZZ V (3)
+  r = S.mul(sel_digit(el == 2, m, P), m);
+  r = sel_digit(el == 0, Spread::add(r, r), r);
+  g = S.from(r, el == 1 ? 2 : el == 2 ? 1 : 0);  // M^2 (1), S (2), W (4)
+  const digit s = sel_digit(el == 2, g, r), mm = sel_digit(el == 2, r, g);
+  // X' = M^2 - 2 S (1, 2); W (0, 4), ZZ' (3)
+  digit x = S.reduce(Spread::sub(Spread::sub(Spread::add(mm, S.multiple(3)), s), s));
+  x = S.norm(sel_digit(el == 1 || el == 2, x, sel_digit(el == 4, g, r)));
+  // W Y (0), M (S - X') (2), ZZZ' = W ZZZ (4)
+  const digit d = S.norm(sel_digit(el == 2, Spread::sub(Spread::add(s, S.multiple(2)), x), x));
+  r = S.mul(sel_digit(el == 2, m, P), d);
+  // Y' = M (S - X') - W Y (0), ZZZ' (4)
+  const digit y = S.reduce(Spread::sub(Spread::add(S.from(r, 2), S.multiple(2)), r));
+  r = S.norm(sel_digit(el == 0, y, r));
+  return sel_digit(el == 0 || el == 4, r, x);
+}
+
+// add-2008-s.  Bounds in units of q: products of coordinates < 1.4, P, R < 3.2,
+// P^2, R^2 < 2.1, P^3 < 1.7, Q < 1.3, R (Q - X') < 2.1.
+__device__ __forceinline__ digit point_add(const Spread &S, const digit &A, const digit &B) {
+  if (point_is_inf(S, B)) return A;
+  if (point_is_inf(S, A)) return B;
+  const uint32_t el = S.el;
+  // s1 = Y1 ZZZ2 (0), u1 = X1 ZZ2 (1), u2 = X2 ZZ1 (2), ZZ1 ZZ2 (3), s2 = Y2 ZZZ1 (4)
+  const digit b1 = S.from(B, el == 2 ? 1 : 0), b2 = S.from(B, el == 0 ? 4 : 3), a1 = S.from(A, 3);
+  digit r = S.mul(sel_digit(el == 2 || el == 4, b1, A), sel_digit(el == 2, a1, sel_digit(el == 4, A, b2)));
+  // R = s2 - s1 (0), P = u2 - u1 (1), u1 (2), ZZ1 ZZ2 (3), s1 (4)
+  digit g = S.from(r, el == 0 ? 4 : el == 1 ? 2 : el == 2 ? 1 : 0);
+  const digit diff = Spread::sub(Spread::add(g, S.multiple(2)), r);
+  const digit d = S.norm(sel_digit(el < 2, diff, sel_digit(el == 3, r, g)));
+  const digit z = S.norm(S.reduce(d));
+  const uint32_t zero = __ballot_sync(0xffffffffu, (z.l | z.h) == 0);
+  const uint32_t isq = __ballot_sync(0xffffffffu, z.l == S.q[0][0] && z.h == S.q[0][1]);
+  if (element_all(zero, 1) || element_all(isq, 1)) {  // equal x: the same point or opposite ones
+    if (element_all(zero, 0) || element_all(isq, 0)) return point_dbl(S, A);
+    return {0, 0, 0};
+  }
+  // R^2 (0), P^2 (1), ZZZ1 ZZZ2 (2)
+  const digit a4 = S.from(A, 4), b4 = S.from(B, 4);
+  const digit r2 = S.mul(sel_digit(el == 2, a4, d), sel_digit(el == 2, b4, d));
+  const digit pp = S.norm(S.from(r2, 1));
+  // P^3 (1), Q = u1 P^2 (2), ZZ' = ZZ1 ZZ2 P^2 (3)
+  const digit r3 = S.mul(d, pp);
+  const digit ppp = S.norm(S.from(r3, 1)), q = S.from(r3, 2);
+  // X' = R^2 - P^3 - 2 Q (all)
+  digit x = Spread::add(Spread::add(S.from(r2, 0), S.multiple(2)), S.multiple(3));
+  x = S.norm(S.reduce(Spread::sub(Spread::sub(Spread::sub(x, ppp), q), q)));
+  const digit e = S.norm(Spread::sub(Spread::add(q, S.multiple(2)), x));
+  // R (Q - X') (0), ZZZ' = ZZZ1 ZZZ2 P^3 (2), s1 P^3 (4)
+  r = S.mul(S.norm(sel_digit(el == 2, r2, d)), sel_digit(el == 0, e, ppp));
+  g = S.from(r, el == 0 ? 4 : 2);
+  const digit y = S.reduce(Spread::sub(Spread::add(r, S.multiple(2)), g));
+  return S.norm(sel_digit(el == 0, y, sel_digit(el == 3, r3, sel_digit(el == 4, g, x))));
+}
+
 // sum of val(j), lo <= j < hi, by a block of kPointThreads (the result in
-// thread 0): strided sums, then a tree in shared memory
+// red[0] for all): strided sums, then a tree in shared memory, its lower levels
+// with a warp to each addition (k_msm_bitreduce at 200003 points: 106 -> 71 us)
+constexpr uint32_t kWarpAdds = 16;
 template <typename F>
 __device__ __forceinline__ g1x block_sum(uint32_t lo, uint32_t hi, g1x *red, F val) {
   g1x acc = g1x_inf();
   for (uint32_t j = lo + threadIdx.x; j < hi; j += kPointThreads) acc = g1x_add(acc, val(j));
   red[threadIdx.x] = acc;
   __syncthreads();
-  for (uint32_t h = kPointThreads / 2; h > 0; h >>= 1) {
+  for (uint32_t h = kPointThreads / 2; h > kWarpAdds; h >>= 1) {
     if (threadIdx.x < h) red[threadIdx.x] = g1x_add(red[threadIdx.x], red[threadIdx.x + h]);
     __syncthreads();
   }
+  const Spread S;
+  for (uint32_t h = kWarpAdds; h > 0; h >>= 1) {
+    for (uint32_t i = threadIdx.x / 32; i < h; i += kPointThreads / 32) {
+      const digit a = point_load(S, red + i), b = point_load(S, red + i + h);
+      if (point_is_inf(S, b)) continue;
+      point_park(S, point_add(S, a, b), red + i);
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x < 32) {
+    const digit a = point_load(S, red);
+    point_store(S, a, red);
+  }
+  __syncthreads();
   const g1x r = red[0];
   __syncthreads();  // red may be used again
   return r;
@@ -700,7 +833,7 @@ __global__ void __launch_bounds__(kPointThreads)
                uint32_t resident, uint32_t small_blocks, const uint2 *__restrict__ items,
                const uint32_t *__restrict__ n_items, g1x *__restrict__ chunk_sum,
                g1x *__restrict__ buckets) {
-  __shared__ g1x red[kPointThreads];
+  __shared__ __align__(16) g1x red[kPointThreads];
   const uint32_t K = run_length(off[nb], resident);
   if (blockIdx.x < small_blocks) {
     const uint32_t few = join_few(off[nb], nb, K);
@@ -729,7 +862,7 @@ __global__ void __launch_bounds__(kPointThreads)
                       const uint2 *__restrict__ multi,
                       const uint32_t *__restrict__ n_items, const g1x *__restrict__ chunk_sum,
                       g1x *__restrict__ buckets) {
-  __shared__ g1x red[kPointThreads];
+  __shared__ __align__(16) g1x red[kPointThreads];
   const uint32_t n = n_items[1], K = run_length(off[nb], resident);
   for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
     const uint2 mb = multi[i];
@@ -766,20 +899,18 @@ __global__ void __launch_bounds__(kPointThreads)
 // sum_s T_s, sum j = 1 + k is Q_k) and one short Horner chain; no sum weights
 // a point by more than one doubling at a time.
 //
-// Each sum is cut into chunks of kChunk terms; one thread adds one chunk (8
+// Each sum is cut into chunks of p.chunk terms; one thread adds one chunk (8
 // instead of 16 terms: 303 -> 118 us of dependent additions).
 // Window w's chunks are part[w ncw + u]: u < nc0 for sum 0, then nc1 chunks
 // for each Q_k in order of k.
-constexpr uint32_t kChunk = 8;
-
 struct ChunkCounts {
   uint32_t nc0, nc1, ncw;
 };
 
 __host__ __device__ __forceinline__ ChunkCounts chunk_counts(const MsmPlan &p) {
   ChunkCounts c;
-  c.nc0 = (p.S + kChunk - 1) / kChunk;
-  c.nc1 = (p.S / 2 + kChunk - 1) / kChunk;
+  c.nc0 = (p.S + p.chunk - 1) / p.chunk;
+  c.nc1 = (p.S / 2 + p.chunk - 1) / p.chunk;
   c.ncw = c.nc0 + p.lgS * c.nc1;
   return c;
 }
@@ -795,13 +926,13 @@ __global__ void __launch_bounds__(kPointThreads)
     g1x acc = g1x_inf();
     if (u < cc.nc0) {
       const g1x *row = seg_t + (uint64_t)w * p.S;
-      const uint32_t lo = u * kChunk, hi = lo + kChunk < p.S ? lo + kChunk : p.S;
+      const uint32_t lo = u * p.chunk, hi = lo + p.chunk < p.S ? lo + p.chunk : p.S;
       for (uint32_t i = lo; i < hi; ++i) acc = g1x_add(acc, row[i]);
     } else {
       const uint32_t k = (u - cc.nc0) / cc.nc1, ch = (u - cc.nc0) - k * cc.nc1;
       const g1x *row = seg_r + (uint64_t)w * p.S;
       const uint32_t half = p.S >> 1;
-      const uint32_t lo = ch * kChunk, hi = lo + kChunk < half ? lo + kChunk : half;
+      const uint32_t lo = ch * p.chunk, hi = lo + p.chunk < half ? lo + p.chunk : half;
       for (uint32_t i = lo; i < hi; ++i) {
         // the i-th segment index with bit k set
         const uint32_t s = ((i >> k) << (k + 1)) | (1u << k) | (i & ((1u << k) - 1));
@@ -815,7 +946,7 @@ __global__ void __launch_bounds__(kPointThreads)
 // One block per (window, sum): the sum's chunks.  sums[w (1 + lg S) + j].
 __global__ void __launch_bounds__(kPointThreads)
     k_msm_bitreduce(const g1x *__restrict__ part, MsmPlan p, g1x *__restrict__ sums) {
-  __shared__ g1x red[kPointThreads];
+  __shared__ __align__(16) g1x red[kPointThreads];
   const ChunkCounts cc = chunk_counts(p);
   const uint32_t L = 1 + p.lgS;
   const uint32_t w = blockIdx.x / L, j = blockIdx.x - w * L;
@@ -824,133 +955,46 @@ __global__ void __launch_bounds__(kPointThreads)
   if (threadIdx.x == 0) sums[blockIdx.x] = sum;
 }
 
-// ---- Horner chains in one warp.  They are bound by the latency of dependent
-// multiplies, so the independent ones of a doubling (3 levels instead of 9
-// multiplies) or of an addition (4 levels instead of 14) run on different
-// lanes and are exchanged by shuffles.
-__device__ __forceinline__ fq shfl_fq(const fq &a, int src) {
-  fq r;
-#pragma unroll
-  for (int i = 0; i < 12; ++i) r.v[i] = __shfl_sync(0xffffffffu, a.v[i], src);
-  return r;
-}
-__device__ __forceinline__ fq sel_fq(bool c, const fq &a, const fq &b) {
-  fq r;
-#pragma unroll
-  for (int i = 0; i < 12; ++i) r.v[i] = c ? a.v[i] : b.v[i];
-  return r;
-}
-
-// 2^n p for a point that every lane holds.  During the chain the coordinates
-// live apart, Y in lane 0, X in lane 1, ZZ and ZZZ in lane 3, so a level of
-// multiplies needs one exchange of 12 words, each lane fetching the one operand
-// it lacks (dbl-2008-s-1; Y = 0 needs no test: it gives ZZ = 0).
-// The multiplies are inlined: the loop is the kernel.  200003 points (247
-// doublings): the final chain took 1.0 ms when every lane held the whole point
-// and each product was broadcast, 0.88 ms so.
-__device__ g1x dbl_chain(const g1x &p, uint32_t n) {
-  if (g1x_is_inf(p)) return p;  // the upper windows of short scalars are empty
-  const int lane = threadIdx.x & 31;
-  const int src1 = lane == 2 ? 1 : 0;
-  const int src2 = lane == 1 ? 2 : lane == 2 ? 1 : 0;
-  fq P = sel_fq(lane == 0, p.y, sel_fq(lane == 1, p.x, p.zz)), Z = p.zzz;
-#pragma unroll 1
-  for (uint32_t k = 0; k < n; ++k) {
-    // u = 2Y (0), X (1), ZZ (3); squares V = u^2 (0), X^2 (1)
-    const fq u = sel_fq(lane == 0, fq_dbl(P), P);
-    fq r = fq_sqr_cells(u);
-    fq g = shfl_fq(r, src1);  // V (0, 1, 3), X^2 (2)
-    const fq m = fq_add(fq_dbl(g), g);  // M = 3 X^2 (2)
-    // W = u V (0), S = X V (1), M^2 (2), ZZ' = ZZ V (3)
-    const fq r2 = fq_mul_cells(sel_fq(lane == 2, m, u), sel_fq(lane == 2, m, g));
-    g = shfl_fq(r2, src2);  // M^2 (1), S (2), W (3)
-    const fq s = sel_fq(lane == 2, g, r2), mm = sel_fq(lane == 2, r2, g);
-    const fq x = fq_sub(mm, fq_dbl(s));  // X' (1, 2)
-    // W Y (0), M (S - X') (2), ZZZ' = W ZZZ (3)
-    const fq a = sel_fq(lane == 0, r2, sel_fq(lane == 2, m, g));
-    const fq b = sel_fq(lane == 0, P, sel_fq(lane == 2, fq_sub(s, x), Z));
-    r = fq_mul_cells(a, b);
-    g = shfl_fq(r, 2);
-    P = sel_fq(lane == 0, fq_sub(g, r), sel_fq(lane == 1, x, r2));
-    Z = r;
-  }
-  g1x o;
-  o.y = shfl_fq(P, 0);
-  o.x = shfl_fq(P, 1);
-  o.zz = shfl_fq(P, 3);
-  o.zzz = shfl_fq(Z, 3);
-  return o;
-}
-
-__device__ g1x add_warp(const g1x &p, const g1x &q) {
-  if (g1x_is_inf(q)) return p;
-  if (g1x_is_inf(p)) return q;
-  const int lane = threadIdx.x & 31;
-  // u1 = X1 ZZ2, u2 = X2 ZZ1, s1 = Y1 ZZZ2, s2 = Y2 ZZZ1, ZZ1 ZZ2, ZZZ1 ZZZ2
-  fq a = lane == 0 ? p.x : lane == 1 ? q.x : lane == 2 ? p.y : lane == 3 ? q.y
-         : lane == 4 ? p.zz : p.zzz;
-  fq b = lane == 0 ? q.zz : lane == 1 ? p.zz : lane == 2 ? q.zzz : lane == 3 ? p.zzz
-         : lane == 4 ? q.zz : q.zzz;
-  fq r = fq_mul(a, b);
-  const fq u1 = shfl_fq(r, 0), u2 = shfl_fq(r, 1), s1 = shfl_fq(r, 2), s2 = shfl_fq(r, 3);
-  const fq zz12 = shfl_fq(r, 4), zzz12 = shfl_fq(r, 5);
-  const fq P = fq_sub(u2, u1), R = fq_sub(s2, s1);
-  if (fq_is_zero(P)) return fq_is_zero(R) ? dbl_chain(p, 1) : g1x_inf();
-  // P^2 (0), R^2 (1)
-  a = lane == 0 ? P : R;
-  r = fq_sqr(a);
-  const fq pp = shfl_fq(r, 0), rr = shfl_fq(r, 1);
-  // P pp (0), u1 pp (1), zz12 pp (2)
-  a = lane == 0 ? P : lane == 1 ? u1 : zz12;
-  r = fq_mul(a, pp);
-  const fq ppp = shfl_fq(r, 0), Q = shfl_fq(r, 1);
-  g1x o;
-  o.zz = shfl_fq(r, 2);
-  o.x = fq_sub(fq_sub(rr, ppp), fq_dbl(Q));
-  // R (Q - x') (0), s1 ppp (1), zzz12 ppp (2)
-  a = lane == 0 ? R : lane == 1 ? s1 : zzz12;
-  b = lane == 0 ? fq_sub(Q, o.x) : ppp;
-  r = fq_mul(a, b);
-  o.y = fq_sub(shfl_fq(r, 0), shfl_fq(r, 1));
-  o.zzz = shfl_fq(r, 2);
-  return o;
-}
-
 // One warp per window: win[w] = sum_s T_s + G sum_k 2^k Q_k (Horner over k)
 __global__ void __launch_bounds__(32) k_msm_wincombine(const g1x *__restrict__ sums, MsmPlan p,
                                                        g1x *__restrict__ win) {
-  const uint32_t w = blockIdx.x;
-  const g1x *q = sums + (uint64_t)w * (1 + p.lgS);  // q[0] = sum T, q[1 + k] = Q_k
-  g1x acc = p.lgS ? q[p.lgS] : g1x_inf();
+  const Spread S;
+  const g1x *q = sums + (uint64_t)blockIdx.x * (1 + p.lgS);  // q[0] = sum T, q[1 + k] = Q_k
+  digit acc = {0, 0, 0};
 #pragma unroll 1
-  for (int k = (int)p.lgS - 2; k >= -1; --k) {
+  for (int k = (int)p.lgS - 1; k >= -1; --k) {
     // Q_k after one doubling, then (k = -1) sum_s T_s after lg G
-    acc = dbl_chain(acc, k >= 0 ? 1 : p.lgG);
-    acc = add_warp(acc, q[1 + k]);
+    for (uint32_t j = k >= 0 ? 1 : p.lgG; j > 0; --j) acc = point_dbl(S, acc);
+    acc = point_add(S, acc, point_load(S, q + 1 + k));
   }
-  if (threadIdx.x == 0) win[w] = acc;
+  point_store(S, acc, win + blockIdx.x);
 }
 
 // Horner over the windows (one warp), then affine; out = Jacobian (x, y, 1),
 // or all zero for the point at infinity
 __global__ void __launch_bounds__(32) k_msm_final(const g1x *__restrict__ win, MsmPlan p,
                                                   fq *__restrict__ out) {
-  g1x acc = win[p.nsets - 1];
+  __shared__ __align__(16) g1x sum;
+  const Spread S;
+  digit acc = {0, 0, 0};
 #pragma unroll 1
-  for (int w = (int)p.nsets - 2; w >= 0; --w) {
-    acc = dbl_chain(acc, p.c);
-    acc = add_warp(acc, win[w]);
+  for (int w = (int)p.nsets - 1; w >= 0; --w) {
+    if (!point_is_inf(S, acc))  // the upper windows of short scalars are empty
+      for (uint32_t j = 0; j < p.c; ++j) acc = point_dbl(S, acc);
+    acc = point_add(S, acc, point_load(S, win + w));
   }
+  point_store(S, acc, &sum);
+  __syncwarp();
   if (threadIdx.x != 0) return;
-  const g1a a = g1x_to_affine(acc);
-  const bool inf = g1x_is_inf(acc);
+  const g1a a = g1x_to_affine(sum);
+  const bool inf = g1x_is_inf(sum);
   out[0] = a.x;
   out[1] = a.y;
   out[2] = inf ? fq_zero() : fq_one();
 }
 
 struct MsmLayout {
-  size_t digits, counts, n_items, offsets, cursor, list, part, items, multi, chunk_sum, buckets, seg_t,
+  size_t digits, counts, n_items, offsets, list, part, items, multi, chunk_sum, buckets, seg_t,
       seg_r, chunks, sums, win, tiles, pairs[2], pair_off, total;
   uint32_t resident; // threads of k_msm_accumulate resident at once
   uint32_t runs;     // runs of the list at most
@@ -984,15 +1028,15 @@ MsmLayout msm_layout(uint64_t n, const MsmPlan &p, uint32_t rounds) {
   L.resident = (uint32_t)device_sm_count() * kAccumulateBlocks * kPointThreads;
   L.runs = most_runs(entries, L.resident, kRunMin, kRunMax);
   // each run leaves at most two partial sums, and a listed bucket has more than
-  // kJoinMin of them: at most 2 runs / 9 buckets, plus one item per full chunk
-  const uint64_t items = L.runs / 4 + 64, multi = 2 * (uint64_t)L.runs / kJoinChunk + 1;
+  // kJoinMin of them: at most 2 runs / 4 buckets, plus one item per full chunk
+  const uint64_t items = L.runs / 2 + 2 * (uint64_t)L.runs / kJoinChunk + 64, multi = 2 * (uint64_t)L.runs / kJoinChunk + 1;
   size_t o = 0;
   L.digits = o, o += up(entries * 4);
   L.counts = o, o += nb * 4;
   L.n_items = o, o = up(o + 8);  // cleared with the counts
   L.offsets = o, o += up((nb + 1) * 4);
-  L.cursor = o, o += up(nb * 4);
   L.list = o, o += up(entries * 4);
+  // the entries' ranks first: 384 bytes per run of at most kRunMax entries
   L.part = o, o += up(2 * (size_t)L.runs * sizeof(g1x));
   L.items = o, o += up(items * sizeof(uint2));
   L.multi = o, o += up(multi * sizeof(uint2));
@@ -1099,7 +1143,7 @@ int msm_run(const g1a *points, const uint32_t *scalars, uint64_t n, const MsmPla
   auto u32 = [&](size_t off) { return reinterpret_cast<uint32_t *>(ws + off); };
   auto pts = [&](size_t off) { return reinterpret_cast<g1x *>(ws + off); };
   uint32_t *digits = u32(L.digits), *counts = u32(L.counts), *offsets = u32(L.offsets);
-  uint32_t *cursor = u32(L.cursor), *list = u32(L.list), *n_items = u32(L.n_items);
+  uint32_t *rank = u32(L.part), *list = u32(L.list), *n_items = u32(L.n_items);
   uint32_t *tiles = u32(L.tiles);
   uint2 *items = reinterpret_cast<uint2 *>(ws + L.items), *multi = reinterpret_cast<uint2 *>(ws + L.multi);
   g1x *buckets = pts(L.buckets), *seg_t = pts(L.seg_t), *seg_r = pts(L.seg_r), *win = pts(L.win);
@@ -1108,11 +1152,11 @@ int msm_run(const g1a *points, const uint32_t *scalars, uint64_t n, const MsmPla
 
   // 1-3: signed digits, bucket sizes, counting sort of (point, sign) by bucket
   PP_CUDA_TRY(cudaMemsetAsync(counts, 0, nb * 4 + 8, s));  // and n_items
-  k_msm_digits<<<grid_for(n, 256), 256, 0, s>>>(scalars, n, p, digits, counts);
+  k_msm_digits<<<grid_for(n, 256), 256, 0, s>>>(scalars, n, p, digits, rank, counts);
   PP_COUNT_LAUNCH();
   PP_LAUNCH_CHECK();
-  if ((st = scan_u32<false>(counts, nb, offsets, cursor, tiles, s))) return st;
-  k_msm_scatter<<<grid_for((uint64_t)p.W * n, 256), 256, 0, s>>>(digits, n, p, cursor, list);
+  if ((st = scan_u32<false>(counts, nb, offsets, tiles, s))) return st;
+  k_msm_scatter<<<grid_for((uint64_t)p.W * n, 256), 256, 0, s>>>(digits, n, p, rank, offsets, list);
   PP_COUNT_LAUNCH();
   PP_LAUNCH_CHECK();
 
@@ -1123,7 +1167,7 @@ int msm_run(const g1a *points, const uint32_t *scalars, uint64_t n, const MsmPla
     PP_CUDA_TRY(cudaFuncSetAttribute(k_msm_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmem));
   uint64_t left = (uint64_t)p.W * n;
   for (uint32_t r = 0; r < rounds; ++r) {
-    if ((st = scan_u32<true>(offsets, nb, spare, nullptr, tiles, s))) return st;
+    if ((st = scan_u32<true>(offsets, nb, spare, tiles, s))) return st;
     left = pair_outputs(left, nb);
     g1a *pair_sums = reinterpret_cast<g1a *>(ws + L.pairs[r & 1]);
     k_msm_pairs<<<grid_for(most_runs(left, L.resident, kPairMin, kPairMax), kPointThreads),
