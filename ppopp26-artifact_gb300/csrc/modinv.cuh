@@ -10,7 +10,9 @@
 //   g even:               (1 + delta, f, g / 2)
 // Starting from (1, M, x) it reaches g = 0 with f = +-gcd(M, x) = +-1 within
 // floor((49 * 256 + 57) / 17) = 741 steps for 256-bit inputs, and within
-// 1101 for 381-bit ones.
+// 1101 for 381-bit ones.  Starting from delta = 1/2 instead it takes fewer: at most
+// 590 and 879 (P. Wuille and G. Maxwell, "Bounds on divsteps iterations in safegcd",
+// 2021).
 //
 // B divsteps depend only on the low B + 2 bits of f and g, so they run on
 // one machine word each and record a 2x2 integer matrix T with
@@ -23,12 +25,12 @@
 // top one are in [0, 2^B) and the top limb carries the sign.  Two widths:
 // B = 30 on 32-bit words with 64-bit sums (the GPU form: every limb product
 // is one 32 x 32 -> 64-bit multiply-add) and B = 62 on 64-bit words with
-// 128-bit sums (a 64-bit host CPU's form).  Measured on a GB300 (ns per
-// Fr inversion, 9728 warps):
-//                         30-bit   62-bit   binary GCD
-//   warp-uniform            21.5     30.5       37.6
-//   one per lane             1.0      1.6        4.6
-//   one thread (latency)   34.8 us  41.8 us    54.0 us
+// 128-bit sums (a 64-bit host CPU's form; on a GB300 it took 1.2 to 1.6 times
+// the 30-bit form's time, a binary GCD 1.6 to 4.6 times).
+//
+// GB300, 30-bit form: a lone thread inverts in 19.4 us (Fr) and 33.3 us (Fq); 34.5
+// and 57.1 us one divstep at a time with d and e reduced after each batch.  One per lane,
+// 9728 warps: 0.65 and 1.18 ns (0.96 and 1.89).
 #pragma once
 #include <cstdint>
 
@@ -76,51 +78,51 @@ PP_HD int ctz_word(uint64_t x) {
 #endif
 }
 
-// ---- B divsteps on the low words.  Returns the updated delta; T in u..r.
+// ---- B divsteps on the low words.  Returns the updated D = delta - 1/2; T in u..r.
+// A divstep with delta <= 0 keeps f and adds it to an odd g before halving, so up to
+// 1/2 - delta = -D of them in a row come to one: g + w f with the w that clears the
+// low bits, w = -g / f modulo a power of two; f (f^2 - 2) = -1 / f modulo 2^6 for odd
+// f, since (f^2 - 1)^2 is a multiple of 64.  One with delta > 0 is an exchange
+// (f, g) -> (g, -f), delta -> -delta, and such a step.
 template <typename L>
-PP_HD int divsteps_word(int delta, typename LimbTraits<L>::U f0, typename LimbTraits<L>::U g0,
+PP_HD int divsteps_word(int D, typename LimbTraits<L>::U f0, typename LimbTraits<L>::U g0,
                         L &u_out, L &v_out, L &q_out, L &r_out) {
   using U = typename LimbTraits<L>::U;
   constexpr int B = LimbTraits<L>::B;
-  L u = 1, v = 0, q = 0, r = 1;
-  int i = 0;
-  while (i < B) {
-    if (!(g0 & 1)) {
-      // a run of zero bits: g / 2^z and the f row times 2^z
-      int z = g0 ? ctz_word(g0) : B;
-      if (z > B - i) z = B - i;
-      g0 >>= z;
-      u = (L)((U)u << z);
-      v = (L)((U)v << z);
-      delta += z;
-      i += z;
-      continue;
+  U u = 1, v = 0, q = 0, r = 1;
+  int left = B;
+  for (;;) {
+    const int z = ctz_word(g0 | ((U)~(U)0 << left));  // a run of zero bits, at most `left`
+    g0 >>= z;
+    u <<= z;
+    v <<= z;
+    D += z;
+    left -= z;
+    if (left == 0) break;
+    if (D >= 0) {
+      D = -D - 1;
+      U t = f0;
+      f0 = g0;
+      g0 = 0 - t;
+      t = u;
+      u = q;
+      q = 0 - t;
+      t = v;
+      v = r;
+      r = 0 - t;
     }
-    if (delta > 0) {
-      const U nf = g0;
-      g0 = (g0 - f0) >> 1;
-      f0 = nf;
-      const L nu = (L)(2 * q), nv = (L)(2 * r);
-      q -= u;
-      r -= v;
-      u = nu;
-      v = nv;
-      delta = 1 - delta;
-    } else {
-      g0 = (g0 + f0) >> 1;
-      q += u;
-      r += v;
-      u = (L)(2 * u);
-      v = (L)(2 * v);
-      delta += 1;
-    }
-    ++i;
+    int bits = -D < left ? -D : left;
+    if (bits > 6) bits = 6;
+    const U w = (f0 * g0 * (f0 * f0 - 2)) & (((U)1 << bits) - 1);
+    g0 += w * f0;
+    q += w * u;
+    r += w * v;
   }
-  u_out = u;
-  v_out = v;
-  q_out = q;
-  r_out = r;
-  return delta;
+  u_out = (L)u;
+  v_out = (L)v;
+  q_out = (L)q;
+  r_out = (L)r;
+  return D;
 }
 
 // [f, g] = T [f, g] / 2^B (exact)
@@ -147,28 +149,16 @@ PP_HD void apply_fg(SLimbs<L, NL> &f, SLimbs<L, NL> &g, L u, L v, L q, L r) {
   g.l[NL - 1] = (L)cg;
 }
 
-// x in (-M, 2M) -> [0, M)
+// x, or -x where neg is all ones, plus M where mask is all ones
 template <typename L, int NL>
-PP_HD void normalize_mod(SLimbs<L, NL> &x, const ModulusB<L, NL> &M) {
+PP_HD void negate_add(SLimbs<L, NL> &x, L neg, L mask, const ModulusB<L, NL> &M) {
   using U = typename LimbTraits<L>::U;
   constexpr int B = LimbTraits<L>::B;
   constexpr U MASK = ((U)1 << B) - 1;
-  int sgn = x.l[NL - 1] < 0 ? -1 : 0;
-  if (!sgn) {
-    // x >= M ?
-    bool ge = true;
-    for (int i = NL - 1; i >= 0; --i)
-      if (x.l[i] != M.m[i]) {
-        ge = x.l[i] > M.m[i];
-        break;
-      }
-    if (ge) sgn = 1;
-  }
-  if (!sgn) return;
   L c = 0;
 #pragma unroll
   for (int i = 0; i < NL; ++i) {
-    c += x.l[i] + (sgn < 0 ? M.m[i] : -M.m[i]);
+    c += ((x.l[i] ^ neg) - neg) + (M.m[i] & mask);
     if (i < NL - 1) {
       x.l[i] = (L)((U)c & MASK);
       c >>= B;
@@ -178,7 +168,9 @@ PP_HD void normalize_mod(SLimbs<L, NL> &x, const ModulusB<L, NL> &M) {
   }
 }
 
-// [d, e] = T [d, e] / 2^B mod M, d and e in [0, M)
+// [d, e] = T [d, e] / 2^B mod M, d and e in (-2M, M) before and after: with M added to
+// negative ones u d + v e lies within 2^B M of 0 (|u| + |v| <= 2^B), and the multiple
+// of M that clears the low B bits, taken in (-2^B M, 0], leaves (-2^(B+1) M, 2^B M).
 template <typename L, int NL>
 PP_HD void apply_de(SLimbs<L, NL> &d, SLimbs<L, NL> &e, L u, L v, L q, L r,
                     const ModulusB<L, NL> &M) {
@@ -186,11 +178,12 @@ PP_HD void apply_de(SLimbs<L, NL> &d, SLimbs<L, NL> &e, L u, L v, L q, L r,
   using U = typename LimbTraits<L>::U;
   constexpr int B = LimbTraits<L>::B;
   constexpr U MASK = ((U)1 << B) - 1;
+  const L sd = d.l[NL - 1] < 0 ? -1 : 0, se = e.l[NL - 1] < 0 ? -1 : 0;
   A cd = (A)u * d.l[0] + (A)v * e.l[0];
   A ce = (A)q * d.l[0] + (A)r * e.l[0];
-  // the multiples of M that clear the low B bits
-  const U md = (U)(0 - (U)cd * M.inv) & MASK;
-  const U me = (U)(0 - (U)ce * M.inv) & MASK;
+  L md = (u & sd) + (v & se), me = (q & sd) + (r & se);
+  md -= (L)(((U)cd * M.inv + (U)md) & MASK);
+  me -= (L)(((U)ce * M.inv + (U)me) & MASK);
   cd += (A)md * M.m[0];
   ce += (A)me * M.m[0];
   cd >>= B;
@@ -206,8 +199,6 @@ PP_HD void apply_de(SLimbs<L, NL> &d, SLimbs<L, NL> &e, L u, L v, L q, L r,
   }
   d.l[NL - 1] = (L)cd;
   e.l[NL - 1] = (L)ce;
-  normalize_mod(d, M);
-  normalize_mod(e, M);
 }
 
 template <typename L, int NL>
@@ -237,13 +228,13 @@ PP_HD SLimbs<L, NL> modinv_divsteps(const SLimbs<L, NL> &x, const ModulusB<L, NL
   }
   e.l[0] = 1;
   if (is_zero_limbs(g)) return d;
-  int delta = 1;
+  int D = 0;
   bool done = false;
   for (int b = 0; b < max_batches && !done; ++b) {
     L u, v, q, r;
     const U f0 = (U)f.l[0] | ((U)f.l[1] << B);
     const U g0 = (U)g.l[0] | ((U)g.l[1] << B);
-    delta = divsteps_word<L>(delta, f0, g0, u, v, q, r);
+    D = divsteps_word<L>(D, f0, g0, u, v, q, r);
     apply_fg(f, g, u, v, q, r);
     apply_de(d, e, u, v, q, r, M);
     done = is_zero_limbs(g);
@@ -253,21 +244,11 @@ PP_HD SLimbs<L, NL> modinv_divsteps(const SLimbs<L, NL> &x, const ModulusB<L, NL
     for (int i = 0; i < NL; ++i) d.l[i] = 0;
     return d;
   }
-  // f = +-1: x^-1 = +-d
-  if (f.l[NL - 1] < 0 && !is_zero_limbs(d)) {
-    constexpr U MASK = ((U)1 << B) - 1;
-    L c = 0;
-#pragma unroll
-    for (int i = 0; i < NL; ++i) {
-      c += M.m[i] - d.l[i];
-      if (i < NL - 1) {
-        d.l[i] = (L)((U)c & MASK);
-        c >>= B;
-      } else {
-        d.l[i] = c;
-      }
-    }
-  }
+  // f = +-1: x^-1 = +-d, d in (-2M, M)
+  negate_add(d, (L)0, d.l[NL - 1] < 0 ? (L)-1 : (L)0, M);
+  const L neg = f.l[NL - 1] < 0 ? (L)-1 : (L)0;
+  negate_add(d, neg, (L)0, M);
+  negate_add(d, (L)0, d.l[NL - 1] < 0 ? (L)-1 : (L)0, M);
   return d;
 }
 
