@@ -6,11 +6,11 @@
 // HBM traffic, plus a <<<1,1>>> squaring launch per step for division.  Here
 // each is two launches with O(N) multiplies and two passes over HBM:
 //  1. every thread folds a contiguous chunk of K elements into one summary
-//     (a product for the grand product; an affine map S_start = a + b*S_end for
-//     the backward recurrence S_i = p_i + m*S_{i+1} behind both evaluation,
-//     m = x, and division, m = -c); a block-wide work-efficient scan over the
-//     256 thread summaries in shared memory gives every thread its in-block
-//     carry and the block its summary (evaluation needs only the summary);
+//     (a product for the grand product; the value S_start for S_end = 0 of the
+//     backward recurrence S_i = p_i + m*S_{i+1} behind both evaluation, m = x,
+//     and division, m = -c); a block-wide scan over the 256 thread summaries
+//     gives every thread its in-block carry and the block its summary
+//     (evaluation needs only the summary);
 //  2. every block folds the summaries of the blocks before it (grand product)
 //     or after it (division) and each thread replays its chunk with the exact
 //     carry; evaluation composes all block maps in one block.
@@ -27,9 +27,10 @@ namespace pp {
 
 // Blocks per SM each operator's geometry aims for (scan_geom): longer chunks
 // cut the summaries to scan, more blocks hide more latency.  Swept over 1, 2,
-// 3 and 4 on GB300 (us at 2^20 / 2^22 / 2^24): division 2 (77 / 170 / 529;
-// 1: 72 / 171 / 559, 4: 115 / 207 / 546).  Evaluation has its own geometry
-// (k_eval_tree), and so has the permutation product (k_perm_local).
+// 3 and 4 on GB300 (us at 2^20 / 2^22 / 2^24): division 2 (57 / 137 / 446; with the
+// general maps before it 77 / 170 / 529, 1: 72 / 171 / 559, 4: 115 / 207 / 546).
+// Evaluation has its own geometry (k_eval_tree), and so has the permutation product
+// (k_perm_local).
 constexpr uint32_t kGpBlocksPerSm = 2, kDivBlocksPerSm = 2;
 // The grand product's chains grow with n while its block trees do not: us with
 // 2 / 3 / 4 blocks per SM at 2^20 57.4 / 57.4 / 65.6, at 2^22 159.5 / 156.1 /
@@ -301,14 +302,12 @@ __device__ void block_scan_pair(const fr &a, const fr &b, fr *s1, fr *s2, fr *to
   }
 }
 
-// Suffix composition of affine maps f_t(x) = a_t + b_t x over the block.
-// Afterwards (a, b) = F_t = f_t o f_{t+1} o ... o f_{n-1} and, when `all`,
-// (sa[t], sb[t]) = F_t for every t; without `all` only F_0 is produced (in
-// thread 0's (a, b) and sa[0], sb[0]).  Scanned in reversed order u = n-1-t,
-// where the running composition is G_u = g_u o G_{u-1}.
+// Composition of affine maps f_t(x) = a_t + b_t x over the block: afterwards thread
+// 0's (a, b) and sa[0], sb[0] hold f_0 o f_1 o ... o f_255.  Reversed order
+// u = 255 - t, where the running composition is G_u = g_u o G_{u-1}.
 // NAMED: the block also has a helper warp past the first 256 threads that
-// does not take part, so the scan synchronises its 256 threads on a named
-// barrier instead of __syncthreads.
+// does not take part, so the threads synchronise on a named barrier instead of
+// __syncthreads.
 template <bool NAMED>
 __device__ __forceinline__ void scan_sync() {
   if (NAMED) asm volatile("bar.sync 1, 256;" ::: "memory");
@@ -316,18 +315,14 @@ __device__ __forceinline__ void scan_sync() {
 }
 
 template <bool NAMED = false>
-__device__ void block_affine_suffix(fr &a, fr &b, fr *sa, fr *sb, bool all = true) {
-  const int t = threadIdx.x, n = NAMED ? kScanThreads : blockDim.x;
+__device__ void block_affine_compose(fr &a, fr &b, fr *sa, fr *sb) {
+  const int t = threadIdx.x, n = kScanThreads;
   const int u = n - 1 - t;
   sts_fr(sa + u, a);
   sts_fr(sb + u, b);
   scan_sync<NAMED>();
-  // The full scan of 256 maps takes the hybrid form of block_exclusive_product:
-  // three up-sweep levels, one warp scanning the 32 run maps, three
-  // down-sweep levels.
-  const bool hybrid = all && n == 256;
   // combine(left = earlier in u, right = later in u) = right o left
-  for (int d = 1; d < (hybrid ? 8 : n); d <<= 1) {
+  for (int d = 1; d < n; d <<= 1) {
     const int idx = (t + 1) * 2 * d - 1;
     if (idx < n) {
       const fr la = lds_fr(sa + idx - d), lb = lds_fr(sb + idx - d), ra = lds_fr(sa + idx), rb = lds_fr(sb + idx);
@@ -336,56 +331,13 @@ __device__ void block_affine_suffix(fr &a, fr &b, fr *sa, fr *sb, bool all = tru
     }
     scan_sync<NAMED>();
   }
-  if (!all) {
-    // sa[n-1], sb[n-1] = G_{n-1} = F_0
-    if (t == 0) {
-      a = lds_fr(sa + n - 1);
-      b = lds_fr(sb + n - 1);
-      sts_fr(sa, a);
-      sts_fr(sb, b);
-    }
-    scan_sync<NAMED>();
-    return;
+  // sa[n-1], sb[n-1] = G_{n-1} = F_0
+  if (t == 0) {
+    a = lds_fr(sa + n - 1);
+    b = lds_fr(sb + n - 1);
+    sts_fr(sa, a);
+    sts_fr(sb, b);
   }
-  if (hybrid) {
-    if (t < 32) {
-      // exclusive scan of the run maps at u = 8k + 7, in u order
-      fr xa = lds_fr(sa + 8 * t + 7), xb = lds_fr(sb + 8 * t + 7);
-      for (int o = 1; o < 32; o <<= 1) {
-        const fr ua = shfl_up_fr(xa, o), ub = shfl_up_fr(xb, o);
-        if (t >= o) {
-          xa = fr_add(xa, fr_mul(xb, ua));
-          xb = fr_mul(xb, ub);
-        }
-      }
-      const fr ea = shfl_up_fr(xa, 1), eb = shfl_up_fr(xb, 1);
-      sts_fr(sa + 8 * t + 7, t ? ea : fr_zero());
-      sts_fr(sb + 8 * t + 7, t ? eb : fr_one());
-    }
-  } else if (t == 0) {
-    sts_fr(sa + n - 1, fr_zero());
-    sts_fr(sb + n - 1, fr_one());
-  }
-  scan_sync<NAMED>();
-  for (int d = hybrid ? 4 : n >> 1; d >= 1; d >>= 1) {
-    const int idx = (t + 1) * 2 * d - 1;
-    if (idx < n) {
-      const fr la = lds_fr(sa + idx - d), lb = lds_fr(sb + idx - d), pa = lds_fr(sa + idx), pb = lds_fr(sb + idx);
-      sts_fr(sa + idx - d, pa);
-      sts_fr(sb + idx - d, pb);
-      sts_fr(sa + idx, fr_add(la, fr_mul(lb, pa)));  // left o P
-      sts_fr(sb + idx, fr_mul(lb, pb));
-    }
-    scan_sync<NAMED>();
-  }
-  // exclusive E_u in (sa[u], sb[u]); inclusive G_u = g_u o E_u = F_t
-  const fr ea = lds_fr(sa + u), eb = lds_fr(sb + u);
-  const fr ia = fr_add(a, fr_mul(b, ea)), ib = fr_mul(b, eb);
-  scan_sync<NAMED>();
-  sts_fr(sa + t, ia);
-  sts_fr(sb + t, ib);
-  a = ia;
-  b = ib;
   scan_sync<NAMED>();
 }
 
@@ -691,21 +643,17 @@ __global__ void __launch_bounds__(kScanThreads)
 // chunk length K is shared by the block: only a shorter (last) chunk computes
 // its own power.
 
-// per-thread exclusive suffix map (optional) and per-block map.  Launched
-// with kScanThreads + 32 threads: the extra warp computes m^K while the
-// others evaluate their chunks (chunk_dot, after the first warp's table of
-// m^0 .. m^16), which do not need it.
+// per-block map.  Launched with kScanThreads + 32 threads: the extra warp
+// computes m^K while the others evaluate their chunks (chunk_dot, after the
+// first warp's table of m^0 .. m^16), which do not need it.
 __global__ void __launch_bounds__(kScanThreads + 32, 2) k_affine_local(const fr *__restrict__ p, ScanGeom g,
                                                                      const fr *__restrict__ m_ptr,
-                                                                     int negate_m, fr *thread_a,
-                                                                     fr *thread_b, fr *block_a,
-                                                                     fr *block_b) {
+                                                                     fr *block_a, fr *block_b) {
   __shared__ uint4 sm[kTileSmemUnits];  // the chunks' tiles, then the scan
   fr *sa = reinterpret_cast<fr *>(sm), *sb = sa + kScanThreads;
   __shared__ fr s_mk;
   __shared__ __align__(16) fr s_pw[17];  // m^k, k <= 16, for the chunks' dot products
-  fr m = ld_fr(m_ptr);
-  if (negate_m) m = fr_neg(m);
+  const fr m = ld_fr(m_ptr);
   if (threadIdx.x >= kScanThreads) {
     if (threadIdx.x == kScanThreads) s_mk = fr_pow_u64(m, g.k);
     __syncthreads();
@@ -720,12 +668,7 @@ __global__ void __launch_bounds__(kScanThreads + 32, 2) k_affine_local(const fr 
   const fr L = chunk_dot(ct, p, s_pw);
   __syncthreads();  // m^K ready, tiles free
   fr a = L, b = hi - lo == g.k ? s_mk : hi > lo ? fr_pow_u64(m, hi - lo) : fr_one();
-  block_affine_suffix<true>(a, b, sa, sb, thread_a != nullptr);
-  if (thread_a && gt < g.threads) {
-    const bool last = threadIdx.x == kScanThreads - 1;
-    st_fr(thread_a + gt, last ? fr_zero() : lds_fr(sa + threadIdx.x + 1));
-    st_fr(thread_b + gt, last ? fr_one() : lds_fr(sb + threadIdx.x + 1));
-  }
+  block_affine_compose<true>(a, b, sa, sb);
   if (threadIdx.x == 0) {
     st_fr(block_a + blockIdx.x, a);
     st_fr(block_b + blockIdx.x, b);
@@ -747,37 +690,149 @@ __device__ void compose_blocks(const fr *block_a, const fr *block_b, uint32_t fi
     a = fr_add(ai, fr_mul(bi, a));
     b = fr_mul(bi, b);
   }
-  block_affine_suffix(a, b, sa, sb, false);
+  block_affine_compose(a, b, sa, sb);
   A = lds_fr(sa);
   B = lds_fr(sb);
 }
 
-__global__ void __launch_bounds__(kScanThreads) k_div_apply(fr *inout, ScanGeom g,
-                                                             const fr *__restrict__ m_ptr,
-                                                             const fr *__restrict__ thread_a,
-                                                             const fr *__restrict__ thread_b,
-                                                             const fr *__restrict__ block_a,
-                                                             const fr *__restrict__ block_b) {
-  __shared__ uint4 sm[kTileSmemUnits];  // the composition's scan, then the tiles
-  fr *sa = reinterpret_cast<fr *>(sm), *sb = sa + kScanThreads;
-  const fr m = fr_neg(ld_fr(m_ptr));
-  fr A, B;
-  compose_blocks(block_a, block_b, blockIdx.x + 1, g.blocks, A, B, sa, sb);
-  __syncthreads();
-  const fr s_end_block = A;  // S at the end of this block (S_n = 0)
+// Division: every S.  The vector counts as padded with zeros to whole chunks and
+// blocks (S = 0 past its end), so each chunk's map is x -> L + q x with the same
+// q = m^K and each block's x -> A + Q x, Q = q^256: a combine of two neighbours is one
+// multiply by a known power instead of two, and a sum over all later blocks is a
+// weighted sum without a chain.  us at 2^20 / 2^22 / 2^24: 77 / 170 / 529 with general
+// maps (two multiplies per combine, 24 and 18 deep), 57 / 137 / 446 so.
+// Powers, by the helper warp beside the chunks; block 0 leaves them for the apply:
+struct DivPowers {
+  fr q[33];     // q^a
+  fr q32[9];    // q^(32 b)
+  fr Q[33];     // Q^a
+  fr Q32[17];   // Q^(32 b): up to 512 blocks
+};
+// pw[k] = x^k for k <= 2^steps (at most 32), by the lanes of one warp
+__device__ __forceinline__ void warp_powers(const fr &x, uint32_t steps, fr *pw) {
+  const uint32_t lane = threadIdx.x & 31;
+  // lane l makes x^(l + 1): in step h lanes h .. 2h - 1 take x^(l + 1 - h) x^h
+  fr v = x;
+#pragma unroll 1
+  for (uint32_t h = 1; h < 1u << steps; h <<= 1) {
+    fr low, hv;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+      low.v[w] = __shfl_sync(0xffffffffu, v.v[w], (int)(lane >= h ? lane - h : 0));
+      hv.v[w] = __shfl_sync(0xffffffffu, v.v[w], (int)h - 1);
+    }
+    if (lane >= h && lane < 2 * h) v = fr_mul(low, hv);
+  }
+  if (lane < 1u << steps) sts_fr(pw + lane + 1, v);
+  if (lane == 0) sts_fr(pw, fr_one());
+  __syncwarp();
+}
+
+__device__ __forceinline__ fr shfl_down_fr(const fr &v, int o) {
+  fr r;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) r.v[i] = __shfl_down_sync(0xffffffffu, v.v[i], o);
+  return r;
+}
+
+// thread_s[t] = S at the end of thread t's chunk if it is 0 at the end of its block,
+// block_s[b] = S at the start of block b likewise
+__global__ void __launch_bounds__(kScanThreads + 32, 2)
+    k_div_local(const fr *__restrict__ p, ScanGeom g, const fr *__restrict__ c_ptr, fr *thread_s, fr *block_s,
+                DivPowers *powers) {
+  __shared__ uint4 sm[kTileSmemUnits];
+  __shared__ __align__(16) fr s_pw[17];  // m^k, k <= 16, for the chunks' dot products
+  __shared__ __align__(16) fr s_q[33], s_q32[9], s_Q[33], s_Q32[17], s_warp[kScanThreads / 32];
+  const fr m = fr_neg(ld_fr(c_ptr));
+  if (threadIdx.x >= kScanThreads) {
+    warp_powers(fr_pow_u64(m, g.k), 5, s_q);
+    warp_powers(lds_fr(s_q + 32), 3, s_q32);
+    __syncthreads();
+    if (blockIdx.x == 0) {
+      const uint32_t lane = threadIdx.x & 31;
+      warp_powers(lds_fr(s_q32 + 8), 5, s_Q);
+      warp_powers(lds_fr(s_Q + 32), 4, s_Q32);
+      for (uint32_t i = lane; i < 33; i += 32) {
+        st_fr(powers->q + i, lds_fr(s_q + i));
+        st_fr(powers->Q + i, lds_fr(s_Q + i));
+      }
+      if (lane < 9) st_fr(powers->q32 + lane, lds_fr(s_q32 + lane));
+      if (lane < 17) st_fr(powers->Q32 + lane, lds_fr(s_Q32 + lane));
+    }
+    return;
+  }
+  if (threadIdx.x < 32) warp_power_table17(m, s_pw);
+  asm volatile("bar.sync 1, 256;" ::: "memory");
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint64_t gt = blockIdx.x * (uint64_t)kScanThreads + threadIdx.x;
+  const ChunkTiles ct(sm, warp, gt - lane, g.n, g.k);
+  fr I = chunk_dot(ct, p, s_pw);
+  __syncthreads();  // the powers are there
+  // I = S at the lane's start if 0 at the warp's end
+#pragma unroll 1
+  for (uint32_t o = 1; o < 32; o <<= 1) {
+    const fr next = shfl_down_fr(I, o);
+    if (lane + o < 32) I = fr_add(I, fr_mul(next, lds_fr(s_q + o)));
+  }
+  if (lane == 0) sts_fr(s_warp + warp, I);
+  asm volatile("bar.sync 1, 256;" ::: "memory");
+  // the same over the warps, by every warp
+  constexpr uint32_t nw = kScanThreads / 32;
+  fr W = lds_fr(s_warp + (lane & (nw - 1)));
+#pragma unroll 1
+  for (uint32_t o = 1; o < nw; o <<= 1) {
+    const fr next = shfl_down_fr(W, o);
+    if ((lane & (nw - 1)) + o < nw) W = fr_add(W, fr_mul(next, lds_fr(s_q32 + o)));
+  }
+  fr C;  // at this warp's end
+#pragma unroll
+  for (int w = 0; w < 8; ++w) C.v[w] = __shfl_sync(0xffffffffu, W.v[w], warp + 1 < nw ? warp + 1 : 0);
+  if (warp + 1 == nw) C = fr_zero();
+  const fr after = shfl_down_fr(I, 1);
+  const fr S = fr_mul(C, lds_fr(s_q + 31 - lane));
+  if (gt < g.threads) st_fr(thread_s + gt, lane == 31 ? S : fr_add(after, S));
+  if (threadIdx.x == 0) st_fr(block_s + blockIdx.x, W);
+}
+
+// The exact S at the block's end, then at the chunk's, then the chunk replayed:
+// m as a four-part constant, S below 2.01 r in between.
+__global__ void __launch_bounds__(kScanThreads, 2)
+    k_div_apply(fr *inout, ScanGeom g, const fr *__restrict__ c_ptr, const fr *__restrict__ thread_s,
+                const fr *__restrict__ block_s, const DivPowers *__restrict__ powers) {
+  __shared__ uint4 sm[kTileSmemUnits];
+  __shared__ __align__(16) fr s_m[4], s_warp[kScanThreads / 32];
+  const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  if (t < 4) sts_fr(s_m + t, fr_mul(fr_neg(ld_fr(c_ptr)), fr_const4_factor(t)));
+  // sum over the later blocks b of block_s[b] Q^(b - this - 1)
+  fr sum = fr_zero();
+  for (uint32_t j = t; blockIdx.x + 1 + j < g.blocks; j += kScanThreads) {
+    const fr w = fr_mul(ldg_fr(powers->Q + (j & 31)), ldg_fr(powers->Q32 + (j >> 5)));
+    sum = fr_add(sum, fr_mul(w, ldg_fr(block_s + blockIdx.x + 1 + j)));
+  }
+#pragma unroll 1
+  for (uint32_t o = 16; o > 0; o >>= 1) sum = fr_add(sum, shfl_down_fr(sum, o));
+  if (lane == 0) sts_fr(s_warp + warp, sum);
+  // q^(255 - t)
+  const fr weight = fr_mul(ldg_fr(powers->q + 31 - lane), ldg_fr(powers->q32 + kScanThreads / 32 - 1 - warp));
+  __syncthreads();
+  fr end = lds_fr(s_warp);
+#pragma unroll 1
+  for (uint32_t w = 1; w < kScanThreads / 32; ++w) end = fr_add(end, lds_fr(s_warp + w));
+  const uint64_t gt = blockIdx.x * (uint64_t)kScanThreads + t;
   // past the vector S = 0 and elements read as zero, so s stays 0 there
-  fr s = gt < g.threads ? fr_add(ld_fr(thread_a + gt), fr_mul(ld_fr(thread_b + gt), s_end_block))
-                        : fr_zero();
-  const ChunkTiles ct(sm, threadIdx.x >> 5, gt - (threadIdx.x & 31), g.n, g.k);
+  fr s = gt < g.threads ? fr_add(ld_fr(thread_s + gt), fr_mul(weight, end)) : fr_zero();
+  fr m[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) m[k] = lds_fr(s_m + k);
+  const ChunkTiles ct(sm, warp, gt - lane, g.n, g.k);
   const uint32_t last = ct.tiles - 1;
-  ct.run(inout, inout, [&](uint32_t st) { return last - st; }, [&](uint32_t, uint32_t t, uint32_t slot) {
+  ct.run(inout, inout, [&](uint32_t st) { return last - st; }, [&](uint32_t, uint32_t tile, uint32_t slot) {
 #pragma unroll
     for (int e = (int)kTileElems - 1; e >= 0; --e)
-      if (e == 0 || t * kTileElems + e < g.k) {
+      if (e == 0 || tile * kTileElems + e < g.k) {
         const fr pi = ct.get(slot, e);
-        ct.put(slot, e, s);  // q_i = S_(i+1)
-        s = fr_add(pi, fr_mul(m, s));
+        ct.put(slot, e, fr_canon(s));  // q_i = S_(i+1)
+        s = fr_add_raw(pi, fr_mul_const4(s, m));
       }
   });
 }
@@ -970,17 +1025,19 @@ extern "C" int pp_div_xplusc(void *d_inout, uint64_t n, const void *d_c, void *s
   cudaStream_t s = (cudaStream_t)stream;
   const pp::ScanGeom g = pp::scan_geom(n, pp::kDivBlocksPerSm);
   int st = PP_OK;
-  fr *ws = static_cast<fr *>(
-      pp::workspace_get((2 * g.threads + 2 * g.blocks) * sizeof(fr), s, 1, &st));
+  static_assert(sizeof(pp::DivPowers) % sizeof(fr) == 0, "in whole elements");
+  fr *ws = static_cast<fr *>(pp::workspace_get(
+      (g.threads + g.blocks) * sizeof(fr) + sizeof(pp::DivPowers), s, 1, &st));
   if (st) return st;
-  fr *ta = ws, *tb = ws + g.threads, *ba = ws + 2 * g.threads, *bb = ba + g.blocks;
+  fr *thread_s = ws, *block_s = ws + g.threads;
+  pp::DivPowers *powers = reinterpret_cast<pp::DivPowers *>(block_s + g.blocks);
   const fr *c = static_cast<const fr *>(d_c);
-  pp::k_affine_local<<<g.blocks, pp::kScanThreads + 32, 0, s>>>(static_cast<const fr *>(d_inout), g, c,
-                                                           1, ta, tb, ba, bb);
+  pp::k_div_local<<<g.blocks, pp::kScanThreads + 32, 0, s>>>(static_cast<const fr *>(d_inout), g, c,
+                                                            thread_s, block_s, powers);
   PP_COUNT_LAUNCH();
   PP_LAUNCH_CHECK();
-  pp::k_div_apply<<<g.blocks, pp::kScanThreads, 0, s>>>(static_cast<fr *>(d_inout), g, c, ta, tb,
-                                                        ba, bb);
+  pp::k_div_apply<<<g.blocks, pp::kScanThreads, 0, s>>>(static_cast<fr *>(d_inout), g, c, thread_s,
+                                                        block_s, powers);
   PP_COUNT_LAUNCH();
   PP_LAUNCH_CHECK();
   return PP_OK;
@@ -1202,7 +1259,7 @@ extern "C" int pp_eval_noalloc(const void *d_poly, uint64_t n, const void *d_x, 
   // the same call, so nothing in the array has to be cleared first
   fr *ba = scratch, *bb = scratch + pp::kEvalNoAllocMaxBlocks;
   pp::k_affine_local<<<g.blocks, pp::kScanThreads + 32, 0, s>>>(
-      static_cast<const fr *>(d_poly), g, static_cast<const fr *>(d_x), 0, nullptr, nullptr, ba, bb);
+      static_cast<const fr *>(d_poly), g, static_cast<const fr *>(d_x), ba, bb);
   PP_COUNT_LAUNCH();
   PP_LAUNCH_CHECK();
   pp::k_eval_final<<<1, pp::kScanThreads, 0, s>>>(ba, bb, g.blocks, static_cast<fr *>(d_y));
