@@ -24,11 +24,11 @@
 //                launch joins each shared bucket's partial sums (one thread
 //                for a few, blocks for many: a bucket can hold up to all n
 //                points: equal scalars, or the few-bit top window)
-//   6. segments  one thread per run of G buckets: running sums T = sum
-//                (j + 1) B and R = sum B over its run
+//   6. segments  one thread (or two lanes) per run of G buckets: running sums T =
+//                sum (j + 1) B and R = sum B over its run
 //   7. windows   sum T + G sum_s s R_s with sum_s s R_s = sum_k 2^k Q_k, Q_k
-//                the R_s whose index has bit k set: plain sums in chunks, a
-//                block tree per sum, then one warp per window for the Horner
+//                the R_s whose index has bit k set: plain sums in chunks, the
+//                chunks a warp to an addition, then one warp per window for the Horner
 //                chain over k
 //   8. final     one warp: Horner over the windows (c doublings each, the
 //                independent multiplies of each step on different lanes), one
@@ -63,12 +63,14 @@ struct MsmPlan {
 // gives 2^15 segment threads.  On GB300 this beat fixed 4, 8 and 16 (2^16
 // points: 16 -> 4.65 ms, 4 -> 3.92 ms; 2^22: 4 -> 53.2 ms, 16 -> 51.3 ms).
 constexpr uint32_t kSegmentMax = 16, kSegmentMin = 4, kSegmentThreads = 1u << 15;
+// Segments of four buckets take two lanes each (k_msm_segments4) while those make no
+// more than one warp per SM sub-partition (152 SMs, four each): 8192 segments 101 ->
+// 74 us, but 20480 segments 131 -> 141.
+constexpr uint32_t kPairedLanes = 152 * 128;
 
-// Terms per thread of the window sums: 8, and 4 where that leaves the chip less
-// than full and a block of k_msm_bitreduce at most two chunks per thread.  8 / 4:
-// 200003 points 2.575 / 2.551 ms, 2^14 1.189 / 1.165; but with one bucket set 2^16
-// points (8192 segments) 1.059 / 1.117, and 2^20 points 7.37 / 7.39.
-constexpr uint32_t kChunkMax = 8, kChunkThreads = 1u << 14, kChunkSum = 2048;
+// Terms per thread of the window sums (k_msm_bitsums): 8, and 4 where that leaves the
+// chip less than full.  With one set of 2^15 buckets 4 terms take 56 us and 8 terms 117.
+constexpr uint32_t kChunkMax = 8, kChunkThreads = 1u << 14;
 
 // the rest of a plan once c and the number of bucket sets are fixed
 MsmPlan msm_plan_for(uint32_t c, uint32_t nsets) {
@@ -83,7 +85,7 @@ MsmPlan msm_plan_for(uint32_t c, uint32_t nsets) {
   while ((1u << p.lgG) < p.G) ++p.lgG;
   while ((1u << p.lgS) < p.S) ++p.lgS;
   p.chunk = kChunkMax;
-  if ((uint64_t)nsets * (2 + p.lgS) * p.S / (2 * kChunkMax) <= kChunkThreads && p.S <= kChunkSum) p.chunk /= 2;
+  if ((uint64_t)nsets * (2 + p.lgS) * p.S / (2 * kChunkMax) <= kChunkThreads) p.chunk /= 2;
   return p;
 }
 
@@ -794,7 +796,7 @@ __device__ __forceinline__ digit point_add(const Spread &S, const digit &A, cons
 
 // sum of val(j), lo <= j < hi, by a block of kPointThreads (the result in
 // red[0] for all): strided sums, then a tree in shared memory, its lower levels
-// with a warp to each addition (k_msm_bitreduce at 200003 points: 106 -> 71 us)
+// with a warp to each addition (128 values in 220 blocks: 106 -> 71 us)
 constexpr uint32_t kWarpAdds = 16;
 template <typename F>
 __device__ __forceinline__ g1x block_sum(uint32_t lo, uint32_t hi, g1x *red, F val) {
@@ -893,6 +895,36 @@ __global__ void __launch_bounds__(kPointThreads)
   }
 }
 
+// The same for segments of four buckets, two lanes each: four dependent additions
+// instead of six.  R = (B0 + B1) + (B2 + B3) and T = (R + B1) + ((B2 + B3) + B3 +
+// (B2 + B3)).  Bound by the additions' latency; kPairedLanes says when.
+__device__ __forceinline__ g1x neighbour(const g1x &a) {  // the other lane's
+  g1x r;
+  const uint32_t *u = reinterpret_cast<const uint32_t *>(&a);
+  uint32_t *v = reinterpret_cast<uint32_t *>(&r);
+#pragma unroll
+  for (uint32_t k = 0; k < sizeof(g1x) / 4; ++k) v[k] = __shfl_xor_sync(0xffffffffu, u[k], 1);
+  return r;
+}
+__global__ void __launch_bounds__(kPointThreads, 3)
+    k_msm_segments4(const g1x *__restrict__ buckets, uint64_t total, g1x *__restrict__ seg_t,
+                    g1x *__restrict__ seg_r) {
+  const uint64_t i = (uint64_t)blockIdx.x * kPointThreads + threadIdx.x;
+  const uint64_t t = i / 2 < total ? i / 2 : total - 1;  // all lanes stay for the exchanges
+  const uint32_t up = (uint32_t)i & 1;                   // buckets 2 and 3
+  const g1x *row = buckets + 4 * t + 2 * up;
+  const g1x odd = row[1];
+  const g1x s = g1x_add(row[0], odd);
+  // R (down), B2 + 2 B3 (up)
+  const g1x other = neighbour(s);
+  g1x a = g1x_add(s, up ? odd : other);
+  if (!up && i / 2 < total) seg_r[t] = a;
+  // R + B1, 2 B2 + 3 B3
+  a = g1x_add(a, up ? s : odd);
+  const g1x b = neighbour(a);
+  if (!up && i / 2 < total) seg_t[t] = g1x_add(a, b);
+}
+
 // Window sums from the segments: sum_b (b + 1) B_b = sum_s T_s + G sum_s s R_s,
 // and sum_s s R_s = sum_k 2^k Q_k, where Q_k adds the R_s of the segments whose
 // index s has bit k set.  So a window needs 1 + lg S plain sums (sum j = 0 is
@@ -943,16 +975,54 @@ __global__ void __launch_bounds__(kPointThreads)
   }
 }
 
-// One block per (window, sum): the sum's chunks.  sums[w (1 + lg S) + j].
-__global__ void __launch_bounds__(kPointThreads)
-    k_msm_bitreduce(const g1x *__restrict__ part, MsmPlan p, g1x *__restrict__ sums) {
-  __shared__ __align__(16) g1x red[kPointThreads];
-  const ChunkCounts cc = chunk_counts(p);
-  const uint32_t L = 1 + p.lgS;
-  const uint32_t w = blockIdx.x / L, j = blockIdx.x - w * L;
-  const uint64_t first = (uint64_t)w * cc.ncw + (j == 0 ? 0 : cc.nc0 + (j - 1) * cc.nc1);
-  const g1x sum = block_sum(0, j == 0 ? cc.nc0 : cc.nc1, red, [&](uint32_t i) { return part[first + i]; });
-  if (threadIdx.x == 0) sums[blockIdx.x] = sum;
+// Sums of every (window, sum)'s chunks, in blocks of at most kReduceSpan: a warp
+// adds up to 8 of them, each addition spread over it, then the warps' sums meet in
+// a tree.  in and out are the numbers of inputs and of blocks per sum; where a sum
+// takes several blocks a second launch adds those.  Bound by the latency of the
+// additions (2.2 us alone, 4.3 with four warps to a sub-partition).  One block of
+// 128 threads per sum, a lane to an addition down to 16 of them, took 170 us for
+// one bucket set of 2^15 buckets against 68 us for both launches (16 to a warp: 80),
+// and 91 us for 20 sets of 2^12 against 92.
+constexpr uint32_t kReduceWarps = 8, kReduceSpan = 8 * kReduceWarps;
+__host__ __device__ __forceinline__ ChunkCounts reduced_counts(const ChunkCounts &in, uint32_t lgS) {
+  ChunkCounts c;
+  c.nc0 = (in.nc0 + kReduceSpan - 1) / kReduceSpan;
+  c.nc1 = (in.nc1 + kReduceSpan - 1) / kReduceSpan;
+  c.ncw = c.nc0 + lgS * c.nc1;
+  return c;
+}
+__global__ void __launch_bounds__(32 * kReduceWarps)
+    k_msm_bitreduce(const g1x *__restrict__ part, ChunkCounts in, ChunkCounts out, g1x *__restrict__ sums) {
+  __shared__ __align__(16) g1x red[kReduceWarps];
+  const uint32_t w = blockIdx.x / out.ncw, u = blockIdx.x - w * out.ncw;
+  const bool t_sum = u < out.nc0;
+  const uint32_t v = t_sum ? u : u - out.nc0, blocks = t_sum ? out.nc0 : out.nc1;
+  const uint32_t k = v / blocks, count = t_sum ? in.nc0 : in.nc1;
+  const uint32_t span = (count + blocks - 1) / blocks, lo = (v - k * blocks) * span;
+  const uint32_t hi = lo + span < count ? lo + span : count;
+  const g1x *row = part + (uint64_t)w * in.ncw + (t_sum ? 0 : in.nc0 + k * in.nc1);
+  const uint32_t warp = threadIdx.x / 32;
+  const Spread S;
+  digit acc = {0, 0, 0}, next = {0, 0, 0};
+  uint32_t i = lo + warp;
+  if (i < hi) next = point_load(S, row + i);
+#pragma unroll 1
+  for (; i < hi; i += kReduceWarps) {
+    const digit p = next;
+    if (i + kReduceWarps < hi) next = point_load(S, row + i + kReduceWarps);
+    acc = point_add(S, acc, p);
+  }
+  point_park(S, acc, red + warp);
+  __syncthreads();
+#pragma unroll 1
+  for (uint32_t h = kReduceWarps / 2; h > 0; h >>= 1) {
+    if (warp < h) {
+      acc = point_add(S, acc, point_load(S, red + warp + h));
+      point_park(S, acc, red + warp);
+    }
+    __syncthreads();
+  }
+  if (warp == 0) point_store(S, acc, sums + blockIdx.x);
 }
 
 // One warp per window: win[w] = sum_s T_s + G sum_k 2^k Q_k (Horner over k)
@@ -995,7 +1065,7 @@ __global__ void __launch_bounds__(32) k_msm_final(const g1x *__restrict__ win, M
 
 struct MsmLayout {
   size_t digits, counts, n_items, offsets, list, part, items, multi, chunk_sum, buckets, seg_t,
-      seg_r, chunks, sums, win, tiles, pairs[2], pair_off, total;
+      seg_r, chunks, chunks2, sums, win, tiles, pairs[2], pair_off, total;
   uint32_t resident; // threads of k_msm_accumulate resident at once
   uint32_t runs;     // runs of the list at most
 };
@@ -1044,7 +1114,9 @@ MsmLayout msm_layout(uint64_t n, const MsmPlan &p, uint32_t rounds) {
   L.buckets = o, o += up(nb * sizeof(g1x));
   L.seg_t = o, o += up((size_t)p.nsets * p.S * sizeof(g1x));
   L.seg_r = o, o += up((size_t)p.nsets * p.S * sizeof(g1x));
-  L.chunks = o, o += up((size_t)p.nsets * chunk_counts(p).ncw * sizeof(g1x));
+  const ChunkCounts chunks = chunk_counts(p);
+  L.chunks = o, o += up((size_t)p.nsets * chunks.ncw * sizeof(g1x));
+  L.chunks2 = o, o += up((size_t)p.nsets * reduced_counts(chunks, p.lgS).ncw * sizeof(g1x));
   L.sums = o, o += up((size_t)p.nsets * (1 + p.lgS) * sizeof(g1x));
   L.win = o, o += up((size_t)p.nsets * sizeof(g1x));
   L.tiles = o, o += up(((nb + kScanTile - 1) / kScanTile + 1) * 4);
@@ -1147,7 +1219,7 @@ int msm_run(const g1a *points, const uint32_t *scalars, uint64_t n, const MsmPla
   uint32_t *tiles = u32(L.tiles);
   uint2 *items = reinterpret_cast<uint2 *>(ws + L.items), *multi = reinterpret_cast<uint2 *>(ws + L.multi);
   g1x *buckets = pts(L.buckets), *seg_t = pts(L.seg_t), *seg_r = pts(L.seg_r), *win = pts(L.win);
-  g1x *chunks = pts(L.chunks), *sums = pts(L.sums), *part = pts(L.part), *chunk_sum = pts(L.chunk_sum);
+  g1x *chunks = pts(L.chunks), *chunks2 = pts(L.chunks2), *sums = pts(L.sums), *part = pts(L.part), *chunk_sum = pts(L.chunk_sum);
   const uint64_t nb = (uint64_t)p.nsets * p.B;
 
   // 1-3: signed digits, bucket sizes, counting sort of (point, sign) by bucket
@@ -1201,17 +1273,26 @@ int msm_run(const g1a *points, const uint32_t *scalars, uint64_t n, const MsmPla
   PP_LAUNCH_CHECK();
 
   // 6-8: weighted bucket sums per bucket set, sets combined, affine result
-  k_msm_segments<<<grid_for((uint64_t)p.nsets * p.S, kPointThreads), kPointThreads, 0, s>>>(
-      buckets, p, seg_t, seg_r);
+  const uint64_t segments = (uint64_t)p.nsets * p.S;
+  if (p.G == 4 && 2 * segments <= kPairedLanes)
+    k_msm_segments4<<<grid_for(2 * segments, kPointThreads), kPointThreads, 0, s>>>(buckets, segments, seg_t, seg_r);
+  else
+    k_msm_segments<<<grid_for(segments, kPointThreads), kPointThreads, 0, s>>>(buckets, p, seg_t, seg_r);
   PP_COUNT_LAUNCH();
   PP_LAUNCH_CHECK();
-  k_msm_bitsums<<<grid_for((uint64_t)p.nsets * chunk_counts(p).ncw, kPointThreads), kPointThreads,
-                  0, s>>>(seg_t, seg_r, p, chunks);
+  const ChunkCounts cc = chunk_counts(p), some = reduced_counts(cc, p.lgS), one{1, 1, 1 + p.lgS};
+  k_msm_bitsums<<<grid_for((uint64_t)p.nsets * cc.ncw, kPointThreads), kPointThreads, 0, s>>>(seg_t, seg_r, p, chunks);
   PP_COUNT_LAUNCH();
   PP_LAUNCH_CHECK();
-  k_msm_bitreduce<<<p.nsets * (1 + p.lgS), kPointThreads, 0, s>>>(chunks, p, sums);
+  const bool twice = some.nc0 > 1;
+  k_msm_bitreduce<<<p.nsets * some.ncw, 32 * kReduceWarps, 0, s>>>(chunks, cc, some, twice ? chunks2 : sums);
   PP_COUNT_LAUNCH();
   PP_LAUNCH_CHECK();
+  if (twice) {
+    k_msm_bitreduce<<<p.nsets * one.ncw, 32 * kReduceWarps, 0, s>>>(chunks2, some, one, sums);
+    PP_COUNT_LAUNCH();
+    PP_LAUNCH_CHECK();
+  }
   k_msm_wincombine<<<p.nsets, 32, 0, s>>>(sums, p, win);
   PP_COUNT_LAUNCH();
   PP_LAUNCH_CHECK();
