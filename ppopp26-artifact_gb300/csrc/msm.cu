@@ -101,11 +101,13 @@ uint32_t ceil_lg(uint64_t n) {
 // Window bits.  Scalars below r < 2^255 leave the top window few digit
 // values unless c is 13, 16 or 20 (the top window then spans 232, 29678 or
 // 29678 values): with other c about n entries share a handful of buckets, or
-// one carry window, and those buckets need extra levels of serial group sums.
-// Swept on GB300 (2^12..2^24 points, c = 10..20), these won: 13 up to 2^19
-// points (2^14: 2.86 ms against 3.45 for the cost model's 11), 16 up to 2^23
-// (2^22: 41.2 against 47.2 for 18), 18 beyond (2^24: 149.8 against 158.6 for
-// 20).  Below 2^10 points the cost model decides.
+// one carry window.  Swept on GB300 (2^8..2^24 points, c = 6..20): 13 up to
+// 2^19 points, 16 up to 2^23 (2^22: 41.2 against 47.2 ms for 18), 18 beyond (2^24:
+// 149.8 against 158.6 for 20).  Below 2^15 points the steps after the bucket sums
+// are the larger part, and they shrink with the buckets: 8 up to 2^9 points, 10 up
+// to 2^15.  Microseconds with 8 / 10 / 13: 1000 points 825 / 829 / 954, 4096 983 /
+// 862 / 980, 2^14 1218 / 1023 / 1073, 2^15 1402 / 1168 / 1196, 2^16 1812 / 1492 /
+// 1443.  With 2^7 points and fewer the cost model decides.
 //
 // The model minimises W (10 n + 14 2^c) Fq multiplies: the bucket sums (one
 // mixed add per point and window) against the aggregation (two adds per
@@ -114,8 +116,8 @@ MsmPlan msm_plan(uint64_t n) {
   const uint32_t lg = ceil_lg(n);
   const uint32_t forced = g_window_bits[lg].load(std::memory_order_relaxed);
   if (forced) return msm_plan_for(forced, 256 / forced + 1);
-  if (lg >= 10) {
-    const uint32_t c = lg <= 19 ? 13 : lg <= 23 ? 16 : 18;
+  if (lg >= 8) {
+    const uint32_t c = lg <= 9 ? 8 : lg <= 15 ? 10 : lg <= 19 ? 13 : lg <= 23 ? 16 : 18;
     return msm_plan_for(c, 256 / c + 1);
   }
   uint32_t best_c = 0;
@@ -336,7 +338,7 @@ __global__ void k_msm_scatter(const uint32_t *__restrict__ digits, uint64_t n, M
 
 constexpr int kPointThreads = 128;
 constexpr int kAccumulateBlocks = 3;       // resident blocks per SM (168 registers)
-constexpr uint32_t kRunMin = 10, kRunMax = 64;
+constexpr uint32_t kRunMin = 4, kRunMax = 64;
 constexpr uint32_t kJoinMin = 3;           // partial sums one thread adds up (3 / 5 / 8:
                                            // 200003 points 2.42 / 2.45 / 2.47 ms)
 constexpr uint32_t kJoinChunk = 1024;      // partial sums one block adds up
@@ -346,8 +348,10 @@ constexpr uint32_t kJoinChunk = 1024;      // partial sums one block adds up
 // Fixed-base 2^20 points (17.8 M entries): 7.85 ms as one wave of 306 entries,
 // 7.33 / 6.98 / 7.05 / 7.03 with runs of at most 128 / 64 / 48 / 32: the SMs do
 // not keep step, and shorter waves even that out.  4 blocks per SM (128
-// registers, spills): no faster.  Runs shorter than kRunMin cost more partial
-// sums and workspace than they save.  The kernels take it from the list's real
+// registers, spills): no faster.  Lists too short to fill the chip take runs of
+// kRunMin, whose additions follow one another (10 us each); 4 / 6 / 10: 2000 points
+// 835 / 852 / 876 us, window tables 1000 points 420 / 430 / 470, 2^13 473 / 500 /
+// 512, but 8000 points 932 / 905 / 934.  The kernels take it from the list's real
 // length (zero digits have no entry): half of 2^18 scalars zero and the rest one
 // took 1638 us with runs sized for a full list.
 __host__ __device__ __forceinline__ uint32_t equal_run(uint64_t items, uint32_t resident, uint32_t least,
@@ -1189,14 +1193,16 @@ __global__ void __launch_bounds__(kPointThreads)
   }
 }
 
-// Window bits for a fixed point set, from the same kind of sweep (c = 12..20,
-// 2^14..2^24 points on GB300) and the same top-window effect: 13 up to 2^14
+// Window bits for a fixed point set, from the same kind of sweep (c = 10..20,
+// 2^8..2^24 points on GB300) and the same top-window effect: 13 up to 2^11
 // points, 16 up to 2^21 (2^20: 10.72 ms against 10.98 for 17 and 11.83 for
 // 15), 20 beyond (2^22: 33.8 against 35.8 for 19).  One bucket set serves all
-// windows, so a large c costs little aggregation.
+// windows, so a large c costs little aggregation, and a bucket of many entries is
+// joined from many runs.  Microseconds with 13 / 16: 4096 points 511 / 454, 8000
+// 688 / 473, 2^14 854 / 528.
 uint32_t fixed_window_bits(uint64_t n) {
   const uint32_t lg = ceil_lg(n);
-  return lg <= 14 ? 13 : lg <= 21 ? 16 : 20;
+  return lg <= 11 ? 13 : lg <= 21 ? 16 : 20;
 }
 
 // The pipeline behind both entry points.  points holds n affine points (one
