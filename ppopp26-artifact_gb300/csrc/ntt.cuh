@@ -62,6 +62,8 @@ struct NttInputDesc {
   // 128-byte lines of the NVLink-C2C traffic
   bool in_host = false;
   bool out_host = false;
+  // the launch before it in the stream is another transform's last pass
+  bool follows = false;
 };
 
 // The transform of 2^lg_m points with every pass reading and writing

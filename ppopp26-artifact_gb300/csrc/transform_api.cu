@@ -77,6 +77,7 @@ int lde_run(const fr *in, fr *out, uint32_t lg_n, uint32_t lambda, uint32_t mode
   if (st) return st;
   desc.kind = pp::NTT_IN_DIAG;
   desc.in_host = false;
+  desc.follows = true;
   desc.diag = pp::pow_table(pp::host_mont_small(7), lg_n, &st);
   if (st) return st;
   return pp::ntt_run(coef, out, L, false, desc, s);
