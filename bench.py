@@ -40,8 +40,9 @@ MM_PER_NTT = (N // 2) * LG_N          # algorithmic Montgomery multiplies (radix
 INSTR_PER_MM = 256                     # 8x8 limbs: 4 n^2 integer multiply instructions
 BYTES_PER_NTT = 2 * 32 * N             # read + write once
 IMAD_PER_CLK_PER_SM = 64               # 32-bit multiply-add lanes per SM per clock (nominal)
-EXEC_MM_PER_NTT = int(11.375 * N)      # multiplies the shipped 9,6,9 split executes (unit twiddles skipped)
-WIDE_PER_MM = 112                      # mad.wide products per Montgomery multiply (r's two low limbs are free)
+# wide products the shipped 9,6,9 split executes (unit twiddles skipped): 9.375 N multiplies by
+# four-part constants of 82 and 2 N by layer twiddles of 112
+EXEC_WIDE_PER_NTT = int((9.375 * 82 + 2 * 112) * N)
 
 
 def parse():
@@ -386,15 +387,15 @@ def run_ours(args, rank, world, local):
                      "measured_rates_T_per_s": {k: round(v / 1e12, 4) for k, v in rates.items()},
                      "traffic": traffic,
                      "frac_of_wide_multiply_rate": round(
-                         EXEC_MM_PER_NTT * WIDE_PER_MM / sec_per_ntt / rates["mad_wide_per_s"], 4),
+                         EXEC_WIDE_PER_NTT / sec_per_ntt / rates["mad_wide_per_s"], 4),
                      "wide_product_ceiling": round(2 * rates["mad_wide_per_s"] / 1e12, 3),
                      "frac_of_wide_product_ceiling": round(achieved_int / (2 * rates["mad_wide_per_s"] / 1e12), 4),
                      "note": "algorithmic (N/2)lgN Montgomery multiplies x 256 32-bit multiply instructions; "
                              "peak = the measured low-half (mad.lo) rate; half of the 256 are high halves, "
                              "which run at 0.38 of that rate; the fastest measured instruction for a low and "
                              "high half is one mad.wide, so wide_product_ceiling = 2 x the measured mad.wide "
-                             "rate bounds the 256 instructions. frac_of_wide_multiply_rate: the 11.375 N multiplies the "
-                             "transform executes x 112 mad.wide products each, over the measured mad.wide "
+                             "rate bounds the 256 instructions. frac_of_wide_multiply_rate: the mad.wide products the "
+                             "transform executes (9.375 N multiplies of 82, 2 N of 112), over the measured mad.wide "
                              "rate"},
         "roofline_hbm": {"bound": "hbm", "achieved": round(achieved_hbm, 2), "peak": peaks.get("hbm_gbs"),
                          "unit": "GB/s", "frac": round(achieved_hbm / peaks.get("hbm_gbs", 6800.0), 4),
