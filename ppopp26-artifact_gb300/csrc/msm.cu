@@ -1075,21 +1075,25 @@ struct MsmLayout {
   uint32_t runs;     // runs of the list at most
 };
 
-// Rounds of pair sums before the buckets are accumulated: while a round has 28
-// outputs per resident thread, over which an inversion and the round's launches
-// spread, and 8 per bucket, below which unpaired entries and steps between buckets
+// Rounds of pair sums before the buckets are accumulated: while a round has 14
+// outputs per resident thread (28 with window tables), over which an inversion and
+// the round's launches spread, and 8 per bucket, below which unpaired entries and steps between buckets
 // take the gain.  Milliseconds with 0, 1, 2, 3 and 4 rounds (rule's choice marked):
 //   200003 points  3.13 3.08* 3.12 3.30 3.55   window tables 2.03 2.00* 2.07 2.25
 //   2^20 points    8.42 7.97 7.87* 7.94 8.10   window tables 6.97 6.46 6.29 6.23* 6.26
 //   2^22 points    26.7 24.4 23.1 22.6 22.5*
 //   2^16 points    2.05* 2.18 2.47             window tables 1.16* 1.35 1.53
+// Since inversions take 33 instead of 57 us the bound is 14 instead of 28: 2^17 points
+// 1937 -> 1893 us, 2^18 2792 -> 2719, 200003 2368 -> 2350; with window tables 2^17
+// 1236 -> 1250, 200003 1605 -> 1623, so it stays 28 there.
 // The bound on the entries keeps the rounds' buffers below 20 GB.
 uint32_t pair_rounds(uint64_t n, const MsmPlan &p) {
   const uint64_t entries = (uint64_t)p.W * n, nb = (uint64_t)p.nsets * p.B;
   const uint64_t resident = (uint64_t)device_sm_count() * kAccumulateBlocks * kPointThreads;
+  const uint64_t per_thread = p.nsets > 1 ? 14 : 28;
   uint32_t r = 0;
   if (entries <= 1ull << 28)
-    while ((entries >> (r + 1)) >= 28 * resident && (entries >> (r + 1)) >= 8 * nb) ++r;
+    while ((entries >> (r + 1)) >= per_thread * resident && (entries >> (r + 1)) >= 8 * nb) ++r;
   return r;
 }
 // outputs of a round over that many inputs, at most: every bucket rounds up
