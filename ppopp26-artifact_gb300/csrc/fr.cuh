@@ -1185,11 +1185,16 @@ PP_HD fr fr_mul_lazy(const fr &a, const fr &b) {
 // 256 bits where a general product needs eight: 64 + 18 = 82 wide products
 // instead of 112.  a is any 256-bit value.  The sum is below 2^66 r, so the
 // result, (sum - M r) / 2^96 + r with 0 <= M < 2^96, is in (0, r + 2^-30 r]:
-// it is a lazy value (below 2r).
+// it is a lazy value (below 2r), and its upper end is reached by small a (a = 0
+// gives r), so the sum of it and a canonical value is not.  Without LAZY r is
+// added to negative values only, which leaves the canonical form: (sum - M r) / 2^96
+// + M 2^160 is below 2^256 - r + 2^-30 r, so taking M 2^160 away from it borrows
+// exactly when the value is negative.
 // Parts of 128 bits would need five steps (94 products) and two constants,
 // of 32 bits two steps (76) and eight.  GB300, two chains per thread: 108 G/s
 // for four, 95 G/s for two, against 78 G/s for the general lazy multiply.
 // ---------------------------------------------------------------------------
+template <bool LAZY = true>
 PP_HD fr fr_mul_const4(const fr &a, const fr w[4]) {
   uint32_t E[12], O[12];  // cells at words 0, 2, .. and 1, 3, ..
   uint32_t c8 = 0;        // carries into word 8, where E holds product words
@@ -1232,8 +1237,14 @@ PP_HD fr fr_mul_const4(const fr &a, const fr w[4]) {
   // - M 2^160 (M's words were collected at 2^256, words 8 .. 10), + r
   o.v[5] = sub_cc(o.v[5], m0);
   o.v[6] = subc_cc(o.v[6], m1);
-  o.v[7] = subc(o.v[7], m2);
-  fr_add_r_masked(o.v, 0xffffffffu);
+  uint32_t add = 0xffffffffu;
+  if constexpr (LAZY) {
+    o.v[7] = subc(o.v[7], m2);
+  } else {
+    o.v[7] = subc_cc(o.v[7], m2);
+    add = subc(0, 0);  // all ones on borrow
+  }
+  fr_add_r_masked(o.v, add);
   return o;
 }
 

@@ -794,8 +794,9 @@ __global__ void __launch_bounds__(kScanThreads + 32, 2)
   if (threadIdx.x == 0) st_fr(block_s + blockIdx.x, W);
 }
 
-// The exact S at the block's end, then at the chunk's, then the chunk replayed:
-// m as a four-part constant, S below 2.01 r in between.
+// The exact S at the block's end, then at the chunk's, then the chunk replayed: m as
+// a four-part constant.  The product is canonical, so S, its unreduced sum with a
+// coefficient, is below 2r as fr_canon needs.
 __global__ void __launch_bounds__(kScanThreads, 2)
     k_div_apply(fr *inout, ScanGeom g, const fr *__restrict__ c_ptr, const fr *__restrict__ thread_s,
                 const fr *__restrict__ block_s, const DivPowers *__restrict__ powers) {
@@ -832,7 +833,7 @@ __global__ void __launch_bounds__(kScanThreads, 2)
       if (e == 0 || tile * kTileElems + e < g.k) {
         const fr pi = ct.get(slot, e);
         ct.put(slot, e, fr_canon(s));  // q_i = S_(i+1)
-        s = fr_add_raw(pi, fr_mul_const4(s, m));
+        s = fr_add_raw(pi, fr_mul_const4<false>(s, m));
       }
   });
 }
