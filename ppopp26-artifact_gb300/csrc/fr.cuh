@@ -534,10 +534,6 @@ PP_HD fr fr_mul_kara(const fr &a, const fr &b) {
   return mont_redc16(t);
 }
 
-#ifndef PP_MUL_VARIANT
-#define PP_MUL_VARIANT 14  // fr_mul_cells
-#endif
-
 // ---------------------------------------------------------------------------
 // Variants 6-8: bare 32x32->64 products (mul.wide, no addend) whose halves
 // are summed by explicit add-with-carry chains.  On sm_103a a wide multiply
@@ -1071,37 +1067,12 @@ PP_HD uint32_t fr_redc8_cells(uint32_t o[8], const uint32_t *t) {
   return subc(top, 0);
 }
 
-PP_HD fr fr_mul(const fr &a, const fr &b) {
-#if PP_MUL_VARIANT == 2
-  return fr_mul_w(a, b);
-#elif PP_MUL_VARIANT == 3
-  return fr_mul_kara<false>(a, b);
-#elif PP_MUL_VARIANT == 4
-  return fr_mul_kara<true>(a, b);
-#elif PP_MUL_VARIANT == 5
-  return fr_mul_sos(a, b);
-#elif PP_MUL_VARIANT == 6
-  return fr_mul_split<1, 1>(a, b);
-#elif PP_MUL_VARIANT == 7
-  return fr_mul_split<1, 0>(a, b);
-#elif PP_MUL_VARIANT == 8
-  return fr_mul_split<0, 1>(a, b);
-#elif PP_MUL_VARIANT == 9
-  return fr_mul_row9(a, b);
-#elif PP_MUL_VARIANT == 10
-  return fr_mul_kara_rows(a, b);
-#elif PP_MUL_VARIANT == 11
-  return fr_mul_mix<0, 1>(a, b);
-#elif PP_MUL_VARIANT == 12
-  return fr_mul_mix<1, 0>(a, b);
-#elif PP_MUL_VARIANT == 13
-  return fr_mul_mix<0, 2>(a, b);
-#elif PP_MUL_VARIANT == 14
-  return fr_mul_cells(a, b);
-#else
-  return fr_mul_v<PP_MUL_VARIANT>(a, b);
-#endif
-}
+// The kernels' multiply.  Canonical when one factor is canonical (the other any
+// 256-bit value); of two factors below 2r the product is below 1.82 r.  The kernels
+// that keep their values lazy (constraint.cu, k_perm_local) rely on the second: the
+// row forms above need one canonical factor, since theirs would pass 2^256, so none of
+// them can stand in here.
+PP_HD fr fr_mul(const fr &a, const fr &b) { return fr_mul_cells(a, b); }
 
 // rows I .. 6 of the cross products a_I a_j (j > I) of a square: words I + j,
 // even ones in E, odd ones in O (word k at O[k - 1])
@@ -1165,15 +1136,7 @@ PP_HD fr fr_sqr(const fr &a) {
 // result.  fr_mul_lazy takes a < 2r and b < r (the twiddle) and returns a
 // value < 2r.
 PP_HD fr fr_mul_lazy(const fr &a, const fr &b) {
-#if PP_MUL_VARIANT == 14
   return fr_mul_cells<true>(a, b);
-#elif PP_MUL_VARIANT == 9
-  return fr_mul_row9<true>(a, b);
-#else
-  fr c = a;
-  fr_reduce_once(c.v);
-  return fr_mul(c, b);
-#endif
 }
 
 // ---------------------------------------------------------------------------
