@@ -1260,11 +1260,12 @@ PP_HD fr fr_add_lazy(const fr &a, const fr &b) {
 
 // a - b mod 2r for a, b < 2r.  On the device the 2r comes back as predicated
 // additions: 18 instructions where masking each word of 2r takes 25 (2^24
-// transform 2874 -> 2845 us).
+// transform 2874 -> 2845 us).  Volatile like every statement that uses the carry flag:
+// the flag passes between statements, and only volatile ones keep their order.
 PP_HD fr fr_sub_lazy(const fr &a, const fr &b) {
   fr d;
 #if defined(__CUDA_ARCH__)
-  asm("{\n\t.reg .pred p;\n\t.reg .u32 m;\n\t"
+  asm volatile("{\n\t.reg .pred p;\n\t.reg .u32 m;\n\t"
       "sub.cc.u32 %0, %8, %16;\n\tsubc.cc.u32 %1, %9, %17;\n\tsubc.cc.u32 %2, %10, %18;\n\tsubc.cc.u32 %3, %11, %19;\n\t"
       "subc.cc.u32 %4, %12, %20;\n\tsubc.cc.u32 %5, %13, %21;\n\tsubc.cc.u32 %6, %14, %22;\n\tsubc.cc.u32 %7, %15, %23;\n\t"
       "subc.u32 m, 0, 0;\n\tsetp.ne.u32 p, m, 0;\n\t"
