@@ -14,12 +14,23 @@
 // 590 and 879 (P. Wuille and G. Maxwell, "Bounds on divsteps iterations in safegcd",
 // 2021).
 //
+// Steps in a row are divisions.  After an exchange at delta the next steps keep f, and
+// the first delta + 1/2 of them (with delta at a half) add f to g or not, as g is odd
+// or even, and halve it: together they add the w f, 0 <= w < 2^(delta + 1/2), that makes
+// g divisible by 2^(delta + 1/2), so
+//   (f, g) -> (g, w g - f),  w = f / g (mod 2^(delta + 1/2)),  and g's zero bits go;
+// as g then has at least that many of them, delta is positive again and the next
+// division follows.  A division is three multiply-adds (f and g, and the two columns of
+// their coefficients), however many steps it stands for.
+//
 // B divsteps depend only on the low B + 2 bits of f and g, so they run on
 // one machine word each and record a 2x2 integer matrix T with
 // 2^B [f', g'] = T [f, g]; |u| + |v| <= 2^B and |q| + |r| <= 2^B.  T is then
 // applied to the full f, g (the division by 2^B is exact) and to the pair
 // d, e with f = d x, g = e x (mod M), where the division by 2^B is done mod
-// M by first adding the multiple of M that clears the low B bits.
+// M by first adding the multiple of M that clears the low B bits.  That multiple is
+// taken from [-2^(B-1), 2^(B-1)) M, so a batch adds at most M / 2 to the larger of |d|
+// and |e|: they stay below (1 + batches / 2) M and are not reduced until the end.
 //
 // Numbers are NL limbs of B bits, least significant first; limbs below the
 // top one are in [0, 2^B) and the top limb carries the sign.  Two widths:
@@ -28,9 +39,8 @@
 // 128-bit sums (a 64-bit host CPU's form; on a GB300 it took 1.2 to 1.6 times
 // the 30-bit form's time, a binary GCD 1.6 to 4.6 times).
 //
-// GB300, 30-bit form: a lone thread inverts in 19.4 us (Fr) and 33.3 us (Fq); 34.5
-// and 57.1 us one divstep at a time with d and e reduced after each batch.  One per lane,
-// 9728 warps: 0.65 and 1.18 ns (0.96 and 1.89).
+// GB300, 30-bit form: a lone thread inverts in 18.6 us (Fr) and 32.0 us (Fq); 34.5
+// and 57.1 us one divstep at a time with d and e reduced after each batch.
 #pragma once
 #include <cstdint>
 
@@ -78,127 +88,129 @@ PP_HD int ctz_word(uint64_t x) {
 #endif
 }
 
-// ---- B divsteps on the low words.  Returns the updated D = delta - 1/2; T in u..r.
-// A divstep with delta <= 0 keeps f and adds it to an odd g before halving, so up to
-// 1/2 - delta = -D of them in a row come to one: g + w f with the w that clears the
-// low bits, w = -g / f modulo a power of two; f (f^2 - 2) = -1 / f modulo 2^6 for odd
-// f, since (f^2 - 1)^2 is a multiple of 64.  One with delta > 0 is an exchange
-// (f, g) -> (g, -f), delta -> -delta, and such a step.
+// a b + s; on the device one instruction, whatever the compiler knows of a and b (left to
+// itself it spends several on the products by M's limbs: 20.0 against 18.6 us)
+PP_HD int64_t mad_limbs(int32_t a, int32_t b, int64_t s) {
+#ifdef __CUDA_ARCH__
+  int64_t r;
+  asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(s));
+  return r;
+#else
+  return (int64_t)a * b + s;
+#endif
+}
+PP_HD __int128 mad_limbs(int64_t a, int64_t b, __int128 s) { return (__int128)a * b + s; }
+
+// B divsteps as a matrix: f' = (u f + v g) / 2^B, g' = (q f + r g) / 2^B
 template <typename L>
-PP_HD int divsteps_word(int D, typename LimbTraits<L>::U f0, typename LimbTraits<L>::U g0,
-                        L &u_out, L &v_out, L &q_out, L &r_out) {
-  using U = typename LimbTraits<L>::U;
-  constexpr int B = LimbTraits<L>::B;
-  U u = 1, v = 0, q = 0, r = 1;
-  int left = B;
-  for (;;) {
-    const int z = ctz_word(g0 | ((U)~(U)0 << left));  // a run of zero bits, at most `left`
-    g0 >>= z;
-    u <<= z;
-    v <<= z;
-    D += z;
-    left -= z;
-    if (left == 0) break;
-    if (D >= 0) {
-      D = -D - 1;
-      U t = f0;
-      f0 = g0;
-      g0 = 0 - t;
-      t = u;
-      u = q;
-      q = 0 - t;
-      t = v;
-      v = r;
-      r = 0 - t;
-    }
-    int bits = -D < left ? -D : left;
-    if (bits > 6) bits = 6;
-    const U w = (f0 * g0 * (f0 * f0 - 2)) & (((U)1 << bits) - 1);
-    g0 += w * f0;
-    q += w * u;
-    r += w * v;
-  }
-  u_out = (L)u;
-  v_out = (L)v;
-  q_out = (L)q;
-  r_out = (L)r;
-  return D;
+struct DivMatrix {
+  L u, v, q, r;
+};
+
+// x / y modulo 2^bits, or 2^10 where that is less; y odd.  3 y with its second bit
+// flipped is 1 / y modulo 2^5 (P. Montgomery's start), one of Newton's steps makes that
+// ten bits.  Longer quotients are rare: a branch for them costs each division more (lone
+// thread 22.3 against 18.6 us) than finishing them in a second piece.
+template <typename U>
+PP_HD U quotient_mod2(U x, U y, int bits) {
+  const U inv = (3 * y) ^ 2;
+  return (x * inv) * (2 - y * inv) & (((U)1 << (bits < 10 ? bits : 10)) - 1);
 }
 
-// [f, g] = T [f, g] / 2^B (exact)
+// ---- B divsteps on the low words; D is delta - 1/2
+template <typename L>
+PP_HD void divide_batch(int &D, typename LimbTraits<L>::U f, typename LimbTraits<L>::U g, DivMatrix<L> &T) {
+  using U = typename LimbTraits<L>::U;
+  // f and g are fF F + fG G and gF F + gG G over a power of two, F and G the words given
+  U fF = 1, fG = 0, gF = 0, gG = 1;
+  int left = LimbTraits<L>::B;
+  const auto strip = [&] {  // g's zero bits, at most `left` of them
+    const int zeros = ctz_word(g | (U)1 << left);
+    g >>= zeros;
+    fF <<= zeros;
+    fG <<= zeros;
+    D += zeros;
+    left -= zeros;
+  };
+  strip();
+  while (left > 0) {
+    if (D < 0) {  // the rest of a long division, or of one that the batch before began
+      const U w = quotient_mod2<U>(0 - g, f, -D < left ? -D : left);
+      g += w * f;
+      gF += w * fF;
+      gG += w * fG;
+      strip();
+    }
+    while (left > 0 && D >= 0) {  // g is odd here
+      const U w = quotient_mod2<U>(f, g, D < left ? D + 1 : left);
+      const U rest = w * g - f, restF = w * gF - fF, restG = w * gG - fG;
+      f = g, fF = gF, fG = gG;
+      g = rest, gF = restF, gG = restG;
+      D = -1 - D;
+      strip();
+    }
+  }
+  T = {(L)fF, (L)fG, (L)gF, (L)gG};
+}
+
+// [x, y] = T [x, y] / 2^B: exact (f and g), or modulo M.  A limb's products are summed
+// before the carry joins them, so the chain along the limbs is two additions a limb.
+template <bool EXACT, typename L, int NL>
+PP_HD void apply_batch(SLimbs<L, NL> &x, SLimbs<L, NL> &y, const DivMatrix<L> &T, const ModulusB<L, NL> &M) {
+  using A = typename LimbTraits<L>::A;
+  using U = typename LimbTraits<L>::U;
+  constexpr int B = LimbTraits<L>::B, PAD = 8 * (int)sizeof(U) - B;
+  constexpr U MASK = ((U)1 << B) - 1;
+  A sx = (A)T.u * x.l[0] + (A)T.v * y.l[0], sy = (A)T.q * x.l[0] + (A)T.r * y.l[0];
+  L mx = 0, my = 0;  // multiples of M
+  if (!EXACT) {
+    mx = (L)((0 - (U)sx * M.inv) << PAD) >> PAD;
+    my = (L)((0 - (U)sy * M.inv) << PAD) >> PAD;
+    sx += (A)mx * M.m[0];
+    sy += (A)my * M.m[0];
+  }
+#pragma unroll
+  for (int i = 1; i < NL; ++i) {
+    A px = mad_limbs(T.v, y.l[i], mad_limbs(T.u, x.l[i], 0)), py = mad_limbs(T.r, y.l[i], mad_limbs(T.q, x.l[i], 0));
+    if (!EXACT) {
+      px = mad_limbs(mx, M.m[i], px);
+      py = mad_limbs(my, M.m[i], py);
+    }
+    sx = (sx >> B) + px;
+    sy = (sy >> B) + py;
+    x.l[i - 1] = (L)((U)sx & MASK);
+    y.l[i - 1] = (L)((U)sy & MASK);
+  }
+  sx >>= B;
+  sy >>= B;
+  x.l[NL - 1] = (L)sx;
+  y.l[NL - 1] = (L)sy;
+}
+
+// sign x modulo M, in [0, 5/4 M), for |x| < 20 M and sign = 1 or -1.  The multiple of M
+// comes from the top limbs: t is at most sign x / 2^s and less than 2 below it (1 where
+// sign is 1), M / 2^s lies between the modulus's top limb and one more, and the quotient
+// is rounded down towards the side where nothing is taken too often.  What is left is
+// below 1 + 22 / (top limb) times M, and the smallest top limb is 115.
 template <typename L, int NL>
-PP_HD void apply_fg(SLimbs<L, NL> &f, SLimbs<L, NL> &g, L u, L v, L q, L r) {
+PP_HD void reduce_once_signed(SLimbs<L, NL> &x, L sign, const ModulusB<L, NL> &M) {
   using A = typename LimbTraits<L>::A;
   using U = typename LimbTraits<L>::U;
   constexpr int B = LimbTraits<L>::B;
   constexpr U MASK = ((U)1 << B) - 1;
-  A cf = (A)u * f.l[0] + (A)v * g.l[0];
-  A cg = (A)q * f.l[0] + (A)r * g.l[0];
-  cf >>= B;
-  cg >>= B;
-#pragma unroll
-  for (int i = 1; i < NL; ++i) {
-    cf += (A)u * f.l[i] + (A)v * g.l[i];
-    cg += (A)q * f.l[i] + (A)r * g.l[i];
-    f.l[i - 1] = (L)((U)cf & MASK);
-    g.l[i - 1] = (L)((U)cg & MASK);
-    cf >>= B;
-    cg >>= B;
-  }
-  f.l[NL - 1] = (L)cf;
-  g.l[NL - 1] = (L)cg;
-}
-
-// x, or -x where neg is all ones, plus M where mask is all ones
-template <typename L, int NL>
-PP_HD void negate_add(SLimbs<L, NL> &x, L neg, L mask, const ModulusB<L, NL> &M) {
-  using U = typename LimbTraits<L>::U;
-  constexpr int B = LimbTraits<L>::B;
-  constexpr U MASK = ((U)1 << B) - 1;
-  L c = 0;
+  const L top = M.m[NL - 1], t = sign < 0 ? -1 - x.l[NL - 1] : x.l[NL - 1];
+  const L k = t < 0 ? -((top - 1 - t) / top) : t / (top + 1);
+  A c = 0;
 #pragma unroll
   for (int i = 0; i < NL; ++i) {
-    c += ((x.l[i] ^ neg) - neg) + (M.m[i] & mask);
+    c += (A)sign * x.l[i] - (A)k * M.m[i];
     if (i < NL - 1) {
       x.l[i] = (L)((U)c & MASK);
       c >>= B;
     } else {
-      x.l[i] = c;
+      x.l[i] = (L)c;
     }
   }
-}
-
-// [d, e] = T [d, e] / 2^B mod M, d and e in (-2M, M) before and after: with M added to
-// negative ones u d + v e lies within 2^B M of 0 (|u| + |v| <= 2^B), and the multiple
-// of M that clears the low B bits, taken in (-2^B M, 0], leaves (-2^(B+1) M, 2^B M).
-template <typename L, int NL>
-PP_HD void apply_de(SLimbs<L, NL> &d, SLimbs<L, NL> &e, L u, L v, L q, L r,
-                    const ModulusB<L, NL> &M) {
-  using A = typename LimbTraits<L>::A;
-  using U = typename LimbTraits<L>::U;
-  constexpr int B = LimbTraits<L>::B;
-  constexpr U MASK = ((U)1 << B) - 1;
-  const L sd = d.l[NL - 1] < 0 ? -1 : 0, se = e.l[NL - 1] < 0 ? -1 : 0;
-  A cd = (A)u * d.l[0] + (A)v * e.l[0];
-  A ce = (A)q * d.l[0] + (A)r * e.l[0];
-  L md = (u & sd) + (v & se), me = (q & sd) + (r & se);
-  md -= (L)(((U)cd * M.inv + (U)md) & MASK);
-  me -= (L)(((U)ce * M.inv + (U)me) & MASK);
-  cd += (A)md * M.m[0];
-  ce += (A)me * M.m[0];
-  cd >>= B;
-  ce >>= B;
-#pragma unroll
-  for (int i = 1; i < NL; ++i) {
-    cd += (A)u * d.l[i] + (A)v * e.l[i] + (A)md * M.m[i];
-    ce += (A)q * d.l[i] + (A)r * e.l[i] + (A)me * M.m[i];
-    d.l[i - 1] = (L)((U)cd & MASK);
-    e.l[i - 1] = (L)((U)ce & MASK);
-    cd >>= B;
-    ce >>= B;
-  }
-  d.l[NL - 1] = (L)cd;
-  e.l[NL - 1] = (L)ce;
 }
 
 template <typename L, int NL>
@@ -209,10 +221,9 @@ PP_HD bool is_zero_limbs(const SLimbs<L, NL> &x) {
   return o == 0;
 }
 
-// x^-1 mod M for 0 <= x < M, M an odd prime; 0 -> 0.  max_batches bounds the
-// loop: it must cover the divstep bound of the modulus's size (741 for
-// 256-bit inputs, 1101 for 381-bit ones) in batches of B.  An input that does
-// not finish within them (not below M) gives 0.
+// x^-1 mod M, in [0, 5/4 M), for 0 <= x < M, M an odd prime; 0 -> 0.  The loop ends
+// when g is 0; max_batches (at most 38) only stops an input that is not below M, which
+// then gives 0, and covers the divstep bound of the modulus's size.
 template <typename L, int NL>
 PP_HD SLimbs<L, NL> modinv_divsteps(const SLimbs<L, NL> &x, const ModulusB<L, NL> &M,
                                     int max_batches) {
@@ -231,12 +242,10 @@ PP_HD SLimbs<L, NL> modinv_divsteps(const SLimbs<L, NL> &x, const ModulusB<L, NL
   int D = 0;
   bool done = false;
   for (int b = 0; b < max_batches && !done; ++b) {
-    L u, v, q, r;
-    const U f0 = (U)f.l[0] | ((U)f.l[1] << B);
-    const U g0 = (U)g.l[0] | ((U)g.l[1] << B);
-    D = divsteps_word<L>(D, f0, g0, u, v, q, r);
-    apply_fg(f, g, u, v, q, r);
-    apply_de(d, e, u, v, q, r, M);
+    DivMatrix<L> T;
+    divide_batch<L>(D, (U)f.l[0] | ((U)f.l[1] << B), (U)g.l[0] | ((U)g.l[1] << B), T);
+    apply_batch<true>(f, g, T, M);
+    apply_batch<false>(d, e, T, M);
     done = is_zero_limbs(g);
   }
   if (!done) {
@@ -244,11 +253,8 @@ PP_HD SLimbs<L, NL> modinv_divsteps(const SLimbs<L, NL> &x, const ModulusB<L, NL
     for (int i = 0; i < NL; ++i) d.l[i] = 0;
     return d;
   }
-  // f = +-1: x^-1 = +-d, d in (-2M, M)
-  negate_add(d, (L)0, d.l[NL - 1] < 0 ? (L)-1 : (L)0, M);
-  const L neg = f.l[NL - 1] < 0 ? (L)-1 : (L)0;
-  negate_add(d, neg, (L)0, M);
-  negate_add(d, (L)0, d.l[NL - 1] < 0 ? (L)-1 : (L)0, M);
+  // f = +-1: x^-1 = +-d
+  reduce_once_signed(d, f.l[NL - 1] < 0 ? (L)-1 : (L)1, M);
   return d;
 }
 
