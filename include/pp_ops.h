@@ -50,7 +50,11 @@ int pp_ntt(const void *d_in, void *d_out, uint32_t lg_n, int inverse, void *stre
 
 /* Builds (synchronously) the cached twiddle tables of a transform size so
  * that later pp_ntt calls of that size only launch the pass kernels (e.g.
- * before CUDA-graph capture).  The reference builds its table blob in the
+ * before CUDA-graph capture), and so do pp_ntt_host calls: where their
+ * endpoints take a split of their own (stored splits with more than 9 bits at
+ * an end, e.g. 2^22), its tables, 32 * 2^lg_n bytes, are built too.  A
+ * capture of a pp_ntt_host call without them keeps the size's stored split.
+ * The reference builds its table blob in the
  * Ntt constructor (function.cu:278 -> zksnark_ntt.cu:17-39). */
 int pp_ntt_prepare(uint32_t lg_n, int inverse);
 

@@ -1023,7 +1023,7 @@ bool g_attr_set[64] = {false};
 
 }  // namespace
 
-int ntt_prepare(uint32_t lg_m, bool inverse) {
+int ntt_prepare(uint32_t lg_m, bool inverse, bool host_endpoints) {
   if (lg_m > PP_MAX_LG_N) return PP_E_UNSUPPORTED;
   int dev = 0;
   PP_CUDA_TRY(cudaGetDevice(&dev));
@@ -1032,6 +1032,11 @@ int ntt_prepare(uint32_t lg_m, bool inverse) {
   Plan *p = nullptr;
   int st = get_plan(dev, lg_m, inverse, &p);
   if (!st && ntt_small_form(lg_m)) st = get_plan(dev, lg_m, inverse, &p, true);
+  if (!st && host_endpoints && !ntt_small_form(lg_m)) {
+    NttInputDesc both;
+    both.in_host = both.out_host = true;
+    if (host_split_differs(lg_m, both)) st = get_plan(dev, lg_m, inverse, &p, false, false, true);
+  }
   return st;
 }
 

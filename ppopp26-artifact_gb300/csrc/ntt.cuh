@@ -121,7 +121,7 @@ int ntt_launch_level(const LevelParams &params, cudaStream_t stream);
 
 // Builds (or fetches) the cached tables for a transform size (for graph capture
 // the tables must exist before capture starts).
-int ntt_prepare(uint32_t lg_m, bool inverse);
+int ntt_prepare(uint32_t lg_m, bool inverse, bool host_endpoints = false);
 
 // h^i for i < n as a cached device table (coset diagonals)
 const fr *pow_table(const fr &h, uint32_t lg_n, int *status);

@@ -103,7 +103,7 @@ extern "C" int pp_lde(const void *d_in, void *d_out, uint32_t lg_n, uint32_t lam
 }
 
 extern "C" int pp_ntt_prepare(uint32_t lg_n, int inverse) {
-  return pp::ntt_prepare(lg_n, inverse != 0);
+  return pp::ntt_prepare(lg_n, inverse != 0, true);
 }
 
 // ------------------------------------------------- host-resident transforms
