@@ -418,8 +418,10 @@ int pp_gate_constraint(const pp_gate_args *a, void *d_out, uint64_t n, void *str
  * window aggregation runs on the GPU.  n < 2^31.  Uses a per-stream device
  * workspace of at most 56 W n + 360 W 2^(c-1) bytes (c = window bits, W =
  * 256 / c + 1 windows; pp_msm_g1_window_bits gives c), and up to 72 W n +
- * 72 W 2^(c-1) more, where the device has them, for the pair sums of large
- * buckets: 1.7 GB for 2^20 points, 6.4 GB for 2^22. */
+ * 72 W 2^(c-1) more, where the device has twice as much free, for the pair
+ * sums of large buckets: 1.7 GB for 2^20 points, 6.4 GB for 2^22.  Whether
+ * it has is asked once per stream and size, and not again before
+ * pp_release(); under capture the workspace at hand is used, and it stays. */
 int pp_msm_g1(const void *d_points, const void *d_scalars, uint64_t n, void *d_out, void *stream);
 int pp_msm_g1_window_bits(uint64_t n);
 /* Tuning: the window bits pp_msm_g1 uses for n with ceil(lg n) = lg_n

@@ -90,8 +90,10 @@ __device__ __forceinline__ fr mul_shared_const(const fr &x, const fr *k) {
 // One buffer per (device, stream, slot): work queued on one stream is ordered,
 // so calls on that stream may reuse it; different streams never share one.
 void *workspace_get(size_t bytes, cudaStream_t stream, int slot, int *status);
-// The same, of `most` bytes if the device has them beside the slot's present
-// buffer, else of `least` (kept, or grown as above); *got is which.
+// The same, of `most` bytes if the device has twice as many free, else of `least` (kept,
+// or grown as above); *got is which.  A size that did not fit is not tried again, and a
+// buffer of `least` bytes that a stream capture was given is not replaced by a larger one
+// (a graph may hold its address), as long as the slot lives.
 void *workspace_get_most(size_t most, size_t least, cudaStream_t stream, int slot, size_t *got, int *status);
 // frees every workspace of `stream` (call before destroying the stream)
 void workspace_release_stream(cudaStream_t stream);

@@ -28,6 +28,10 @@ struct WsKey {
 struct WsBuf {
   void *ptr = nullptr;
   size_t bytes = 0;
+  // workspace_get_most: the smallest larger size the device had no room for (0: none),
+  // and whether a capture took the buffer, so that a graph may hold its address
+  size_t refused = 0;
+  bool captured = false;
 };
 std::mutex g_ws_mu;
 std::map<WsKey, WsBuf> g_ws;
@@ -104,25 +108,30 @@ void *workspace_get_most(size_t most, size_t least, cudaStream_t stream, int slo
   {
     std::lock_guard<std::mutex> lk(g_ws_mu);
     WsBuf &b = g_ws[WsKey{dev, stream, slot}];
-    void *larger = nullptr;
-    // a capture must not allocate: the buffer at hand does
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (b.bytes < most && b.bytes >= least) cudaStreamIsCapturing(stream, &capture);
-    if (b.bytes < most && capture == cudaStreamCaptureStatusNone) {
-      PP_COUNT_ALLOC(most);
-      if (cudaMalloc(&larger, most) != cudaSuccess) {
+    cudaStreamIsCapturing(stream, &capture);
+    const bool capturing = capture != cudaStreamCaptureStatusNone, enough = b.bytes >= least;
+    if (capturing && enough) b.captured = true;
+    // a capture must not allocate, and a captured buffer stays where it is: the buffer at
+    // hand does
+    if (b.bytes < most && !(enough && b.captured) && !capturing && (b.refused == 0 || most < b.refused)) {
+      // as much again stays free for the process's other allocations
+      size_t free_bytes = 0, total_bytes = 0;
+      void *larger = nullptr;
+      if (cudaMemGetInfo(&free_bytes, &total_bytes) == cudaSuccess && most <= free_bytes / 2 &&
+          cudaMalloc(&larger, most) == cudaSuccess) {
+        PP_COUNT_ALLOC(most);
+        if (b.ptr) {
+          // the old buffer may still be in use by queued work on this stream
+          cudaStreamSynchronize(stream);
+          cudaFree(b.ptr);
+        }
+        b.ptr = larger;
+        b.bytes = most;
+      } else {
         cudaGetLastError();
-        larger = nullptr;
+        b.refused = most;
       }
-    }
-    if (larger) {
-      if (b.ptr) {
-        // the old buffer may still be in use by queued work on this stream
-        cudaStreamSynchronize(stream);
-        cudaFree(b.ptr);
-      }
-      b.ptr = larger;
-      b.bytes = most;
     }
     if (b.bytes >= most) {
       *got = most;
