@@ -416,10 +416,12 @@ int pp_gate_constraint(const pp_gate_args *a, void *d_out, uint64_t n, void *str
  * cuda::msm_zkp_cuda (PLONK/utils/zkp/cuda/zksnark_msm.cu:48-88) and
  * cpu::msm_collect_cpu (PLONK/utils/zkp/cpu/msmcollect.cpp:5-41); the final
  * window aggregation runs on the GPU.  n < 2^31.  Uses a per-stream device
- * workspace of at most 56 W n + 360 W 2^(c-1) bytes (c = window bits, W =
- * 256 / c + 1 windows; pp_msm_g1_window_bits gives c), and up to 72 W n +
- * 72 W 2^(c-1) more, where the device has twice as much free, for the pair
- * sums of large buckets: 1.7 GB for 2^20 points, 6.4 GB for 2^22.  Whether
+ * workspace of at most 131 W n bytes (16 W n + 30 MB where that is less) +
+ * 400 W 2^(c-1) + 32 KB (c = window bits, W = 256 / c + 1 windows;
+ * pp_msm_g1_window_bits gives c): 8.1 MB for 1000 points, 36 MB for 2^14.
+ * Up to 72 W n + 128 W 2^(c-1) more, where the device has twice as much free
+ * as both together, serve the pair sums of large buckets: 1.8 GB in all for
+ * 2^20 points, 6.5 GB for 2^22.  Whether
  * it has is asked once per stream and size, and not again before
  * pp_release(); under capture the workspace at hand is used, and it stays. */
 int pp_msm_g1(const void *d_points, const void *d_scalars, uint64_t n, void *d_out, void *stream);
@@ -441,7 +443,8 @@ int pp_msm_g1_set_window_bits(uint32_t lg_n, uint32_t window_bits);
  * done) and allocates with cudaMalloc; W n must stay below 2^31.
  * pp_msm_g1_fixed then computes sum_i s_i P_i for n scalars like pp_msm_g1:
  * every window's digits go to one shared set of 2^(c-1) buckets, so the
- * window sums run once and there is no Horner chain over the windows.  Call
+ * window sums run once and there is no Horner chain over the windows.  Its
+ * workspace is pp_msm_g1's with one set of 2^(c-1) buckets for the W.  Call
  * it with the device of the tables current.  pp_msm_g1_bases_destroy frees
  * the tables (a null handle is fine). */
 typedef struct pp_msm_bases pp_msm_bases;
