@@ -979,6 +979,29 @@ __global__ void k_zero1(fr *y) { st_fr(y, fr_zero()); }
 
 static bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
+static uint32_t perm_blocks(uint64_t n) { return (uint32_t)((n + kPermBlockRows - 1) / kPermBlockRows); }
+
+// scan_geom's rule with kEvalHorner threads per block
+static ScanGeom eval_geom(uint64_t n) {
+  const uint32_t bps = n <= kEvalSmallMax ? kEvalBlocksPerSmSmall : kEvalBlocksPerSm;
+  ScanGeom g;
+  g.n = n;
+  const uint64_t target = (uint64_t)device_sm_count() * bps * kEvalHorner;
+  g.k = (n + target - 1) / target;
+  if (g.k < 4) g.k = 4;
+  g.threads = (n + g.k - 1) / g.k;
+  g.blocks = (uint32_t)((g.threads + kEvalHorner - 1) / kEvalHorner);
+  return g;
+}
+
+size_t gp_perm_workspace(uint64_t n) { return 2 * (size_t)perm_blocks(n) * sizeof(fr); }
+size_t div_workspace(uint64_t n) {
+  const ScanGeom g = scan_geom(n, kDivBlocksPerSm);
+  return (g.threads + g.blocks) * sizeof(fr) + sizeof(DivPowers);
+}
+// block sums, then the ticket counter in a slot of its own
+size_t eval_workspace(uint64_t n) { return ((size_t)eval_geom(n).blocks + 1) * sizeof(fr); }
+
 }  // namespace pp
 
 using pp::fr;
@@ -1027,8 +1050,7 @@ extern "C" int pp_div_xplusc(void *d_inout, uint64_t n, const void *d_c, void *s
   const pp::ScanGeom g = pp::scan_geom(n, pp::kDivBlocksPerSm);
   int st = PP_OK;
   static_assert(sizeof(pp::DivPowers) % sizeof(fr) == 0, "in whole elements");
-  fr *ws = static_cast<fr *>(pp::workspace_get(
-      (g.threads + g.blocks) * sizeof(fr) + sizeof(pp::DivPowers), s, 1, &st));
+  fr *ws = static_cast<fr *>(pp::workspace_get(pp::div_workspace(n), s, 1, &st));
   if (st) return st;
   fr *thread_s = ws, *block_s = ws + g.threads;
   pp::DivPowers *powers = reinterpret_cast<pp::DivPowers *>(block_s + g.blocks);
@@ -1057,20 +1079,12 @@ extern "C" int pp_eval(const void *d_poly, uint64_t n, const void *d_x, void *d_
     PP_LAUNCH_CHECK();
     return PP_OK;
   }
-  // scan_geom's rule with kEvalHorner threads per block
   constexpr uint32_t HT = pp::kEvalHorner;
-  const uint32_t bps = n <= pp::kEvalSmallMax ? pp::kEvalBlocksPerSmSmall : pp::kEvalBlocksPerSm;
-  pp::ScanGeom g;
-  g.n = n;
-  const uint64_t target = (uint64_t)pp::device_sm_count() * bps * HT;
-  g.k = (n + target - 1) / target;
-  if (g.k < 4) g.k = 4;
-  g.threads = (n + g.k - 1) / g.k;
-  g.blocks = (uint32_t)((g.threads + HT - 1) / HT);
+  const pp::ScanGeom g = pp::eval_geom(n);
   const uint32_t nb = g.blocks;
   int st = PP_OK;
   // block sums, then the ticket counter in its own 32-byte slot
-  char *ws = static_cast<char *>(pp::workspace_get((nb + 1) * sizeof(fr), s, 1, &st));
+  char *ws = static_cast<char *>(pp::workspace_get(pp::eval_workspace(n), s, 1, &st));
   if (st) return st;
   fr *block_val = reinterpret_cast<fr *>(ws);
   uint32_t *ticket = reinterpret_cast<uint32_t *>(ws + nb * sizeof(fr));
@@ -1101,13 +1115,11 @@ extern "C" int pp_gp_perm(const void *const *d_w, const void *const *d_sigma, co
   }
   cudaStream_t s = (cudaStream_t)stream;
   const uint64_t n = 1ull << lg_n;
-  const uint64_t nb64 = (n + pp::kPermBlockRows - 1) / pp::kPermBlockRows;
-  const uint32_t nb = (uint32_t)nb64;
+  const uint32_t nb = pp::perm_blocks(n);
   int st = PP_OK;
   const fr *omega_pow = pp::pow_table(pp::host_root_of_unity((int)lg_n, false), lg_n, &st);
   if (st) return st;
-  fr *ws = static_cast<fr *>(
-      pp::workspace_get(2 * (size_t)nb * sizeof(fr), s, 1, &st));
+  fr *ws = static_cast<fr *>(pp::workspace_get(pp::gp_perm_workspace(n), s, 1, &st));
   if (st) return st;
   pp::PermArgs a;
   for (int j = 0; j < 3; ++j) {

@@ -34,6 +34,11 @@ inline ScanGeom scan_geom(uint64_t n, uint32_t blocks_per_sm = 4) {
   return g;
 }
 
+// bytes of workspace slot 1 that one call takes (the server reserves them ahead)
+size_t gp_perm_workspace(uint64_t n);
+size_t div_workspace(uint64_t n);
+size_t eval_workspace(uint64_t n);
+
 // one grand product of a batch: exclusive prefix product in -> out (may alias)
 struct GpBatchJob {
   const fr *in;

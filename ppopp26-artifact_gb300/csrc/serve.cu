@@ -249,15 +249,17 @@ extern "C" int pp_server_create(const pp_server_config *cfg, void **srv) {
   S->streams.resize(cfg->slots);
   S->slot_owner.assign(cfg->slots, 0);
   const size_t nmax = size_t{1} << (cfg->max_lg + cfg->lambda);
-  // the grand product of the largest bundle needs the most scan workspace
-  const size_t npoly = size_t{1} << cfg->max_lg;
-  const pp::ScanGeom sg = pp::scan_geom(npoly);
-  const size_t scan_elems = 2 * npoly + sg.threads + sg.blocks;
+  // what any call of a bundle takes, so that none allocates while serving
+  size_t scan_bytes = 0;
+  for (uint32_t lg = cfg->min_lg; lg <= cfg->max_lg; ++lg) {
+    const uint64_t n = 1ull << lg;
+    scan_bytes = std::max({scan_bytes, pp::gp_perm_workspace(n), pp::div_workspace(n), pp::eval_workspace(n)});
+  }
   for (uint32_t i = 0; i < cfg->slots; ++i) {
     PP_CUDA_TRY(cudaStreamCreateWithFlags(&S->streams[i], cudaStreamNonBlocking));
     int st = PP_OK;
     pp::workspace_get(nmax * sizeof(pp::fr), S->streams[i], 0, &st);
-    if (!st) pp::workspace_get(scan_elems * sizeof(pp::fr), S->streams[i], 1, &st);
+    if (!st) pp::workspace_get(scan_bytes, S->streams[i], 1, &st);
     if (st) {
       delete S;
       return st;
