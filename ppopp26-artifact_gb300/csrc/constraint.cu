@@ -327,13 +327,11 @@ __global__ void __launch_bounds__(kThreads, 2) k_gate_groups(const GateArgs a,
 
 bool aligned16(const void *p) { return p && (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-// capped: at most 8 blocks per SM, each striding over points; otherwise one
-// thread per point, as every kernel here launches (the permutation terms:
-// 2^22 points in 1.45 ms, against 1.85 ms with the cap)
-unsigned grid_for(uint64_t n, bool capped = true) {
+// one thread per point (at most 2^31 - 1 blocks; the kernels stride beyond): 2^22 points'
+// permutation terms took 1.45 ms so, 1.85 ms with at most 8 blocks per SM
+unsigned grid_for(uint64_t n) {
   const uint64_t want = (n + kThreads - 1) / kThreads;
-  const uint64_t cap = capped ? (uint64_t)device_sm_count() * 8 : 0x7fffffffull;
-  return (unsigned)(want < cap ? want : cap);
+  return (unsigned)(want < 0x7fffffffull ? want : 0x7fffffffull);
 }
 
 // which fields each term reads
@@ -382,7 +380,7 @@ int perm_launch(const pp_perm_quotient_args *a, void *result, uint64_t n, void *
   p.gamma = static_cast<const fr *>(a->gamma);
   for (int j = 0; j < 3; ++j) p.k[j] = static_cast<const fr *>(a->k[j]);
   p.one = static_cast<const fr *>(a->one);
-  k_perm_quotient<TERMS><<<grid_for(n, false), kThreads, 0, (cudaStream_t)stream>>>(
+  k_perm_quotient<TERMS><<<grid_for(n), kThreads, 0, (cudaStream_t)stream>>>(
       p, static_cast<fr *>(result), n);
   PP_COUNT_LAUNCH();
   PP_LAUNCH_CHECK();
@@ -448,7 +446,7 @@ extern "C" int pp_gate_constraint(const pp_gate_args *a, void *d_out, uint64_t n
   PP_LAUNCH_CHECK();
   // one thread per point; of each pair, the form that does not match the
   // scalars returns at once
-  const unsigned grid = pp::grid_for(n, false);
+  const unsigned grid = pp::grid_for(n);
   pp::fr *out = static_cast<pp::fr *>(d_out);
   pp::k_gate_range_logic<true><<<grid, pp::kThreads, 0, s>>>(g, gs, out, n);
   PP_COUNT_LAUNCH();

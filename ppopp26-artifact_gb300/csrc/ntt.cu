@@ -777,7 +777,6 @@ struct Plan {
   uint32_t P = 0;
   uint32_t lgR[4] = {0, 0, 0, 0};
   uint32_t lgT[4] = {0, 0, 0, 0};
-  const fr *tw_inner[4] = {nullptr, nullptr, nullptr, nullptr};
   const uint4 *tw_round = nullptr;
   fr *tw_layer[4] = {nullptr, nullptr, nullptr, nullptr};
   // host-pass plans: split layer tables instead of tw_layer
