@@ -13,7 +13,7 @@
 // what counts: with binary-GCD inversions 2^24 divisions took 3.71 ms with
 // one divergent inversion per lane and 32 elements, 5.09 ms with one per
 // warp and 256 elements in registers (118 registers), 1.81 ms as here; with
-// the divstep inversion (modinv.cuh) 1.73 ms, 1.19 ms with its present form and
+// the divstep inversion (modinv.cuh) 1.73 ms, 1.18 ms with its present form and
 // multiply.  As in the reference, the
 // inverse of 0 is taken as 0.
 #include "common.cuh"

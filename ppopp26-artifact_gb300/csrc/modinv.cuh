@@ -39,8 +39,9 @@
 // 128-bit sums (a 64-bit host CPU's form; on a GB300 it took 1.2 to 1.6 times
 // the 30-bit form's time, a binary GCD 1.6 to 4.6 times).
 //
-// GB300, 30-bit form: a lone thread inverts in 18.6 us (Fr) and 32.0 us (Fq); 34.5
-// and 57.1 us one divstep at a time with d and e reduced after each batch.
+// GB300, 30-bit form: a lone thread inverts in 18.5 us (Fr) and 31.5 us (Fq), 32 lanes
+// with a value each in 25.9 and 42.1; the lone thread took 34.5 and 57.1 us one divstep
+// at a time with d and e reduced after each batch.
 #pragma once
 #include <cstdint>
 
@@ -89,7 +90,7 @@ PP_HD int ctz_word(uint64_t x) {
 }
 
 // a b + s; on the device one instruction, whatever the compiler knows of a and b (left to
-// itself it spends several on the products by M's limbs: 20.0 against 18.6 us)
+// itself it spends several on the products by M's limbs: 20.5 against 18.5 us)
 PP_HD int64_t mad_limbs(int32_t a, int32_t b, int64_t s) {
 #ifdef __CUDA_ARCH__
   int64_t r;
@@ -110,7 +111,7 @@ struct DivMatrix {
 // x / y modulo 2^bits, or 2^10 where that is less; y odd.  3 y with its second bit
 // flipped is 1 / y modulo 2^5 (P. Montgomery's start), one of Newton's steps makes that
 // ten bits.  Longer quotients are rare: a branch for them costs each division more (lone
-// thread 22.3 against 18.6 us) than finishing them in a second piece.
+// thread 22.3 against 18.5 us) than finishing them in a second piece.
 template <typename U>
 PP_HD U quotient_mod2(U x, U y, int bits) {
   const U inv = (3 * y) ^ 2;
@@ -124,31 +125,25 @@ PP_HD void divide_batch(int &D, typename LimbTraits<L>::U f, typename LimbTraits
   // f and g are fF F + fG G and gF F + gG G over a power of two, F and G the words given
   U fF = 1, fG = 0, gF = 0, gG = 1;
   int left = LimbTraits<L>::B;
-  const auto strip = [&] {  // g's zero bits, at most `left` of them
+  for (;;) {
+    // g's zero bits, at most `left` of them
     const int zeros = ctz_word(g | (U)1 << left);
     g >>= zeros;
     fF <<= zeros;
     fG <<= zeros;
     D += zeros;
     left -= zeros;
-  };
-  strip();
-  while (left > 0) {
-    if (D < 0) {  // the rest of a long division, or of one that the batch before began
-      const U w = quotient_mod2<U>(0 - g, f, -D < left ? -D : left);
-      g += w * f;
-      gF += w * fF;
-      gG += w * fG;
-      strip();
-    }
-    while (left > 0 && D >= 0) {  // g is odd here
-      const U w = quotient_mod2<U>(f, g, D < left ? D + 1 : left);
-      const U rest = w * g - f, restF = w * gF - fF, restG = w * gG - fG;
-      f = g, fF = gF, fG = gG;
-      g = rest, gF = restF, gG = restG;
-      D = -1 - D;
-      strip();
-    }
+    if (left == 0) break;
+    // the next division, (f, g) -> (g, w g - f); or, with D < 0, the rest of a long one
+    // or of one that the batch before began, (f, g) -> (f, w f + g)
+    const bool next = D >= 0;
+    const U b = next ? 0 - f : g, bF = next ? 0 - fF : gF, bG = next ? 0 - fG : gG;
+    f = next ? g : f, fF = next ? gF : fF, fG = next ? gG : fG;
+    D = next ? -1 - D : D;
+    const U w = quotient_mod2<U>(0 - b, f, -D < left ? -D : left);
+    g = w * f + b;
+    gF = w * fF + bF;
+    gG = w * fG + bG;
   }
   T = {(L)fF, (L)fG, (L)gF, (L)gG};
 }
