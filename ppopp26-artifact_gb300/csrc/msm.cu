@@ -1083,7 +1083,7 @@ struct MsmLayout {
 //   2^20 points    8.42 7.97 7.87* 7.94 8.10   window tables 6.97 6.46 6.29 6.23* 6.26
 //   2^22 points    26.7 24.4 23.1 22.6 22.5*
 //   2^16 points    2.05* 2.18 2.47             window tables 1.16* 1.35 1.53
-// Since inversions take 33 instead of 57 us the bound is 14 instead of 28: 2^17 points
+// Since inversions take 32 instead of 57 us the bound is 14 instead of 28: 2^17 points
 // 1937 -> 1893 us, 2^18 2792 -> 2719, 200003 2368 -> 2350; with window tables 2^17
 // 1236 -> 1250, 200003 1605 -> 1623, so it stays 28 there.
 // The bound on the entries keeps the rounds' buffers below 20 GB.

@@ -27,7 +27,7 @@ namespace pp {
 
 // Blocks per SM each operator's geometry aims for (scan_geom): longer chunks
 // cut the summaries to scan, more blocks hide more latency.  Swept over 1, 2,
-// 3 and 4 on GB300 (us at 2^20 / 2^22 / 2^24): division 2 (57 / 137 / 446; with the
+// 3 and 4 on GB300 (us at 2^20 / 2^22 / 2^24): division 2 (58 / 139 / 453; with the
 // general maps before it 77 / 170 / 529, 1: 72 / 171 / 559, 4: 115 / 207 / 546).
 // Evaluation has its own geometry (k_eval_tree), and so has the permutation product
 // (k_perm_local).
@@ -700,7 +700,7 @@ __device__ void compose_blocks(const fr *block_a, const fr *block_b, uint32_t fi
 // q = m^K and each block's x -> A + Q x, Q = q^256: a combine of two neighbours is one
 // multiply by a known power instead of two, and a sum over all later blocks is a
 // weighted sum without a chain.  us at 2^20 / 2^22 / 2^24: 77 / 170 / 529 with general
-// maps (two multiplies per combine, 24 and 18 deep), 57 / 137 / 446 so.
+// maps (two multiplies per combine, 24 and 18 deep), 58 / 139 / 453 so.
 // Powers, by the helper warp beside the chunks; block 0 leaves them for the apply:
 struct DivPowers {
   fr q[33];     // q^a
