@@ -83,6 +83,7 @@ void *workspace_get(size_t bytes, cudaStream_t stream, int slot, int *status) {
     cudaFree(b.ptr);
     b.ptr = nullptr;
     b.bytes = 0;
+    b.captured = false;
   }
   PP_COUNT_ALLOC(bytes);
   cudaError_t e = cudaMalloc(&b.ptr, bytes);
@@ -128,6 +129,7 @@ void *workspace_get_most(size_t most, size_t least, cudaStream_t stream, int slo
         }
         b.ptr = larger;
         b.bytes = most;
+        b.captured = false;
       } else {
         cudaGetLastError();
         b.refused = most;
