@@ -39,9 +39,9 @@
 // 128-bit sums (a 64-bit host CPU's form; on a GB300 it took 1.2 to 1.6 times
 // the 30-bit form's time, a binary GCD 1.6 to 4.6 times).
 //
-// GB300, 30-bit form: a lone thread inverts in 18.5 us (Fr) and 31.5 us (Fq), 32 lanes
-// with a value each in 25.9 and 42.1; the lone thread took 34.5 and 57.1 us one divstep
-// at a time with d and e reduced after each batch.
+// GB300, 30-bit form: a lone thread that only inverts takes 20.0 us (Fr) and 34.6 us
+// (Fq), 32 lanes with a value each 28.4 and 47.1; the lone thread took 34.5 and 57.1 us
+// one divstep at a time with d and e reduced after each batch.
 #pragma once
 #include <cstdint>
 
@@ -89,8 +89,10 @@ PP_HD int ctz_word(uint64_t x) {
 #endif
 }
 
-// a b + s; on the device one instruction, whatever the compiler knows of a and b (left to
-// itself it spends several on the products by M's limbs: 20.5 against 18.5 us)
+// a b + s; on the device one instruction, whatever the compiler makes of the sum.  For the
+// products by T, not for those by M's limbs, which are constants: the permutation product
+// of 2^13 rows, half of it the inversion, takes 66.9 us so, 69.2 with no product and 72.4
+// with all of them written like this.
 PP_HD int64_t mad_limbs(int32_t a, int32_t b, int64_t s) {
 #ifdef __CUDA_ARCH__
   int64_t r;
@@ -111,7 +113,8 @@ struct DivMatrix {
 // x / y modulo 2^bits, or 2^10 where that is less; y odd.  3 y with its second bit
 // flipped is 1 / y modulo 2^5 (P. Montgomery's start), one of Newton's steps makes that
 // ten bits.  Longer quotients are rare: a branch for them costs each division more (lone
-// thread 22.3 against 18.5 us) than finishing them in a second piece.
+// thread 22.3 against 18.5 us, with products by M's limbs as mad_limbs) than finishing
+// them in a second piece.
 template <typename U>
 PP_HD U quotient_mod2(U x, U y, int bits) {
   const U inv = (3 * y) ^ 2;
@@ -168,8 +171,8 @@ PP_HD void apply_batch(SLimbs<L, NL> &x, SLimbs<L, NL> &y, const DivMatrix<L> &T
   for (int i = 1; i < NL; ++i) {
     A px = mad_limbs(T.v, y.l[i], mad_limbs(T.u, x.l[i], 0)), py = mad_limbs(T.r, y.l[i], mad_limbs(T.q, x.l[i], 0));
     if (!EXACT) {
-      px = mad_limbs(mx, M.m[i], px);
-      py = mad_limbs(my, M.m[i], py);
+      px += (A)mx * M.m[i];
+      py += (A)my * M.m[i];
     }
     sx = (sx >> B) + px;
     sy = (sy >> B) + py;
