@@ -491,9 +491,9 @@ struct PermArgs {
 // products by beta and beta k_j take the four-part constant form.
 //
 // GB300, 2^20 rows, us: first pass / carry / last pass 257 / 55 / 110 with
-// numerators and denominators kept in memory, 221 / 48 / 21 so (561 -> 292 per
-// call with the general multiply's rows counted in; 3, 4 and 5 rows per thread:
-// 293, 292 and 308; at 2^22 1029, 1002 and 1005).
+// numerators and denominators kept in memory, 221 / 33 / 21 so (561 -> 285 per
+// call with the general multiply's rows counted in; with an inversion 7 us longer 3, 4
+// and 5 rows per thread took 293, 292 and 308, at 2^22 1029, 1002 and 1005).
 constexpr uint32_t kPermRows = 4, kPermBlockRows = kPermRows * kScanThreads;
 constexpr uint32_t kPermSlots = 2 * kPermRows * 2 * kScanThreads;  // 16-byte units: 64 KiB
 
